@@ -382,6 +382,22 @@ int moc_sparse_attn_bwd(const moc_sparse_attn_shape* s, const void* q, const voi
                         const int32_t* block_indices, const void* o, const float* lse, const void* d_o,
                         void* d_q, float* d_k, float* d_v, int32_t* status, void* stream);
 
+/* The same contract on the tensor cores (bf16, head_dim 64, block_size a multiple of 64, at most 128 query heads per
+ * KV head): an inverted index key unit -> (token, slot) pairs is built on the device, every unit's K / V tile is
+ * multiplied with the gathered query rows that selected it, and a token's partial results are merged.  d_k / d_v are
+ * bf16 like k / v, written in full.  `index` (index_bytes) is filled by the forward call; the backward call reads it
+ * when have_index != 0 and fills it from block_indices otherwise.  `scratch`: fwd_bytes / bwd_bytes.  All three are
+ * 16-byte aligned.  Chapter ids outside [0, TK / block_size) raise MOC_DEV_BAD_INDEX and contribute nothing. */
+int moc_sparse_attn_tc_sizes(const moc_sparse_attn_shape* s, int64_t* index_bytes, int64_t* fwd_bytes,
+                             int64_t* bwd_bytes);
+int moc_sparse_attn_tc_fwd(const moc_sparse_attn_shape* s, const void* q, const void* k, const void* v,
+                           const int32_t* block_indices, void* index, void* scratch, void* o, float* lse,
+                           int32_t* status, void* stream);
+int moc_sparse_attn_tc_bwd(const moc_sparse_attn_shape* s, const void* q, const void* k, const void* v,
+                           const int32_t* block_indices, void* index, int32_t have_index, void* scratch, const void* o,
+                           const float* lse, const void* d_o, void* d_q, void* d_k, void* d_v, int32_t* status,
+                           void* stream);
+
 /* out[r] = <a[r, :], b[r, :]> in fp32 for contiguous [rows, dim] operands: the per-(token, head) delta = <o, do> of
  * memory_cross_attn_preprocess_delta (kernels-final/memory_cross_attn.py:1369-1384). */
 int moc_row_dot(const void* a, const void* b, int32_t dtype, float* out, int64_t rows, int32_t dim, void* stream);

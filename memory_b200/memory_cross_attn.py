@@ -28,13 +28,31 @@ def _check(q, k, v, block_indices, block_size):
         raise ValueError("value head dim must equal key head dim")
 
 
+def _same_dtype(q, k, v):
+    return q.dtype == k.dtype == v.dtype
+
+
+def _forward(q, k, v, bi, block_size, scale):
+    """(o, lse, index or None): the tensor-core kernels where they apply, else a warp per (token, head)."""
+    if _same_dtype(q, k, v) and ops.sparse_attn_tc_supported(q, k, block_size):
+        return ops.sparse_attn_tc_fwd(q, k, v, bi, block_size, scale)
+    return (*ops.sparse_attn_fwd(q, k, v, bi, block_size, scale), None)
+
+
+def _backward(q, k, v, bi, o, lse, do, block_size, scale, index=None):
+    if _same_dtype(q, k, v) and do.dtype == q.dtype and ops.sparse_attn_tc_supported(q, k, block_size):
+        return ops.sparse_attn_tc_bwd(q, k, v, bi, o, lse, do.contiguous(), block_size, scale, index)
+    dq, dk, dv = ops.sparse_attn_bwd(q, k, v, bi, o, lse, do.contiguous(), block_size, scale)
+    return dq, dk.to(k.dtype), dv.to(v.dtype)
+
+
 def memory_cross_attn_forward(q, k, v, block_indices, block_size: int,
                               scale: Optional[float] = None) -> Tuple[torch.Tensor, torch.Tensor]:
     """(o [B,TQ,HQ,D] in v's dtype, lse [B,TQ,HQ] fp32)."""
     _check(q, k, v, block_indices, block_size)
     if scale is None:
         scale = q.shape[-1] ** -0.5
-    return ops.sparse_attn_fwd(q, k, v, block_indices.to(torch.int32).contiguous(), block_size, scale)
+    return _forward(q, k, v, block_indices.to(torch.int32).contiguous(), block_size, scale)[:2]
 
 
 def memory_cross_attn_preprocess_delta(o: torch.Tensor, do: torch.Tensor) -> torch.Tensor:
@@ -57,8 +75,7 @@ def memory_cross_attn_backward(q, k, v, o, lse, do, block_indices, block_size: i
     _check(q, k, v, bi, block_size)
     if scale is None:
         scale = q.shape[-1] ** -0.5
-    dq, dk, dv = ops.sparse_attn_bwd(q, k, v, bi, o, lse, do.contiguous(), block_size, scale)
-    return dq, dk.to(k.dtype), dv.to(v.dtype)
+    return _backward(q, k, v, bi, o, lse, do, block_size, scale)
 
 
 class MemoryCrossAttnFunction(torch.autograd.Function):
@@ -68,16 +85,15 @@ class MemoryCrossAttnFunction(torch.autograd.Function):
             scale = q.shape[-1] ** -0.5
         bi = block_indices.to(torch.int32).contiguous()
         _check(q, k, v, bi, block_size)
-        o, lse = ops.sparse_attn_fwd(q, k, v, bi, block_size, scale)
-        ctx.save_for_backward(q, k, v, o, lse, bi)
+        o, lse, index = _forward(q, k, v, bi, block_size, scale)
+        ctx.save_for_backward(q, k, v, o, lse, bi, index)
         ctx.block_size, ctx.scale = block_size, scale
         return o
 
     @staticmethod
     def backward(ctx, do):
-        q, k, v, o, lse, bi = ctx.saved_tensors
-        dq, dk, dv = ops.sparse_attn_bwd(q, k, v, bi, o, lse, do.contiguous(), ctx.block_size, ctx.scale)
-        return dq, dk.to(k.dtype), dv.to(v.dtype), None, None, None
+        q, k, v, o, lse, bi, index = ctx.saved_tensors
+        return (*_backward(q, k, v, bi, o, lse, do, ctx.block_size, ctx.scale, index), None, None, None)
 
 
 def memory_cross_attn(q, k, v, block_indices, block_size: int, scale: Optional[float] = None,

@@ -647,6 +647,58 @@ def sparse_attn_bwd(q, k, v, block_indices, o, lse, d_o, block_size: int, scale:
     return d_q, d_k, d_v
 
 
+def sparse_attn_tc_supported(q: torch.Tensor, k: torch.Tensor, block_size: int) -> bool:
+    """Whether the tensor-core kernels take this joint-softmax problem: bf16, head_dim 64, chapters of a multiple of 64
+    rows.  They are the faster ones at every size measured (100 tokens up), so nothing else decides."""
+    return (q.dtype == torch.bfloat16 and k.dtype == torch.bfloat16 and q.shape[-1] == 64 and int(block_size) % 64 == 0
+            and q.shape[2] // k.shape[2] <= 128)
+
+
+def _sparse_tc_sizes(s):
+    n = [C.c_int64() for _ in range(3)]
+    L.check(L.lib().moc_sparse_attn_tc_sizes(C.byref(s), *[C.addressof(v) for v in n]), "moc_sparse_attn_tc_sizes")
+    return [v.value for v in n]
+
+
+@_instrument("sparse_attn_tc_fwd", 6)
+def sparse_attn_tc_fwd(q, k, v, block_indices, block_size: int, scale: float):
+    """(o, lse, index) of the tensor-core path; ``index`` goes to :func:`sparse_attn_tc_bwd`."""
+    L.require_cuda(q, k, v, block_indices)
+    b, tq, hq, d = q.shape
+    s = L.SparseAttnShape(b, tq, k.shape[1], hq, k.shape[2], d, block_indices.shape[-1], int(block_size), float(scale),
+                          L.dtype_code(q.dtype))
+    n_index, n_fwd, _ = _sparse_tc_sizes(s)
+    o = torch.empty_like(q)
+    lse = torch.empty(b, tq, hq, dtype=torch.float32, device=q.device)
+    index = torch.empty(n_index, dtype=torch.uint8, device=q.device)
+    scratch = torch.empty(n_fwd, dtype=torch.uint8, device=q.device)
+    rc = L.lib().moc_sparse_attn_tc_fwd(C.byref(s), L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(block_indices), L.ptr(index),
+                                        L.ptr(scratch), L.ptr(o), L.ptr(lse), L.ptr(L.status_word(q.device)),
+                                        L.stream_ptr(q.device))
+    L.check(rc, "moc_sparse_attn_tc_fwd")
+    return o, lse, index
+
+
+@_instrument("sparse_attn_tc_bwd", 4)
+def sparse_attn_tc_bwd(q, k, v, block_indices, o, lse, d_o, block_size: int, scale: float,
+                       index: Optional[torch.Tensor] = None):
+    """(dq, dk, dv) in the inputs' dtype; without ``index`` it is built again from ``block_indices``."""
+    b, tq, hq, d = q.shape
+    s = L.SparseAttnShape(b, tq, k.shape[1], hq, k.shape[2], d, block_indices.shape[-1], int(block_size), float(scale),
+                          L.dtype_code(q.dtype))
+    n_index, _, n_bwd = _sparse_tc_sizes(s)
+    have = index is not None
+    if not have:
+        index = torch.empty(n_index, dtype=torch.uint8, device=q.device)
+    scratch = torch.empty(n_bwd, dtype=torch.uint8, device=q.device)
+    d_q, d_k, d_v = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+    rc = L.lib().moc_sparse_attn_tc_bwd(C.byref(s), L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(block_indices), L.ptr(index),
+                                        int(have), L.ptr(scratch), L.ptr(o), L.ptr(lse), L.ptr(_contig(d_o)), L.ptr(d_q),
+                                        L.ptr(d_k), L.ptr(d_v), L.ptr(L.status_word(q.device)), L.stream_ptr(q.device))
+    L.check(rc, "moc_sparse_attn_tc_bwd")
+    return d_q, d_k, d_v
+
+
 @_instrument("sparse_attn_weighted_fwd", 1)
 def sparse_attn_weighted_fwd(q, k, v, block_indices, weights, block_size: int, scale: float,
                              base: Optional[torch.Tensor] = None, out_scale: float = 1.0):
