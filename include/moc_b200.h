@@ -468,6 +468,61 @@ int moc_bank_adamw_step(float* param, float* exp_avg, float* exp_avg_sq, int64_t
 int moc_rows_sqnorm(const float* rows, const int32_t* num_unique, int32_t tokens_per_chapter, int32_t dim,
                     float* out, void* workspace, size_t workspace_bytes, void* stream);
 
+/* ------------------------------------------------------------------------------------------------
+ * One memory layer in two calls (bf16 arithmetic): router, chapter gather (fused into the K/V projection when
+ * `fused`, materialised otherwise), normalisation, projections and joint-softmax attention -- the chain of
+ * memory_transformer/model.py:624-692 and memory_block.py:549-558 -- and the backward pass of all of it.  Each call
+ * issues every kernel of its pass on two streams (`side_stream` forks from and joins `stream`), so a host pays one
+ * call per pass instead of one per kernel.
+ *   weights of one dtype (weight_dtype), row-major nn.Linear layout; row_norm / pre_norm: MOC_NORM_*; row_norm is the
+ *   one in effect (MOC_NORM_NONE when there is no shared or no routed slice).  h_attn / out share attn_dtype.
+ *   arena: moc_layer_arena_bytes(); what the forward call leaves in it is the saved state the backward call reads.
+ *   uniq [B*(S+k)], num_unique [1]: the touched chapters (written when for_backward).
+ * ---------------------------------------------------------------------------------------------- */
+typedef struct {
+  int32_t batch, seq, router_seq, hidden_dim, num_heads, num_kv_heads;
+  int32_t num_chapters, tokens_per_chapter, top_k, num_shared;
+  int32_t router_dtype, attn_dtype, bank_dtype, weight_dtype;
+  int32_t row_norm, pre_norm, add_residual, with_losses, fused, for_backward;
+  float routed_scale, row_eps, pre_eps;
+  int64_t bank_rows;       /* rows of bank and of bank_shadow */
+  const void *h_router, *h_attn, *bank, *bank_shadow;
+  const float *bank_inv_rms, *router_w, *router_b;
+  const void *wq, *wk, *wv, *wo;
+  const float *norm_w, *norm_b;
+  void* out;
+  int64_t* idx;
+  float* weights;
+  int32_t* comb_idx;
+  float *comb_w, *losses;
+  int32_t *uniq, *num_unique;
+  void* arena;
+  int32_t* status;
+  void *stream, *side_stream;
+} moc_layer_desc;
+
+int64_t moc_layer_arena_bytes(const moc_layer_desc* s);
+int moc_layer_fwd(const moc_layer_desc* s);
+
+/* g: gradient of `out`; g_weights / g_comb_w / g_losses may be NULL.  d_h_router NULL: the router's share is added
+ * into d_h_attn (the two inputs are one tensor).  want_dh_router 0: that share is not computed.  The bank gradient
+ * leaves as compact rows in bank_rows (fp32) and / or bank_rows_bf16, or dense in bank_dense; all NULL: not wanted.
+ * d_wkv: K rows then V rows.  scratch: moc_layer_bwd_scratch_bytes(). */
+typedef struct {
+  const void* g;
+  const float *g_weights, *g_comb_w, *g_losses;
+  int32_t want_dh_router, dq_on_side_stream, wkv_grad_in_place, want_router_w;
+  void *d_h_attn, *d_h_router;
+  float* bank_rows;
+  void* bank_rows_bf16;
+  float* bank_dense;
+  float *d_router_w, *d_router_b, *d_wq, *d_wkv, *d_wo, *d_norm_w, *d_norm_b;
+  void* scratch;
+} moc_layer_bwd_desc;
+
+int64_t moc_layer_bwd_scratch_bytes(const moc_layer_desc* s, const moc_layer_bwd_desc* b);
+int moc_layer_bwd(const moc_layer_desc* s, const moc_layer_bwd_desc* b);
+
 /* Element-wise helpers used by the host layer (device pointers, n elements). */
 int moc_cast_f32_to_bf16(const float* src, void* dst, int64_t n, void* stream);
 int moc_cast_bf16_to_f32(const void* src, float* dst, int64_t n, void* stream);

@@ -55,6 +55,33 @@ class DecodeShape(C.Structure):
                 ("scale", C.c_float)]
 
 
+def _fields(spec: str):
+    """``"i: a b; f: c; p: d"`` -> ctypes fields of int32 (i), int64 (l), float (f) or pointer (p) type."""
+    kinds = {"i": C.c_int32, "l": C.c_int64, "f": C.c_float, "p": C.c_void_p}
+    out = []
+    for group in spec.split(";"):
+        kind, names = group.split(":")
+        out += [(n, kinds[kind.strip()]) for n in names.split()]
+    return out
+
+
+class LayerDesc(C.Structure):
+    _fields_ = _fields(
+        "i: batch seq router_seq hidden_dim num_heads num_kv_heads num_chapters tokens_per_chapter top_k num_shared"
+        " router_dtype attn_dtype bank_dtype weight_dtype row_norm pre_norm add_residual with_losses fused for_backward;"
+        "f: routed_scale row_eps pre_eps; l: bank_rows;"
+        "p: h_router h_attn bank bank_shadow bank_inv_rms router_w router_b wq wk wv wo norm_w norm_b"
+        " out idx weights comb_idx comb_w losses uniq num_unique arena status stream side_stream")
+
+
+class LayerBwdDesc(C.Structure):
+    _fields_ = _fields(
+        "p: g g_weights g_comb_w g_losses;"
+        "i: want_dh_router dq_on_side_stream wkv_grad_in_place want_router_w;"
+        "p: d_h_attn d_h_router bank_rows bank_rows_bf16 bank_dense d_router_w d_router_b d_wq d_wkv d_wo d_norm_w"
+        " d_norm_b scratch")
+
+
 P = C.c_void_p
 _PROTOTYPES = {
     "moc_last_error": (C.c_char_p, []),
@@ -97,6 +124,10 @@ _PROTOTYPES = {
                                                P, P, P, P]),
     "moc_sparse_attn_weighted_bwd": (C.c_int, [C.POINTER(SparseAttnShape), P, P, P, C.c_int64, P, P, C.c_float, P,
                                                P, P, C.c_int32, P, P, C.c_int64, P, P, P]),
+    "moc_layer_arena_bytes": (C.c_int64, [C.POINTER(LayerDesc)]),
+    "moc_layer_fwd": (C.c_int, [C.POINTER(LayerDesc)]),
+    "moc_layer_bwd_scratch_bytes": (C.c_int64, [C.POINTER(LayerDesc), C.POINTER(LayerBwdDesc)]),
+    "moc_layer_bwd": (C.c_int, [C.POINTER(LayerDesc), C.POINTER(LayerBwdDesc)]),
     "moc_sparse_attn_tc_sizes": (C.c_int, [C.POINTER(SparseAttnShape), P, P, P]),
     "moc_sparse_attn_tc_fwd": (C.c_int, [C.POINTER(SparseAttnShape), P, P, P, P, P, P, P, P, P, P]),
     "moc_sparse_attn_tc_bwd": (C.c_int, [C.POINTER(SparseAttnShape), P, P, P, P, P, C.c_int32, P, P, P, P, P, P, P, P, P]),
@@ -168,13 +199,21 @@ def ptr(t) -> int:
     return t.data_ptr()
 
 
+def device_index(device: torch.device) -> int:
+    return device.index if device.index is not None else torch.cuda.current_device()
+
+
 def stream_ptr(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    if not isinstance(device, torch.device):
+        device = torch.device(device)
+    return torch._C._cuda_getCurrentRawStream(device_index(device))
 
 
 def status_word(device) -> torch.Tensor:
     """Per-device int32 the kernels raise on device-side errors."""
-    key = torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device()
+    if not isinstance(device, torch.device):
+        device = torch.device(device)
+    key = device_index(device)
     t = _status.get(key)
     if t is None:
         t = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", key))

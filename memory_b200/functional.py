@@ -18,6 +18,7 @@ from typing import Dict, Optional, Tuple
 
 import torch
 
+from . import _lib as L
 from . import ops
 
 LOSS_KEYS = ("load_balance", "auxiliary", "z_loss", "entropy")
@@ -313,17 +314,21 @@ def cross_attention(h: torch.Tensor, memory: torch.Tensor, wq, wk, wv, wo, num_h
 # the whole layer as one node with two streams (bf16 path)
 # --------------------------------------------------------------------------------------------
 _side_streams: Dict[tuple, "torch.cuda.Stream"] = {}
+_side_handles: Dict[tuple, int] = {}
 
 
-def _side_stream(device: torch.device) -> "torch.cuda.Stream":
+def _side_stream(dev_index: int, main_handle: int) -> int:
     """Second stream of the layer, with the priority of the stream it runs beside (a step captured on a
-    high-priority stream keeps both of its streams ahead of background work such as a gradient exchange)."""
-    idx = device.index if device.index is not None else torch.cuda.current_device()
-    prio = torch.cuda.current_stream(device).priority
-    key = (idx, prio)
-    if key not in _side_streams:
-        _side_streams[key] = torch.cuda.Stream(device=device, priority=prio)
-    return _side_streams[key]
+    high-priority stream keeps both of its streams ahead of background work such as a gradient exchange).
+    ``main_handle`` is the raw handle of the current stream; so is the result."""
+    handle = _side_handles.get((dev_index, main_handle))
+    if handle is None:
+        device = torch.device("cuda", dev_index)
+        key = (dev_index, torch.cuda.current_stream(device).priority)
+        if key not in _side_streams:
+            _side_streams[key] = torch.cuda.Stream(device=device, priority=key[1])
+        handle = _side_handles[(dev_index, main_handle)] = _side_streams[key].cuda_stream
+    return handle
 
 
 # The dQ kernel runs on the side stream beside the dK/dV kernel (fused route): 768 CTAs over 296 slots leave the last
@@ -333,9 +338,10 @@ _DQ_ON_SIDE_STREAM = os.environ.get("MOC_DQ_ON_SIDE_STREAM", "1") != "0"
 
 
 class _MemoryLayerTwoStream(torch.autograd.Function):
-    """Router, gather, projections and attention of one layer as a single autograd node, so that the
-    bandwidth- and latency-bound kernels (router, chapter bookkeeping, gather backward) run on a second
-    stream beside the tensor-core kernels instead of in front of or behind them:
+    """Router, gather, projections and attention of one layer as a single autograd node of one native call per pass
+    (``moc_layer_fwd`` / ``moc_layer_bwd``): the bandwidth- and latency-bound kernels (router, chapter bookkeeping,
+    gather backward) run on a second stream beside the tensor-core kernels, and the host pays one call instead of one
+    per kernel.
 
       forward   side: router, chapter segments      | main: weight pack, (norm,) query projection
                 join, then gather, K/V projection, attention, output projection on main
@@ -344,7 +350,8 @@ class _MemoryLayerTwoStream(torch.autograd.Function):
                                                        projections, normalisation backward
 
     Both streams fork from and join the caller's stream with events, which a CUDA-graph capture records as
-    ordinary dependencies.  Every tensor that crosses streams stays referenced until after the join.
+    ordinary dependencies.  Every buffer is allocated on the caller's stream, behind which the side stream is joined
+    before the call returns.
     """
 
     @staticmethod
@@ -352,248 +359,133 @@ class _MemoryLayerTwoStream(torch.autograd.Function):
                 fused=None):
         (num_heads, num_kv_heads, t, top_k, num_shared, routed_scale, row_norm, row_eps, with_losses,
          pre_norm, pre_eps, add_residual) = cfg
-        cd = torch.bfloat16
+        L.require_cuda(h_router, h_attn, bank, router_w)
+        if h_router.dim() != 3:
+            raise ValueError(f"hidden_states must be 3D (B, T, D), got shape {tuple(h_router.shape)}")
         dev = h_attn.device
         b, l, d = h_attn.shape
-        dkv = wk.shape[0]
-        main, side = torch.cuda.current_stream(dev), _side_stream(dev)
-        num_chapters = bank.shape[0] // t
-
-        side.wait_stream(main)
-        with torch.cuda.stream(side):
-            r = ops.router_fwd(h_router, router_w, router_b, top_k, num_shared, routed_scale, with_losses, parts=1)
-            routed = torch.cuda.Event()
-            routed.record(side)          # the gather needs nothing after this point of the side stream
-            if with_losses:
-                ops.router_fwd(h_router, router_w, router_b, top_k, num_shared, routed_scale, with_losses, parts=2,
-                               out=r)
-            seg = ops.chapter_segments(r["comb_idx"], num_chapters)
-
-        # main stream meanwhile: bf16 weights (+ transposes for the backward pass), query projection
-        need_t = any(ctx.needs_input_grad[:11])
-        w_all = torch.empty(2 * d + 2 * dkv, d, dtype=cd, device=dev)
-        wq_c, wkv_c, wo_c = w_all[:d], w_all[d:d + 2 * dkv], w_all[d + 2 * dkv:]
-        wq_t = torch.empty(d, d, dtype=cd, device=dev) if need_t else None
-        wkv_t = torch.empty(d, 2 * dkv, dtype=cd, device=dev) if need_t else None
-        wo_t = torch.empty(d, d, dtype=cd, device=dev) if need_t else None
-        ops.pack_weights([wq, wk, wv, wo], [wq_c, wkv_c[:dkv], wkv_c[dkv:], wo_c],
-                         [wq_t, wkv_t, wkv_t[:, dkv:] if need_t else None, wo_t], [0, 2 * dkv, 2 * dkv, 0])
-        x2 = h_attn.reshape(b * l, d)
-        stats_n = None
-        if pre_norm is not None:
-            x2 = x2.float()
-            h2, stats_n = ops.norm_fwd(x2, norm_w.float(), None if norm_b is None else norm_b.float(), pre_norm,
-                                       pre_eps, cd)
-        else:
-            h2 = ops.cast(x2, cd)
-        q = ops.gemm(h2, wq_c, tag="q_proj")
-
-        main.wait_event(routed)
-        k_sel = r["idx"].shape[1]
+        rows, c = bank.shape[0], router_w.shape[0]
+        # the kernels take fp32 or bf16 activations; anything else computes in bf16 and is cast back
+        in_dtype = h_attn.dtype
+        ha = ops._contig(h_attn if in_dtype in (torch.float32, torch.bfloat16) else h_attn.to(torch.bfloat16))
+        hr = ha if h_router is h_attn else ops._contig(h_router)
+        k_sel = ops.router_selected_k(c, top_k, num_shared)
         # the reference only normalises when both a shared and a routed slice exist (model.py:413-418)
         norm = row_norm if (num_shared > 0 and k_sel > 0) else None
         if fused is not None and (norm not in (None, "rms") or (norm == "rms" and fused.get("inv_rms") is None)):
             fused = None                      # affine-free LayerNorm rows are not a row scale: two-pass route
-        row_scale = None
-        if fused is not None:
-            # Gather, normalisation, weight multiply and the K/V projection in one kernel: chapters are read from
-            # the bf16 copy of the bank through the TMA gather list, u~ (and 1/rms) is the epilogue row scale.
-            n_sel = r["comb_idx"].shape[1] * t
-            row_scale = ops.chapter_row_scale(r["comb_idx"], r["comb_w"], fused["inv_rms"] if norm == "rms" else None,
-                                              bank.shape[0], t)
-            kv = ops.gemm(fused["shadow"], wkv_c, a_row_blocks=r["comb_idx"].reshape(-1), a_block_rows=t,
-                          m=b * n_sel, row_scale=row_scale, scale_block_rows=1, tag="kv_proj").view(b, n_sel, -1)
-            m2 = stats_m = None
-        else:
-            memory, stats_m = ops.gather_rows_fwd(bank, t, r["comb_idx"], r["comb_w"], norm, row_eps, cd)
-            n_sel = memory.shape[-2]
-            m2 = memory.reshape(-1, d)
-            kv = ops.gemm(m2, wkv_c, tag="kv_proj").view(b, n_sel, -1)
-        scale = (d // num_heads) ** -0.5
-        o, lse = ops.attn_fwd(q.view(b, l, -1), kv, num_heads, num_kv_heads, scale)
-        res = (x2 if x2.dtype == torch.float32 else x2.float()) if add_residual else None
-        out_dtype = h_attn.dtype if h_attn.dtype in (torch.float32, cd) else cd
-        out = ops.gemm(o.view(b * l, -1), wo_c, out_dtype=out_dtype, residual=res, tag="o_proj")
-        main.wait_stream(side)           # loss terms and chapter segments finished beside the attention
+        shadow = None if fused is None else ops._contig(fused["shadow"])
+        if shadow is not None and (shadow.dtype != torch.bfloat16 or shadow.shape != bank.shape):
+            raise TypeError("bank_shadow must be a bf16 tensor shaped like the bank")
+        inv_rms = ops._contig(fused["inv_rms"]) if (fused is not None and norm == "rms") else None
+        bank_c = ops._contig(bank)
+        rw = ops._contig(router_w.float())
+        rb = None if router_b is None else ops._contig(router_b.float())
+        ws = [ops._contig(w) for w in (wq, wk, wv, wo)]
+        nw = None if norm_w is None else ops._contig(norm_w.float())
+        nb = None if norm_b is None else ops._contig(norm_b.float())
+        need_grad = any(ctx.needs_input_grad[:11])
+        n_pairs = b * (num_shared + k_sel)
+        f32, i32 = torch.float32, torch.int32
+        out = torch.empty(b, l, d, dtype=ha.dtype, device=dev)
+        idx = torch.empty(b, k_sel, dtype=torch.int64, device=dev)
+        weights = torch.empty(b, k_sel, dtype=f32, device=dev)
+        comb_idx = torch.empty(b, num_shared + k_sel, dtype=i32, device=dev)
+        comb_w = torch.empty(b, num_shared + k_sel, dtype=f32, device=dev)
+        losses = torch.empty(4, dtype=f32, device=dev) if with_losses else torch.zeros(4, dtype=f32, device=dev)
+        touched = torch.empty(n_pairs + 1, dtype=i32, device=dev) if need_grad else None    # ids, then their count
+        index = L.device_index(dev)
+        main = L.stream_ptr(dev)
+        s = L.LayerDesc(
+            b, l, hr.shape[1], d, num_heads, num_kv_heads, c, t, top_k, num_shared, L.dtype_code(hr.dtype),
+            L.dtype_code(ha.dtype), L.dtype_code(bank.dtype), L.dtype_code(wq.dtype), L.NORM_CODES[norm],
+            ops.NORM_KINDS[pre_norm] if pre_norm is not None else 0, int(add_residual), int(with_losses),
+            int(fused is not None), int(need_grad), routed_scale, row_eps, pre_eps, rows, hr.data_ptr(), ha.data_ptr(),
+            bank_c.data_ptr(), L.ptr(shadow), L.ptr(inv_rms), rw.data_ptr(), L.ptr(rb), ws[0].data_ptr(),
+            ws[1].data_ptr(), ws[2].data_ptr(), ws[3].data_ptr(), L.ptr(nw), L.ptr(nb), out.data_ptr(), idx.data_ptr(),
+            weights.data_ptr(), comb_idx.data_ptr(), comb_w.data_ptr(), losses.data_ptr(), L.ptr(touched),
+            None if touched is None else touched.data_ptr() + 4 * n_pairs, None, L.status_word(dev).data_ptr(), main,
+            _side_stream(index, main))
+        arena = torch.empty(ops.layer_arena_bytes(s), dtype=torch.uint8, device=dev)
+        s.arena = arena.data_ptr()
+        ops.layer_fwd(s)
 
-        ctx.cfg = cfg
-        ctx.norm_row = norm
-        ctx.fused = None if fused is None else dict(fused, row_scale=row_scale)
-        ctx.scale = scale
-        # outputs of this node (weights, combined weights, losses) are saved through save_for_backward below:
-        # kept as attributes they would tie the node to its own outputs in a reference cycle
-        ctx.router_saved = {k: r[k] for k in ("pooled", "probs", "idx", "comb_idx", "row_stats", "chapter_stats", "_ws")}
-        ctx.seg = seg
-        ctx.sink = sink
+        ctx.cfg, ctx.desc, ctx.sink = cfg, s, sink
         ctx.same_h = h_router is h_attn
-        ctx.shapes = (tuple(h_router.shape), h_router.dtype, h_attn.dtype, router_b is not None,
+        ctx.wkv_in_place = bool(fused is not None and fused.get("wkv_grad_in_place"))
+        ctx.shapes = (tuple(h_router.shape), h_router.dtype, in_dtype, router_b is not None,
                       (wq.dtype, wk.dtype, wv.dtype, wo.dtype), None if norm_w is None else norm_w.dtype,
-                      None if norm_b is None else norm_b.dtype)
-        ctx.wt = (wq_t, wkv_t, wo_t)
-        ctx.save_for_backward(h2, m2, wq_c, wkv_c, wo_c, q, kv, o, lse, bank, router_w, stats_m,
-                              x2 if pre_norm is not None else None, stats_n,
-                              norm_w.float() if pre_norm is not None else None, r["weights"], r["comb_w"])
-        ctx.mark_non_differentiable(r["idx"], r["comb_idx"])
-        losses = r["losses"] if with_losses else torch.zeros(4, dtype=torch.float32, device=dev)
-        return out.view(b, l, -1).to(h_attn.dtype), r["idx"], r["weights"], r["comb_idx"], r["comb_w"], losses
+                      None if norm_b is None else norm_b.dtype, wk.shape[0])
+        if need_grad:
+            # outputs of this node (weights, combined lists) go through save_for_backward: kept as attributes they
+            # would tie the node to its own outputs in a reference cycle.  The attention input is saved where the
+            # backward pass reads it itself: as the bf16 projection operand, or for the normalisation.
+            keep_h = ha if (pre_norm is not None or ha.dtype == torch.bfloat16) else None
+            ctx.save_for_backward(arena, touched, keep_h, bank_c, shadow, inv_rms, rw, nw, idx, weights, comb_idx, comb_w)
+        ctx.mark_non_differentiable(idx, comb_idx)
+        return out if in_dtype == out.dtype else out.to(in_dtype), idx, weights, comb_idx, comb_w, losses
 
     @staticmethod
     def backward(ctx, g, _g_idx, g_w, _g_cidx, g_cw, g_losses):
-        (h2, m2, wq_c, wkv_c, wo_c, q, kv, o, lse, bank, router_w, stats_m, x2, stats_n,
-         norm_w, r_weights, r_comb_w) = ctx.saved_tensors
-        (num_heads, num_kv_heads, t, top_k, num_shared, routed_scale, _row_norm, row_eps, _with_losses,
-         pre_norm, _pre_eps, add_residual) = ctx.cfg
-        hr_shape, hr_dtype, ha_dtype, has_rbias, wdt, nw_dtype, nb_dtype = ctx.shapes
-        wq_t, wkv_t, wo_t = ctx.wt
-        r, seg = dict(ctx.router_saved, weights=r_weights, comb_w=r_comb_w), ctx.seg
-        cd, f32 = torch.bfloat16, torch.float32
-        dev = q.device
-        b, l, _ = o.shape
-        d = h2.shape[1]
-        main, side = torch.cuda.current_stream(dev), _side_stream(dev)
+        arena, touched, ha, bank, shadow, inv_rms, rw, nw, idx, weights, comb_idx, comb_w = ctx.saved_tensors
+        s, sink = ctx.desc, ctx.sink
+        hr_shape, hr_dtype, in_dtype, has_rbias, wdt, nw_dtype, nb_dtype, dkv = ctx.shapes
+        t = s.tokens_per_chapter
         need = ctx.needs_input_grad
-        num_chapters = bank.shape[0] // t
+        dev = arena.device
+        f32 = torch.float32
+        b, l, d = s.batch, s.seq, s.hidden_dim
+        n_pairs = touched.numel() - 1
+        attn_dtype = f32 if s.attn_dtype == L.MOC_F32 else torch.bfloat16
+        # saved tensors may have been moved (hooks): take their addresses again
+        p = L.ptr
+        s.arena, s.uniq, s.num_unique = p(arena), p(touched), p(touched) + 4 * n_pairs
+        s.h_attn, s.bank, s.bank_shadow, s.bank_inv_rms, s.router_w, s.norm_w = p(ha), p(bank), p(shadow), p(inv_rms), p(rw), p(nw)
+        s.idx, s.weights, s.comb_idx, s.comb_w = p(idx), p(weights), p(comb_idx), p(comb_w)
+        s.stream = L.stream_ptr(dev)
+        s.side_stream = _side_stream(L.device_index(dev), s.stream)
 
-        def splits(rows, out_rows, out_cols):
-            tiles = -(-out_rows // 128) * -(-out_cols // 256)
-            return max(1, min(148 // max(tiles, 1), rows // 512))
-
-        g2f = g.reshape(b * l, -1)
-        g2 = ops.cast(g2f.contiguous(), cd)
-        side.wait_stream(main)
-        with torch.cuda.stream(side):
-            d_wo = ops.gemm(g2, o.view(b * l, -1), a_kmajor=False, b_kmajor=False, out_dtype=f32,
-                            split_k=splits(b * l, d, d), tag="d_wo")
-        d_o = ops.gemm(g2, wo_t, tag="d_attn_out")
-        fused = ctx.fused
-        # 64-row chapters: the chapter-weight gradient is taken in the dK/dV epilogue, where K and V are still in
-        # shared memory, instead of by a pass over the memory-row gradient and the bank rows
-        kv_dot = None
-        if fused is not None and t == 64:
-            kv_dot = torch.empty(b, kv.shape[1] // 64, num_kv_heads, dtype=f32, device=dev)
-        split_bwd = _DQ_ON_SIDE_STREAM and fused is not None
-        if split_bwd:
-            # per-row constants here, then the dQ kernel on the side stream (its consumers follow it there) beside
-            # the dK/dV kernel on this one: each fills the tail of the other's last round of CTAs
-            q3, do3 = q.view(b, l, -1), d_o.view(b, l, -1)
-            bufs = (torch.empty_like(q3), torch.empty_like(kv),
-                    torch.empty(6, b, num_heads, l, dtype=f32, device=dev))
-            akw = dict(buffers=bufs, kv_row_scale=fused["row_scale"], kv_dot=kv_dot)
-            ops.attn_bwd(q3, kv, o, lse, do3, num_heads, num_kv_heads, ctx.scale, parts=1, **akw)
-            side.wait_stream(main)
-            with torch.cuda.stream(side):
-                ops.attn_bwd(q3, kv, o, lse, do3, num_heads, num_kv_heads, ctx.scale, parts=2, **akw)
-            ops.attn_bwd(q3, kv, o, lse, do3, num_heads, num_kv_heads, ctx.scale, parts=4, **akw)
-            d_q, d_kv = bufs[0], bufs[1]
-        else:
-            d_q, d_kv = ops.attn_bwd(q.view(b, l, -1), kv, o, lse, d_o.view(b, l, -1), num_heads, num_kv_heads,
-                                     ctx.scale, kv_row_scale=None if fused is None else fused["row_scale"],
-                                     kv_dot=kv_dot)
-        d_q2 = d_q.view(b * l, -1)
-        d_kv2 = d_kv.view(-1, d_kv.shape[-1])
-
-        if not split_bwd:
-            side.wait_stream(main)
-        with torch.cuda.stream(side):
-            d_wq = ops.gemm(d_q2, h2, a_kmajor=False, b_kmajor=False, out_dtype=f32, split_k=splits(b * l, d, d),
-                            tag="d_wq")
-            # gradient of the (normalised) attention input, in the hidden-state dtype so that the router's
-            # gradient can be added into it
-            d_h = ops.gemm(d_q2, wq_t, out_dtype=f32 if (pre_norm is not None or ha_dtype == f32) else cd, tag="d_h")
-            d_nw = d_nb = None
-            g_res = g2f if add_residual else None
-            if pre_norm is not None:
-                d_h, d_nw, d_nb = ops.norm_bwd(d_h, x2, norm_w, stats_n, None if g_res is None else g_res.float(),
-                                               pre_norm, nb_dtype is not None)
-                d_nw = d_nw.to(nw_dtype)
-                d_nb = None if d_nb is None else d_nb.to(nb_dtype)
-            elif add_residual:
-                d_h = d_h.float() + g_res.float()
-            d_h = d_h.view(b, l, d).to(ha_dtype)
-            ev_dh = torch.cuda.Event()
-            ev_dh.record(side)              # the router's hidden-state gradient is added into d_h later
-            if split_bwd:
-                side.wait_stream(main)      # dK/dV was issued on the main stream
-            if fused is None:
-                d_wkv = ops.gemm(d_kv2, m2, a_kmajor=False, b_kmajor=False, out_dtype=f32,
-                                 split_k=splits(d_kv2.shape[0], wkv_c.shape[0], d), tag="d_wkv")
-            elif fused.get("wkv_grad_in_place"):
-                # dKV' already carries the row scale, so the weight gradient can read the raw bank rows in place
-                # through the gather list on its B operand
-                d_wkv = ops.gemm(d_kv2, fused["shadow"], a_kmajor=False, b_kmajor=False, out_dtype=f32,
-                                 split_k=splits(d_kv2.shape[0], wkv_c.shape[0], d), tag="d_wkv",
-                                 b_row_blocks=r["comb_idx"].reshape(-1), b_block_rows=t, k=d_kv2.shape[0])
+        g = ops._contig(g if g.dtype == attn_dtype else g.to(attn_dtype))
+        as_f32 = lambda v: None if v is None else ops._contig(v.float())     # noqa: E731
+        g_w, g_cw, g_losses = as_f32(g_w), as_f32(g_cw), as_f32(g_losses)
+        fuse_dh = ctx.same_h and need[0] and hr_dtype == in_dtype and in_dtype == attn_dtype
+        d_ha = torch.empty(b, l, d, dtype=attn_dtype, device=dev)
+        d_hr = None if fuse_dh or not need[0] else torch.empty(hr_shape, dtype=hr_dtype, device=dev)
+        rows = wire = dense = None
+        if need[2]:
+            n_rows = n_pairs * t
+            if sink is None:
+                dense = torch.empty(bank.shape, dtype=f32, device=dev)
             else:
-                # ... but with the contraction running over chapters, every K step of that projection lands in
-                # another chapter of the 403 MB copy and it measured twice as slow as over contiguous rows.  This
-                # stream has slack, so the raw selected rows (no norm, no weight: dKV' carries both) are copied out
-                # once here, off the critical path, and the projection runs over the contiguous copy.
-                m_raw, _ = ops.gather_rows_fwd(fused["shadow"], t, r["comb_idx"], None, None, row_eps, cd)
-                d_wkv = ops.gemm(d_kv2, m_raw.view(-1, d), a_kmajor=False, b_kmajor=False, out_dtype=f32,
-                                 split_k=splits(d_kv2.shape[0], wkv_c.shape[0], d), tag="d_wkv")
+                wire_only = sink.wire_only and s.fused and d % 8 == 0 and d <= 1024
+                if not wire_only:
+                    rows = torch.empty(n_rows, d, dtype=f32, device=dev)
+                if sink.wire_dtype == torch.bfloat16:
+                    wire = torch.empty(n_rows, d, dtype=torch.bfloat16, device=dev)
+        d_rw = torch.empty(rw.shape, dtype=f32, device=dev) if (need[3] or need[4]) else None
+        d_rb = torch.empty(rw.shape[0], dtype=f32, device=dev) if (has_rbias and need[4]) else None
+        d_wq = torch.empty(d, d, dtype=f32, device=dev)
+        d_wkv = torch.empty(2 * dkv, d, dtype=f32, device=dev)
+        d_wo = torch.empty(d, d, dtype=f32, device=dev)
+        d_nw = torch.empty(d, dtype=f32, device=dev) if nw is not None else None
+        d_nb = torch.empty(d, dtype=f32, device=dev) if nb_dtype is not None else None
+        q = L.LayerBwdDesc(p(g), p(g_w), p(g_cw), p(g_losses), int(need[0]), int(_DQ_ON_SIDE_STREAM), int(ctx.wkv_in_place),
+                           int(d_rw is not None), p(d_ha), p(d_hr), p(rows), p(wire), p(dense), p(d_rw), p(d_rb), p(d_wq),
+                           p(d_wkv), p(d_wo), p(d_nw), p(d_nb), None)
+        scratch = torch.empty(ops.layer_bwd_scratch_bytes(s, q), dtype=torch.uint8, device=dev)
+        q.scratch = scratch.data_ptr()
+        ops.layer_bwd(s, q)
+        if rows is not None or wire is not None:
+            sink.add(touched[:n_pairs], touched[n_pairs:], wire if rows is None else rows, t, wire=wire)
 
-        d_mem = ops.gemm(d_kv2, wkv_t, tag="d_mem")
-        want_bank = need[2]
-        wire = [] if (ctx.sink is not None and ctx.sink.wire_dtype == torch.bfloat16) else None
-        d_bank = None
-
-        def emit_bank(rows):
-            nonlocal d_bank
-            if not want_bank:
-                return
-            if ctx.sink is not None:
-                ctx.sink.add(seg["uniq"], seg["num_unique"], rows, t, wire=wire[0] if wire else None)
-            else:
-                d_bank = torch.zeros(bank.shape, dtype=f32, device=dev)
-                ops.scatter_bank_grad(rows, seg, t, d_bank)
-                d_bank = d_bank.to(bank.dtype)
-
-        if fused is None:
-            d_cw, rows = ops.gather_rows_bwd(d_mem, bank, t, r["comb_idx"], r["comb_w"], ctx.norm_row, row_eps,
-                                             stats_m, seg, want_dw=True, want_bank=want_bank, wire_copy=wire)
-            emit_bank(rows)
-        else:
-            pre = dict(want_bank=want_bank, wire_copy=wire,
-                       wire_only=ctx.sink is not None and getattr(ctx.sink, "wire_only", False))
-            pargs = (d_mem, fused["shadow"], t, r["comb_idx"], r["comb_w"],
-                     fused["inv_rms"] if ctx.norm_row == "rms" else None, seg)
-            if kv_dot is not None:
-                # the chapter-weight gradient came out of the dK/dV epilogue, so nothing downstream reads the bank
-                # gradient: its kernel runs on the side stream, off the path to the router's backward
-                d_cw = kv_dot.sum(dim=2) / r["comb_w"].clamp_min(1e-30)
-                ev_mem = torch.cuda.Event()
-                ev_mem.record(main)
-                with torch.cuda.stream(side):
-                    side.wait_event(ev_mem)
-                    _, rows = ops.gather_rows_bwd_prescaled(*pargs, want_dw=False, **pre)
-                    emit_bank(rows if rows is not None else (wire[0] if wire else None))
-            else:
-                d_cw, rows = ops.gather_rows_bwd_prescaled(*pargs, want_dw=True, **pre)
-                emit_bank(rows if rows is not None else (wire[0] if wire else None))
-        if g_cw is not None:
-            d_cw = d_cw + g_cw.float()
-        fuse_dh = ctx.same_h and need[0] and hr_dtype == ha_dtype
+        def cast(v, dtype):
+            return v if v is None or v.dtype == dtype else v.to(dtype)
+        d_ha = cast(d_ha, in_dtype)
         if fuse_dh:
-            main.wait_event(ev_dh)      # the attention branch's d_h must be complete before the router adds to it
-        # logit gradient on the main stream; the router-weight gradient (nothing downstream reads it) on the side
-        # stream beside the pooled / hidden-state gradient
-        rargs = (hr_shape, hr_dtype, router_w, r, top_k, num_shared, routed_scale,
-                 None if g_w is None else g_w.float(), d_cw, None if g_losses is None else g_losses.float())
-        rb = ops.router_bwd(*rargs, want_dh=need[0], parts=1)
-        side.wait_stream(main)
-        with torch.cuda.stream(side):
-            ops.router_bwd(*rargs, want_dh=need[0], parts=2, out=rb)
-        ops.router_bwd(*rargs, want_dh=need[0], d_h_accum=d_h if fuse_dh else None, parts=4, out=rb)
-        main.wait_stream(side)
-        d_rw = rb["d_w"].to(router_w.dtype) if need[3] else None
-        d_rb = rb["d_bias"] if (has_rbias and need[4]) else None
-        dkv_dim = wkv_c.shape[0] // 2
-        if fuse_dh:
-            d_hr, d_ha = rb["d_h"], None
-        else:
-            d_hr, d_ha = rb["d_h"], d_h
-        return (d_hr, d_ha, d_bank, d_rw, d_rb, d_wq.to(wdt[0]), d_wkv[:dkv_dim].to(wdt[1]),
-                d_wkv[dkv_dim:].to(wdt[2]), d_wo.to(wdt[3]), d_nw, d_nb, None, None, None)
+            d_hr, d_ha = d_ha, None
+        return (d_hr, d_ha, cast(dense, bank.dtype), cast(d_rw, rw.dtype) if need[3] else None, d_rb, cast(d_wq, wdt[0]),
+                cast(d_wkv[:dkv], wdt[1]), cast(d_wkv[dkv:], wdt[2]), cast(d_wo, wdt[3]),
+                cast(d_nw, nw_dtype), cast(d_nb, nb_dtype), None, None, None)
 
 
 # --------------------------------------------------------------------------------------------
@@ -644,7 +536,7 @@ def memory_layer(h_router: torch.Tensor, h_attn: torch.Tensor, bank: torch.Tenso
                                               "wkv_grad_in_place": wkv_grad_in_place})
         losses = {}
         if with_losses:
-            losses = _LossDict({k: lv[i] for i, k in enumerate(LOSS_KEYS)})
+            losses = _LossDict(zip(LOSS_KEYS, lv.unbind()))
             losses.vector = lv
         return out, losses, {"indices": idx, "weights": w, "combined_indices": cidx, "combined_weights": cw}
     idx, w, cidx, cw, losses = route(h_router, router_weight, router_bias, top_k, num_shared_chapters,

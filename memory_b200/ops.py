@@ -465,6 +465,83 @@ def scatter_bank_grad(bank_grad: torch.Tensor, seg: Dict[str, torch.Tensor], tok
 
 
 # --------------------------------------------------------------------------------------------
+# a whole layer per call
+# --------------------------------------------------------------------------------------------
+def layer_arena_bytes(s) -> int:
+    n = L.lib().moc_layer_arena_bytes(C.byref(s))
+    L.check(-1 if n < 0 else 0, "moc_layer_arena_bytes")
+    return n
+
+
+def layer_bwd_scratch_bytes(s, b) -> int:
+    n = L.lib().moc_layer_bwd_scratch_bytes(C.byref(s), C.byref(b))
+    L.check(-1 if n < 0 else 0, "moc_layer_bwd_scratch_bytes")
+    return n
+
+
+def _report(label: str, launches: int, parts) -> None:
+    """Accounting of a call that issues several operators' kernels: the count, and one hook call per operator."""
+    global LAUNCHES
+    LAUNCHES += launches
+    if LAUNCH_HOOK is not None:
+        for name in parts():
+            LAUNCH_HOOK(name)
+
+
+def _timed(label: str, call) -> int:
+    if TIMER is None:
+        return call()
+    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    e0.record()
+    rc = call()
+    e1.record()
+    TIMER.setdefault(label, []).append((e0, e1))
+    return rc
+
+
+_TAG_OF_CODE = {L.MOC_F32: "f32", L.MOC_BF16: "bf16"}
+
+
+def layer_fwd(s) -> None:
+    """``moc_layer_fwd`` on a filled ``_lib.LayerDesc``."""
+    L.check(_timed("layer_fwd", lambda: L.lib().moc_layer_fwd(C.byref(s))), "moc_layer_fwd")
+    f32_in, norm = s.attn_dtype == L.MOC_F32, s.pre_norm != 0
+
+    def parts():
+        yield "router_fwd:" + _TAG_OF_CODE[s.router_dtype]
+        yield "pack_weights:" + _TAG_OF_CODE[s.weight_dtype]
+        if norm:
+            yield "norm_fwd:f32"
+        yield from ("gemm:bf16",) * 3
+        yield "chapter_row_scale:i32" if s.fused else "gather_rows_fwd:" + _TAG_OF_CODE[s.bank_dtype]
+        yield "attn_fwd:bf16"
+    casts = int(norm or f32_in) + int((norm or s.add_residual) and not f32_in)
+    _report("layer_fwd", 10 + 2 * s.with_losses + s.for_backward + casts, parts)
+
+
+def layer_bwd(s, b) -> None:
+    """``moc_layer_bwd`` on the forward call's descriptor and a filled ``_lib.LayerBwdDesc``."""
+    L.check(_timed("layer_bwd", lambda: L.lib().moc_layer_bwd(C.byref(s), C.byref(b))), "moc_layer_bwd")
+    f32_in, norm = s.attn_dtype == L.MOC_F32, s.pre_norm != 0
+    copies_rows = bool(s.fused) and not b.wkv_grad_in_place
+    want_bank = bool(b.bank_rows or b.bank_rows_bf16 or b.bank_dense)
+
+    def parts():
+        yield from ("gemm:bf16",) * 6
+        yield "attn_bwd:bf16"
+        if norm:
+            yield "norm_bwd:f32"
+        if copies_rows:
+            yield "gather_rows_fwd:bf16"
+        if want_bank:
+            yield "gather_rows_bwd_prescaled:bf16" if s.fused else "gather_rows_bwd:bf16"
+        yield "router_bwd:f32"
+    n = 6 + 3 + int(f32_in) + 2 * int(norm) + int(copies_rows) + int(want_bank) + int(bool(b.bank_dense)) + 1
+    n += 1 + b.want_router_w + 3 * b.want_dh_router
+    _report("layer_bwd", n, parts)
+
+
+# --------------------------------------------------------------------------------------------
 # projections
 # --------------------------------------------------------------------------------------------
 def _gemm_label(a, b, **k):
