@@ -129,6 +129,27 @@ int moc_router_bwd_parts(const moc_router_shape* s, const float* w, const float*
                          void* d_h, int32_t accumulate_dh, void* workspace, size_t workspace_bytes, int32_t parts,
                          int32_t* status, void* stream);
 
+/* The router (moc_router_fwd / _bwd, or position-weighted pooling in front of it when pos_weight [L] is not NULL) with
+ * its scratch and saved state in one buffer: what ChapterRouter.forward issues.  losses NULL: not computed.  Backward:
+ * any of g_* may be NULL; d_h / d_w / d_bias NULL: not wanted (d_bias goes with d_w). */
+typedef struct {
+  moc_router_shape shape;
+  const void* h;
+  const float *w, *bias, *pos_weight;
+  int64_t* idx;
+  float* weights;
+  int32_t* comb_idx;
+  float *comb_w, *losses;
+  void* arena;
+  int32_t* status;
+  void* stream;
+} moc_route_desc;
+int64_t moc_route_arena_bytes(const moc_route_desc* s);
+int64_t moc_route_bwd_scratch_bytes(const moc_route_desc* s);
+int moc_route_fwd(const moc_route_desc* s);
+int moc_route_bwd(const moc_route_desc* s, const float* g_weights, const float* g_comb_w, const float* g_losses,
+                  void* d_h, float* d_w, float* d_bias, void* scratch);
+
 /* Position-weighted pooling: pooled[b, :] = sum_t pos_weight[t] * h[b, t, :] (fp32 accumulation), and its
  * backward d_h[b, t, :] (+)= pos_weight[t] * d_pooled[b, :].  With the coefficients of the rolling-window rule this
  * replaces ChapterRouter._sequence_rolling_pool (memory_transformer/router.py:159-195): the average over t of the
@@ -155,6 +176,15 @@ int moc_gather_rows_fwd(const void* bank, int32_t bank_dtype, int64_t bank_rows,
                         int32_t batch, int32_t k_sel, int32_t norm_type, float eps, void* out,
                         int32_t out_dtype, float* row_stats, int32_t* status, void* stream);
 
+/* idx32[i] = idx[i] (int64 when idx64 != 0, else int32) and flat[i*T + r] = idx[i]*T + r: the row ids that
+ * ChapteredMemoryBank.get_chapters_batched returns beside the rows (memory_bank.py:279-293). */
+int moc_chapter_lists(const void* idx, int32_t idx64, int32_t n, int32_t tokens_per_chapter, int32_t* idx32,
+                      int64_t* flat, void* stream);
+/* The weighted sum of the four router losses (router.py:490-527): out[0] = sum_i c_i losses[i]; with grad != NULL its
+ * gradient instead, out[i] = grad[0] * c_i. */
+int moc_loss_total(const float* losses, const float* grad, float c0, float c1, float c2, float c3, float* out,
+                   void* stream);
+
 /* Groups the B*K (batch, slot) pairs by chapter id, deterministically.
  * uniq [<=n_pairs] ascending chapter ids, seg_offsets [n_pairs+1], seg_pairs [n_pairs] pair ids grouped by
  * chapter and ascending inside a group, pair_to_uniq [n_pairs], num_unique [1].  One CTA; n_pairs <= 65536. */
@@ -174,6 +204,15 @@ int moc_gather_rows_bwd(const void* d_mem, int32_t d_mem_dtype, const void* bank
                         const float* row_stats, const int32_t* uniq, const int32_t* seg_offsets,
                         const int32_t* seg_pairs, const int32_t* num_unique, float* d_comb_w,
                         float* bank_grad, void* bank_grad_bf16, int32_t* status, void* stream);
+
+/* The same from the chapter lists alone: groups the pairs (segments: 4*B*K + 2 ints; its first B*K + 1 come back as the
+ * touched chapters and their count), then the gradients as above -- compact rows in bank_grad / bank_grad_bf16, or, with
+ * bank_dense [bank_rows, dim] instead of bank_grad, written in place there with zeros everywhere else. */
+int moc_gather_rows_bwd_lists(const void* d_mem, int32_t d_mem_dtype, const void* bank, int32_t bank_dtype,
+                              int64_t bank_rows, int32_t dim, int32_t tokens_per_chapter, const int32_t* comb_idx,
+                              const float* comb_w, int32_t batch, int32_t k_sel, int32_t norm_type, float eps,
+                              const float* row_stats, int32_t* segments, float* d_comb_w, float* bank_grad,
+                              void* bank_grad_bf16, float* bank_dense, int32_t* status, void* stream);
 
 /* ---- Fused gather-and-project path (no gathered rows are materialised) ----------------------------------------
  * Forward: moc_gemm with the TMA gather list over a bf16 copy of the bank and row_scale[pair*T + r] = u~[pair]
@@ -522,6 +561,41 @@ typedef struct {
 
 int64_t moc_layer_bwd_scratch_bytes(const moc_layer_desc* s, const moc_layer_bwd_desc* b);
 int moc_layer_bwd(const moc_layer_desc* s, const moc_layer_bwd_desc* b);
+
+/* ------------------------------------------------------------------------------------------------
+ * Cross attention over memory rows that are already gathered and weighted, projections included, in two calls:
+ * out = [h +] Wo attn(Wq [norm](h), Wk memory, Wv memory) (memory_transformer/memory_attention.py:209-261, 298-316,
+ * 452-478; memory_block.py:549-558 with pre_norm / add_residual), and its backward pass.  compute_dtype MOC_BF16 runs
+ * on the tensor cores, MOC_F32 on the FMA pipes.  memory [B, n_sel, mem_dim], or [n_sel, mem_dim] with mem_shared.
+ * out has out_dtype (fp32, or compute_dtype).  The arena of the forward call is the backward call's saved state.
+ * ---------------------------------------------------------------------------------------------- */
+typedef struct {
+  int32_t batch, seq, n_sel, hidden_dim, mem_dim, num_heads, num_kv_heads, mem_shared;
+  int32_t h_dtype, mem_dtype, weight_dtype, compute_dtype, out_dtype;
+  int32_t pre_norm, add_residual, for_backward;
+  float pre_eps;
+  const void *h, *memory, *wq, *wk, *wv, *wo;
+  const float *norm_w, *norm_b;
+  void *out, *arena;
+  int32_t* status;
+  void *stream, *side_stream;
+} moc_xattn_desc;
+
+int64_t moc_xattn_arena_bytes(const moc_xattn_desc* s);
+int moc_xattn_fwd(const moc_xattn_desc* s);
+
+/* g: gradient of `out`, g_dtype.  d_h / d_memory have dtypes d_h_dtype / d_mem_dtype (each fp32 or compute_dtype) and
+ * may be NULL (not wanted); the weight gradients are fp32, d_wkv the K rows then the V rows. */
+typedef struct {
+  const void* g;
+  int32_t g_dtype, d_h_dtype, d_mem_dtype;
+  void *d_h, *d_memory;
+  float *d_wq, *d_wkv, *d_wo, *d_norm_w, *d_norm_b;
+  void* scratch;
+} moc_xattn_bwd_desc;
+
+int64_t moc_xattn_bwd_scratch_bytes(const moc_xattn_desc* s, const moc_xattn_bwd_desc* b);
+int moc_xattn_bwd(const moc_xattn_desc* s, const moc_xattn_bwd_desc* b);
 
 /* Element-wise helpers used by the host layer (device pointers, n elements). */
 int moc_cast_f32_to_bf16(const float* src, void* dst, int64_t n, void* stream);

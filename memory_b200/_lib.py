@@ -65,6 +65,11 @@ def _fields(spec: str):
     return out
 
 
+class RouteDesc(C.Structure):
+    _fields_ = [("shape", RouterShape)] + _fields(
+        "p: h w bias pos_weight idx weights comb_idx comb_w losses arena status stream")
+
+
 class LayerDesc(C.Structure):
     _fields_ = _fields(
         "i: batch seq router_seq hidden_dim num_heads num_kv_heads num_chapters tokens_per_chapter top_k num_shared"
@@ -80,6 +85,18 @@ class LayerBwdDesc(C.Structure):
         "i: want_dh_router dq_on_side_stream wkv_grad_in_place want_router_w;"
         "p: d_h_attn d_h_router bank_rows bank_rows_bf16 bank_dense d_router_w d_router_b d_wq d_wkv d_wo d_norm_w"
         " d_norm_b scratch")
+
+
+class XattnDesc(C.Structure):
+    _fields_ = _fields(
+        "i: batch seq n_sel hidden_dim mem_dim num_heads num_kv_heads mem_shared h_dtype mem_dtype weight_dtype"
+        " compute_dtype out_dtype pre_norm add_residual for_backward; f: pre_eps;"
+        "p: h memory wq wk wv wo norm_w norm_b out arena status stream side_stream")
+
+
+class XattnBwdDesc(C.Structure):
+    _fields_ = _fields("p: g; i: g_dtype d_h_dtype d_mem_dtype;"
+                       "p: d_h d_memory d_wq d_wkv d_wo d_norm_w d_norm_b scratch")
 
 
 P = C.c_void_p
@@ -101,6 +118,8 @@ _PROTOTYPES = {
     "moc_chapter_segments": (C.c_int, [P, C.c_int32, C.c_int32, P, P, P, P, P, P, P]),
     "moc_gather_rows_bwd": (C.c_int, [P, C.c_int32, P, C.c_int32, C.c_int64, C.c_int32, C.c_int32, P, P,
                                       C.c_int32, C.c_int32, C.c_int32, C.c_float, P, P, P, P, P, P, P, P, P, P]),
+    "moc_gather_rows_bwd_lists": (C.c_int, [P, C.c_int32, P, C.c_int32, C.c_int64, C.c_int32, C.c_int32, P, P, C.c_int32,
+                                            C.c_int32, C.c_int32, C.c_float, P, P, P, P, P, P, P, P]),
     "moc_bank_grad_merge": (C.c_int, [P, C.c_int32, C.c_int32, P, P, C.c_int32, C.c_int32, C.c_int32, C.c_int32,
                                       C.c_float, P, P, P, P, P, P, C.c_int64, P, P]),
     "moc_bank_grad_merge_to": (C.c_int, [P, C.c_int32, C.c_int32, P, P, C.c_int32, C.c_int32, C.c_int32, C.c_int32,
@@ -128,6 +147,16 @@ _PROTOTYPES = {
     "moc_layer_fwd": (C.c_int, [C.POINTER(LayerDesc)]),
     "moc_layer_bwd_scratch_bytes": (C.c_int64, [C.POINTER(LayerDesc), C.POINTER(LayerBwdDesc)]),
     "moc_layer_bwd": (C.c_int, [C.POINTER(LayerDesc), C.POINTER(LayerBwdDesc)]),
+    "moc_xattn_arena_bytes": (C.c_int64, [C.POINTER(XattnDesc)]),
+    "moc_xattn_fwd": (C.c_int, [C.POINTER(XattnDesc)]),
+    "moc_xattn_bwd_scratch_bytes": (C.c_int64, [C.POINTER(XattnDesc), C.POINTER(XattnBwdDesc)]),
+    "moc_xattn_bwd": (C.c_int, [C.POINTER(XattnDesc), C.POINTER(XattnBwdDesc)]),
+    "moc_route_arena_bytes": (C.c_int64, [C.POINTER(RouteDesc)]),
+    "moc_route_bwd_scratch_bytes": (C.c_int64, [C.POINTER(RouteDesc)]),
+    "moc_route_fwd": (C.c_int, [C.POINTER(RouteDesc)]),
+    "moc_route_bwd": (C.c_int, [C.POINTER(RouteDesc), P, P, P, P, P, P, P]),
+    "moc_chapter_lists": (C.c_int, [P, C.c_int32, C.c_int32, C.c_int32, P, P, P]),
+    "moc_loss_total": (C.c_int, [P, P, C.c_float, C.c_float, C.c_float, C.c_float, P, P]),
     "moc_sparse_attn_tc_sizes": (C.c_int, [C.POINTER(SparseAttnShape), P, P, P]),
     "moc_sparse_attn_tc_fwd": (C.c_int, [C.POINTER(SparseAttnShape), P, P, P, P, P, P, P, P, P, P]),
     "moc_sparse_attn_tc_bwd": (C.c_int, [C.POINTER(SparseAttnShape), P, P, P, P, P, C.c_int32, P, P, P, P, P, P, P, P, P]),

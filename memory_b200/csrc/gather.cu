@@ -3,7 +3,7 @@
 // All kernels are HBM bound: one warp per 1-D row, vector accesses where alignment allows.
 #include <math.h>
 
-#include "moc_common.cuh"
+#include "host_pass.cuh"
 
 namespace moc {
 namespace {
@@ -352,7 +352,7 @@ __global__ void bank_grad_kernel(const TG* __restrict__ d_mem, const TB* __restr
                                  int norm_type, const int* __restrict__ uniq,
                                  const int* __restrict__ seg_offsets, const int* __restrict__ seg_pairs,
                                  const int* __restrict__ num_unique, long long max_rows,
-                                 float* __restrict__ bank_grad, __nv_bfloat16* __restrict__ bank_grad_wire) {
+                                 float* __restrict__ bank_grad, __nv_bfloat16* __restrict__ bank_grad_wire, int dense) {
   const int lane = threadIdx.x & 31;
   const long long r = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
   if (r >= max_rows) return;
@@ -360,7 +360,8 @@ __global__ void bank_grad_kernel(const TG* __restrict__ d_mem, const TB* __restr
   if (u >= num_unique[0]) return;
   const int within = static_cast<int>(r - static_cast<long long>(u) * T);
   const int p0 = seg_offsets[u], p1 = seg_offsets[u + 1];
-  float* dst = bank_grad + r * dim;
+  // dense: bank_grad is shaped like the bank, rows go to their place in it (the caller has cleared it)
+  float* dst = bank_grad + (dense ? static_cast<long long>(uniq[u]) * T + within : r) * dim;
   // optional second copy in bf16: what travels between ranks when the exchange is asked to halve its volume
   __nv_bfloat16* wire = bank_grad_wire ? bank_grad_wire + r * dim : nullptr;
   if (norm_type == MOC_NORM_NONE && (dim & 7) == 0) {
@@ -440,6 +441,17 @@ __global__ void row_inv_rms_kernel(const TB* __restrict__ bank, long long rows, 
   acc = warp_sum(acc);
   if (lane == 0) out[r] = rsqrtf(acc / static_cast<float>(dim) + eps);
 }
+// idx32[i] = idx[i], flat[i * T + r] = idx[i] * T + r
+template <typename I>
+__global__ void chapter_lists_kernel(const I* __restrict__ idx, int n, int T, int* __restrict__ idx32,
+                                     long long* __restrict__ flat) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= n * T) return;
+  const int i = e / T, r = e - i * T;
+  const long long c = idx[i];
+  flat[e] = c * T + r;
+  if (r == 0) idx32[i] = static_cast<int>(c);
+}
 // scale[pair * T + r] = comb_w[pair] * (inv_rms ? inv_rms[comb_idx[pair] * T + r] : 1)
 __global__ void row_scale_kernel(const int* __restrict__ comb_idx, const float* __restrict__ comb_w,
                                  const float* __restrict__ inv_rms, long long bank_rows, int n_pairs, int T,
@@ -496,7 +508,7 @@ __global__ void bank_grad_prescaled_kernel(const TG* __restrict__ g, const TB* _
                                            const float* __restrict__ inv_rms, const int* __restrict__ uniq,
                                            const int* __restrict__ seg_offsets, const int* __restrict__ seg_pairs,
                                            const int* __restrict__ num_unique, long long max_rows,
-                                           float* __restrict__ bank_grad, __nv_bfloat16* __restrict__ bank_grad_wire) {
+                                           float* __restrict__ bank_grad, __nv_bfloat16* __restrict__ bank_grad_wire, int dense) {
   const int lane = threadIdx.x & 31;
   const long long r = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
   if (r >= max_rows) return;
@@ -506,9 +518,9 @@ __global__ void bank_grad_prescaled_kernel(const TG* __restrict__ g, const TB* _
   const int p0 = seg_offsets[u], p1 = seg_offsets[u + 1];
   // bank_grad may be NULL when only the bf16 rows are wanted (a data-parallel step whose mean gradient is formed
   // from the ranks' bf16 rows): the vector path below then skips the fp32 store
-  float* dst = bank_grad ? bank_grad + r * dim : nullptr;
   __nv_bfloat16* wire = bank_grad_wire ? bank_grad_wire + r * dim : nullptr;
   const long long brow = static_cast<long long>(uniq[u]) * T + within;
+  float* dst = bank_grad ? bank_grad + (dense ? brow : r) * dim : nullptr;
   const TB* row = bank + brow * dim;
   if ((dim & 7) == 0 && dim <= 8 * 32 * 4) {
     // 16-byte accesses: lane l owns columns [8 l + 256 n, +8); the sums stay in registers for the norm term
@@ -750,13 +762,13 @@ extern "C" int moc_bank_grad_merge(const void* const* rank_rows, int32_t rows_dt
                                 rows_out_capacity, status, stream_);
 }
 
-extern "C" int moc_gather_rows_bwd(const void* d_mem, int32_t d_mem_dtype, const void* bank, int32_t bank_dtype,
+int moc::gather_rows_bwd_impl(const void* d_mem, int32_t d_mem_dtype, const void* bank, int32_t bank_dtype,
                                    int64_t bank_rows, int32_t dim, int32_t T, const int32_t* comb_idx,
                                    const float* comb_w, int32_t batch, int32_t k_sel, int32_t norm_type,
                                    float eps, const float* row_stats, const int32_t* uniq,
                                    const int32_t* seg_offsets, const int32_t* seg_pairs,
                                    const int32_t* num_unique, float* d_comb_w, float* bank_grad,
-                                   void* bank_grad_bf16, int32_t* status, void* stream_) {
+                                   void* bank_grad_bf16, int32_t* status, void* stream_, int dense) {
   (void)eps; (void)status;
   MOC_REQUIRE(d_mem && bank && comb_idx && uniq && seg_offsets && seg_pairs && num_unique, "NULL buffer");
   MOC_REQUIRE(norm_type == MOC_NORM_NONE || row_stats != nullptr, "row_stats needed for normalised rows");
@@ -775,7 +787,7 @@ extern "C" int moc_gather_rows_bwd(const void* d_mem, int32_t d_mem_dtype, const
                                                            static_cast<const TB*>(bank), dim, T, comb_w,      \
                                                            row_stats, norm_type, uniq, seg_offsets,           \
                                                            seg_pairs, num_unique, max_rows, bank_grad,        \
-                                                           static_cast<__nv_bfloat16*>(bank_grad_bf16));      \
+                                                           static_cast<__nv_bfloat16*>(bank_grad_bf16), dense);\
   } while (0)
   if (d_mem_dtype == MOC_F32 && bank_dtype == MOC_F32) MOC_GBWD(float, float);
   else if (d_mem_dtype == MOC_F32 && bank_dtype == MOC_BF16) MOC_GBWD(float, __nv_bfloat16);
@@ -786,6 +798,16 @@ extern "C" int moc_gather_rows_bwd(const void* d_mem, int32_t d_mem_dtype, const
   MOC_CUDA_OK(cudaGetLastError());
   return MOC_OK;
 }
+extern "C" int moc_gather_rows_bwd(const void* d_mem, int32_t d_mem_dtype, const void* bank, int32_t bank_dtype,
+                                   int64_t bank_rows, int32_t dim, int32_t T, const int32_t* comb_idx,
+                                   const float* comb_w, int32_t batch, int32_t k_sel, int32_t norm_type,
+                                   float eps, const float* row_stats, const int32_t* uniq,
+                                   const int32_t* seg_offsets, const int32_t* seg_pairs,
+                                   const int32_t* num_unique, float* d_comb_w, float* bank_grad,
+                                   void* bank_grad_bf16, int32_t* status, void* stream_) {
+  return gather_rows_bwd_impl(d_mem, d_mem_dtype, bank, bank_dtype, bank_rows, dim, T, comb_idx, comb_w, batch, k_sel, norm_type, eps, row_stats, uniq, seg_offsets, seg_pairs, num_unique, d_comb_w, bank_grad, bank_grad_bf16, status, stream_, 0);
+}
+
 
 extern "C" int moc_scatter_bank_grad(const float* bank_grad, const int32_t* uniq, const int32_t* num_unique,
                                      int32_t max_unique, int32_t T, int32_t dim, float* bank_dense,
@@ -896,6 +918,18 @@ extern "C" int moc_row_inv_rms(const void* bank, int32_t bank_dtype, int64_t row
   return MOC_OK;
 }
 
+extern "C" int moc_chapter_lists(const void* idx, int32_t idx64, int32_t n, int32_t T, int32_t* idx32, int64_t* flat,
+                                 void* stream_) {
+  MOC_REQUIRE(idx && idx32 && flat && n > 0 && T > 0 && static_cast<int64_t>(n) * T < (1ll << 31), "bad chapter list");
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  const int blocks = ceil_div(n * T, 256);
+  long long* out = reinterpret_cast<long long*>(flat);
+  if (idx64) chapter_lists_kernel<long long><<<blocks, 256, 0, stream>>>(static_cast<const long long*>(idx), n, T, idx32, out);
+  else chapter_lists_kernel<int><<<blocks, 256, 0, stream>>>(static_cast<const int*>(idx), n, T, idx32, out);
+  MOC_CUDA_OK(cudaGetLastError());
+  return MOC_OK;
+}
+
 extern "C" int moc_chapter_row_scale(const int32_t* comb_idx, const float* comb_w, const float* inv_rms,
                                      int64_t bank_rows, int32_t n_pairs, int32_t T, float* scale, int32_t* status,
                                      void* stream_) {
@@ -907,12 +941,12 @@ extern "C" int moc_chapter_row_scale(const int32_t* comb_idx, const float* comb_
   return MOC_OK;
 }
 
-extern "C" int moc_gather_rows_bwd_prescaled(const void* g, int32_t g_dtype, const void* bank, int32_t bank_dtype,
+int moc::gather_rows_bwd_prescaled_impl(const void* g, int32_t g_dtype, const void* bank, int32_t bank_dtype,
                                              int64_t bank_rows, int32_t dim, int32_t T, const int32_t* comb_idx,
                                              const float* comb_w, int32_t n_pairs, const float* inv_rms,
                                              const int32_t* uniq, const int32_t* seg_offsets,
                                              const int32_t* seg_pairs, const int32_t* num_unique, float* d_comb_w,
-                                             float* bank_grad, void* bank_grad_bf16, int32_t* status, void* stream_) {
+                                             float* bank_grad, void* bank_grad_bf16, int32_t* status, void* stream_, int dense) {
   (void)status;
   MOC_REQUIRE(g && bank && comb_idx && uniq && seg_offsets && seg_pairs && num_unique, "NULL buffer");
   MOC_REQUIRE(bank_grad != nullptr || bank_grad_bf16 == nullptr || ((dim & 7) == 0 && dim <= 1024),
@@ -929,7 +963,7 @@ extern "C" int moc_gather_rows_bwd_prescaled(const void* g, int32_t g_dtype, con
     if (bank_grad != nullptr || bank_grad_bf16 != nullptr)                                                        \
       bank_grad_prescaled_kernel<TG, TB><<<blocks, 256, 0, stream>>>(                                             \
           static_cast<const TG*>(g), static_cast<const TB*>(bank), dim, T, inv_rms, uniq, seg_offsets, seg_pairs, \
-          num_unique, max_rows, bank_grad, static_cast<__nv_bfloat16*>(bank_grad_bf16));                          \
+          num_unique, max_rows, bank_grad, static_cast<__nv_bfloat16*>(bank_grad_bf16), dense);                   \
   } while (0)
   if (g_dtype == MOC_F32 && bank_dtype == MOC_F32) MOC_GPRE(float, float);
   else if (g_dtype == MOC_F32 && bank_dtype == MOC_BF16) MOC_GPRE(float, __nv_bfloat16);
@@ -940,3 +974,12 @@ extern "C" int moc_gather_rows_bwd_prescaled(const void* g, int32_t g_dtype, con
   MOC_CUDA_OK(cudaGetLastError());
   return MOC_OK;
 }
+extern "C" int moc_gather_rows_bwd_prescaled(const void* g, int32_t g_dtype, const void* bank, int32_t bank_dtype,
+                                             int64_t bank_rows, int32_t dim, int32_t T, const int32_t* comb_idx,
+                                             const float* comb_w, int32_t n_pairs, const float* inv_rms,
+                                             const int32_t* uniq, const int32_t* seg_offsets,
+                                             const int32_t* seg_pairs, const int32_t* num_unique, float* d_comb_w,
+                                             float* bank_grad, void* bank_grad_bf16, int32_t* status, void* stream_) {
+  return gather_rows_bwd_prescaled_impl(g, g_dtype, bank, bank_dtype, bank_rows, dim, T, comb_idx, comb_w, n_pairs, inv_rms, uniq, seg_offsets, seg_pairs, num_unique, d_comb_w, bank_grad, bank_grad_bf16, status, stream_, 0);
+}
+

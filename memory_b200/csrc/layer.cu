@@ -3,9 +3,7 @@
 // Issued one operator at a time from Python, a training step of this layer is 38 launches at 25 to 45 us of host time
 // each (tensor allocation, argument conversion, stream look-ups): 1.15 ms for a step whose kernels take 0.36 ms on one
 // 320-token sequence, 0.43 ms for a forward whose kernels take 0.18 ms.  Here a pass is one call with one arena.
-#include <algorithm>
-
-#include "moc_common.cuh"
+#include "host_pass.cuh"
 
 namespace moc {
 namespace {
@@ -25,16 +23,6 @@ __global__ void add_kernel(float* __restrict__ a, const float* __restrict__ b, i
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) a[i] += b[i];
 }
-
-struct Carver {
-  char* base;
-  int64_t off;
-  template <typename T> T* take(int64_t n) {
-    T* r = reinterpret_cast<T*>(base + off);
-    off += (n * static_cast<int64_t>(sizeof(T)) + 255) & ~int64_t(255);
-    return r;
-  }
-};
 
 struct Dims {
   int64_t rows, n_sel, sel_rows, pairs, d, dkv;
@@ -94,68 +82,6 @@ int64_t carve(const moc_layer_desc* s, const Dims& x, void* arena, Saved* a) {
   return c.off;
 }
 
-// Events that order the two streams of one pass.  A wait refers to the record before it, so a thread can use the same
-// few events for every pass it issues; they belong to the device they were made on.
-struct EventRing {
-  static constexpr int kMax = 16;
-  cudaEvent_t ev[kMax];
-  int device = -1, next = 0;
-};
-int fork_event(cudaStream_t from, cudaEvent_t* out) {
-  thread_local EventRing ring[16];
-  int dev = 0;
-  MOC_CUDA_OK(cudaGetDevice(&dev));
-  MOC_REQUIRE(dev >= 0 && dev < 16, "device index out of range");
-  EventRing& r = ring[dev];
-  if (r.device != dev) {
-    for (int i = 0; i < EventRing::kMax; ++i) MOC_CUDA_OK(cudaEventCreateWithFlags(&r.ev[i], cudaEventDisableTiming));
-    r.device = dev;
-  }
-  *out = r.ev[r.next];
-  r.next = (r.next + 1) % EventRing::kMax;
-  MOC_CUDA_OK(cudaEventRecord(*out, from));
-  return MOC_OK;
-}
-int order(cudaStream_t before, cudaStream_t after) {      // `after` continues behind what `before` holds now
-  cudaEvent_t e;
-  const int rc = fork_event(before, &e);
-  if (rc != MOC_OK) return rc;
-  MOC_CUDA_OK(cudaStreamWaitEvent(after, e, 0));
-  return MOC_OK;
-}
-
-#define MOC_TRY(expr)                    \
-  do {                                   \
-    const int _rc = (expr);              \
-    if (_rc != MOC_OK) return _rc;       \
-  } while (0)
-
-struct Gemm : moc_gemm_desc {
-  // C [m, n] = op(A) op(B), dense operands
-  Gemm(int64_t m_, int64_t n_, int64_t k_, bool a_k, bool b_k, int c_dt) {
-    dtype = MOC_BF16; c_dtype = c_dt;
-    m = static_cast<int>(m_); n = static_cast<int>(n_); k = static_cast<int>(k_);
-    a_kmajor = a_k; b_kmajor = b_k;
-    lda = a_k ? k : m; ldb = b_k ? k : n; ldc = n;
-    accumulate = 0; split_k = 1; scale_block_rows = 1; a_block_rows = 0;
-    a_stored_rows = a_k ? m : k;
-    residual = nullptr; ldr = 0;
-  }
-};
-// K-splits of a weight gradient [out_rows, out_cols] over `rows`: enough (tile, split) items to fill the SMs once
-int splits(int64_t rows, int64_t out_rows, int64_t out_cols) {
-  const int64_t tiles = ((out_rows + 127) / 128) * ((out_cols + 255) / 256);
-  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(148 / std::max<int64_t>(tiles, 1), rows / 512)));
-}
-// dW [m, n] fp32 = A^T B over `rows`
-int weight_grad(int64_t m, int64_t n, int64_t rows, const void* a, const void* b, float* out, int* status, void* stream) {
-  Gemm g(m, n, rows, false, false, MOC_F32);
-  g.split_k = splits(rows, m, n);
-  if (g.split_k > 1)
-    MOC_CUDA_OK(cudaMemsetAsync(out, 0, static_cast<size_t>(m * n) * 4, static_cast<cudaStream_t>(stream)));
-  return moc_gemm(&g, a, b, out, nullptr, nullptr, status, stream);
-}
-
 int check(const moc_layer_desc* s) {
   MOC_REQUIRE(s != nullptr, "layer descriptor is NULL");
   MOC_REQUIRE(s->batch > 0 && s->seq > 0 && s->hidden_dim > 0 && s->num_heads > 0 && s->num_kv_heads > 0 &&
@@ -171,6 +97,43 @@ int check(const moc_layer_desc* s) {
 }
 
 }  // namespace
+
+struct EventRing {
+  static constexpr int kMax = 16;
+  cudaEvent_t ev[kMax];
+  bool made = false;
+  int next = 0;
+};
+int fork_event(cudaStream_t from, cudaEvent_t* out) {
+  thread_local EventRing ring[16];
+  int dev = 0;
+  MOC_CUDA_OK(cudaGetDevice(&dev));
+  MOC_REQUIRE(dev >= 0 && dev < 16, "device index out of range");
+  EventRing& r = ring[dev];
+  if (!r.made) {
+    for (int i = 0; i < EventRing::kMax; ++i) MOC_CUDA_OK(cudaEventCreateWithFlags(&r.ev[i], cudaEventDisableTiming));
+    r.made = true;
+  }
+  *out = r.ev[r.next];
+  r.next = (r.next + 1) % EventRing::kMax;
+  MOC_CUDA_OK(cudaEventRecord(*out, from));
+  return MOC_OK;
+}
+int order(cudaStream_t before, cudaStream_t after) {
+  cudaEvent_t e;
+  MOC_TRY(fork_event(before, &e));
+  MOC_CUDA_OK(cudaStreamWaitEvent(after, e, 0));
+  return MOC_OK;
+}
+int weight_grad(int dtype, int64_t m, int64_t n, int64_t rows, const void* a, const void* b, float* out, int* status,
+                void* stream) {
+  Gemm g(dtype, m, n, rows, false, false, MOC_F32);
+  if (dtype == MOC_BF16) g.split_k = splits(rows, m, n);
+  if (g.split_k > 1)
+    MOC_CUDA_OK(cudaMemsetAsync(out, 0, static_cast<size_t>(m * n) * 4, static_cast<cudaStream_t>(stream)));
+  return moc_gemm(&g, a, b, out, nullptr, nullptr, status, stream);
+}
+
 }  // namespace moc
 
 using namespace moc;
@@ -226,12 +189,12 @@ extern "C" int moc_layer_fwd(const moc_layer_desc* s) {
   else if (a.h2)
     MOC_TRY(moc_cast_f32_to_bf16(static_cast<const float*>(s->h_attn), a.h2, x.rows * d, main));
   {
-    const Gemm g(x.rows, d, d, true, true, MOC_BF16);
+    const Gemm g(MOC_BF16, x.rows, d, d, true, true, MOC_BF16);
     MOC_TRY(moc_gemm(&g, h2, a.wq, a.q, nullptr, nullptr, s->status, main));
   }
 
   MOC_CUDA_OK(cudaStreamWaitEvent(main, routed, 0));
-  Gemm g(x.sel_rows, 2 * x.dkv, d, true, true, MOC_BF16);
+  Gemm g(MOC_BF16, x.sel_rows, 2 * x.dkv, d, true, true, MOC_BF16);
   if (s->fused) {
     // gather, normalisation, weight multiply and the K/V projection in one kernel: chapters are read from the bf16 copy
     // of the bank through the TMA gather list, u~ (and 1/rms) is the epilogue's row scale
@@ -249,7 +212,7 @@ extern "C" int moc_layer_fwd(const moc_layer_desc* s) {
   const moc_attn_shape as = {B, L, static_cast<int32_t>(x.n_sel), s->num_heads, s->num_kv_heads, hd,
                              1.0f / sqrtf(static_cast<float>(hd)), MOC_BF16};
   MOC_TRY(moc_attn_fwd(&as, a.q, a.kv, a.o, a.lse, s->status, main));
-  Gemm go(x.rows, d, d, true, true, s->attn_dtype);
+  Gemm go(MOC_BF16, x.rows, d, d, true, true, s->attn_dtype);
   if (s->add_residual) { go.residual = x2; go.ldr = d; }
   MOC_TRY(moc_gemm(&go, a.o, a.wo, s->out, nullptr, nullptr, s->status, main));
   return order(side, main);
@@ -261,7 +224,7 @@ namespace {
 struct Scratch {
   __nv_bfloat16 *g2, *d_o, *d_q, *d_kv, *d_mem, *m_raw;
   float *g32, *dh32, *dx32;         // fp32 forms of the output gradient / the attention input's gradient
-  float *attn, *kv_dot, *d_comb_w, *d_logits, *d_pooled, *dummy_b, *bank_rows;
+  float *attn, *kv_dot, *d_comb_w, *d_logits, *d_pooled, *dummy_b;
   char *router_ws, *norm_ws;
 };
 int64_t carve_bwd(const moc_layer_desc* s, const moc_layer_bwd_desc* b, const Dims& x, void* scratch, Scratch* t) {
@@ -283,7 +246,6 @@ int64_t carve_bwd(const moc_layer_desc* s, const moc_layer_bwd_desc* b, const Di
   t->d_pooled = c.take<float>(static_cast<int64_t>(s->batch) * x.d);
   t->dummy_b = c.take<float>(s->num_chapters);
   t->router_ws = c.take<char>(static_cast<int64_t>(moc_router_workspace_bytes(&rs)));
-  t->bank_rows = b->bank_dense && !b->bank_rows ? c.take<float>(x.sel_rows * x.d) : nullptr;
   return c.off;
 }
 
@@ -319,9 +281,9 @@ extern "C" int moc_layer_bwd(const moc_layer_desc* s, const moc_layer_bwd_desc* 
     g2 = t.g2;
   }
   MOC_TRY(order(main, side));
-  MOC_TRY(weight_grad(d, d, x.rows, g2, a.o, b->d_wo, st, side));
+  MOC_TRY(weight_grad(MOC_BF16, d, d, x.rows, g2, a.o, b->d_wo, st, side));
   {
-    const Gemm g(x.rows, d, d, true, true, MOC_BF16);
+    const Gemm g(MOC_BF16, x.rows, d, d, true, true, MOC_BF16);
     MOC_TRY(moc_gemm(&g, g2, a.wo_t, t.d_o, nullptr, nullptr, st, main));
   }
   // With 64-row chapters the chapter-weight gradient is taken in the dK/dV epilogue, where K and V are still in shared
@@ -346,9 +308,9 @@ extern "C" int moc_layer_bwd(const moc_layer_desc* s, const moc_layer_bwd_desc* 
   }
 
   // side stream: what only the dQ path feeds
-  MOC_TRY(weight_grad(d, d, x.rows, t.d_q, h2, b->d_wq, st, side));
+  MOC_TRY(weight_grad(MOC_BF16, d, d, x.rows, t.d_q, h2, b->d_wq, st, side));
   {
-    Gemm g(x.rows, d, d, true, true, norm ? MOC_F32 : s->attn_dtype);
+    Gemm g(MOC_BF16, x.rows, d, d, true, true, norm ? MOC_F32 : s->attn_dtype);
     const float* g32 = f32 ? static_cast<const float*>(b->g) : t.g32;
     if (s->add_residual && t.g32) MOC_TRY(moc_cast_bf16_to_f32(b->g, t.g32, n_el, side));
     if (norm) {
@@ -367,10 +329,10 @@ extern "C" int moc_layer_bwd(const moc_layer_desc* s, const moc_layer_bwd_desc* 
   MOC_TRY(fork_event(side, &dh_done));
   if (split) MOC_TRY(order(main, side));          // dK/dV is on the main stream
   if (!s->fused) {
-    MOC_TRY(weight_grad(2 * x.dkv, d, x.sel_rows, t.d_kv, a.m2, b->d_wkv, st, side));
+    MOC_TRY(weight_grad(MOC_BF16, 2 * x.dkv, d, x.sel_rows, t.d_kv, a.m2, b->d_wkv, st, side));
   } else if (b->wkv_grad_in_place) {
     // dKV' already carries the row scale, so the raw bank rows can be read in place through a gather list on B
-    Gemm g(2 * x.dkv, d, x.sel_rows, false, false, MOC_F32);
+    Gemm g(MOC_BF16, 2 * x.dkv, d, x.sel_rows, false, false, MOC_F32);
     g.split_k = splits(x.sel_rows, 2 * x.dkv, d);
     if (g.split_k > 1) MOC_CUDA_OK(cudaMemsetAsync(b->d_wkv, 0, static_cast<size_t>(2 * x.dkv * d) * 4, side));
     MOC_TRY(moc_gemm_gather_b(&g, t.d_kv, s->bank_shadow, b->d_wkv, nullptr, s->comb_idx, s->tokens_per_chapter, bank_rows_n,
@@ -380,34 +342,28 @@ extern "C" int moc_layer_bwd(const moc_layer_desc* s, const moc_layer_bwd_desc* 
     // 403 MB copy, which measured twice as slow; the raw selected rows are copied out once, off the critical path
     MOC_TRY(moc_gather_rows_fwd(s->bank_shadow, MOC_BF16, bank_rows_n, d, s->tokens_per_chapter, s->comb_idx, nullptr, B,
                                 s->num_shared + x.k_sel, MOC_NORM_NONE, s->row_eps, t.m_raw, MOC_BF16, nullptr, st, side));
-    MOC_TRY(weight_grad(2 * x.dkv, d, x.sel_rows, t.d_kv, t.m_raw, b->d_wkv, st, side));
+    MOC_TRY(weight_grad(MOC_BF16, 2 * x.dkv, d, x.sel_rows, t.d_kv, t.m_raw, b->d_wkv, st, side));
   }
 
   {
-    const Gemm g(x.sel_rows, d, 2 * x.dkv, true, true, MOC_BF16);
+    const Gemm g(MOC_BF16, x.sel_rows, d, 2 * x.dkv, true, true, MOC_BF16);
     MOC_TRY(moc_gemm(&g, t.d_kv, a.wkv_t, t.d_mem, nullptr, nullptr, st, main));
   }
   const bool want_bank = b->bank_rows || b->bank_rows_bf16 || b->bank_dense;
-  float* rows_out = b->bank_rows ? b->bank_rows : t.bank_rows;
+  const int dense = b->bank_dense != nullptr;
+  float* rows_out = dense ? b->bank_dense : b->bank_rows;
   auto bank_grad = [&](float* d_cw, cudaStream_t stream) -> int {
+    if (dense) MOC_TRY(clear_dense(b->bank_dense, bank_rows_n * d, stream));
     if (s->fused) {
-      if (d_cw || want_bank)
-        MOC_TRY(moc_gather_rows_bwd_prescaled(t.d_mem, MOC_BF16, s->bank_shadow, MOC_BF16, bank_rows_n, d,
-                                              s->tokens_per_chapter, s->comb_idx, s->comb_w, static_cast<int>(x.pairs),
-                                              s->row_norm == MOC_NORM_RMS ? s->bank_inv_rms : nullptr, s->uniq, a.seg_off,
-                                              a.seg_pairs, s->num_unique, d_cw, rows_out, b->bank_rows_bf16, st, stream));
-    } else {
-      MOC_TRY(moc_gather_rows_bwd(t.d_mem, MOC_BF16, s->bank, s->bank_dtype, bank_rows_n, d, s->tokens_per_chapter,
-                                  s->comb_idx, s->comb_w, B, s->num_shared + x.k_sel, s->row_norm, s->row_eps, a.stats_m,
-                                  s->uniq, a.seg_off, a.seg_pairs, s->num_unique, d_cw, rows_out, b->bank_rows_bf16, st,
-                                  stream));
+      if (!d_cw && !want_bank) return MOC_OK;
+      return gather_rows_bwd_prescaled_impl(t.d_mem, MOC_BF16, s->bank_shadow, MOC_BF16, bank_rows_n, d,
+                                            s->tokens_per_chapter, s->comb_idx, s->comb_w, static_cast<int>(x.pairs),
+                                            s->row_norm == MOC_NORM_RMS ? s->bank_inv_rms : nullptr, s->uniq, a.seg_off,
+                                            a.seg_pairs, s->num_unique, d_cw, rows_out, b->bank_rows_bf16, st, stream, dense);
     }
-    if (b->bank_dense) {
-      MOC_CUDA_OK(cudaMemsetAsync(b->bank_dense, 0, static_cast<size_t>(bank_rows_n) * d * 4, stream));
-      MOC_TRY(moc_scatter_bank_grad(rows_out, s->uniq, s->num_unique, static_cast<int>(x.pairs), s->tokens_per_chapter, d,
-                                    b->bank_dense, bank_rows_n, st, stream));
-    }
-    return MOC_OK;
+    return gather_rows_bwd_impl(t.d_mem, MOC_BF16, s->bank, s->bank_dtype, bank_rows_n, d, s->tokens_per_chapter, s->comb_idx,
+                                s->comb_w, B, s->num_shared + x.k_sel, s->row_norm, s->row_eps, a.stats_m, s->uniq,
+                                a.seg_off, a.seg_pairs, s->num_unique, d_cw, rows_out, b->bank_rows_bf16, st, stream, dense);
   };
   const int n_pairs = static_cast<int>(x.pairs), pair_blocks = ceil_div(n_pairs, 256);
   if (t.kv_dot) {

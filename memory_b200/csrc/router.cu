@@ -524,6 +524,20 @@ __global__ void loss_finish_kernel(const float* __restrict__ partial, const floa
   }
 }
 
+// out[0] = c . losses, or with grad: out[0..3] = grad * c
+__global__ void loss_total_kernel(const float* __restrict__ losses, const float* __restrict__ grad, float4 c,
+                                  float* __restrict__ out) {
+  const float cs[4] = {c.x, c.y, c.z, c.w};
+  if (grad != nullptr) {
+    if (threadIdx.x < 4) out[threadIdx.x] = grad[0] * cs[threadIdx.x];
+  } else if (threadIdx.x == 0) {
+    float t = 0.f;
+    for (int i = 0; i < 4; ++i)
+      if (cs[i] != 0.f) t += cs[i] * losses[i];
+    out[0] = t;
+  }
+}
+
 // logits[r, c] += bias[c]
 __global__ void add_bias_kernel(float* __restrict__ logits, const float* __restrict__ bias, long long total, int C) {
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
@@ -1009,6 +1023,14 @@ extern "C" int moc_sum_terms(const float* src, const float* bias, float* dst, in
   if (blocks > 148LL * 32) blocks = 148LL * 32;
   sum_terms_kernel<<<static_cast<int>(blocks), 256, 0, static_cast<cudaStream_t>(stream_)>>>(src, bias, dst, rows, cols,
                                                                                              ld, terms);
+  MOC_CUDA_OK(cudaGetLastError());
+  return MOC_OK;
+}
+
+extern "C" int moc_loss_total(const float* losses, const float* grad, float c0, float c1, float c2, float c3, float* out,
+                              void* stream_) {
+  MOC_REQUIRE(losses && out, "NULL buffer");
+  loss_total_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream_)>>>(losses, grad, make_float4(c0, c1, c2, c3), out);
   MOC_CUDA_OK(cudaGetLastError());
   return MOC_OK;
 }

@@ -24,9 +24,51 @@ from . import ops
 LOSS_KEYS = ("load_balance", "auxiliary", "z_loss", "entropy")
 
 
+_KERNEL_DTYPES = (torch.float32, torch.bfloat16)
+
+
+def _cast(v, dtype):
+    return v if v is None or v.dtype == dtype else v.to(dtype)
+
+
 class _LossDict(dict):
-    """Router loss dict (same keys as the reference) that also carries the raw 4-vector as ``.vector``."""
-    vector = None
+    """Router loss dict (same keys as the reference) that also carries the raw 4-vector as ``.vector`` (order of
+    LOSS_KEYS), for a single backward seed and a single-kernel weighted sum.  A dict somebody has changed no longer
+    says what the vector does and drops it."""
+
+    def __init__(self, vector: torch.Tensor):
+        super().__init__(zip(LOSS_KEYS, vector.unbind()))
+        self.vector = vector
+
+    def _changed(name):
+        method = getattr(dict, name)
+
+        def change(self, *args, **kwargs):
+            self.vector = None
+            return method(self, *args, **kwargs)
+        return change
+
+    __setitem__, __delitem__, __ior__ = _changed("__setitem__"), _changed("__delitem__"), _changed("__ior__")
+    update, pop, popitem = _changed("update"), _changed("pop"), _changed("popitem")
+    clear, setdefault = _changed("clear"), _changed("setdefault")
+    del _changed
+
+
+class _WeightedLosses(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, vector, coefs):
+        ctx.coefs = coefs
+        ctx.save_for_backward(vector)
+        return ops.loss_total(vector, coefs)
+
+    @staticmethod
+    def backward(ctx, g):
+        return ops.loss_total(ctx.saved_tensors[0], ctx.coefs, g.float()), None
+
+
+def weighted_losses(losses: _LossDict, **coefs: float) -> torch.Tensor:
+    """sum of coefficient * loss over the coefficients that are positive (router.py:490-527), one kernel each way."""
+    return _WeightedLosses.apply(losses.vector, tuple(max(0.0, float(coefs.get(k, 0.0))) for k in LOSS_KEYS))
 
 
 class SparseBankGrad:
@@ -63,46 +105,77 @@ class SparseBankGrad:
         return dense
 
 
+_side_streams: Dict[tuple, "torch.cuda.Stream"] = {}
+_side_handles: Dict[tuple, int] = {}
+
+
+def _side_stream(dev_index: int, main_handle: int) -> int:
+    """Second stream of the layer, with the priority of the stream it runs beside (a step captured on a
+    high-priority stream keeps both of its streams ahead of background work such as a gradient exchange).
+    ``main_handle`` is the raw handle of the current stream; so is the result."""
+    handle = _side_handles.get((dev_index, main_handle))
+    if handle is None:
+        device = torch.device("cuda", dev_index)
+        key = (dev_index, torch.cuda.current_stream(device).priority)
+        if key not in _side_streams:
+            _side_streams[key] = torch.cuda.Stream(device=device, priority=key[1])
+        handle = _side_handles[(dev_index, main_handle)] = _side_streams[key].cuda_stream
+    return handle
+
+
 # --------------------------------------------------------------------------------------------
 # router
 # --------------------------------------------------------------------------------------------
 class _Route(torch.autograd.Function):
     @staticmethod
     def forward(ctx, h, weight, bias, top_k, num_shared, routed_scale, with_losses, pos_weight):
-        pooled = ops.pool_weighted_fwd(h, pos_weight) if pos_weight is not None else None
-        r = ops.router_fwd(h, weight, bias, top_k, num_shared, routed_scale, with_losses, pooled=pooled)
-        ctx.cfg = (tuple(h.shape), h.dtype, int(top_k), int(num_shared), float(routed_scale), bias is not None)
-        # Output tensors go through save_for_backward (autograd handles a node's own outputs there without a
-        # reference cycle); only tensors that are not outputs stay as attributes, so the node and its buffers
-        # are released by reference counting as soon as the graph is.
-        ctx.internals = {k: r[k] for k in ("pooled", "probs", "idx", "row_stats", "chapter_stats", "_ws")}
-        ctx.pos_weight = pos_weight
-        ctx.save_for_backward(weight, r["weights"], r["comb_w"])
-        ctx.mark_non_differentiable(r["idx"], r["comb_idx"])
-        losses = r["losses"] if with_losses else torch.zeros(4, dtype=torch.float32, device=h.device)
-        return r["idx"], r["weights"], r["comb_idx"], r["comb_w"], losses
+        L.require_cuda(h, weight, bias)
+        if h.dim() != 3:
+            raise ValueError(f"hidden_states must be 3D (B, T, D), got shape {tuple(h.shape)}")
+        dev, f32 = h.device, torch.float32
+        hc, w = ops._contig(h), ops._contig(weight.float())
+        bc = None if bias is None else ops._contig(bias.float())
+        pw = None if pos_weight is None else ops._contig(pos_weight.float())
+        b, l, d = h.shape
+        c = w.shape[0]
+        k = ops.router_selected_k(c, top_k, num_shared)
+        idx = torch.empty(b, k, dtype=torch.int64, device=dev)
+        weights = torch.empty(b, k, dtype=f32, device=dev)
+        comb_idx = torch.empty(b, num_shared + k, dtype=torch.int32, device=dev)
+        comb_w = torch.empty(b, num_shared + k, dtype=f32, device=dev)
+        losses = torch.empty(4, dtype=f32, device=dev) if with_losses else None
+        p = L.ptr
+        s = L.RouteDesc(L.RouterShape(b, l, d, c, top_k, num_shared, routed_scale, L.dtype_code(h.dtype)), p(hc), p(w), p(bc),
+                        p(pw), p(idx), p(weights), p(comb_idx), p(comb_w), p(losses), None, p(L.status_word(dev)),
+                        L.stream_ptr(dev))
+        arena = torch.empty(ops.route_arena_bytes(s), dtype=torch.uint8, device=dev)
+        s.arena = p(arena)
+        ops.route_fwd(s)
+        if any(ctx.needs_input_grad[:3]):
+            ctx.desc = s
+            ctx.meta = (tuple(h.shape), h.dtype, weight.dtype, None if bias is None else bias.dtype)
+            # Output tensors go through save_for_backward (autograd handles a node's own outputs there without a
+            # reference cycle), so the node and its buffers are released by reference counting as soon as the graph is.
+            ctx.save_for_backward(w, arena, idx, weights, comb_w, pw)
+        ctx.mark_non_differentiable(idx, comb_idx)
+        return idx, weights, comb_idx, comb_w, losses if with_losses else torch.zeros(4, dtype=f32, device=dev)
 
     @staticmethod
     def backward(ctx, _g_idx, g_w, _g_cidx, g_cw, g_losses):
-        weight, weights, comb_w = ctx.saved_tensors
-        saved = dict(ctx.internals, weights=weights, comb_w=comb_w)
-        h_shape, h_dtype, top_k, num_shared, routed_scale, has_bias = ctx.cfg
-        if g_w is not None:
-            g_w = g_w.float()
-        if g_cw is not None:
-            g_cw = g_cw.float()
-        if g_losses is not None:
-            g_losses = g_losses.float()
-        want_dh = ctx.needs_input_grad[0]
-        rolling = ctx.pos_weight is not None
-        r = ops.router_bwd(h_shape, h_dtype, weight, saved, top_k, num_shared, routed_scale,
-                           g_w, g_cw, g_losses, want_dh=want_dh and not rolling)
-        d_h = r["d_h"]
-        if rolling and want_dh:
-            d_h = ops.pool_weighted_bwd(r["d_pooled"], ctx.pos_weight, h_shape, h_dtype)
-        d_w = r["d_w"].to(weight.dtype) if ctx.needs_input_grad[1] else None
-        d_b = r["d_bias"] if (has_bias and ctx.needs_input_grad[2]) else None
-        return d_h, d_w, d_b, None, None, None, None, None
+        w, arena, idx, weights, comb_w, pw = ctx.saved_tensors
+        s, p = ctx.desc, L.ptr
+        h_shape, h_dtype, w_dtype, b_dtype = ctx.meta
+        need, dev, f32 = ctx.needs_input_grad, w.device, torch.float32
+        s.w, s.arena, s.idx, s.weights, s.comb_w, s.pos_weight = p(w), p(arena), p(idx), p(weights), p(comb_w), p(pw)
+        s.stream = L.stream_ptr(dev)
+        g_w, g_cw, g_losses = (None if g is None else ops._contig(g.float()) for g in (g_w, g_cw, g_losses))
+        d_h = torch.empty(h_shape, dtype=h_dtype, device=dev) if need[0] else None
+        want_b = b_dtype is not None and need[2]
+        d_w = torch.empty(w.shape, dtype=f32, device=dev) if (need[1] or want_b) else None
+        d_b = torch.empty(w.shape[0], dtype=f32, device=dev) if want_b else None
+        scratch = torch.empty(ops.route_bwd_scratch_bytes(s), dtype=torch.uint8, device=dev)
+        ops.route_bwd(s, g_w, g_cw, g_losses, d_h, d_w, d_b, scratch)
+        return d_h, _cast(d_w, w_dtype) if need[1] else None, d_b, None, None, None, None, None
 
 
 def route(h: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], top_k: int, num_shared: int,
@@ -112,37 +185,17 @@ def route(h: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], t
     sequence-rolling rule, see :func:`ops.rolling_pool_coefficients`)."""
     idx, w, cidx, cw, lv = _Route.apply(h, weight, bias, int(top_k), int(num_shared), float(routed_scale),
                                         bool(with_losses), pos_weight)
-    losses = {k: lv[i] for i, k in enumerate(LOSS_KEYS)} if with_losses else {}
-    if with_losses:
-        losses = _LossDict(losses)
-        losses.vector = lv          # the four losses as one tensor (order of LOSS_KEYS), for a single backward seed
-    return idx, w, cidx, cw, losses
+    return idx, w, cidx, cw, _LossDict(lv) if with_losses else {}
 
 
 # --------------------------------------------------------------------------------------------
 # gather
 # --------------------------------------------------------------------------------------------
-def _bank_backward(sink, d_mem, bank, t, comb_idx, comb_w, norm, eps, stats, num_chapters, want_dw, want_bank):
-    seg = ops.chapter_segments(comb_idx, num_chapters)
-    wire = [] if (sink is not None and sink.wire_dtype == torch.bfloat16) else None
-    d_cw, rows = ops.gather_rows_bwd(d_mem, bank, t, comb_idx, comb_w, norm, eps, stats, seg,
-                                     want_dw=want_dw, want_bank=want_bank, wire_copy=wire)
-    d_bank = None
-    if want_bank:
-        if sink is not None:
-            sink.add(seg["uniq"], seg["num_unique"], rows, t, wire=wire[0] if wire else None)
-        else:
-            d_bank = torch.zeros(bank.shape, dtype=torch.float32, device=bank.device)
-            ops.scatter_bank_grad(rows, seg, t, d_bank)
-            d_bank = d_bank.to(bank.dtype)
-    return d_cw, d_bank
-
-
 class _GatherChapters(torch.autograd.Function):
     @staticmethod
     def forward(ctx, bank, comb_idx, comb_w, tokens_per_chapter, norm_type, eps, out_dtype, sink):
         out, stats = ops.gather_rows_fwd(bank, tokens_per_chapter, comb_idx, comb_w, norm_type, eps, out_dtype)
-        ctx.cfg = (int(tokens_per_chapter), norm_type, float(eps), bank.shape[0] // int(tokens_per_chapter))
+        ctx.cfg = (int(tokens_per_chapter), norm_type, float(eps))
         ctx.sink = sink
         ctx.save_for_backward(bank, comb_idx, comb_w, stats)
         return out
@@ -150,11 +203,15 @@ class _GatherChapters(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         bank, comb_idx, comb_w, stats = ctx.saved_tensors
-        t, norm, eps, num_chapters = ctx.cfg
-        g2 = g.reshape(-1, g.shape[-1])
-        d_cw, d_bank = _bank_backward(ctx.sink, g2, bank, t, comb_idx, comb_w, norm, eps, stats, num_chapters,
-                                      want_dw=comb_w is not None and ctx.needs_input_grad[2],
-                                      want_bank=ctx.needs_input_grad[0])
+        t, norm, eps = ctx.cfg
+        want_dw = comb_w is not None and ctx.needs_input_grad[2]
+        want_bank = ctx.needs_input_grad[0]
+        d_cw, rows, wire, dense, uniq, count = ops.gather_rows_bwd_lists(
+            g, bank, t, comb_idx, comb_w, norm, eps, stats, want_dw, want_bank,
+            dense=ctx.sink is None, wire=ctx.sink is not None and ctx.sink.wire_dtype == torch.bfloat16)
+        if want_bank and ctx.sink is not None:
+            ctx.sink.add(uniq, count, rows, t, wire=wire)
+        d_bank = _cast(dense, bank.dtype)
         return d_bank, None, d_cw, None, None, None, None, None
 
 
@@ -171,119 +228,88 @@ def gather_chapters(bank: torch.Tensor, comb_idx: torch.Tensor, comb_w: Optional
 # cross attention over gathered rows
 # --------------------------------------------------------------------------------------------
 class _CrossAttention(torch.autograd.Function):
+    """One native call per pass (``moc_xattn_fwd`` / ``moc_xattn_bwd``)."""
+
     @staticmethod
     def forward(ctx, h, memory, wq, wk, wv, wo, norm_w, norm_b, num_heads, num_kv_heads, compute_dtype,
                 norm_kind, norm_eps, add_residual):
+        L.require_cuda(h, memory, wq, wk, wv, wo)
         b, l, d = h.shape
         cd = compute_dtype
-        n_sel = memory.shape[-2]
+        dev = h.device
         mem_shared = memory.dim() == 2
-        x2 = h.reshape(b * l, d)
-        stats = None
-        if norm_kind is not None:
-            # the normalisation writes the projection operand in the compute dtype: no separate cast
-            x2 = x2.float()
-            h2, stats = ops.norm_fwd(x2, norm_w.float(), None if norm_b is None else norm_b.float(), norm_kind,
-                                     norm_eps, cd)
-        else:
-            h2 = ops.cast(x2, cd)
-        m2 = ops.cast(memory.reshape(-1, memory.shape[-1]), cd)
-        dkv = wk.shape[0]
-        wt = None
-        if cd == torch.bfloat16 and wq.dtype == wk.dtype == wv.dtype == wo.dtype:
-            # one launch: bf16 working copies of the four weights (Wk and Wv stacked) and, for the backward
-            # pass, their transposes, so every input-gradient projection has K-major operands
-            w_all = torch.empty(2 * d + 2 * dkv, d, dtype=cd, device=h.device)
-            wq_c, wkv_c, wo_c = w_all[:d], w_all[d:d + 2 * dkv], w_all[d + 2 * dkv:]
-            need_t = any(ctx.needs_input_grad[:6])
-            wq_t = torch.empty(d, d, dtype=cd, device=h.device) if need_t else None
-            wkv_t = torch.empty(d, 2 * dkv, dtype=cd, device=h.device) if need_t else None
-            wo_t = torch.empty(d, d, dtype=cd, device=h.device) if need_t else None
-            ops.pack_weights([wq, wk, wv, wo], [wq_c, wkv_c[:dkv], wkv_c[dkv:], wo_c],
-                             [wq_t, wkv_t, wkv_t[:, dkv:] if need_t else None, wo_t], [0, 2 * dkv, 2 * dkv, 0])
-            wt = (wq_t, wkv_t, wo_t)
-        else:
-            wq_c, wo_c = ops.cast(wq, cd), ops.cast(wo, cd)
-            wkv_c = ops.cast(torch.cat([wk, wv], dim=0), cd)
-        q = ops.gemm(h2, wq_c, tag="q_proj")                                   # [B*L, H*D]
-        kv = ops.gemm(m2, wkv_c, tag="kv_proj")                                 # [(B*)n_sel, 2*HK*D]
-        if mem_shared:
-            kv = kv.unsqueeze(0).expand(b, -1, -1).contiguous()
-        head_dim = d // num_heads
-        scale = head_dim ** -0.5
-        kv = kv.view(b, n_sel, -1)
-        o, lse = ops.attn_fwd(q.view(b, l, -1), kv, num_heads, num_kv_heads, scale)
-        # the output projection writes the caller's dtype; the residual connection of the enclosing block
-        # (memory_block.py:558) is added in its epilogue
-        res = (x2 if x2.dtype == torch.float32 else x2.float()) if add_residual else None
-        out = ops.gemm(o.view(b * l, -1), wo_c, out_dtype=h.dtype if h.dtype in (torch.float32, cd) else cd,
-                       residual=res, tag="o_proj")
-        ctx.cfg = (num_heads, num_kv_heads, scale, cd, mem_shared, h.dtype, memory.dtype)
-        ctx.norm = (norm_kind, norm_b is not None, add_residual,
-                    None if norm_w is None else norm_w.dtype, None if norm_b is None else norm_b.dtype)
-        ctx.save_for_backward(h2, m2, wq_c, wkv_c, wo_c, q, kv, o, lse,
-                              x2 if norm_kind is not None else None, stats,
-                              norm_w.float() if norm_kind is not None else None)
-        ctx.wt = wt
-        ctx.w_dtypes = (wq.dtype, wk.dtype, wv.dtype, wo.dtype)
-        return out.view(b, l, -1).to(h.dtype)
+        in_dtype, mem_dtype = h.dtype, memory.dtype
+        # the kernels take fp32 or bf16; anything else goes through the compute dtype
+        hc = ops._contig(h if in_dtype in _KERNEL_DTYPES else h.to(cd))
+        mc = ops._contig(memory if mem_dtype in _KERNEL_DTYPES else memory.to(cd))
+        if mc.dim() == 3 and mc.shape[0] != b:
+            raise ValueError("memory must be (N, d) or (B, N, d) with the batch size of the hidden states")
+        w_dtypes = (wq.dtype, wk.dtype, wv.dtype, wo.dtype)
+        same = len(set(w_dtypes)) == 1 and wq.dtype in _KERNEL_DTYPES
+        ws = [ops._contig(w if same else w.float()) for w in (wq, wk, wv, wo)]
+        nw = None if norm_w is None else ops._contig(norm_w.float())
+        nb = None if norm_b is None else ops._contig(norm_b.float())
+        need_grad = any(ctx.needs_input_grad[:8])
+        out = torch.empty(b, l, d, dtype=in_dtype if in_dtype in (torch.float32, cd) else cd, device=dev)
+        if cd == torch.float32 and out.dtype != cd:
+            out = torch.empty(b, l, d, dtype=cd, device=dev)
+        main = L.stream_ptr(dev)
+        code, p = L.dtype_code, L.ptr
+        s = L.XattnDesc(b, l, mc.shape[-2], d, mc.shape[-1], num_heads, num_kv_heads, int(mem_shared), code(hc.dtype),
+                        code(mc.dtype), code(ws[0].dtype), code(cd), code(out.dtype),
+                        ops.NORM_KINDS[norm_kind] if norm_kind is not None else 0, int(add_residual), int(need_grad),
+                        norm_eps, p(hc), p(mc), p(ws[0]), p(ws[1]), p(ws[2]), p(ws[3]), p(nw), p(nb), p(out), None,
+                        p(L.status_word(dev)), main, _side_stream(L.device_index(dev), main))
+        arena = torch.empty(ops.xattn_arena_bytes(s), dtype=torch.uint8, device=dev)
+        s.arena = p(arena)
+        ops.xattn_fwd(s)
+        if need_grad:
+            ctx.desc = s
+            ctx.dtypes = (in_dtype, mem_dtype, w_dtypes, None if norm_w is None else norm_w.dtype,
+                          None if norm_b is None else norm_b.dtype, wk.shape[0])
+            # inputs the backward pass reads itself: as projection operands, or for the normalisation
+            keep_h = hc if (norm_kind is not None or hc.dtype == cd) else None
+            keep_m = mc if mc.dtype == cd else None
+            keep_w = (ws[0], ws[3]) if (cd == torch.float32 and ws[0].dtype == cd) else (None, None)
+            ctx.save_for_backward(arena, keep_h, keep_m, *keep_w, nw)
+        return _cast(out, in_dtype)
 
     @staticmethod
     def backward(ctx, g):
-        h2, m2, wq_c, wkv_c, wo_c, q, kv, o, lse, x2, stats, norm_w = ctx.saved_tensors
-        num_heads, num_kv_heads, scale, cd, mem_shared, h_dtype, mem_dtype = ctx.cfg
-        norm_kind, norm_has_bias, add_residual, nw_dtype, nb_dtype = ctx.norm
-        b, l, _ = o.shape
-        d = h2.shape[1]
-        g2 = ops.cast(g.reshape(b * l, -1).contiguous(), cd)
-        f32 = torch.float32
-        # K-splits of the weight-gradient projections: enough (tile, split) items to fill the SMs once
-        def splits(rows, out_rows, out_cols):
-            if cd == torch.float32:
-                return 1
-            tiles = -(-out_rows // 128) * -(-out_cols // 256)
-            return max(1, min(148 // max(tiles, 1), rows // 512))
-        split = splits(b * l, d, d)
-        tc = cd == torch.bfloat16
-
-        wt = ctx.wt
-
-        def grad_in(dy, w_c, w_t, tag, out_dtype=None):
-            """dX = dY W.  The tensor-core kernel is fastest with both operands K-major, so it takes the
-            transposed copy of the small weight; the fp32 kernel takes the strided operand directly."""
-            if tc:
-                return ops.gemm(dy, w_t if w_t is not None else ops.transpose(w_c), out_dtype=out_dtype, tag=tag)
-            return ops.gemm(dy, w_c, b_kmajor=False, tag=tag)
-
-        d_o = grad_in(g2, wo_c, wt[2] if wt else None, "d_attn_out")                                      # [B*L, H*D]
-        d_wo = ops.gemm(g2, o.view(b * l, -1), a_kmajor=False, b_kmajor=False, out_dtype=f32, split_k=split,
-                        tag="d_wo")
-        d_q, d_kv = ops.attn_bwd(q.view(b, l, -1), kv, o, lse, d_o.view(b, l, -1), num_heads, num_kv_heads, scale)
-        d_q2 = d_q.view(b * l, -1)
-        # gradient of the (normalised) attention input; fp32 when the normalisation's backward consumes it
-        d_h = grad_in(d_q2, wq_c, wt[0] if wt else None, "d_h", f32 if norm_kind is not None else None)
-        d_nw = d_nb = None
-        g_res = g.reshape(b * l, -1) if add_residual else None
-        if norm_kind is not None:
-            d_h, d_nw, d_nb = ops.norm_bwd(d_h, x2, norm_w, stats, None if g_res is None else g_res.float(),
-                                           norm_kind, norm_has_bias)
-            d_nw = d_nw.to(nw_dtype)
-            d_nb = None if d_nb is None else d_nb.to(nb_dtype)
-        elif add_residual:
-            d_h = d_h.float() + g_res.float()
-        d_wq = ops.gemm(d_q2, h2, a_kmajor=False, b_kmajor=False, out_dtype=f32, split_k=split, tag="d_wq")
-        d_kv2 = d_kv.view(-1, d_kv.shape[-1])
-        if mem_shared:
-            d_kv2 = d_kv.float().sum(dim=0).to(cd)
-        rows = d_kv2.shape[0]
-        split_kv = splits(rows, wkv_c.shape[0], d)
-        d_mem = grad_in(d_kv2, wkv_c, wt[1] if wt else None, "d_mem")
-        d_wkv = ops.gemm(d_kv2, m2, a_kmajor=False, b_kmajor=False, out_dtype=f32, split_k=split_kv, tag="d_wkv")
-        dkv_dim = wkv_c.shape[0] // 2
-        wdt = ctx.w_dtypes
-        d_mem = d_mem.view(-1, d_mem.shape[-1]) if mem_shared else d_mem.view(b, -1, d_mem.shape[-1])
-        return (d_h.view(b, l, d).to(h_dtype), d_mem.to(mem_dtype), d_wq.to(wdt[0]), d_wkv[:dkv_dim].to(wdt[1]),
-                d_wkv[dkv_dim:].to(wdt[2]), d_wo.to(wdt[3]), d_nw, d_nb, None, None, None, None, None, None)
+        arena, hc, mc, wq, wo, nw = ctx.saved_tensors
+        s = ctx.desc
+        in_dtype, mem_dtype, wdt, nw_dtype, nb_dtype, dkv = ctx.dtypes
+        dev, f32, p = arena.device, torch.float32, L.ptr
+        need = ctx.needs_input_grad
+        cd = f32 if s.compute_dtype == L.MOC_F32 else torch.bfloat16
+        s.arena, s.h, s.memory, s.wq, s.wo, s.norm_w = p(arena), p(hc), p(mc), p(wq), p(wo), p(nw)
+        s.stream = L.stream_ptr(dev)
+        s.side_stream = _side_stream(L.device_index(dev), s.stream)
+        g = ops._contig(g if g.dtype in _KERNEL_DTYPES else g.to(cd))
+        b, l, d, md = s.batch, s.seq, s.hidden_dim, s.mem_dim
+        dh_dtype = in_dtype if in_dtype in (f32, cd) else cd
+        dm_dtype = mem_dtype if mem_dtype in (f32, cd) else cd
+        if nw is not None and cd == torch.bfloat16 and in_dtype not in _KERNEL_DTYPES:
+            dh_dtype = f32
+        d_h = torch.empty(b, l, d, dtype=dh_dtype if cd != f32 else f32, device=dev) if (need[0] or nw is not None) else None
+        d_mem = None
+        if need[1]:
+            shape = (s.n_sel, md) if s.mem_shared else (b, s.n_sel, md)
+            d_mem = torch.empty(shape, dtype=dm_dtype if cd != f32 else f32, device=dev)
+        d_wq = torch.empty(d, d, dtype=f32, device=dev)
+        d_wkv = torch.empty(2 * dkv, md, dtype=f32, device=dev)
+        d_wo = torch.empty(d, d, dtype=f32, device=dev)
+        d_nw = torch.empty(d, dtype=f32, device=dev) if nw is not None else None
+        d_nb = torch.empty(d, dtype=f32, device=dev) if nb_dtype is not None else None
+        q = L.XattnBwdDesc(p(g), L.dtype_code(g.dtype), L.dtype_code(d_h.dtype) if d_h is not None else 0,
+                           L.dtype_code(d_mem.dtype) if d_mem is not None else 0, p(d_h), p(d_mem), p(d_wq), p(d_wkv),
+                           p(d_wo), p(d_nw), p(d_nb), None)
+        scratch = torch.empty(ops.xattn_bwd_scratch_bytes(s, q), dtype=torch.uint8, device=dev)
+        q.scratch = p(scratch)
+        ops.xattn_bwd(s, q)
+        return (_cast(d_h, in_dtype) if need[0] else None, _cast(d_mem, mem_dtype), _cast(d_wq, wdt[0]),
+                _cast(d_wkv[:dkv], wdt[1]), _cast(d_wkv[dkv:], wdt[2]), _cast(d_wo, wdt[3]), _cast(d_nw, nw_dtype),
+                _cast(d_nb, nb_dtype), None, None, None, None, None, None)
 
 
 def cross_attention(h: torch.Tensor, memory: torch.Tensor, wq, wk, wv, wo, num_heads: int,
@@ -313,24 +339,6 @@ def cross_attention(h: torch.Tensor, memory: torch.Tensor, wq, wk, wv, wo, num_h
 # --------------------------------------------------------------------------------------------
 # the whole layer as one node with two streams (bf16 path)
 # --------------------------------------------------------------------------------------------
-_side_streams: Dict[tuple, "torch.cuda.Stream"] = {}
-_side_handles: Dict[tuple, int] = {}
-
-
-def _side_stream(dev_index: int, main_handle: int) -> int:
-    """Second stream of the layer, with the priority of the stream it runs beside (a step captured on a
-    high-priority stream keeps both of its streams ahead of background work such as a gradient exchange).
-    ``main_handle`` is the raw handle of the current stream; so is the result."""
-    handle = _side_handles.get((dev_index, main_handle))
-    if handle is None:
-        device = torch.device("cuda", dev_index)
-        key = (dev_index, torch.cuda.current_stream(device).priority)
-        if key not in _side_streams:
-            _side_streams[key] = torch.cuda.Stream(device=device, priority=key[1])
-        handle = _side_handles[(dev_index, main_handle)] = _side_streams[key].cuda_stream
-    return handle
-
-
 # The dQ kernel runs on the side stream beside the dK/dV kernel (fused route): 768 CTAs over 296 slots leave the last
 # of dQ's three rounds 59 % full, and the other kernel's CTAs take the free slots (measured 1.189 -> 1.177 ms per
 # step).  MOC_DQ_ON_SIDE_STREAM=0 puts both back on the main stream.
@@ -478,14 +486,12 @@ class _MemoryLayerTwoStream(torch.autograd.Function):
         if rows is not None or wire is not None:
             sink.add(touched[:n_pairs], touched[n_pairs:], wire if rows is None else rows, t, wire=wire)
 
-        def cast(v, dtype):
-            return v if v is None or v.dtype == dtype else v.to(dtype)
-        d_ha = cast(d_ha, in_dtype)
+        d_ha = _cast(d_ha, in_dtype)
         if fuse_dh:
             d_hr, d_ha = d_ha, None
-        return (d_hr, d_ha, cast(dense, bank.dtype), cast(d_rw, rw.dtype) if need[3] else None, d_rb, cast(d_wq, wdt[0]),
-                cast(d_wkv[:dkv], wdt[1]), cast(d_wkv[dkv:], wdt[2]), cast(d_wo, wdt[3]),
-                cast(d_nw, nw_dtype), cast(d_nb, nb_dtype), None, None, None)
+        return (d_hr, d_ha, _cast(dense, bank.dtype), _cast(d_rw, rw.dtype) if need[3] else None, d_rb, _cast(d_wq, wdt[0]),
+                _cast(d_wkv[:dkv], wdt[1]), _cast(d_wkv[dkv:], wdt[2]), _cast(d_wo, wdt[3]),
+                _cast(d_nw, nw_dtype), _cast(d_nb, nb_dtype), None, None, None)
 
 
 # --------------------------------------------------------------------------------------------
@@ -534,10 +540,7 @@ def memory_layer(h_router: torch.Tensor, h_attn: torch.Tensor, bank: torch.Tenso
             getattr(bank, "moc_sparse_grad", None),
             None if bank_shadow is None else {"shadow": bank_shadow, "inv_rms": bank_inv_rms,
                                               "wkv_grad_in_place": wkv_grad_in_place})
-        losses = {}
-        if with_losses:
-            losses = _LossDict(zip(LOSS_KEYS, lv.unbind()))
-            losses.vector = lv
+        losses = _LossDict(lv) if with_losses else {}
         return out, losses, {"indices": idx, "weights": w, "combined_indices": cidx, "combined_weights": cw}
     idx, w, cidx, cw, losses = route(h_router, router_weight, router_bias, top_k, num_shared_chapters,
                                      routed_scaling_factor, with_losses)
@@ -644,11 +647,7 @@ def route_tokens(h: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Ten
                  with_losses: bool = True):
     """Returns (global chapter ids int64 [B,L,k'], weights [B,L,k'], losses dict); k' = min(k, C - num_shared)."""
     idx, w, lv = _RouteTokens.apply(h, weight, bias, int(top_k), int(num_shared), bool(with_losses))
-    losses = {}
-    if with_losses:
-        losses = _LossDict({k: lv[i] for i, k in enumerate(LOSS_KEYS)})
-        losses.vector = lv
-    return idx, w, losses
+    return idx, w, _LossDict(lv) if with_losses else {}
 
 
 class _TokenRoutedAttention(torch.autograd.Function):

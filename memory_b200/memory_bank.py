@@ -58,11 +58,8 @@ class ChapteredMemoryBank(nn.Module):
         """(rows [B, K*T, d], flat row ids [B, K*T]) of the selected chapters; the gradient of the
         rows is scattered only into the touched chapters."""
         memory = self.get_memory()
-        rows = F_moc.gather_chapters(memory, chapter_indices, None, self.tokens_per_chapter)
-        t = self.tokens_per_chapter
-        flat = (chapter_indices.long().unsqueeze(-1) * t
-                + torch.arange(t, device=chapter_indices.device).view(1, 1, -1)).view(chapter_indices.shape[0], -1)
-        return rows, flat
+        idx32, flat = ops.chapter_lists(chapter_indices, self.tokens_per_chapter)
+        return F_moc.gather_chapters(memory, idx32, None, self.tokens_per_chapter), flat
 
     def bf16_shadow(self) -> torch.Tensor:
         """bf16 copy of the bank for the TMA-gather projection; refreshed when the parameter changed."""

@@ -274,6 +274,30 @@ def gather_rows_fwd(bank: torch.Tensor, tokens_per_chapter: int, comb_idx: torch
     return out, stats
 
 
+@_instrument("chapter_lists", 1)
+def chapter_lists(chapter_idx: torch.Tensor, tokens_per_chapter: int):
+    """(int32 copy of an int64 / int32 [B, K] list, flat row ids [B, K*T] int64 of the listed chapters) in one launch."""
+    L.require_cuda(chapter_idx)
+    idx = _contig(chapter_idx if chapter_idx.dtype in (torch.int64, torch.int32) else chapter_idx.long())
+    b, k = idx.shape
+    t = int(tokens_per_chapter)
+    idx32 = torch.empty(b, k, dtype=torch.int32, device=idx.device)
+    flat = torch.empty(b, k * t, dtype=torch.int64, device=idx.device)
+    if flat.numel():
+        L.check(L.lib().moc_chapter_lists(L.ptr(idx), int(idx.dtype == torch.int64), b * k, t, L.ptr(idx32), L.ptr(flat),
+                                          L.stream_ptr(idx.device)), "moc_chapter_lists")
+    return idx32, flat
+
+
+@_instrument("loss_total", 1)
+def loss_total(losses: torch.Tensor, coefs, grad: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """sum_i coefs[i] * losses[i] of four fp32 losses (0-d); with ``grad`` (0-d) its gradient grad * coefs [4]."""
+    out = torch.empty((4,) if grad is not None else (), dtype=torch.float32, device=losses.device)
+    L.check(L.lib().moc_loss_total(L.ptr(losses), L.ptr(grad), *[float(c) for c in coefs], L.ptr(out),
+                                   L.stream_ptr(losses.device)), "moc_loss_total")
+    return out
+
+
 @_instrument("chapter_segments", 1)
 def chapter_segments(comb_idx: torch.Tensor, num_chapters: int) -> Dict[str, torch.Tensor]:
     comb_idx = _contig(comb_idx.to(torch.int32))
@@ -320,6 +344,32 @@ def gather_rows_bwd(d_mem: torch.Tensor, bank: torch.Tensor, tokens_per_chapter:
                                      L.stream_ptr(dev))
     L.check(rc, "moc_gather_rows_bwd")
     return d_comb_w, bank_grad
+
+
+@_instrument("gather_rows_bwd", lambda *a, **k: 2 + int(bool(a[8])))
+def gather_rows_bwd_lists(d_mem, bank, tokens_per_chapter, comb_idx, comb_w, norm_type, eps, row_stats, want_dw, want_bank,
+                          dense: bool, wire: bool):
+    """Chapter-weight and bank gradients from the chapter lists alone (they are grouped here).  The bank's leaves dense
+    (bank-shaped, zero outside the touched chapters) or as compact rows, with a bf16 copy when ``wire``; returns
+    (d_comb_w, rows, wire rows, dense, touched chapters, their count), None where not wanted."""
+    d_mem, bank, comb_idx = _contig(d_mem), _contig(bank), _contig(comb_idx)
+    b, k = comb_idx.shape
+    n_rows, d = bank.shape
+    t, dev, n = int(tokens_per_chapter), bank.device, b * k
+    seg = torch.empty(4 * n + 2, dtype=torch.int32, device=dev)
+    d_cw = torch.empty(b, k, dtype=torch.float32, device=dev) if want_dw else None
+    rows = wire_rows = full = None
+    if want_bank and dense:
+        full = torch.empty(n_rows, d, dtype=torch.float32, device=dev)
+    elif want_bank:
+        rows = torch.empty(n * t, d, dtype=torch.float32, device=dev)
+        wire_rows = torch.empty(n * t, d, dtype=torch.bfloat16, device=dev) if wire else None
+    rc = L.lib().moc_gather_rows_bwd_lists(
+        L.ptr(d_mem), L.dtype_code(d_mem.dtype), L.ptr(bank), L.dtype_code(bank.dtype), n_rows, d, t, L.ptr(comb_idx),
+        L.ptr(_contig(comb_w)), b, k, L.NORM_CODES[norm_type], float(eps), L.ptr(row_stats), L.ptr(seg), L.ptr(d_cw),
+        L.ptr(rows), L.ptr(wire_rows), L.ptr(full), L.ptr(L.status_word(dev)), L.stream_ptr(dev))
+    L.check(rc, "moc_gather_rows_bwd_lists")
+    return d_cw, rows, wire_rows, full, seg[:n], seg[n:n + 1]
 
 
 @_instrument("row_inv_rms", 1)
@@ -467,19 +517,21 @@ def scatter_bank_grad(bank_grad: torch.Tensor, seg: Dict[str, torch.Tensor], tok
 # --------------------------------------------------------------------------------------------
 # a whole layer per call
 # --------------------------------------------------------------------------------------------
-def layer_arena_bytes(s) -> int:
-    n = L.lib().moc_layer_arena_bytes(C.byref(s))
-    L.check(-1 if n < 0 else 0, "moc_layer_arena_bytes")
+def _size(fn: str, *descs) -> int:
+    n = getattr(L.lib(), fn)(*[C.byref(d) for d in descs])
+    L.check(-1 if n < 0 else 0, fn)
     return n
+
+
+def layer_arena_bytes(s) -> int:
+    return _size("moc_layer_arena_bytes", s)
 
 
 def layer_bwd_scratch_bytes(s, b) -> int:
-    n = L.lib().moc_layer_bwd_scratch_bytes(C.byref(s), C.byref(b))
-    L.check(-1 if n < 0 else 0, "moc_layer_bwd_scratch_bytes")
-    return n
+    return _size("moc_layer_bwd_scratch_bytes", s, b)
 
 
-def _report(label: str, launches: int, parts) -> None:
+def _report(launches: int, parts) -> None:
     """Accounting of a call that issues several operators' kernels: the count, and one hook call per operator."""
     global LAUNCHES
     LAUNCHES += launches
@@ -516,7 +568,7 @@ def layer_fwd(s) -> None:
         yield "chapter_row_scale:i32" if s.fused else "gather_rows_fwd:" + _TAG_OF_CODE[s.bank_dtype]
         yield "attn_fwd:bf16"
     casts = int(norm or f32_in) + int((norm or s.add_residual) and not f32_in)
-    _report("layer_fwd", 10 + 2 * s.with_losses + s.for_backward + casts, parts)
+    _report(10 + 2 * s.with_losses + s.for_backward + casts, parts)
 
 
 def layer_bwd(s, b) -> None:
@@ -538,7 +590,65 @@ def layer_bwd(s, b) -> None:
         yield "router_bwd:f32"
     n = 6 + 3 + int(f32_in) + 2 * int(norm) + int(copies_rows) + int(want_bank) + int(bool(b.bank_dense)) + 1
     n += 1 + b.want_router_w + 3 * b.want_dh_router
-    _report("layer_bwd", n, parts)
+    _report(n, parts)
+
+
+def route_arena_bytes(s) -> int:
+    return _size("moc_route_arena_bytes", s)
+
+
+def route_bwd_scratch_bytes(s) -> int:
+    return _size("moc_route_bwd_scratch_bytes", s)
+
+
+def route_fwd(s) -> None:
+    """``moc_route_fwd`` on a filled ``_lib.RouteDesc``."""
+    L.check(_timed("router_fwd", lambda: L.lib().moc_route_fwd(C.byref(s))), "moc_route_fwd")
+    _report(4 + 2 * int(bool(s.losses)), lambda: ("router_fwd:" + _TAG_OF_CODE[s.shape.h_dtype],))
+
+
+def route_bwd(s, g_w, g_cw, g_losses, d_h, d_w, d_bias, scratch) -> None:
+    """``moc_route_bwd`` on the forward call's descriptor."""
+    rc = _timed("router_bwd", lambda: L.lib().moc_route_bwd(C.byref(s), L.ptr(g_w), L.ptr(g_cw), L.ptr(g_losses), L.ptr(d_h),
+                                                            L.ptr(d_w), L.ptr(d_bias), L.ptr(scratch)))
+    L.check(rc, "moc_route_bwd")
+    _report(1 + int(d_w is not None) + 3 * int(d_h is not None), lambda: ("router_bwd:f32",))
+
+
+def xattn_arena_bytes(s) -> int:
+    return _size("moc_xattn_arena_bytes", s)
+
+
+def xattn_bwd_scratch_bytes(s, b) -> int:
+    return _size("moc_xattn_bwd_scratch_bytes", s, b)
+
+
+def xattn_fwd(s) -> None:
+    """``moc_xattn_fwd`` on a filled ``_lib.XattnDesc``."""
+    L.check(_timed("xattn_fwd", lambda: L.lib().moc_xattn_fwd(C.byref(s))), "moc_xattn_fwd")
+    tag = _TAG_OF_CODE[s.compute_dtype]
+
+    def parts():
+        yield from ("gemm:" + tag,) * 3
+        yield "attn_fwd:" + tag
+        if s.pre_norm:
+            yield "norm_fwd:f32"
+    casts = sum(dt != s.compute_dtype for dt in (s.h_dtype, s.mem_dtype))
+    _report(4 + casts + int(s.compute_dtype == L.MOC_BF16) + s.mem_shared, parts)
+
+
+def xattn_bwd(s, b) -> None:
+    """``moc_xattn_bwd`` on the forward call's descriptor and a filled ``_lib.XattnBwdDesc``."""
+    L.check(_timed("xattn_bwd", lambda: L.lib().moc_xattn_bwd(C.byref(s), C.byref(b))), "moc_xattn_bwd")
+    tag = _TAG_OF_CODE[s.compute_dtype]
+
+    def parts():
+        yield from ("gemm:" + tag,) * 6
+        yield "attn_bwd:" + tag
+        if s.pre_norm:
+            yield "norm_bwd:f32"
+    n = 6 + (3 if s.compute_dtype == L.MOC_BF16 else 4) + int(b.g_dtype != s.compute_dtype)
+    _report(n + 2 * int(bool(s.pre_norm)) + s.mem_shared, parts)
 
 
 # --------------------------------------------------------------------------------------------

@@ -94,6 +94,8 @@ def compute_total_router_loss(losses: Dict[str, torch.Tensor], load_balance_coef
     """Weighted sum of the router losses (router.py:490-527); empty dicts give a zero scalar."""
     if not losses:
         return reference_tensor.new_tensor(0.0) if reference_tensor is not None else torch.tensor(0.0)
+    if getattr(losses, "vector", None) is not None:
+        return F_moc.weighted_losses(losses, load_balance=load_balance_coef, auxiliary=auxiliary_coef, z_loss=z_loss_coef)
     total = next(iter(losses.values())).new_tensor(0.0)
     for key, coef in (("load_balance", load_balance_coef), ("auxiliary", auxiliary_coef), ("z_loss", z_loss_coef)):
         if key in losses and coef > 0:
