@@ -283,8 +283,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       const int kt_begin = split * p.k_tiles_per_split;
       const bool has_k = kt_begin < p.k_tiles_total;
       const uint32_t buf = (MT == 1) ? (t & 1) : 0;
-      bool have_acc = mbar_wait(&acc_full[buf], MT == 1 ? ((t >> 1) & 1) : (t & 1), &abort_flag, p.status);
-      have_acc = __all_sync(0xffffffffu, have_acc);   // tcgen05.ld below is warp-collective
+      bool have_acc = mbar_wait_w(&acc_full[buf], MT == 1 ? ((t >> 1) & 1) : (t & 1), &abort_flag, p.status);
       if (!have_acc) break;
       tc_fence_after();
       const uint32_t tmem_acc = tmem_base + (MT == 1 ? buf : static_cast<uint32_t>(sub)) * 256;

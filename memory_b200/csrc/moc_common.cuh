@@ -94,8 +94,12 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 #ifndef MOC_KERNEL_TAG
 #define MOC_KERNEL_TAG 0
 #endif
-__device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                                  int* status, uint32_t limit, int where = 0) {
+//
+// The first try stands outside the loop and looks at nothing but the barrier: a wait whose phase is complete -- most of
+// them, in a pipeline that keeps up -- costs about 100 cycles with its warp vote instead of 175 (290 beside busy warps),
+// and every tile of every kernel here passes two to six waits.
+static __device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
+                                            uint32_t limit, int where) {
   if (*abort_flag) return false;
   for (uint32_t it = 0; it < limit; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
@@ -104,6 +108,18 @@ __device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity
   *abort_flag = 1;
   atomicMax(status, MOC_DEV_TIMEOUT | (MOC_KERNEL_TAG << 8) | (where << 12));
   return false;
+}
+__device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                                  int* status, uint32_t limit, int where = 0) {
+  if (mbar_try_wait(bar, parity)) return true;
+  return mbar_wait_slow(bar, parity, abort_flag, status, limit, where);
+}
+// for a whole converged warp, with a warp-uniform result
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
+                                               int where) {
+  const bool ok = mbar_try_wait(bar, parity);
+  if (__all_sync(0xffffffffu, ok)) return true;
+  return __all_sync(0xffffffffu, ok || mbar_wait_slow(bar, parity, abort_flag, status, kWaitPollLimit, where));
 }
 #define mbar_wait(bar, parity, abort_flag, status) \
   mbar_wait_limited(bar, parity, abort_flag, status, kWaitPollLimit, __LINE__)
@@ -291,8 +307,63 @@ __device__ __forceinline__ void tc_commit_w(uint64_t* bar) {
       : "memory");
 }
 // mbar_wait for a whole warp with a warp-uniform result
-#define mbar_wait_w(bar, parity, abort_flag, status) \
-  __all_sync(0xffffffffu, mbar_wait_limited(bar, parity, abort_flag, status, kWaitPollLimit, __LINE__))
+#define mbar_wait_w(bar, parity, abort_flag, status) mbar_wait_warp(bar, parity, abort_flag, status, __LINE__)
+
+// ----- two fp32 operations per instruction (a register pair holds {lo, hi}) -----
+__device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void f2_unpack(uint64_t v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+// ----- thread-block clusters -----
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {       // every thread of every CTA of the cluster
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// address of this CTA's shared-memory location `p` in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t cluster_map(uint32_t p, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(p), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float4 cluster_ld4(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ float2 cluster_ld2(uint32_t a) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+  return v;
+}
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);   // .x = lo (low 16 bits), .y = hi
@@ -308,6 +379,36 @@ __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
+}
+
+// Runs the key tiles of a query tile are cut into (the CTAs of a cluster), for `ctas` query tiles and a chip with room for
+// `slots` CTAs: the count (at most eight, at least four key tiles per run) with the least rounds * (tiles per run + 3), where
+// 3 stands for a CTA's start-up and its share of the merge.
+inline int attn_key_split(int ctas, int key_tiles, int slots) {
+  int best = 1;
+  double best_cost = 0.0;
+  for (int n = 1; n <= 8 && (n == 1 || key_tiles / n >= 4); ++n) {
+    const long long rounds = (static_cast<long long>(ctas) * n + slots - 1) / slots;
+    const double cost = static_cast<double>(rounds) * ((key_tiles + n - 1) / n + 3);
+    if (n == 1 || cost < 0.97 * best_cost) { best = n; best_cost = cost; }
+  }
+  return best;
+}
+// Launch on clusters of `cluster` CTAs along x (1: a plain launch).
+template <typename... Params, typename... Args>
+inline cudaError_t launch_clustered(void (*kernel)(Params...), dim3 grid, int threads, int smem, int cluster,
+                                    cudaStream_t stream, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = cluster; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = cluster > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 #endif  // __CUDACC__
 

@@ -297,8 +297,7 @@ token_mix_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
         gather_row(q_s, r, p.q + tokrow * (x.HQ * kD) + hq * kD, valid);
         fence_proxy_async();
         mbar_arrive(&q_ready);
-        ok = mbar_wait(&s_bar, it & 1, &abort_flag, p.status);
-        ok = __all_sync(0xffffffffu, ok);
+        ok = mbar_wait_w(&s_bar, it & 1, &abort_flag, p.status);
         if (!ok) break;
         tc_fence_after();
         float m, l = 0.f;
@@ -326,8 +325,7 @@ token_mix_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
         }
         tc_fence_before();
         mbar_arrive(&p_bar);
-        ok = mbar_wait(&o_bar, it & 1, &abort_flag, p.status);
-        ok = __all_sync(0xffffffffu, ok);
+        ok = mbar_wait_w(&o_bar, it & 1, &abort_flag, p.status);
         if (!ok) break;
         tc_fence_after();
         const float f = x.out_scale * wv / l;
@@ -615,8 +613,7 @@ token_mix_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
         if (last) { ngi.next(p, r); nu = 0; }
         if (!ngi.done(p)) next_m = fetch_meta(ngi, nu);
         if (pending) flush_d();
-        ok = mbar_wait(&sdp_bar, it & 1, &abort_flag, p.status);
-        ok = __all_sync(0xffffffffu, ok);
+        ok = mbar_wait_w(&sdp_bar, it & 1, &abort_flag, p.status);
         if (!ok) break;
         tc_fence_after();
         float pr[64];
@@ -660,8 +657,7 @@ token_mix_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
         tc_fence_before();
         fence_proxy_async();
         mbar_arrive(&ds_ready);
-        ok = mbar_wait(&done_bar, it & 1, &abort_flag, p.status);
-        ok = __all_sync(0xffffffffu, ok);
+        ok = mbar_wait_w(&done_bar, it & 1, &abort_flag, p.status);
         if (!ok) break;
         tc_fence_after();
         __nv_bfloat16* dst = p.dq_partial + ((tokrow * x.S + s) * x.HQ + hq) * kD;
