@@ -27,7 +27,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 
 __device__ __forceinline__ float ex2(float x) {
   float y;
-  asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 
@@ -194,11 +194,13 @@ struct DqParams {
   __nv_bfloat16* d_q;
   const float* delta;
   const float* nlse2;
-  int L, n_sel, H, HK;
+  int L, n_sel, H, HK, split;
   float scale, scale_log2;
   int* status;
 };
 
+// A cluster of p.split CTAs shares one query tile when there are few of them (see attn_key_split): each takes a run of
+// the key tiles, their dQ parts are added through distributed shared memory.
 __global__ void __launch_bounds__(kThreads, 2)
 attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_do,
                       const __grid_constant__ CUtensorMap tmap_kv, DqParams p) {
@@ -211,9 +213,11 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   uint8_t* q_s = base;
   uint8_t* do_s = base + kQBytes;
   uint8_t* kv_s = base + 2 * kQBytes;
-  const int q0 = blockIdx.x * kQ, h = blockIdx.y, b = blockIdx.z;
+  const int rank = p.split > 1 ? static_cast<int>(cluster_rank()) : 0;
+  const int q0 = blockIdx.x / p.split * kQ, h = blockIdx.y, b = blockIdx.z;
   const int kh = h / (p.H / p.HK);
-  const int n_tiles = (p.n_sel + kKeys - 1) / kKeys;
+  const int all_tiles = (p.n_sel + kKeys - 1) / kKeys;
+  const int tile0 = rank * all_tiles / p.split, n_tiles = (rank + 1) * all_tiles / p.split - tile0;
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
@@ -241,7 +245,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         if (!mbar_wait(&kv_empty[s], ((j / kStages) & 1) ^ 1, &abort_flag, p.status)) break;
         mbar_arrive_expect_tx(&kv_full[s], 2 * kKvBytes);
         uint8_t* k_s = kv_s + s * 2 * kKvBytes;
-        const int row = b * p.n_sel + j * kKeys;
+        const int row = b * p.n_sel + (tile0 + j) * kKeys;
         tma_load_2d(k_s, &tmap_kv, &kv_full[s], kh * kD, row);
         tma_load_2d(k_s + kKvBytes, &tmap_kv, &kv_full[s], p.HK * kD + kh * kD, row);
       }
@@ -291,11 +295,10 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     const float nl = p.nlse2[sidx], dl = p.delta[sidx];
     bool ok = true;
     for (int j = 0; j < n_tiles; ++j) {
-      ok = mbar_wait(&sdp_full, j & 1, &abort_flag, p.status);
-      ok = __all_sync(0xffffffffu, ok);
+      ok = mbar_wait_w(&sdp_full, j & 1, &abort_flag, p.status);
       if (!ok) break;
       tc_fence_after();
-      const int valid = p.n_sel - j * kKeys - half * 32;   // columns of this half that are real keys
+      const int valid = p.n_sel - (tile0 + j) * kKeys - half * 32;   // columns of this half that are real keys
       uint32_t pk[16];
       {
         uint32_t rs[32], rd[32];
@@ -304,11 +307,15 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         tmem_wait_ld();
         tc_fence_before();
         mbar_arrive(&sdp_free);          // S / dP may be overwritten by the next tile's MMAs
-        // dS without the softmax scale: it is applied once when dQ is written
+        // dS without the softmax scale: it is applied once when dQ is written.  Two columns per instruction around
+        // the exponentials.
+        const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2), nl2 = f2_pack(nl, nl), nd2 = f2_pack(-dl, -dl);
 #pragma unroll
         for (int c = 0; c < 32; c += 2) {
-          const float d0 = ex2(fmaf(__uint_as_float(rs[c]), p.scale_log2, nl)) * (__uint_as_float(rd[c]) - dl);
-          const float d1 = ex2(fmaf(__uint_as_float(rs[c + 1]), p.scale_log2, nl)) * (__uint_as_float(rd[c + 1]) - dl);
+          float e0, e1, d0, d1;
+          f2_unpack(f2_fma(f2_pack(__uint_as_float(rs[c]), __uint_as_float(rs[c + 1])), sc2, nl2), e0, e1);
+          f2_unpack(f2_mul(f2_pack(ex2(e0), ex2(e1)),
+                           f2_add(f2_pack(__uint_as_float(rd[c]), __uint_as_float(rd[c + 1])), nd2)), d0, d1);
           pk[c / 2] = pack_bf16x2(d0, d1);
         }
         if (valid < 32) {
@@ -320,8 +327,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         }
       }
       if (j > 0) {
-        ok = mbar_wait(&dq_bar, (j - 1) & 1, &abort_flag, p.status);   // previous dS consumed
-        ok = __all_sync(0xffffffffu, ok);
+        ok = mbar_wait_w(&dq_bar, (j - 1) & 1, &abort_flag, p.status);   // previous dS consumed
         if (!ok) break;
         tc_fence_after();
       }
@@ -331,8 +337,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       mbar_arrive(&ds_full);
     }
     if (ok) {
-      ok = mbar_wait(&dq_bar, (n_tiles - 1) & 1, &abort_flag, p.status);
-      ok = __all_sync(0xffffffffu, ok);
+      ok = mbar_wait_w(&dq_bar, (n_tiles - 1) & 1, &abort_flag, p.status);
     }
     if (ok) {
       tc_fence_after();
@@ -340,7 +345,15 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       uint32_t r[32];
       tmem_ld32(tmem + lane_sel + kDqColDQ + half * 32, r);
       tmem_wait_ld();
-      if (l < p.L) {
+      if (p.split > 1) {
+        // fp32 rows over the Q and dO tiles, which no product reads any more; chunks rotated against bank conflicts
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const uint32_t addr = smem_u32(q_s) + row * 256 + (((half * 8 + c) ^ (row & 15)) << 4);
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r[4 * c]), "r"(r[4 * c + 1]),
+                       "r"(r[4 * c + 2]), "r"(r[4 * c + 3]) : "memory");
+        }
+      } else if (l < p.L) {
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           uint4 v;
@@ -356,6 +369,24 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   }
   __syncthreads();
   if (abort_flag) { for (int i = 0; i < 200; ++i) __nanosleep(1000); }
+  if (p.split > 1) {
+    cluster_sync();
+    if (!abort_flag) {
+      const int row_lo = rank * kQ / p.split, row_hi = (rank + 1) * kQ / p.split;
+      const int c = threadIdx.x & 15;
+      for (int row = row_lo + static_cast<int>(threadIdx.x >> 4); row < row_hi && q0 + row < p.L; row += kThreads / 16) {
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i = 0; i < p.split; ++i) {
+          const float4 v = cluster_ld4(cluster_map(smem_u32(q_s) + row * 256 + ((c ^ (row & 15)) << 4), i));
+          acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+        }
+        __nv_bfloat16* dst = p.d_q + (static_cast<long long>(b) * p.L + q0 + row) * (p.H * kD) + h * kD;
+        reinterpret_cast<uint2*>(dst)[c] = make_uint2(pack_bf16x2(acc.x * p.scale, acc.y * p.scale),
+                                                      pack_bf16x2(acc.z * p.scale, acc.w * p.scale));
+      }
+    }
+    cluster_sync();                            // no CTA leaves while another still reads its rows
+  }
   if (warp == 9) { tc_fence_after(); tmem_dealloc(tmem, 256); }
 }
 
@@ -541,10 +572,10 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     // this thread's 64 bytes of P^T row `row`: 16-byte chunks 4*half .. 4*half+3 under the 128-byte swizzle
     const uint32_t pt_row = smem_u32(pt_s) + row * 128;
     const uint32_t sw = static_cast<uint32_t>(row & 7);
+    const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2);
     bool ok = true;
     for (int it = 0; it < n_iter; ++it) {
-      ok = mbar_wait(&s_full, it & 1, &abort_flag, p.status);
-      ok = __all_sync(0xffffffffu, ok);
+      ok = mbar_wait_w(&s_full, it & 1, &abort_flag, p.status);
       if (!ok) break;
       tc_fence_after();
       float pf[32];
@@ -556,11 +587,14 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         mbar_arrive(&s_free);          // S^T_j is in registers: its columns may take S^T_{j+1}
         // the tensor core already added -lse / scale to every column
 #pragma unroll
-        for (int c = 0; c < 32; ++c) pf[c] = ex2(__uint_as_float(rs[c]) * p.scale_log2);
+        for (int c = 0; c < 32; c += 2) {
+          float e0, e1;
+          f2_unpack(f2_mul(f2_pack(__uint_as_float(rs[c]), __uint_as_float(rs[c + 1])), sc2), e0, e1);
+          pf[c] = ex2(e0); pf[c + 1] = ex2(e1);
+        }
       }
       if (it > 0) {
-        ok = mbar_wait(&p_free, (it - 1) & 1, &abort_flag, p.status);   // dV_{j-1} has read the P^T tile
-        ok = __all_sync(0xffffffffu, ok);
+        ok = mbar_wait_w(&p_free, (it - 1) & 1, &abort_flag, p.status);   // dV_{j-1} has read the P^T tile
         if (!ok) break;
       }
 #pragma unroll
@@ -573,8 +607,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
       }
       fence_proxy_async();
       mbar_arrive(&p_full);
-      ok = mbar_wait(&dp_full, it & 1, &abort_flag, p.status);
-      ok = __all_sync(0xffffffffu, ok);
+      ok = mbar_wait_w(&dp_full, it & 1, &abort_flag, p.status);
       if (!ok) break;
       tc_fence_after();
       {
@@ -584,8 +617,11 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         // dS^T = P^T (dP^T - delta) without the softmax scale (applied once when dK is written); the
         // tensor core already subtracted delta from every column
 #pragma unroll
-        for (int c = 0; c < 32; c += 2)
-          pd[c / 2] = pack_bf16x2(pf[c] * __uint_as_float(rd[c]), pf[c + 1] * __uint_as_float(rd[c + 1]));
+        for (int c = 0; c < 32; c += 2) {
+          float d0, d1;
+          f2_unpack(f2_mul(f2_pack(pf[c], pf[c + 1]), f2_pack(__uint_as_float(rd[c]), __uint_as_float(rd[c + 1]))), d0, d1);
+          pd[c / 2] = pack_bf16x2(d0, d1);
+        }
         // this thread has read every fp32 value of its row in this column half: overwrite its first 16 columns
         tmem_st16(tmem + lane_sel + kColDPT + half * 32, pd);
         tmem_wait_st();
@@ -594,8 +630,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
       mbar_arrive(&ds_full);
     }
     if (ok) {
-      ok = mbar_wait(&acc_bar, 0, &abort_flag, p.status);
-      ok = __all_sync(0xffffffffu, ok);
+      ok = mbar_wait_w(&acc_bar, 0, &abort_flag, p.status);
     }
     float kv_dot_part = 0.f;        // this thread's share of sum_rows (<dK, K> + <dV, V>) for its key row and column half
     if (p.dkv_tma) {
@@ -737,8 +772,9 @@ int launch_attn_tc_bwd(const moc_attn_shape* s, const void* q, const void* kv, c
     p.d_q = static_cast<__nv_bfloat16*>(d_q); p.delta = delta; p.nlse2 = nlse2;
     p.L = L; p.n_sel = s->n_sel; p.H = H; p.HK = HK;
     p.scale = s->scale; p.scale_log2 = s->scale * kLog2e; p.status = status;
-    dim3 grid(ceil_div(L, kQ), H, B);
-    attn_bwd_dq_tc_kernel<<<grid, kThreads, kDqSmem, stream>>>(tq128, tdo128, tkv, p);
+    p.split = attn_key_split(ceil_div(L, kQ) * H * B, ceil_div(s->n_sel, kKeys), 296);
+    dim3 grid(ceil_div(L, kQ) * p.split, H, B);
+    MOC_CUDA_OK(launch_clustered(attn_bwd_dq_tc_kernel, grid, kThreads, kDqSmem, p.split, stream, tq128, tdo128, tkv, p));
   }
   if (parts & 4) {
     DkvParams p;

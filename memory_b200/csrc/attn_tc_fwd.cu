@@ -5,13 +5,19 @@
 // accumulator in tensor memory) -> online softmax by 128 threads that each own one query row
 // (tcgen05.ld, exp2 on the scaled scores, P written back to tensor memory as packed bf16) ->
 // O += P_j V_j (tcgen05.mma with A = P from tensor memory, B = the V tile as an MN-major operand).
-// A CTA holds 256 TMEM columns -- two 64-column score buffers (tile j uses buffer j & 1; P_j is written
-// as packed bf16 over the first 32 columns of its own buffer) and the 64-column O accumulator -- about
-// 65 KiB of shared memory and 192 threads, and two CTAs share an SM (__launch_bounds__(192, 2)).  S_{j+1}
-// is issued before PV_j, so the tensor pipe computes the next scores while the row owners run the softmax
-// of the current ones; the second CTA fills what is left of the strictly ordered chain.  The
+// A CTA holds 256 TMEM columns -- three 64-column score buffers (P_j is written as packed bf16 over the first 32 columns
+// of its own buffer) and the 64-column O accumulator -- about 97 KiB of shared memory and 192 threads, and two CTAs share
+// an SM (__launch_bounds__(192, 2)).  Scores run three tiles ahead of PV.  The
 // running maximum is only raised (and O rescaled) when it grows by more than 2^8, which keeps P
 // within bf16 range while skipping almost every rescale.
+//
+// What bounds it: at 8 x 1024 queries, 12 heads, 4,160 keys a 128 x 64 tile takes an SM about 410 ns (770 cycles) of which
+// the exponential unit is busy 450 and the tensor pipe 256; the rest is the chain wait -> tensor-memory load ->
+// exponentials -> store -> wait with two row-owning warps per scheduler.  Four CTAs per SM with one score buffer each, and
+// two query tiles per CTA sharing the K / V tiles, measured the same or worse (460 and 445 ns).  190 us before, 167 us now.
+//
+// With few query tiles (short or few sequences) the key range is cut into up to eight runs, one CTA of a cluster each,
+// merged through distributed shared memory at the end: 320 queries of one sequence 52 -> 25 us.
 #define MOC_KERNEL_TAG 2
 #include "moc_common.cuh"
 
@@ -21,31 +27,58 @@ namespace {
 constexpr int kQ = 128;          // queries per CTA
 constexpr int kKeys = 64;        // keys per tile
 constexpr int kD = 64;           // head dim
-constexpr int kStages = 3;       // K/V ring depth (K_j is read one tile before V_j)
-constexpr int kThreads = 192;    // 4 softmax warps + TMA warp + MMA warp
+constexpr int kStages = 5;       // K/V ring depth (K_j is read three tiles before V_j)
+constexpr int kBufs = 3;         // score buffers
+constexpr int kThreads = 192;    // 4 softmax warps + a warp for loads and scores + a warp for P V
 constexpr int kQBytes = kQ * kD * 2;
 constexpr int kTileBytes = kKeys * kD * 2;
 constexpr int kSmemBytes = kQBytes + kStages * 2 * kTileBytes + 1024;
 constexpr int kTmemCols = 256;
-constexpr uint32_t kColS = 0;      // S buffers: columns [0,64) and [64,128), tile j uses buffer j & 1
+constexpr uint32_t kColS = 0;      // S buffers of 64 columns, tile j uses buffer j % 3
 constexpr uint32_t kColP = 0;      // P_j as packed bf16 over the first 32 columns of its S buffer
-constexpr uint32_t kColO = 128;    // O accumulator: 64 columns
+constexpr uint32_t kColO = 192;    // O accumulator: 64 columns
+// Of every eight columns, how many take the polynomial instead of the exponential unit (0, 1, 2, 3 pairs of four in the
+// second half measured 428, 416, 428, 462 ns per 128 x 64 tile and SM).
+constexpr int kPolyOf4 = 1;
 constexpr float kRescaleThreshold = 8.0f;
 
 struct FwdParams {
   __nv_bfloat16* o;
   float* lse;
-  int L, n_sel, H, HK;
+  int L, n_sel, H, HK, split;
   float scale_log2;   // softmax scale * log2(e)
   int* status;
 };
 
 __device__ __forceinline__ float ex2(float x) {
   float y;
-  asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 
+// 2^x for two values on the FMA pipe: x = n + f with |f| <= 1/2 (Cody-Waite with the round-to-nearest addition of
+// 1.5 * 2^23), a degree-5 polynomial fitted to 2^f for least relative error (2.3e-7 in fp32, that of the hardware
+// instruction), n added to the exponent.  Arguments below -126 count as -126.
+__device__ __forceinline__ void ex2_poly2(uint64_t x, float& y0, float& y1) {
+  float x0, x1;
+  f2_unpack(x, x0, x1);
+  x = f2_pack(fmaxf(x0, -126.f), fmaxf(x1, -126.f));
+  const uint64_t magic = f2_pack(12582912.f, 12582912.f), nmagic = f2_pack(-12582912.f, -12582912.f);
+  const uint64_t t = f2_add(x, magic);
+  const uint64_t n = f2_add(t, nmagic);
+  const uint64_t f = f2_fma(n, f2_pack(-1.f, -1.f), x);
+  uint64_t p = f2_pack(0.001327647129073739f, 0.001327647129073739f);
+  p = f2_fma(p, f, f2_pack(0.009675540961325169f, 0.009675540961325169f));
+  p = f2_fma(p, f, f2_pack(0.05550713092088699f, 0.05550713092088699f));
+  p = f2_fma(p, f, f2_pack(0.24022120237350464f, 0.24022120237350464f));
+  p = f2_fma(p, f, f2_pack(0.6931469440460205f, 0.6931469440460205f));
+  p = f2_fma(p, f, f2_pack(1.0000001192092896f, 1.0000001192092896f));
+  float p0, p1, t0, t1;
+  f2_unpack(p, p0, p1);
+  f2_unpack(t, t0, t1);
+  y0 = __int_as_float(__float_as_int(p0) + (__float_as_int(t0) << 23));
+  y1 = __int_as_float(__float_as_int(p1) + (__float_as_int(t1) << 23));
+}
 
 // MMA groups issued as one instruction block by one elected lane (~3 instructions per MMA): the MMA warp
 // shares its scheduler partition with busy row-owning warps, so instructions per MMA set the issue rate.
@@ -86,10 +119,10 @@ __global__ void __launch_bounds__(kThreads, 2)
 attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_kv,
                    FwdParams p) {
   extern __shared__ uint8_t smem_raw[];
-  // p_full is one barrier per score buffer: S_{j+1} is issued before the MMA warp waits for P_j, so the row owners
-  // can finish tile j+1 (the other buffer) while that wait has not yet observed tile j's phase; with a single barrier
-  // two completed phases would look like none to a parity wait and the warp would wait forever.
-  __shared__ __align__(8) uint64_t q_bar, kv_full[kStages], kv_empty[kStages], s_full[2], p_full[2], pv_bar;
+  // p_full is one barrier per score buffer: scores are issued ahead of P, so the row owners can finish tile j+1 (the next
+  // buffer) while the MMA warp has not yet observed tile j's phase; with a single barrier two completed phases would look
+  // like none to a parity wait and the warp would wait forever.
+  __shared__ __align__(8) uint64_t q_bar, kv_full[kStages], s_full[kBufs], p_full[kBufs], pv_done[kBufs], o_bar;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
@@ -98,20 +131,20 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   uint8_t* q_s = base;
   uint8_t* kv_s = base + kQBytes;
 
-  const int q0 = blockIdx.x * kQ;
+  // a cluster of p.split CTAs shares one query tile; each takes a run of the key tiles
+  const int rank = p.split > 1 ? static_cast<int>(cluster_rank()) : 0;
+  const int q0 = blockIdx.x / p.split * kQ;
   const int h = blockIdx.y, b = blockIdx.z;
   const int kh = h / (p.H / p.HK);
-  const int n_tiles = (p.n_sel + kKeys - 1) / kKeys;
+  const int all_tiles = (p.n_sel + kKeys - 1) / kKeys;
+  const int tile0 = rank * all_tiles / p.split, n_tiles = (rank + 1) * all_tiles / p.split - tile0;
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
     mbar_init(&q_bar, 1);
-    for (int s = 0; s < kStages; ++s) { mbar_init(&kv_full[s], 1); mbar_init(&kv_empty[s], 1); }
-    mbar_init(&s_full[0], 1);
-    mbar_init(&s_full[1], 1);
-    mbar_init(&p_full[0], 128);
-    mbar_init(&p_full[1], 128);
-    mbar_init(&pv_bar, 1);
+    for (int s = 0; s < kStages; ++s) mbar_init(&kv_full[s], 1);
+    for (int i = 0; i < kBufs; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 128); mbar_init(&pv_done[i], 1); }
+    mbar_init(&o_bar, 1);
     fence_mbar_init();
     prefetch_tmap(&tmap_q);
     prefetch_tmap(&tmap_kv);
@@ -125,75 +158,81 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
 
+  // Two control warps, warp-uniform, one elected lane issues.  Each passes one or two waits and four MMAs per tile; as one
+  // warp, competing for issue slots with the softmax warps of its scheduler, their chain took longer than the softmax.
   if (warp == 4) {
-    // ---------------- TMA producer ----------------
+    // ---------------- loads and scores ----------------
+    const uint32_t idesc_s = umma_idesc_bf16(kQ, kKeys, 0, 0);
+    const uint64_t q_desc = umma_desc_sw128(smem_u32(q_s), 16, 1024);
+    const uint64_t k_desc0 = umma_desc_sw128(smem_u32(kv_s), 16, 1024);
+    constexpr uint64_t kStageOff = (2 * kTileBytes) >> 4;
+    auto load = [&](int j, int stage) {
+      if (lane == 0) {
+        uint8_t* k_s = kv_s + stage * 2 * kTileBytes;
+        const int row = b * p.n_sel + (tile0 + j) * kKeys;
+        mbar_arrive_expect_tx(&kv_full[stage], 2 * kTileBytes);
+        tma_load_2d(k_s, &tmap_kv, &kv_full[stage], kh * kD, row);
+        tma_load_2d(k_s + kTileBytes, &tmap_kv, &kv_full[stage], p.HK * kD + kh * kD, row);
+      }
+      __syncwarp();
+    };
     if (lane == 0) {
       mbar_arrive_expect_tx(&q_bar, kQBytes);
       tma_load_2d(q_s, &tmap_q, &q_bar, h * kD, b * p.L + q0);
-      for (int j = 0; j < n_tiles; ++j) {
-        const int s = j % kStages;
-        const uint32_t ph = (j / kStages) & 1;
-        if (!mbar_wait(&kv_empty[s], ph ^ 1, &abort_flag, p.status)) break;
-        mbar_arrive_expect_tx(&kv_full[s], 2 * kTileBytes);
-        uint8_t* k_s = kv_s + s * 2 * kTileBytes;
-        const int row = b * p.n_sel + j * kKeys;
-        tma_load_2d(k_s, &tmap_kv, &kv_full[s], kh * kD, row);
-        tma_load_2d(k_s + kTileBytes, &tmap_kv, &kv_full[s], p.HK * kD + kh * kD, row);
+    }
+    for (int j = 0; j < kStages && j < n_tiles; ++j) load(j, j);
+    bool ok = mbar_wait_w(&q_bar, 0, &abort_flag, p.status);
+    // Scores run three tiles ahead: S_j takes the buffer of P_{j-3} as soon as P_{j-3} V_{j-3} is complete, which also
+    // frees that tile's stage.
+    int buf = 0, s = 0, s3 = kStages - kBufs;       // j % 3, j % kStages, (j - 3) % kStages
+    uint32_t bph = 1, sph = 0;                      // parities: PV that last used `buf`, fill of stage s
+    for (int j = 0; j < n_tiles && ok; ++j) {
+      if (j >= kBufs) {
+        ok = mbar_wait_w(&pv_done[buf], bph, &abort_flag, p.status);
+        if (!ok) break;
+        if (j - kBufs + kStages < n_tiles) load(j - kBufs + kStages, s3);
       }
+      ok = mbar_wait_w(&kv_full[s], sph, &abort_flag, p.status);
+      if (!ok) break;
+      tc_fence_after();
+      issue_ss_single(tmem + kColS + buf * 64, q_desc, k_desc0 + s * kStageOff, idesc_s);
+      tc_commit_w(&s_full[buf]);
+      if (++buf == kBufs) { buf = 0; bph ^= 1; }
+      if (++s == kStages) { s = 0; sph ^= 1; }
+      if (++s3 == kStages) s3 = 0;
     }
   } else if (warp == 5) {
-    // ---------------- MMA issuer ----------------
-    {   // warp-uniform: every lane runs the loop, one elected lane issues
-      const uint32_t idesc_s = umma_idesc_bf16(kQ, kKeys, 0, 0);
-      const uint32_t idesc_o = umma_idesc_bf16(kQ, kD, 0, 1);
-      // descriptors are built once; a stage or K step only adds a constant to the address field
-      const uint64_t q_desc = umma_desc_sw128(smem_u32(q_s), 16, 1024);
-      const uint64_t k_desc0 = umma_desc_sw128(smem_u32(kv_s), 16, 1024);
-      const uint64_t v_desc0 = umma_desc_sw128(smem_u32(kv_s) + kTileBytes, 8192, 1024);
-      constexpr uint64_t kStageOff = (2 * kTileBytes) >> 4;
-      bool ok = mbar_wait_w(&q_bar, 0, &abort_flag, p.status);
-      // Two S buffers: S_{j+1} is issued before PV_j, so the tensor pipe computes the next scores while the row
-      // owners exponentiate the current ones.  S_{j+1} overwrites the buffer P_{j-1} lived in; tcgen05.mma
-      // instructions of one thread execute in issue order, so PV_{j-1} has read it.
-      if (ok && n_tiles > 0) {
-        ok = mbar_wait_w(&kv_full[0], 0, &abort_flag, p.status);
-        if (ok) {
-          tc_fence_after();
-          issue_ss_single(tmem + kColS, q_desc, k_desc0, idesc_s);
-          tc_commit_w(&s_full[0]);
-        }
-      }
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        if (j + 1 < n_tiles) {
-          const int sn = (j + 1) % kStages;
-          ok = mbar_wait_w(&kv_full[sn], ((j + 1) / kStages) & 1, &abort_flag, p.status);
-          if (!ok) break;
-          tc_fence_after();
-          issue_ss_single(tmem + kColS + ((j + 1) & 1) * 64, q_desc, k_desc0 + sn * kStageOff, idesc_s);
-          tc_commit_w(&s_full[(j + 1) & 1]);
-        }
-        const int s = j % kStages;
-        ok = mbar_wait_w(&p_full[j & 1], (j >> 1) & 1, &abort_flag, p.status);
-        if (!ok) break;
-        tc_fence_after();
-        issue_ts_single(tmem + kColO, tmem + kColP + (j & 1) * 64, v_desc0 + s * kStageOff, idesc_o, j > 0 ? 1u : 0u);
-        tc_commit_w(&kv_empty[s]);
-        tc_commit_w(&pv_bar);
-      }
+    // ---------------- P V ----------------
+    const uint32_t idesc_o = umma_idesc_bf16(kQ, kD, 0, 1);
+    const uint64_t v_desc0 = umma_desc_sw128(smem_u32(kv_s) + kTileBytes, 8192, 1024);
+    constexpr uint64_t kStageOff = (2 * kTileBytes) >> 4;
+    bool ok = true;
+    int buf = 0, s = 0;
+    uint32_t bph = 0;
+    for (int j = 0; j < n_tiles && ok; ++j) {
+      ok = mbar_wait_w(&p_full[buf], bph, &abort_flag, p.status);    // (S_j was complete before, and K_j / V_j with it)
+      if (!ok) break;
+      tc_fence_after();
+      issue_ts_single(tmem + kColO, tmem + kColP + buf * 64, v_desc0 + s * kStageOff, idesc_o, j > 0 ? 1u : 0u);
+      tc_commit_w(&pv_done[buf]);
+      if (++buf == kBufs) { buf = 0; bph ^= 1; }
+      if (++s == kStages) s = 0;
     }
+    tc_commit_w(&o_bar);
   } else {
     // ---------------- softmax: thread <-> query row ----------------
     const uint32_t lane_sel = static_cast<uint32_t>(warp * 32) << 16;
     const int row = warp * 32 + lane;
     float m_used = -INFINITY, l_sum = 0.f;
     bool ok = true;
+    int buf = 0;
+    uint32_t bph = 0;
     for (int j = 0; j < n_tiles; ++j) {
-      ok = mbar_wait(&s_full[j & 1], (j >> 1) & 1, &abort_flag, p.status);
-      ok = __all_sync(0xffffffffu, ok);
+      ok = mbar_wait_w(&s_full[buf], bph, &abort_flag, p.status);
       if (!ok) break;
       tc_fence_after();
-      const uint32_t s_addr = tmem + lane_sel + kColS + (j & 1) * 64;
-      const int valid = p.n_sel - j * kKeys;   // keys of this tile that exist
+      const uint32_t s_addr = tmem + lane_sel + kColS + buf * 64;
+      const int valid = p.n_sel - (tile0 + j) * kKeys;   // keys of this tile that exist
       uint32_t r0[32], r1[32];                 // the whole score row stays in registers
       tmem_ld32(s_addr, r0);
       tmem_ld32(s_addr + 32, r1);
@@ -205,59 +244,82 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
           if (32 + c >= valid) r1[c] = 0xFF800000u;
         }
       }
-      float tmax = -INFINITY;
-#pragma unroll
-      for (int c = 0; c < 32; ++c) tmax = fmaxf(tmax, fmaxf(__uint_as_float(r0[c]), __uint_as_float(r1[c])));
-      const float m_new = fmaxf(m_used, tmax * p.scale_log2);
-      const bool need = (j == 0) || (m_new - m_used > kRescaleThreshold);
-      const bool any_need = __any_sync(0xffffffffu, need);
-      if (j > 0 && any_need) {
-        ok = mbar_wait(&pv_bar, (j - 1) & 1, &abort_flag, p.status);   // O is complete up to tile j-1
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        tc_fence_after();
-        const float alpha = need ? ex2(m_used - m_new) : 1.f;
-        uint32_t r[32];
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          tmem_ld32(tmem + lane_sel + kColO + half * 32, r);
-          tmem_wait_ld();
-#pragma unroll
-          for (int c = 0; c < 32; ++c) r[c] = __float_as_uint(__uint_as_float(r[c]) * alpha);
-          tmem_st32(tmem + lane_sel + kColO + half * 32, r);
-        }
-        l_sum *= alpha;
-      }
-      if (need) m_used = m_new;
       uint32_t pk[32];
-      float psum0 = 0.f, psum1 = 0.f;
-      // exp2 of -inf is 0, so masked columns add nothing
+      float psum;
+      // exp2 of the scaled scores against the running maximum; exp2 of -inf is 0, so masked columns add nothing.  Scaling
+      // and the row sum take two columns per instruction.
+      auto exps = [&]() {
+        const uint64_t sc = f2_pack(p.scale_log2, p.scale_log2), nm = f2_pack(-m_used, -m_used);
+        uint64_t sum0 = 0ull, sum1 = 0ull;
 #pragma unroll
-      for (int c = 0; c < 32; c += 2) {
-        const float e0 = ex2(fmaf(__uint_as_float(r0[c]), p.scale_log2, -m_used));
-        const float e1 = ex2(fmaf(__uint_as_float(r0[c + 1]), p.scale_log2, -m_used));
-        psum0 += e0;
-        psum1 += e1;
-        pk[c / 2] = pack_bf16x2(e0, e1);
-      }
+        for (int c = 0; c < 32; c += 2) {
+          float e0, e1, g0, g1;
+          const uint64_t xe = f2_fma(f2_pack(__uint_as_float(r0[c]), __uint_as_float(r0[c + 1])), sc, nm);
+          const uint64_t xg = f2_fma(f2_pack(__uint_as_float(r1[c]), __uint_as_float(r1[c + 1])), sc, nm);
+          f2_unpack(xe, e0, e1);
+          e0 = ex2(e0); e1 = ex2(e1);
+          if ((c & 7) / 2 < kPolyOf4) {
+            ex2_poly2(xg, g0, g1);
+          } else {
+            f2_unpack(xg, g0, g1);
+            g0 = ex2(g0); g1 = ex2(g1);
+          }
+          sum0 = f2_add(sum0, f2_pack(e0, e1));
+          sum1 = f2_add(sum1, f2_pack(g0, g1));
+          pk[c / 2] = pack_bf16x2(e0, e1);
+          pk[16 + c / 2] = pack_bf16x2(g0, g1);
+        }
+        float x0, x1;
+        f2_unpack(f2_add(sum0, sum1), x0, x1);
+        psum = x0 + x1;
+      };
+      auto row_max = [&]() {
+        float t[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int c = 0; c < 32; c += 2) {
-        const float e0 = ex2(fmaf(__uint_as_float(r1[c]), p.scale_log2, -m_used));
-        const float e1 = ex2(fmaf(__uint_as_float(r1[c + 1]), p.scale_log2, -m_used));
-        psum0 += e0;
-        psum1 += e1;
-        pk[16 + c / 2] = pack_bf16x2(e0, e1);
+        for (int c = 0; c < 32; c += 4)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) t[i] = max3(t[i], __uint_as_float(r0[c + i]), __uint_as_float(r1[c + i]));
+        return fmaxf(max3(t[0], t[1], t[2]), t[3]);
+      };
+      // The maximum is off the critical path: from the second tile on the exponentials are taken against the running
+      // maximum at once, and only a tile that exceeds it by more than 2^8 (P would leave bf16's accurate range) is taken
+      // again after the rescale.
+      if (j > 0) exps();
+      const float m_new = fmaxf(m_used, row_max() * p.scale_log2);
+      const bool need = (j == 0) || (m_new - m_used > kRescaleThreshold);
+      if (__any_sync(0xffffffffu, need)) {
+        if (j > 0) {
+          const int pb = buf == 0 ? kBufs - 1 : buf - 1;      // O is complete up to tile j-1
+          ok = mbar_wait_w(&pv_done[pb], buf == 0 ? bph ^ 1 : bph, &abort_flag, p.status);
+          if (!ok) break;
+          tc_fence_after();
+          const float alpha = need ? ex2(m_used - m_new) : 1.f;
+          uint32_t r[32];
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            tmem_ld32(tmem + lane_sel + kColO + half * 32, r);
+            tmem_wait_ld();
+#pragma unroll
+            for (int c = 0; c < 32; ++c) r[c] = __float_as_uint(__uint_as_float(r[c]) * alpha);
+            tmem_st32(tmem + lane_sel + kColO + half * 32, r);
+          }
+          l_sum *= alpha;
+        }
+        if (need) m_used = m_new;
+        exps();
       }
-      l_sum += psum0 + psum1;
+      l_sum += psum;
       // every S value of this row is in registers: P goes over the first 32 columns of this tile's S buffer
-      tmem_st32(tmem + lane_sel + kColP + (j & 1) * 64, pk);
+      tmem_st32(tmem + lane_sel + kColP + buf * 64, pk);
       tmem_wait_st();
       tc_fence_before();
-      mbar_arrive(&p_full[j & 1]);
+      mbar_arrive(&p_full[buf]);
+      if (++buf == kBufs) { buf = 0; bph ^= 1; }
     }
     if (ok) {
-      ok = mbar_wait(&pv_bar, (n_tiles - 1) & 1, &abort_flag, p.status);
-      ok = __all_sync(0xffffffffu, ok);
+      // A barrier of its own for the finished accumulator: when this warp has handed over its last tile, the products of
+      // up to two tiles before may still be waiting for another warp's rows (scores run ahead of them).
+      ok = mbar_wait_w(&o_bar, 0, &abort_flag, p.status);
     }
     if (ok) {
       tc_fence_after();
@@ -269,7 +331,15 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         uint32_t r[32];
         tmem_ld32(tmem + lane_sel + kColO + half * 32, r);
         tmem_wait_ld();
-        if (l < p.L) {
+        if (p.split > 1) {
+          // unnormalised rows into the idle tile ring, 16-byte chunks rotated by the row against bank conflicts
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const uint32_t addr = smem_u32(kv_s) + row * 256 + (((half * 8 + c) ^ (row & 15)) << 4);
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r[4 * c]), "r"(r[4 * c + 1]),
+                         "r"(r[4 * c + 2]), "r"(r[4 * c + 3]) : "memory");
+          }
+        } else if (l < p.L) {
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
             uint4 v;
@@ -281,7 +351,9 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
           }
         }
       }
-      if (l < p.L)
+      if (p.split > 1)
+        reinterpret_cast<float2*>(q_s)[row] = make_float2(m_used, l_sum);
+      else if (l < p.L)
         p.lse[(static_cast<long long>(b) * p.H + h) * p.L + l] = (m_used + log2f(l_sum)) * 0.6931471805599453f;
     }
     tc_fence_before();
@@ -290,6 +362,35 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   __syncthreads();
   if (abort_flag) {
     for (int i = 0; i < 200; ++i) __nanosleep(1000);
+  }
+  if (p.split > 1) {
+    // The CTAs of the cluster merge their parts of the key range: each takes a share of the query rows and reads every
+    // CTA's (maximum, sum, row) through distributed shared memory; 16 lanes per row, four columns each.
+    cluster_sync();
+    if (!abort_flag) {
+      const int row_lo = rank * kQ / p.split, row_hi = (rank + 1) * kQ / p.split;
+      const int c = threadIdx.x & 15;
+      for (int row = row_lo + static_cast<int>(threadIdx.x >> 4); row < row_hi && q0 + row < p.L; row += kThreads / 16) {
+        float m = -INFINITY, l = 0.f;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i = 0; i < p.split; ++i) {
+          const float2 ml = cluster_ld2(cluster_map(smem_u32(q_s) + row * 8, i));
+          const float4 v = cluster_ld4(cluster_map(smem_u32(kv_s) + row * 256 + ((c ^ (row & 15)) << 4), i));
+          const float mn = fmaxf(m, ml.x), a = ex2(m - mn), f = ex2(ml.x - mn);
+          l = l * a + ml.y * f;
+          acc.x = acc.x * a + v.x * f; acc.y = acc.y * a + v.y * f;
+          acc.z = acc.z * a + v.z * f; acc.w = acc.w * a + v.w * f;
+          m = mn;
+        }
+        const float inv = 1.f / l;
+        __nv_bfloat16* dst = p.o + (static_cast<long long>(b) * p.L + q0 + row) * (p.H * kD) + h * kD;
+        reinterpret_cast<uint2*>(dst)[c] =
+            make_uint2(pack_bf16x2(acc.x * inv, acc.y * inv), pack_bf16x2(acc.z * inv, acc.w * inv));
+        if (c == 0)
+          p.lse[(static_cast<long long>(b) * p.H + h) * p.L + q0 + row] = (m + log2f(l)) * 0.6931471805599453f;
+      }
+    }
+    cluster_sync();                            // no CTA leaves while another still reads its rows
   }
   if (warp == 5) {
     tc_fence_after();
@@ -320,9 +421,9 @@ int launch_attn_tc_fwd(const moc_attn_shape* s, const void* q, const void* kv, v
   p.L = s->seq; p.n_sel = s->n_sel; p.H = s->num_heads; p.HK = s->num_kv_heads;
   p.scale_log2 = s->scale * 1.4426950408889634f;
   p.status = status;
-  dim3 grid(ceil_div(s->seq, kQ), s->num_heads, s->batch);
-  attn_fwd_tc_kernel<<<grid, kThreads, kSmemBytes, stream>>>(tq, tkv, p);
-  MOC_CUDA_OK(cudaGetLastError());
+  p.split = attn_key_split(ceil_div(s->seq, kQ) * s->num_heads * s->batch, ceil_div(s->n_sel, kKeys), 296);
+  dim3 grid(ceil_div(s->seq, kQ) * p.split, s->num_heads, s->batch);
+  MOC_CUDA_OK(launch_clustered(attn_fwd_tc_kernel, grid, kThreads, kSmemBytes, p.split, stream, tq, tkv, p));
   return MOC_OK;
 }
 

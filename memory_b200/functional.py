@@ -232,7 +232,7 @@ class _CrossAttention(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, h, memory, wq, wk, wv, wo, norm_w, norm_b, num_heads, num_kv_heads, compute_dtype,
-                norm_kind, norm_eps, add_residual):
+                norm_kind, norm_eps, add_residual, grad_on):
         L.require_cuda(h, memory, wq, wk, wv, wo)
         b, l, d = h.shape
         cd = compute_dtype
@@ -249,7 +249,7 @@ class _CrossAttention(torch.autograd.Function):
         ws = [ops._contig(w if same else w.float()) for w in (wq, wk, wv, wo)]
         nw = None if norm_w is None else ops._contig(norm_w.float())
         nb = None if norm_b is None else ops._contig(norm_b.float())
-        need_grad = any(ctx.needs_input_grad[:8])
+        need_grad = grad_on and any(ctx.needs_input_grad[:8])
         out = torch.empty(b, l, d, dtype=in_dtype if in_dtype in (torch.float32, cd) else cd, device=dev)
         if cd == torch.float32 and out.dtype != cd:
             out = torch.empty(b, l, d, dtype=cd, device=dev)
@@ -309,7 +309,7 @@ class _CrossAttention(torch.autograd.Function):
         ops.xattn_bwd(s, q)
         return (_cast(d_h, in_dtype) if need[0] else None, _cast(d_mem, mem_dtype), _cast(d_wq, wdt[0]),
                 _cast(d_wkv[:dkv], wdt[1]), _cast(d_wkv[dkv:], wdt[2]), _cast(d_wo, wdt[3]), _cast(d_nw, nw_dtype),
-                _cast(d_nb, nb_dtype), None, None, None, None, None, None)
+                _cast(d_nb, nb_dtype), None, None, None, None, None, None, None)
 
 
 def cross_attention(h: torch.Tensor, memory: torch.Tensor, wq, wk, wv, wo, num_heads: int,
@@ -333,7 +333,8 @@ def cross_attention(h: torch.Tensor, memory: torch.Tensor, wq, wk, wv, wo, num_h
             norm_bias = None
     return _CrossAttention.apply(h, memory, wq, wk, wv, wo, norm_weight if pre_norm else None,
                                  norm_bias if pre_norm else None, int(num_heads), int(num_kv_heads or num_heads),
-                                 compute_dtype or h.dtype, pre_norm, float(norm_eps), bool(add_residual))
+                                 compute_dtype or h.dtype, pre_norm, float(norm_eps), bool(add_residual),
+                                 torch.is_grad_enabled())
 
 
 # --------------------------------------------------------------------------------------------
@@ -366,7 +367,7 @@ class _MemoryLayerTwoStream(torch.autograd.Function):
     def forward(ctx, h_router, h_attn, bank, router_w, router_b, wq, wk, wv, wo, norm_w, norm_b, cfg, sink,
                 fused=None):
         (num_heads, num_kv_heads, t, top_k, num_shared, routed_scale, row_norm, row_eps, with_losses,
-         pre_norm, pre_eps, add_residual) = cfg
+         pre_norm, pre_eps, add_residual, grad_on) = cfg
         L.require_cuda(h_router, h_attn, bank, router_w)
         if h_router.dim() != 3:
             raise ValueError(f"hidden_states must be 3D (B, T, D), got shape {tuple(h_router.shape)}")
@@ -392,7 +393,8 @@ class _MemoryLayerTwoStream(torch.autograd.Function):
         ws = [ops._contig(w) for w in (wq, wk, wv, wo)]
         nw = None if norm_w is None else ops._contig(norm_w.float())
         nb = None if norm_b is None else ops._contig(norm_b.float())
-        need_grad = any(ctx.needs_input_grad[:11])
+        # (a node's forward always runs with gradients off; needs_input_grad says nothing about the caller's mode)
+        need_grad = grad_on and any(ctx.needs_input_grad[:11])
         n_pairs = b * (num_shared + k_sel)
         f32, i32 = torch.float32, torch.int32
         out = torch.empty(b, l, d, dtype=ha.dtype, device=dev)
@@ -418,7 +420,7 @@ class _MemoryLayerTwoStream(torch.autograd.Function):
         s.arena = arena.data_ptr()
         ops.layer_fwd(s)
 
-        ctx.cfg, ctx.desc, ctx.sink = cfg, s, sink
+        ctx.desc, ctx.sink = s, sink
         ctx.same_h = h_router is h_attn
         ctx.wkv_in_place = bool(fused is not None and fused.get("wkv_grad_in_place"))
         ctx.shapes = (tuple(h_router.shape), h_router.dtype, in_dtype, router_b is not None,
@@ -529,7 +531,7 @@ def memory_layer(h_router: torch.Tensor, h_attn: torch.Tensor, bank: torch.Tenso
             and bank.shape[1] == h_attn.shape[-1]):
         cfg = (int(num_heads), int(num_kv_heads or num_heads), int(tokens_per_chapter), int(top_k),
                int(num_shared_chapters), float(routed_scaling_factor), norm_type, float(norm_eps), bool(with_losses),
-               pre_norm, float(pre_norm_eps), bool(add_residual))
+               pre_norm, float(pre_norm_eps), bool(add_residual), torch.is_grad_enabled())
         if pre_norm is not None and pre_norm not in ops.NORM_KINDS:
             raise ValueError(f"unknown pre_norm {pre_norm!r}")
         if pre_norm in ("rms", "rmsnorm"):

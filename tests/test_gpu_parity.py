@@ -737,3 +737,32 @@ def test_backward_entered_first_on_a_fresh_autograd_thread():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "ok" in r.stdout, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("B,L,H,HK,N", [(1, 64, 2, 2, 257), (1, 320, 3, 1, 512), (2, 128, 2, 2, 2049), (1, 65, 1, 1, 40),
+                                        (1, 192, 12, 12, 4160)])
+def test_attention_split_over_clusters_and_large_scores(B, L, H, HK, N, dev):
+    """Few query tiles: the key range is shared by a cluster of CTAs (runs of unequal length, a ragged last tile).  Scores
+    that keep growing along the keys (by far more than the 2^8 the lazy maximum allows) take the rescale path."""
+    from memory_b200 import ops
+    D = 64
+    g = torch.Generator().manual_seed(N + L)
+    q = torch.randn(B, L, H * D, generator=g)
+    kv = torch.randn(B, N, 2 * HK * D, generator=g)
+    for growing in (False, True):
+        kvx = kv.clone()
+        if growing:
+            kvx[..., :HK * D] *= torch.linspace(0.05, 12.0, N).view(1, N, 1)
+        qb, kb = q.bfloat16().to(dev), kvx.bfloat16().to(dev)
+        ref, lref = attn_reference(qb.float().requires_grad_(True), kb.float().requires_grad_(True), H, HK, D)
+        o, lse = ops.attn_fwd(qb, kb, H, HK, D ** -0.5)
+        assert rel_err(o, ref) < BF16 and rel_err(lse, lref) < 1e-3
+        assert torch.equal(o, ops.attn_fwd(qb, kb, H, HK, D ** -0.5)[0])
+        if L % 64 == 0 and not growing:
+            qr, kr = qb.float().requires_grad_(True), kb.float().requires_grad_(True)
+            r2, _ = attn_reference(qr, kr, H, HK, D)
+            do = torch.randn(B, L, H * D, generator=g).bfloat16().to(dev)
+            r2.backward(do.float())
+            dq, dkv = ops.attn_bwd(qb, kb, o, lse, do, H, HK, D ** -0.5)
+            assert rel_err(dq, qr.grad) < 3e-2 and rel_err(dkv, kr.grad) < 3e-2
+    _status_ok(dev)
