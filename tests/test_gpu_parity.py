@@ -142,6 +142,26 @@ def test_router_tie_break_prefers_lower_chapter_id(dev):
         assert tied == list(range(5, 5 + len(tied)))
 
 
+@pytest.mark.parametrize("c,k,s", [(5, 4, 0), (2048, 64, 1), (2049, 64, 0), (5120, 1024, 3), (5121, 64, 1),
+                                   (9216, 64, 1), (9217, 64, 1)])
+def test_router_selection_is_the_stable_sort(dev, c, k, s):
+    """Rows that differ in how their values crowd: spread out, a grid with ties at the boundary, two values, one value."""
+    g = torch.Generator().manual_seed(c)
+    rows = [3 * torch.randn(c, generator=g), torch.randint(0, 12, (c,), generator=g) / 4, torch.randint(0, 2, (c,), generator=g) * 1.0,
+            torch.zeros(c)]
+    rows[0] = (rows[0] * 64).round() / 64
+    z = torch.stack(rows).to(dev)
+    h = torch.zeros(len(rows), 1, 8, device=dev)
+    from memory_b200 import ops
+    f = ops.router_fwd(h, torch.zeros(c, 8, device=dev), None, k, s, 2.5, False, pooled=h[:, 0].contiguous(), logits=z.clone())
+    want = torch.sort(z[:, s:], dim=-1, descending=True, stable=True).indices[:, :k] + s
+    assert torch.equal(f["idx"], want)
+    p = torch.softmax(z.double(), -1)
+    p[:, :s] = 0
+    p = p.gather(1, want)
+    torch.testing.assert_close(f["weights"].double(), p / p.sum(-1, keepdim=True), rtol=1e-4, atol=0)
+
+
 def test_router_bf16_hidden_states_use_fp32_arithmetic(dev):
     import memory_b200 as M
     case = CASES["cfg0"]
