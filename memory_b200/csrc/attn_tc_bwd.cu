@@ -772,7 +772,7 @@ int launch_attn_tc_bwd(const moc_attn_shape* s, const void* q, const void* kv, c
     p.d_q = static_cast<__nv_bfloat16*>(d_q); p.delta = delta; p.nlse2 = nlse2;
     p.L = L; p.n_sel = s->n_sel; p.H = H; p.HK = HK;
     p.scale = s->scale; p.scale_log2 = s->scale * kLog2e; p.status = status;
-    p.split = attn_key_split(ceil_div(L, kQ) * H * B, ceil_div(s->n_sel, kKeys), 296);
+    p.split = attn_key_split(ceil_div(L, kQ) * H * B, ceil_div(s->n_sel, kKeys));
     dim3 grid(ceil_div(L, kQ) * p.split, H, B);
     MOC_CUDA_OK(launch_clustered(attn_bwd_dq_tc_kernel, grid, kThreads, kDqSmem, p.split, stream, tq128, tdo128, tkv, p));
   }

@@ -421,7 +421,7 @@ int launch_attn_tc_fwd(const moc_attn_shape* s, const void* q, const void* kv, v
   p.L = s->seq; p.n_sel = s->n_sel; p.H = s->num_heads; p.HK = s->num_kv_heads;
   p.scale_log2 = s->scale * 1.4426950408889634f;
   p.status = status;
-  p.split = attn_key_split(ceil_div(s->seq, kQ) * s->num_heads * s->batch, ceil_div(s->n_sel, kKeys), 296);
+  p.split = attn_key_split(ceil_div(s->seq, kQ) * s->num_heads * s->batch, ceil_div(s->n_sel, kKeys));
   dim3 grid(ceil_div(s->seq, kQ) * p.split, s->num_heads, s->batch);
   MOC_CUDA_OK(launch_clustered(attn_fwd_tc_kernel, grid, kThreads, kSmemBytes, p.split, stream, tq, tkv, p));
   return MOC_OK;

@@ -381,15 +381,21 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
-// Runs the key tiles of a query tile are cut into (the CTAs of a cluster), for `ctas` query tiles and a chip with room for
-// `slots` CTAs: the count (at most eight, at least four key tiles per run) with the least rounds * (tiles per run + 3), where
-// 3 stands for a CTA's start-up and its share of the merge.
-inline int attn_key_split(int ctas, int key_tiles, int slots) {
+// Runs the key tiles of a query tile are cut into (the CTAs of a cluster), for `ctas` query tiles of a kernel of which two
+// CTAs fit on an SM.  The rule follows what was measured at 1 to 8 runs (12 to 768 query tiles, 17 to 65 key tiles):
+// a pair of CTAs on an SM takes 1.33 of the time of one that has it alone; a CTA's start-up and end cost 6 key tiles, 12
+// with the merge; a cluster stays within one of eight GPCs of at least 32 CTA slots, so a size that does not divide them
+// leaves slots empty (36 clusters of eight need a second round, of six they do not).  Splitting pays below about 150 query
+// tiles (96: 45 -> 36 us with two runs, 12: 43 -> 12 us with eight) and costs above (384: 97 -> 115 us with three).
+inline int attn_key_split(int ctas, int key_tiles) {
+  constexpr int kSms = 148, kGpcs = 8, kGpcSlots = 32;
   int best = 1;
   double best_cost = 0.0;
   for (int n = 1; n <= 8 && (n == 1 || key_tiles / n >= 4); ++n) {
-    const long long rounds = (static_cast<long long>(ctas) * n + slots - 1) / slots;
-    const double cost = static_cast<double>(rounds) * ((key_tiles + n - 1) / n + 3);
+    const int resident = n == 1 ? 2 * kSms : kGpcs * (kGpcSlots / n);
+    const int full = ctas / resident, rest = ctas % resident;
+    const double rounds = 1.33 * full + (rest == 0 ? 0.0 : rest * n <= kSms ? 1.0 : 1.33);
+    const double cost = rounds * ((key_tiles + n - 1) / n + (n == 1 ? 6 : 12));
     if (n == 1 || cost < 0.97 * best_cost) { best = n; best_cost = cost; }
   }
   return best;
