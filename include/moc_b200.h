@@ -403,6 +403,34 @@ int moc_decode_attn(const moc_decode_shape* s, const void* q, const void* kv_ban
                     const int32_t* comb_idx, const float* comb_w, void* out, float* lse, int32_t* status,
                     void* stream);
 
+/* The routing window of a generated token: dst [batch, dst_rows] = the last dst_rows rows of cache [batch, cache_rows]
+ * followed by h [batch, h_rows]; rows of row_bytes (a multiple of 16) lie behind each other, *_stride bytes lead from one
+ * sequence to the next (dst is dense).  model.py:630-660 concatenates and slices. */
+int moc_roll_window(const void* cache, int64_t cache_stride, int32_t cache_rows, const void* h, int64_t h_stride,
+                    int32_t h_rows, void* dst, int32_t dst_rows, int32_t batch, int32_t row_bytes, void* stream);
+
+/* One decoding step of a memory layer in one call: router on routing_states, query projection of hidden
+ * [batch * n_q, hidden_dim] (hidden_dtype), moc_decode_attn, output projection into out [batch * n_q, out_dim]
+ * (hidden_dtype).  wq / wo bf16. */
+typedef struct {
+  moc_router_shape router;
+  moc_decode_shape attn;
+  int32_t hidden_dtype, out_dim;
+  int64_t bank_rows;
+  const void *routing_states, *hidden;
+  const float *router_w, *router_b;
+  const void *wq, *wo, *kv_bank;
+  int64_t* idx;
+  float* weights;
+  int32_t* comb_idx;
+  float* comb_w;
+  void *out, *arena;
+  int32_t* status;
+  void* stream;
+} moc_decode_step_desc;
+int64_t moc_decode_step_arena_bytes(const moc_decode_step_desc* s);
+int moc_decode_step(const moc_decode_step_desc* s);
+
 /* ------------------------------------------------------------------------------------------------
  * Per-token chapter-sparse attention: the contract of memory_cross_attn(q, k, v, block_indices,
  * block_size, scale) (kernels-final/memory_cross_attn.py:1310-1366, 1387-1603, 1639-1652).

@@ -70,6 +70,12 @@ class RouteDesc(C.Structure):
         "p: h w bias pos_weight idx weights comb_idx comb_w losses arena status stream")
 
 
+class DecodeStepDesc(C.Structure):
+    _fields_ = [("router", RouterShape), ("attn", DecodeShape)] + _fields(
+        "i: hidden_dtype out_dim; l: bank_rows;"
+        "p: routing_states hidden router_w router_b wq wo kv_bank idx weights comb_idx comb_w out arena status stream")
+
+
 class LayerDesc(C.Structure):
     _fields_ = _fields(
         "i: batch seq router_seq hidden_dim num_heads num_kv_heads num_chapters tokens_per_chapter top_k num_shared"
@@ -180,6 +186,9 @@ _PROTOTYPES = {
     "moc_transpose": (C.c_int, [P, C.c_int32, P, C.c_int32, C.c_int32, C.c_int32, P]),
     "moc_pack_weights": (C.c_int, [C.c_int32, P, C.c_int32, P, P, P, P, P, P]),
     "moc_decode_attn": (C.c_int, [P, P, P, C.c_int64, P, P, P, P, P, P]),
+    "moc_roll_window": (C.c_int, [P, C.c_int64, C.c_int32, P, C.c_int64, C.c_int32, P, C.c_int32, C.c_int32, C.c_int32, P]),
+    "moc_decode_step_arena_bytes": (C.c_int64, [C.POINTER(DecodeStepDesc)]),
+    "moc_decode_step": (C.c_int, [C.POINTER(DecodeStepDesc)]),
     "moc_norm_bwd_workspace_bytes": (C.c_size_t, [C.c_int64, C.c_int32]),
     "moc_norm_fwd": (C.c_int, [P, P, P, C.c_int32, C.c_float, C.c_int64, C.c_int32, P, P, P, P]),
     "moc_norm_bwd": (C.c_int, [P, P, P, P, P, C.c_int32, C.c_int64, C.c_int32, P, P, P, P, P]),

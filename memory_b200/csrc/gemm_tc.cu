@@ -447,6 +447,10 @@ int sm_count() {
 
 }  // namespace
 
+bool gemm_rows_supported(const moc_gemm_desc* g, const float* row_scale, const int32_t* a_row_blocks,
+                         const int32_t* b_row_blocks);
+int launch_gemm_rows(const moc_gemm_desc* g, const void* a, const void* b, void* c, cudaStream_t stream);
+
 int launch_gemm_tc(const moc_gemm_desc* g, const void* a, const void* b, void* c, const float* row_scale,
                    const int32_t* a_row_blocks, int32_t* status, cudaStream_t stream,
                    const int32_t* b_row_blocks, int32_t b_block_rows, int64_t b_stored_rows) {
@@ -457,6 +461,7 @@ int launch_gemm_tc(const moc_gemm_desc* g, const void* a, const void* b, void* c
   MOC_REQUIRE(g->c_dtype == MOC_BF16 || g->c_dtype == MOC_F32, "bad c_dtype");
   const int split = g->split_k > 1 ? g->split_k : 1;
   if (split > 1 || g->accumulate) MOC_REQUIRE(g->c_dtype == MOC_F32, "accumulate / split_k need an fp32 C");
+  if (gemm_rows_supported(g, row_scale, a_row_blocks, b_row_blocks)) return launch_gemm_rows(g, a, b, c, stream);
   int a_box_rows = 64;
   int a_num_blocks = 0;
   long long a_stored_rows = g->a_kmajor ? g->m : g->k;

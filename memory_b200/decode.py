@@ -18,7 +18,6 @@ from typing import Optional, Tuple
 
 import torch
 
-from . import functional as F_moc
 from . import ops
 
 
@@ -73,6 +72,12 @@ class RoutingWindow:
         return hidden_states
 
     def step(self, hidden_states: torch.Tensor) -> torch.Tensor:
+        if self.cache is not None and hidden_states.dim() == 3 and not (torch.is_grad_enabled() and hidden_states.requires_grad):
+            rows = min(self.window_size, self.cache.shape[1] + hidden_states.shape[1])
+            window = ops.roll_window(self.cache, hidden_states, rows)
+            if window is not None:
+                self.cache = window
+                return window
         combined = hidden_states if self.cache is None else torch.cat([self.cache, hidden_states], dim=1)
         if combined.shape[1] > self.window_size:
             combined = combined[:, -self.window_size:]
@@ -96,19 +101,12 @@ class MemoryDecoder:
         self.wq_c, self.wo_c = ops.cast(wq.contiguous(), cd), ops.cast(wo.contiguous(), cd)
         self.scale = (wq.shape[0] // self.num_heads) ** -0.5
 
-    @torch.no_grad()
     def step(self, hidden_states: torch.Tensor, routing_states: torch.Tensor) -> Tuple[torch.Tensor, dict]:
         """``hidden_states`` [B, n_q, d]: the tokens being decoded (input of the cross attention);
         ``routing_states`` [B, W, d]: the states the router mean-pools (a :class:`RoutingWindow` result).
         Returns (output [B, n_q, d] in the dtype of ``hidden_states``, routing info)."""
-        b, n_q, d = hidden_states.shape
-        idx, w, cidx, cw, _ = F_moc.route(routing_states, self.router_weight, self.router_bias, self.top_k,
-                                          self.num_shared, self.routed_scale, with_losses=False)
-        cd = torch.bfloat16
-        q = ops.gemm(ops.cast(hidden_states.reshape(b * n_q, d), cd), self.wq_c, tag="q_proj")
-        o = ops.decode_attn(q.view(b, n_q, -1), self.cache.kv_bank, cidx, cw, self.num_heads, self.num_kv_heads,
-                            self.cache.tokens_per_chapter, self.scale)
-        out_dtype = hidden_states.dtype if hidden_states.dtype in (torch.float32, cd) else cd
-        out = ops.gemm(o.view(b * n_q, -1), self.wo_c, out_dtype=out_dtype, tag="o_proj")
-        return out.view(b, n_q, d).to(hidden_states.dtype), {"indices": idx, "weights": w, "combined_indices": cidx,
-                                                              "combined_weights": cw}
+        out, idx, w, cidx, cw = ops.decode_step(
+            hidden_states, routing_states, self.router_weight, self.router_bias, self.wq_c, self.wo_c, self.cache.kv_bank,
+            num_heads=self.num_heads, num_kv_heads=self.num_kv_heads, tokens_per_chapter=self.cache.tokens_per_chapter,
+            top_k=self.top_k, num_shared=self.num_shared, routed_scale=self.routed_scale, scale=self.scale)
+        return out, {"indices": idx, "weights": w, "combined_indices": cidx, "combined_weights": cw}

@@ -68,7 +68,7 @@ def router_selected_k(num_chapters: int, top_k: int, num_shared: int) -> int:
 def _router_fwd_launches(*a, **k):
     parts = k.get("parts", 3)
     with_losses = a[6] if len(a) > 6 else k.get("with_losses")
-    return (4 if parts & 1 else 0) + (2 if (parts & 2) and with_losses else 0)
+    return (3 if parts & 1 else 0) + (2 if (parts & 2) and with_losses else 0)
 
 
 @_instrument(lambda *a, **k: "router_fwd" if k.get("parts", 3) == 3 else "router_fwd:parts%d" % k["parts"],
@@ -568,7 +568,7 @@ def layer_fwd(s) -> None:
         yield "chapter_row_scale:i32" if s.fused else "gather_rows_fwd:" + _TAG_OF_CODE[s.bank_dtype]
         yield "attn_fwd:bf16"
     casts = int(norm or f32_in) + int((norm or s.add_residual) and not f32_in)
-    _report(10 + 2 * s.with_losses + s.for_backward + casts, parts)
+    _report(9 + int(s.router_seq > 1024) + 2 * s.with_losses + s.for_backward + casts, parts)
 
 
 def layer_bwd(s, b) -> None:
@@ -604,7 +604,7 @@ def route_bwd_scratch_bytes(s) -> int:
 def route_fwd(s) -> None:
     """``moc_route_fwd`` on a filled ``_lib.RouteDesc``."""
     L.check(_timed("router_fwd", lambda: L.lib().moc_route_fwd(C.byref(s))), "moc_route_fwd")
-    _report(4 + 2 * int(bool(s.losses)), lambda: ("router_fwd:" + _TAG_OF_CODE[s.shape.h_dtype],))
+    _report(3 + int(s.shape.seq > 1024) + 2 * int(bool(s.losses)), lambda: ("router_fwd:" + _TAG_OF_CODE[s.shape.h_dtype],))
 
 
 def route_bwd(s, g_w, g_cw, g_losses, d_h, d_w, d_bias, scratch) -> None:
@@ -1203,3 +1203,67 @@ def decode_attn(q: torch.Tensor, kv_bank: torch.Tensor, comb_idx: torch.Tensor, 
                                  L.stream_ptr(q.device))
     L.check(rc, "moc_decode_attn")
     return (out, lse) if want_lse else out
+
+
+def roll_window(cache: torch.Tensor, h: torch.Tensor, rows: int) -> Optional[torch.Tensor]:
+    """The last ``rows`` positions of ``cat([cache, h], dim=1)`` as a new [B, rows, d] tensor, or None where the rows are
+    no whole 16-byte pieces of CUDA memory (the caller concatenates)."""
+    b, d = h.shape[0], h.shape[2]
+    size = h.element_size()
+    if (not h.is_cuda or h.device != cache.device or h.dtype != cache.dtype or cache.shape[0] != b or cache.shape[2] != d
+            or d * size % 16 or b == 0 or b > 65535):
+        return None
+    for t in (cache, h):
+        sb, st, sd = t.stride()
+        if (sd != 1 and d > 1) or (st != d and t.shape[1] > 1) or sb * size % 16 or t.data_ptr() % 16:
+            return None
+    out = torch.empty(b, rows, d, dtype=h.dtype, device=h.device)
+    rc = _timed("roll_window", lambda: L.lib().moc_roll_window(
+        cache.data_ptr(), cache.stride(0) * size, cache.shape[1], h.data_ptr(), h.stride(0) * size, h.shape[1], out.data_ptr(),
+        rows, b, d * size, L.stream_ptr(h.device)))
+    L.check(rc, "moc_roll_window")
+    _report(1, lambda: ("roll_window:" + _DTYPE_TAG.get(h.dtype, str(h.dtype)),))
+    return out
+
+
+def decode_step(hidden: torch.Tensor, routing_states: torch.Tensor, router_w: torch.Tensor,
+                router_b: Optional[torch.Tensor], wq: torch.Tensor, wo: torch.Tensor, kv_bank: torch.Tensor, *,
+                num_heads: int, num_kv_heads: int, tokens_per_chapter: int, top_k: int, num_shared: int,
+                routed_scale: float, scale: float):
+    """One decoding step (``moc_decode_step``): out [B, n_q, d] in the dtype of ``hidden``, then indices int64, weights,
+    combined indices int32 and combined weights of the router."""
+    L.require_cuda(hidden, routing_states, router_w, router_b, wq, wo, kv_bank)
+    if routing_states.dim() != 3:
+        raise ValueError(f"hidden_states must be 3D (B, T, D), got shape {tuple(routing_states.shape)}")
+    b, n_q, d = hidden.shape
+    rb, window, rd = routing_states.shape
+    c, head_dim, dev = router_w.shape[0], wq.shape[0] // num_heads, hidden.device
+    if wq.shape[1] != d or wo.shape[1] != wq.shape[0]:
+        raise ValueError(f"inner dimensions differ: {d} / {wq.shape[0]} vs {wq.shape[1]} / {wo.shape[1]}")
+    if rd != router_w.shape[1]:
+        raise ValueError(f"inner dimensions differ: {rd} vs {router_w.shape[1]}")
+    if kv_bank.shape[1] != 2 * num_kv_heads * head_dim:
+        raise ValueError("kv_bank must be [rows, 2 * num_kv_heads * head_dim]")
+    if rb != b:
+        raise ValueError("hidden_states and routing_states must share the batch")
+    k = router_selected_k(c, top_k, num_shared)
+    f32 = torch.float32
+    h, states, w = _contig(hidden), _contig(routing_states), _contig(router_w.float())
+    bias = None if router_b is None else _contig(router_b.float())
+    out = torch.empty(b, n_q, wo.shape[0], dtype=h.dtype, device=dev)
+    idx = torch.empty(b, k, dtype=torch.int64, device=dev)
+    weights = torch.empty(b, k, dtype=f32, device=dev)
+    comb_idx = torch.empty(b, num_shared + k, dtype=torch.int32, device=dev)
+    comb_w = torch.empty(b, num_shared + k, dtype=f32, device=dev)
+    p = L.ptr
+    s = L.DecodeStepDesc(
+        L.RouterShape(b, window, rd, c, top_k, num_shared, routed_scale, L.dtype_code(states.dtype)),
+        L.DecodeShape(b, n_q, num_heads, num_kv_heads, head_dim, num_shared + k, tokens_per_chapter, scale),
+        L.dtype_code(h.dtype), wo.shape[0], kv_bank.shape[0], p(states), p(h), p(w), p(bias), p(wq), p(wo), p(kv_bank), p(idx),
+        p(weights), p(comb_idx), p(comb_w), p(out), None, p(L.status_word(dev)), L.stream_ptr(dev))
+    arena = torch.empty(_size("moc_decode_step_arena_bytes", s), dtype=torch.uint8, device=dev)
+    s.arena = p(arena)
+    L.check(_timed("decode_step", lambda: L.lib().moc_decode_step(C.byref(s))), "moc_decode_step")
+    _report(5 + int(window <= 1024) + 2 * int(window > 1024) + int(h.dtype == f32), lambda: (
+        "router_fwd:" + _TAG_OF_CODE[s.router.h_dtype], "gemm:bf16", "decode_attn:bf16", "gemm:bf16"))
+    return out, idx, weights, comb_idx, comb_w

@@ -1,0 +1,82 @@
+"""The kernels of a decoding step at the edges of their ranges, against the same arithmetic in fp64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-30))
+
+
+@pytest.fixture(scope="module")
+def dev():
+    return torch.device("cuda:0")
+
+
+@pytest.mark.parametrize("b,l,d,c", [(1, 1, 4, 3), (8, 33, 256, 65), (9, 5, 260, 70), (64, 128, 768, 4097), (3, 1024, 1024, 33),
+                                     (17, 40, 1028, 41), (2, 1025, 30, 9)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_router_rows(dev, b, l, d, c, dtype):
+    """Pooling, logits, d_w and d_pooled for few and many rows, widths that fill the register tile or not, both poolings."""
+    from memory_b200 import ops
+    torch.manual_seed(b + d)
+    h = torch.randn(b, l, d, device=dev).to(dtype)
+    w, bias = torch.randn(c, d, device=dev), torch.randn(c, device=dev)
+    f = ops.router_fwd(h, w, bias, 2, 1, 1.0, True)
+    pooled = h.double().mean(1)
+    assert _rel(f["pooled"], pooled) < 1e-6
+    assert _rel(f["logits"], pooled @ w.double().t() + bias.double()) < 1e-6
+    g = torch.randn_like(f["weights"])
+    r = ops.router_bwd((b, l, d), dtype, w, f, 2, 1, 1.0, g, None, torch.ones(4, device=dev), True)
+    dl = r["d_logits"].double()
+    assert _rel(r["d_w"], dl.t() @ f["pooled"].double()) < 1e-5 and _rel(r["d_bias"], dl.sum(0)) < 1e-5
+    assert _rel(r["d_h"], ((dl @ w.double()) / l).unsqueeze(1).expand(b, l, d)) < (1e-5 if dtype == torch.float32 else 5e-3)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 1, 8), (8, 768, 768), (9, 7, 264), (63, 100, 1024), (64, 520, 512), (65, 64, 768), (5, 64, 1032)])
+@pytest.mark.parametrize("out", [torch.float32, torch.bfloat16])
+def test_projection_of_few_rows(dev, m, n, k, out):
+    from memory_b200 import ops
+    torch.manual_seed(m + n)
+    a, w = torch.randn(m, k, device=dev).bfloat16(), torch.randn(n, k, device=dev).bfloat16()
+    y = ops.gemm(a, w, out_dtype=out)
+    assert y.dtype == out and _rel(y, a.double() @ w.double().t()) < (1e-5 if out == torch.float32 else 4e-3)
+
+
+@pytest.mark.parametrize("b,nq,h,hk,t,n_ch", [(1, 1, 12, 12, 64, 65), (1, 1, 4, 1, 5, 3), (2, 3, 6, 2, 33, 4), (1, 1, 1, 1, 1, 1),
+                                              (40, 1, 8, 4, 16, 9), (3, 2, 5, 1, 70, 2)])
+def test_decode_attention_shapes(dev, b, nq, h, hk, t, n_ch):
+    """Clusters of one to eight CTAs, one to four query heads a CTA, chapters that fill no run of 32 rows."""
+    from memory_b200 import ops
+    torch.manual_seed(b + t)
+    c = n_ch + 3
+    q = torch.randn(b, nq, h * 64, device=dev).bfloat16()
+    kv = torch.randn(c * t, 2 * hk * 64, device=dev).bfloat16()
+    idx = torch.stack([torch.randperm(c, device=dev)[:n_ch] for _ in range(b)]).int()
+    u = torch.rand(b, n_ch, device=dev) + 0.1
+    o, lse = ops.decode_attn(q, kv, idx, u, h, hk, t, 0.125, want_lse=True)
+    rows = (idx.long() * t).unsqueeze(-1) + torch.arange(t, device=dev)
+    x = kv[rows.view(b, -1)].double() * u.double().repeat_interleave(t, 1).unsqueeze(-1)
+    k, v = (y.view(b, n_ch * t, hk, 64).repeat_interleave(h // hk, 2) for y in x.chunk(2, dim=-1))
+    s = torch.einsum("bqhd,bkhd->bhqk", q.view(b, nq, h, 64).double(), k) * 0.125
+    want = torch.einsum("bhqk,bkhd->bqhd", s.softmax(-1), v).reshape(b, nq, h * 64)
+    assert _rel(o, want) < 5e-3 and _rel(lse, torch.logsumexp(s, -1).transpose(1, 2)) < 1e-4
+
+
+@pytest.mark.parametrize("dtype,d", [(torch.bfloat16, 768), (torch.float32, 12), (torch.bfloat16, 12)])
+def test_routing_window_is_the_sliced_concatenation(dev, dtype, d):
+    import memory_b200 as M
+    torch.manual_seed(d)
+    prompt = torch.randn(3, 9, d, device=dev).to(dtype)
+    window, want = M.RoutingWindow(6, "hybrid"), prompt[:, -6:]
+    window.prefill(prompt)
+    for n in (1, 2, 1, 7, 6):
+        h = torch.randn(3, n, d, device=dev).to(dtype)
+        want = torch.cat([want, h], 1)[:, -6:]
+        assert torch.equal(window.step(h), want)
+    window = M.RoutingWindow(6, "rolling")
+    want = window.prefill(prompt[:, :2])
+    for n in (1, 2, 3):
+        want = torch.cat([want, prompt[:, :n]], 1)[:, -6:]
+        assert torch.equal(window.step(prompt[:, :n]), want)
