@@ -150,6 +150,26 @@ int moc_route_fwd(const moc_route_desc* s);
 int moc_route_bwd(const moc_route_desc* s, const float* g_weights, const float* g_comb_w, const float* g_losses,
                   void* d_h, float* d_w, float* d_bias, void* scratch);
 
+/* Token-level routing (router.py:262-340) of bf16 states h [rows, hidden_dim]: every token is a routing row.  The fp32 weight
+ * [C, hidden_dim] and the fp32 logit gradients go to the tensor cores as three bf16 terms each.  idx [rows, k'] / weights as
+ * in moc_router_fwd; losses NULL: not computed.  arena holds what the backward pass reads; scratch is free after each call.
+ * Backward: g_weights [rows, k'] / g_losses [4] may be NULL; d_h bf16, d_w, d_bias fp32, NULL: not wanted. */
+typedef struct {
+  int32_t rows, hidden_dim, num_chapters, top_k, num_shared;
+  const void* h;
+  const float *w, *bias;
+  int64_t* idx;
+  float *weights, *losses;
+  void* arena;
+  int32_t* status;
+  void* stream;
+} moc_token_route_desc;
+int64_t moc_token_route_arena_bytes(const moc_token_route_desc* s);
+int64_t moc_token_route_scratch_bytes(const moc_token_route_desc* s, int32_t backward);
+int moc_token_route_fwd(const moc_token_route_desc* s, void* scratch);
+int moc_token_route_bwd(const moc_token_route_desc* s, const float* g_weights, const float* g_losses, void* d_h, float* d_w,
+                        float* d_bias, void* scratch);
+
 /* Position-weighted pooling: pooled[b, :] = sum_t pos_weight[t] * h[b, t, :] (fp32 accumulation), and its
  * backward d_h[b, t, :] (+)= pos_weight[t] * d_pooled[b, :].  With the coefficients of the rolling-window rule this
  * replaces ChapterRouter._sequence_rolling_pool (memory_transformer/router.py:159-195): the average over t of the
@@ -281,7 +301,9 @@ int moc_scatter_bank_grad(const float* bank_grad, const int32_t* uniq, const int
  * (fp32 C only, C must be pre-zeroed or accumulate set).
  * residual (device fp32 [M,N], row stride ldr, may be NULL): added to the product before it is stored,
  * C = row_scale * (A B) + residual -- the residual add that follows the output projection in the
- * reference's block (memory_block.py:558) done in the projection's epilogue. */
+ * reference's block (memory_block.py:558) done in the projection's epilogue.
+ * terms > 1 (bf16 kernel): C = sum over t of op(A_t) op(B_t), all in one accumulator, the last term first; A_t / B_t start
+ * t * a_term_rows / b_term_rows stored rows behind A / B (0: the same operand in every term). */
 typedef struct {
   int32_t dtype, c_dtype;
   int32_t m, n, k;
@@ -293,6 +315,7 @@ typedef struct {
   int64_t a_stored_rows;   /* rows of the stored A when a gather list is used */
   const float* residual;
   int64_t ldr;
+  int32_t terms, a_term_rows, b_term_rows;
 } moc_gemm_desc;
 
 int moc_gemm(const moc_gemm_desc* g, const void* a, const void* b, void* c, const float* row_scale,

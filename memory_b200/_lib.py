@@ -34,7 +34,8 @@ class GemmDesc(C.Structure):
                 ("lda", C.c_int64), ("ldb", C.c_int64), ("ldc", C.c_int64),
                 ("accumulate", C.c_int32), ("split_k", C.c_int32), ("scale_block_rows", C.c_int32),
                 ("a_block_rows", C.c_int32), ("a_stored_rows", C.c_int64),
-                ("residual", C.c_void_p), ("ldr", C.c_int64)]
+                ("residual", C.c_void_p), ("ldr", C.c_int64),
+                ("terms", C.c_int32), ("a_term_rows", C.c_int32), ("b_term_rows", C.c_int32)]
 
 
 class AttnShape(C.Structure):
@@ -68,6 +69,10 @@ def _fields(spec: str):
 class RouteDesc(C.Structure):
     _fields_ = [("shape", RouterShape)] + _fields(
         "p: h w bias pos_weight idx weights comb_idx comb_w losses arena status stream")
+
+
+class TokenRouteDesc(C.Structure):
+    _fields_ = _fields("i: rows hidden_dim num_chapters top_k num_shared; p: h w bias idx weights losses arena status stream")
 
 
 class DecodeStepDesc(C.Structure):
@@ -161,6 +166,10 @@ _PROTOTYPES = {
     "moc_route_bwd_scratch_bytes": (C.c_int64, [C.POINTER(RouteDesc)]),
     "moc_route_fwd": (C.c_int, [C.POINTER(RouteDesc)]),
     "moc_route_bwd": (C.c_int, [C.POINTER(RouteDesc), P, P, P, P, P, P, P]),
+    "moc_token_route_arena_bytes": (C.c_int64, [C.POINTER(TokenRouteDesc)]),
+    "moc_token_route_scratch_bytes": (C.c_int64, [C.POINTER(TokenRouteDesc), C.c_int32]),
+    "moc_token_route_fwd": (C.c_int, [C.POINTER(TokenRouteDesc), P]),
+    "moc_token_route_bwd": (C.c_int, [C.POINTER(TokenRouteDesc), P, P, P, P, P, P]),
     "moc_chapter_lists": (C.c_int, [P, C.c_int32, C.c_int32, C.c_int32, P, P, P]),
     "moc_loss_total": (C.c_int, [P, P, C.c_float, C.c_float, C.c_float, C.c_float, P, P]),
     "moc_sparse_attn_tc_sizes": (C.c_int, [C.POINTER(SparseAttnShape), P, P, P]),

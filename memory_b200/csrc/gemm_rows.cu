@@ -1,7 +1,7 @@
 // Projection of a few rows, C [M <= 64, N] = A [M, K] W [N, K]^T with bf16 operands and fp32 accumulation: the query and
 // output projections of a decoding step.  A 128-row tensor-core tile would leave all but a few SMs idle behind one serial
 // chain of K steps (10 us at K 768 whatever M is); bound by latency, the work goes to a warp per column and eight rows, with
-// the weight row in registers and the sums of the eight rows reduced together.  768 x 768: 9.5 -> 2.5 us for one row, 11 -> 4
+// the weight row in registers and the sums of the eight rows reduced together.  768 x 768: 9.5 -> 2.5 us for one row, 11 -> 10
 // for 64.
 #include "moc_common.cuh"
 
@@ -84,10 +84,11 @@ gemm_rows_kernel(const __nv_bfloat16* __restrict__ a, long long lda, const __nv_
 }  // namespace
 
 // Whether the kernel takes this projection: plain operands, rows of at most 1,024 (32 registers of operands a lane and row),
-// and at most 64 of them, beyond which the tensor-core tiles are as fast.
+// and few enough of them: the work grows with M N while the tensor-core tiles stay at the length of their K chain until N
+// fills the chip (64 x 1,536: 16 us here, 10 there).
 bool gemm_rows_supported(const moc_gemm_desc* g, const float* row_scale, const int32_t* a_row_blocks,
                          const int32_t* b_row_blocks) {
-  return g->m <= 64 && g->k <= 1024 && g->a_kmajor && g->b_kmajor && !g->accumulate && g->split_k <= 1 &&
+  return g->m <= 64 && static_cast<long long>(g->m) * g->n <= 64 * 1024 && g->k <= 1024 && g->a_kmajor && g->b_kmajor && !g->accumulate && g->split_k <= 1 && g->terms <= 1 &&
          g->residual == nullptr && row_scale == nullptr && a_row_blocks == nullptr && b_row_blocks == nullptr;
 }
 int launch_gemm_rows(const moc_gemm_desc* g, const void* a, const void* b, void* c, cudaStream_t stream) {

@@ -57,6 +57,8 @@ struct GemmTcParams {
   int b_num_blocks;
   long long b_stored_rows;
   int k_tiles_total;
+  int k_tiles_per_term, terms; // the K range of one term and the number of terms (see moc_gemm_desc)
+  int a_term_rows, b_term_rows;
   int k_tiles_per_split;
   int splits;
   int m_tiles, n_tiles;
@@ -184,24 +186,30 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           mbar_arrive_expect_tx(&full_bar[s], C::kStageBytes);
           uint8_t* a_s = tiles + s * C::kStageBytes;
           uint8_t* b_s = a_s + C::kABytes;
-          const int k0 = (kt_begin + kt) * BK;
+          int k0 = (kt_begin + kt) * BK, a_off = 0, b_off = 0;
+          if (p.terms > 1) {                                   // the last term first
+            const int t = (kt_begin + kt) / p.k_tiles_per_term;
+            k0 -= t * p.k_tiles_per_term * BK;
+            a_off = (p.terms - 1 - t) * p.a_term_rows;
+            b_off = (p.terms - 1 - t) * p.b_term_rows;
+          }
           if (p.a_kmajor) {
             for (int i = 0; i < nbox_a; ++i) {
-              const int row = (p.a_row_blocks != nullptr) ? a_rows[i] : m0 + i * p.a_box_rows;
+              const int row = (p.a_row_blocks != nullptr) ? a_rows[i] : m0 + i * p.a_box_rows + a_off;
               tma_load_2d(a_s + i * p.a_box_rows * 128, &tmap_a, &full_bar[s], k0, row);
             }
           } else {
 #pragma unroll
-            for (int i = 0; i < 2 * MT; ++i) tma_load_2d(a_s + i * 8192, &tmap_a, &full_bar[s], m0 + 64 * i, k0);
+            for (int i = 0; i < 2 * MT; ++i) tma_load_2d(a_s + i * 8192, &tmap_a, &full_bar[s], m0 + 64 * i, k0 + a_off);
           }
           if (p.b_kmajor) {
 #pragma unroll
             for (int j = 0; j < BN / 128; ++j)
-              tma_load_2d(b_s + j * 16384, &tmap_b, &full_bar[s], k0, n0 + j * 128);
+              tma_load_2d(b_s + j * 16384, &tmap_b, &full_bar[s], k0, n0 + j * 128 + b_off);
           } else if (p.b_row_blocks == nullptr) {
 #pragma unroll
             for (int j = 0; j < BN / 64; ++j)
-              tma_load_2d(b_s + j * 8192, &tmap_b, &full_bar[s], n0 + j * 64, k0);
+              tma_load_2d(b_s + j * 8192, &tmap_b, &full_bar[s], n0 + j * 64, k0 + b_off);
           } else {
             // the K rows of this stage are rows of listed blocks (chapters of the bank): one box per run of rows
             // that is contiguous in the stored matrix
@@ -487,6 +495,12 @@ int launch_gemm_tc(const moc_gemm_desc* g, const void* a, const void* b, void* c
     b_num_blocks = g->k / b_block_rows;
   }
 
+  const int terms = g->terms > 1 ? g->terms : 1;
+  MOC_REQUIRE(terms == 1 || (a_row_blocks == nullptr && b_row_blocks == nullptr && g->a_term_rows >= 0 && g->b_term_rows >= 0),
+              "operands in terms take no gather list");
+  const uint64_t a_more = static_cast<uint64_t>(terms - 1) * static_cast<uint64_t>(terms > 1 ? g->a_term_rows : 0);
+  const uint64_t b_more = static_cast<uint64_t>(terms - 1) * static_cast<uint64_t>(terms > 1 ? g->b_term_rows : 0);
+
   // Tile width.  The kernel is fed from L2 (~8.4 TB/s measured over all SMs), so a tile's time goes with the
   // bytes it loads per K step, (BM + BN) * 128: the cost of a width is rounds-of-items times that.
   const int sms = sm_count();
@@ -509,21 +523,21 @@ int launch_gemm_tc(const moc_gemm_desc* g, const void* a, const void* b, void* c
   CUtensorMap tmap_a, tmap_b;
   int rc;
   if (g->a_kmajor) {
-    rc = make_tmap_bf16_2d(&tmap_a, a, static_cast<uint64_t>(a_stored_rows), static_cast<uint64_t>(g->k),
+    rc = make_tmap_bf16_2d(&tmap_a, a, static_cast<uint64_t>(a_stored_rows) + a_more, static_cast<uint64_t>(g->k),
                            static_cast<uint64_t>(g->lda), static_cast<uint32_t>(a_box_rows), 64);
   } else {
-    rc = make_tmap_bf16_2d(&tmap_a, a, static_cast<uint64_t>(g->k), static_cast<uint64_t>(g->m),
+    rc = make_tmap_bf16_2d(&tmap_a, a, static_cast<uint64_t>(g->k) + a_more, static_cast<uint64_t>(g->m),
                            static_cast<uint64_t>(g->lda), 64, 64);
   }
   if (rc != MOC_OK) return rc;
   if (g->b_kmajor) {
-    rc = make_tmap_bf16_2d(&tmap_b, b, static_cast<uint64_t>(g->n), static_cast<uint64_t>(g->k),
+    rc = make_tmap_bf16_2d(&tmap_b, b, static_cast<uint64_t>(g->n) + b_more, static_cast<uint64_t>(g->k),
                            static_cast<uint64_t>(g->ldb), 128, 64);
   } else if (b_row_blocks != nullptr) {
     rc = make_tmap_bf16_2d(&tmap_b, b, static_cast<uint64_t>(b_stored_rows), static_cast<uint64_t>(g->n),
                            static_cast<uint64_t>(g->ldb), static_cast<uint32_t>(b_box_rows), 64);
   } else {
-    rc = make_tmap_bf16_2d(&tmap_b, b, static_cast<uint64_t>(g->k), static_cast<uint64_t>(g->n),
+    rc = make_tmap_bf16_2d(&tmap_b, b, static_cast<uint64_t>(g->k) + b_more, static_cast<uint64_t>(g->n),
                            static_cast<uint64_t>(g->ldb), 64, 64);
   }
   if (rc != MOC_OK) return rc;
@@ -548,7 +562,9 @@ int launch_gemm_tc(const moc_gemm_desc* g, const void* a, const void* b, void* c
   p.a_stored_rows = a_stored_rows;
   p.b_row_blocks = b_row_blocks; p.b_block_rows = b_block_rows; p.b_box_rows = b_box_rows;
   p.b_num_blocks = b_num_blocks; p.b_stored_rows = b_stored_rows;
-  p.k_tiles_total = ceil_div(g->k, BK);
+  p.terms = terms; p.k_tiles_per_term = ceil_div(g->k, BK);
+  p.a_term_rows = g->a_term_rows; p.b_term_rows = g->b_term_rows;
+  p.k_tiles_total = terms * p.k_tiles_per_term;
   p.k_tiles_per_split = ceil_div(p.k_tiles_total, split);
   p.splits = ceil_div(p.k_tiles_total, p.k_tiles_per_split);   // no empty splits
   p.m_tiles = tall ? ceil_div(g->m, 2 * BM) : m_tiles;

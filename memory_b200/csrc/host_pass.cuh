@@ -42,6 +42,7 @@ struct Gemm : moc_gemm_desc {
     accumulate = 0; split_k = 1; scale_block_rows = 1; a_block_rows = 0;
     a_stored_rows = a_k ? m : k;
     residual = nullptr; ldr = 0;
+    terms = 1; a_term_rows = b_term_rows = 0;
   }
 };
 // K-splits of a weight gradient [out_rows, out_cols] over `rows`: enough (tile, split) items to fill the SMs once

@@ -8,19 +8,24 @@
 
 #include <type_traits>
 
-#include "moc_common.cuh"
+#include "host_pass.cuh"
 
 namespace moc {
 namespace {
 
 constexpr int kPoolSplits = 32;       // sequence splits of the mean-pool
-constexpr int kSelectThreads = 1024;  // one CTA per batch row in the select / dlogits kernels
 constexpr int kLossChunk = 256;       // chapters per CTA in the loss kernels
 constexpr int kDpChunk = 16;          // chapters per CTA in the d_pooled kernel
 
 template <typename T> __device__ __forceinline__ float to_f32(T v);
 template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
+
+// x / d for many x and one d, r = 1 / d: the quotient of the rounded reciprocal, corrected by its remainder (Markstein)
+__device__ __forceinline__ float quotient(float x, float d, float r) {
+  const float q = x * r;
+  return fmaf(fmaf(-q, d, x), r, q);
+}
 
 // ---- block reductions (fixed order) ----------------------------------------------------------
 __device__ __forceinline__ float block_sum(float v, float* red) {
@@ -316,12 +321,13 @@ __global__ void logits_kernel(const float* __restrict__ pooled, const float* __r
 }
 
 // One CTA per batch row: softmax, prefix mask + renormalise, exact top-k, weights, shared prefix.  NV: values per thread
-// (rows of up to 1,024 NV chapters), 0 for longer rows.  Bound by its chain of block-wide steps on one SM: at 4,097
-// chapters, k 64, 16 -> 12 us for a few rows and 392 -> 252 us for 8,192 against four radix passes over shared memory.
-constexpr int kBinThreads = 512, kBinBits = 10, kCand = 512;
-template <int NV>
-__global__ void __launch_bounds__(kSelectThreads)
-select_kernel(const float* __restrict__ logits, float* __restrict__ probs, long long* __restrict__ idx,
+// (rows of up to TH NV chapters), 0 for longer rows.  Bound by its chain of block-wide steps: at 4,097 chapters, k 64, 16 ->
+// 10 us for a few rows with TH 1,024 against four radix passes over shared memory.  Thousands of rows take CTAs of 256
+// threads, whose barriers are shorter and chains more: 8,192 rows, k 16: 252 us with TH 1,024 -> 152.
+constexpr int kBins = 512, kBinBits = 9, kCand = 512;
+template <int NV, int TH>
+__global__ void __launch_bounds__(TH)
+select_kernel(const float* __restrict__ logits, long long ld, const float* __restrict__ bias, float* __restrict__ probs, long long* __restrict__ idx,
               float* __restrict__ weights, int* __restrict__ comb_idx, float* __restrict__ comb_w,
               float* __restrict__ row_stats, int C, int k_sel, int S, float rho) {
   extern __shared__ float sm[];            // [C] masked probabilities, then selection scratch
@@ -332,11 +338,12 @@ select_kernel(const float* __restrict__ logits, float* __restrict__ probs, long 
   __shared__ int hist[256];
   __shared__ uint32_t s_prefix;
   __shared__ int s_krem, s_count, s_ties;
-  __shared__ int bins[NV > 0 ? 2 * kBinThreads : 1], wsum[16], cand_idx[NV > 0 ? kCand : 1];
+  __shared__ int bins[NV > 0 ? kBins : 1], wsum[32], cand_idx[NV > 0 ? kCand : 1];
   __shared__ uint32_t mm[64], cand_key[NV > 0 ? kCand : 1];
 
   const int b = blockIdx.x;
-  const float* z = logits + static_cast<long long>(b) * C;
+  const float* z = logits + b * ld;       // (bias: not yet in the logits, or nullptr)
+  auto logit = [&](int c) { return bias != nullptr ? z[c] + bias[c] : z[c]; };
   float* p = probs + static_cast<long long>(b) * C;
 
   // NV > 0: the row's values stay in registers between the passes (c = threadIdx.x + i * blockDim.x), and the shared copy
@@ -347,34 +354,40 @@ select_kernel(const float* __restrict__ logits, float* __restrict__ probs, long 
   if constexpr (NV > 0) {
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      const int c = threadIdx.x + i * kSelectThreads;
-      v[i] = c < C ? z[c] : -INFINITY;
-      m = fmaxf(m, v[i]);
+      const int c = threadIdx.x + i * TH;     // (all loads first: they are independent)
+      v[i] = z[min(c, C - 1)];
     }
+    if (bias != nullptr) {
+#pragma unroll
+      for (int i = 0; i < NV; ++i) v[i] += bias[min(static_cast<int>(threadIdx.x) + i * TH, C - 1)];
+    }
+#pragma unroll
+    for (int i = 0; i < NV; ++i) m = fmaxf(m, v[i]);       // (a repeated last entry changes no maximum)
   } else {
-    for (int c = threadIdx.x; c < C; c += blockDim.x) m = fmaxf(m, z[c]);
+    for (int c = threadIdx.x; c < C; c += blockDim.x) m = fmaxf(m, logit(c));
   }
   m = block_max(m, red);
   float s = 0.f;
   if constexpr (NV > 0) {
 #pragma unroll
     for (int i = 0; i < NV; ++i)
-      if (threadIdx.x + i * kSelectThreads < C) { v[i] = expf(v[i] - m); s += v[i]; }
+      if (threadIdx.x + i * TH < C) { v[i] = expf(v[i] - m); s += v[i]; }
   } else {
     for (int c = threadIdx.x; c < C; c += blockDim.x) {
-      const float e = expf(z[c] - m);
+      const float e = expf(logit(c) - m);
       pt[c] = e;
       s += e;
     }
   }
   const float denom = block_sum(s, red);
+  const float r_denom = 1.f / denom;
   float ms = 0.f;
   if constexpr (NV > 0) {
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      const int c = threadIdx.x + i * kSelectThreads;
+      const int c = threadIdx.x + i * TH;
       if (c < C) {
-        const float pv = v[i] / denom;
+        const float pv = quotient(v[i], denom, r_denom);
         p[c] = pv;
         v[i] = (c < S) ? 0.f : pv;
         ms += v[i];
@@ -392,9 +405,11 @@ select_kernel(const float* __restrict__ logits, float* __restrict__ probs, long 
   const float masked_mass = block_sum(ms, red);
   const float dn0 = fmaxf(masked_mass, 1e-12f);
   if constexpr (NV > 0) {
-    if (S > 0)
+    if (S > 0) {
+      const float r_dn0 = 1.f / dn0;
 #pragma unroll
-      for (int i = 0; i < NV; ++i) v[i] = v[i] / dn0;
+      for (int i = 0; i < NV; ++i) v[i] = quotient(v[i], dn0, r_dn0);
+    }
   } else {
     if (S > 0)
       for (int c = threadIdx.x; c < C; c += blockDim.x) pt[c] = pt[c] / dn0;
@@ -403,85 +418,81 @@ select_kernel(const float* __restrict__ logits, float* __restrict__ probs, long 
 
   float topk_mass = 0.f, comb_mass = static_cast<float>(S);
   if (k_sel > 0) {
+    float* srt_w = sm;                         // sorted: weight and id, over p~ (no longer needed by then)
+    int* srt_i = reinterpret_cast<int*>(sm + k_sel);
     bool selected = false;
     if constexpr (NV > 0) {
-      // Probabilities of one row share their leading bits, so a radix pass over them piles up in a few bins (and in their
-      // atomics: 4,096 of them serialised).  One histogram over the row's own range instead: the bins above the one in
-      // which the running count reaches k are selected, the few entries of that bin are ranked.
+      // At least k values are as large as the k-th largest of the threads' own maxima, and few more: a histogram of the TH
+      // maxima over their range (one atomic per thread; the probabilities of one row share their leading bits, so radix
+      // passes over all of them pile up in a few bins) gives a bound, and what lies above it is ranked.
       const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-      uint32_t lo = 0xFFFFFFFFu, hi = 0u;
+      constexpr int kPer = kBins / TH > 2 ? kBins / TH : 2, kOwners = kBins / kPer, kWarps = TH / 32;
+      uint32_t top = 0u;
 #pragma unroll
       for (int i = 0; i < NV; ++i) {
-        const int c = threadIdx.x + i * kSelectThreads;
-        if (c < C && c >= S) { lo = min(lo, __float_as_uint(v[i])); hi = max(hi, __float_as_uint(v[i])); }
+        const int c = threadIdx.x + i * TH;
+        if (c < C && c >= S) top = max(top, __float_as_uint(v[i]));
       }
-      lo = __reduce_min_sync(0xffffffffu, lo);
-      hi = __reduce_max_sync(0xffffffffu, hi);
-      if (threadIdx.x < 2 * kBinThreads) bins[threadIdx.x] = 0;
+      uint32_t lo = __reduce_min_sync(0xffffffffu, top), hi = __reduce_max_sync(0xffffffffu, top);
+      for (int i = threadIdx.x; i < kBins; i += TH) bins[i] = 0;
       if (lane == 0) { mm[warp] = lo; mm[32 + warp] = hi; }
-      if (threadIdx.x == 0) { s_count = 0; s_ties = 0; s_prefix = 0u; }
+      if (threadIdx.x == 0) { s_count = 0; s_prefix = 0u; }
       __syncthreads();
-      lo = __reduce_min_sync(0xffffffffu, mm[lane]);
-      hi = __reduce_max_sync(0xffffffffu, mm[32 + lane]);
+      lo = __reduce_min_sync(0xffffffffu, lane < kWarps ? mm[lane] : 0xFFFFFFFFu);
+      hi = __reduce_max_sync(0xffffffffu, lane < kWarps ? mm[32 + lane] : 0u);
       const int sh = max(0, 32 - __clz(hi - lo) - kBinBits);
-      auto bin_of = [&](float x) {
-        const uint32_t key = __float_as_uint(x);
-        return key <= lo ? 0u : (key - lo) >> sh;
-      };
+      if (k_sel <= TH / 2) {
+        atomicAdd(&bins[(top - lo) >> sh], 1);
+        __syncthreads();
+        // an owner has kPer bins, from the top down; the one whose bin reaches k publishes it
+        if (threadIdx.x < kOwners) {
+          const int first = kBins - 1 - kPer * static_cast<int>(threadIdx.x);
+          int h[kPer], incl = 0;
 #pragma unroll
-      for (int i = 0; i < NV; ++i)
-        if (threadIdx.x + i * kSelectThreads < C) atomicAdd(&bins[bin_of(v[i])], 1);
-      __syncthreads();
-      // thread t < 512 owns two bins, from the top down; the owner of the bin that reaches k publishes it
-      if (threadIdx.x < kBinThreads) {
-        const int top = 2 * (kBinThreads - 1 - static_cast<int>(threadIdx.x));
-        const int h1 = bins[top + 1], h0 = bins[top];
-        int incl = h0 + h1;
+          for (int i = 0; i < kPer; ++i) { h[i] = bins[first - i]; incl += h[i]; }
+          const int mine = incl;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int t = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += t;
-        }
-        if (lane == 31) wsum[warp] = incl;
-        asm volatile("bar.sync 1, 512;" ::: "memory");
-        int before = 0;
-        for (int w = 0; w < warp; ++w) before += wsum[w];
-        const int above = before + incl - h0 - h1;
-        if (above < k_sel && k_sel <= above + h1) { s_prefix = top + 1; s_krem = k_sel - above; }
-        else if (above + h1 < k_sel && k_sel <= above + h1 + h0) { s_prefix = top; s_krem = k_sel - above - h1; }
-      }
-      __syncthreads();
-      const uint32_t tb = s_prefix;
-      const int need = s_krem, in_bin = bins[tb];
-      // (bin 0 also holds the masked chapters; a crowded bin is better left to the radix select)
-      if (tb > 0u && in_bin <= kCand) {
+          for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+          }
+          if (lane == 31) wsum[warp] = incl;
+          asm volatile("bar.sync 1, %0;" ::"n"(kOwners) : "memory");
+          int above = incl - mine;
+          for (int w = 0; w < warp; ++w) above += wsum[w];
 #pragma unroll
-        for (int i = 0; i < NV; ++i) {
-          const int c = threadIdx.x + i * kSelectThreads;
-          if (c < C) {
-            const uint32_t bn = bin_of(v[i]);
-            if (bn > tb) {
-              const int pos = atomicAdd(&s_count, 1);
-              sel_key[pos] = __float_as_uint(v[i]); sel_idx[pos] = c;
-            } else if (bn == tb) {
-              const int pos = atomicAdd(&s_ties, 1);
-              cand_key[pos] = __float_as_uint(v[i]); cand_idx[pos] = c;
-            }
+          for (int i = 0; i < kPer; ++i) {
+            if (above < k_sel && k_sel <= above + h[i]) s_prefix = first - i;
+            above += h[i];
           }
         }
         __syncthreads();
-        for (int t = threadIdx.x; t < in_bin; t += kSelectThreads) {
-          const uint32_t kt = cand_key[t];
-          const int it = cand_idx[t];
-          int rank = 0;
-          for (int j = 0; j < in_bin; ++j) rank += (cand_key[j] > kt) || (cand_key[j] == kt && cand_idx[j] < it);
-          if (rank < need) { sel_key[k_sel - need + rank] = kt; sel_idx[k_sel - need + rank] = it; }
+        const uint32_t edge = lo + (s_prefix << sh);
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+          const int c = threadIdx.x + i * TH;
+          if (c < C && c >= S && __float_as_uint(v[i]) >= edge) {
+            const int pos = atomicAdd(&s_count, 1);
+            if (pos < kCand) { cand_key[pos] = __float_as_uint(v[i]); cand_idx[pos] = c; }
+          }
         }
-        selected = true;
-      } else {
+        __syncthreads();
+        const int n = s_count;
+        if (n >= k_sel && n <= kCand) {
+          for (int t = threadIdx.x; t < n; t += TH) {
+            const uint32_t kt = cand_key[t];
+            const int it = cand_idx[t];
+            int rank = 0;
+            for (int j = 0; j < n; ++j) rank += (cand_key[j] > kt) || (cand_key[j] == kt && cand_idx[j] < it);
+            if (rank < k_sel) { srt_w[rank] = __uint_as_float(kt); srt_i[rank] = it; }
+          }
+          selected = true;
+        }
+      }
+      if (!selected) {
 #pragma unroll
         for (int i = 0; i < NV; ++i)
-          if (threadIdx.x + i * kSelectThreads < C) pt[threadIdx.x + i * kSelectThreads] = v[i];
+          if (threadIdx.x + i * TH < C) pt[threadIdx.x + i * TH] = v[i];
       }
       __syncthreads();
     }
@@ -553,13 +564,12 @@ select_kernel(const float* __restrict__ logits, float* __restrict__ probs, long 
       }
     }
     __syncthreads();
-    }
     // rank sort of the k selected entries: value descending, chapter id ascending (shared memory)
-    float* srt_w = sm;                         // p~ is no longer needed: reuse its first 2k words
-    int* srt_i = reinterpret_cast<int*>(sm + k_sel);
-    uint32_t kt_reg[1]; int it_reg[1]; int rk_reg[1];
-    {
-      const int t = threadIdx.x;
+    constexpr int kMine = 1024 / TH;           // k_sel <= 1024
+    uint32_t kt_reg[kMine]; int it_reg[kMine]; int rk_reg[kMine];
+#pragma unroll
+    for (int q = 0; q < kMine; ++q) {
+      const int t = threadIdx.x + q * TH;
       if (t < k_sel) {
         const uint32_t kt = sel_key[t];
         const int it = sel_idx[t];
@@ -568,12 +578,15 @@ select_kernel(const float* __restrict__ logits, float* __restrict__ probs, long 
           const uint32_t kj = sel_key[j];
           rank += (kj > kt) || (kj == kt && sel_idx[j] < it);
         }
-        kt_reg[0] = kt; it_reg[0] = it; rk_reg[0] = rank;
+        kt_reg[q] = kt; it_reg[q] = it; rk_reg[q] = rank;
       }
     }
     __syncthreads();
-    if (threadIdx.x < k_sel) { srt_w[rk_reg[0]] = __uint_as_float(kt_reg[0]); srt_i[rk_reg[0]] = it_reg[0]; }
+#pragma unroll
+    for (int q = 0; q < kMine; ++q)
+      if (threadIdx.x + q * TH < k_sel) { srt_w[rk_reg[q]] = __uint_as_float(kt_reg[q]); srt_i[rk_reg[q]] = it_reg[q]; }
     __syncthreads();
+    }
     float part = 0.f;
     for (int j = threadIdx.x; j < k_sel; j += blockDim.x) part += srt_w[j];
     topk_mass = block_sum(part, red);
@@ -597,6 +610,7 @@ select_kernel(const float* __restrict__ logits, float* __restrict__ probs, long 
     int ci; float u;
     if (j < S) { ci = j; u = 1.f; }
     else { ci = reinterpret_cast<int*>(sm + k_sel)[j - S]; u = sm[j - S] * (S > 0 ? rho : 1.f); }
+    if (comb_idx == nullptr) break;        // (uniform: a caller of token rows has no use for the joint list)
     comb_idx[static_cast<long long>(b) * kc + j] = ci;
     comb_w[static_cast<long long>(b) * kc + j] = (S > 0) ? u / fmaxf(comb_mass, 1e-12f) : u;
   }
@@ -742,12 +756,6 @@ __global__ void loss_total_kernel(const float* __restrict__ losses, const float*
   }
 }
 
-// logits[r, c] += bias[c]
-__global__ void add_bias_kernel(float* __restrict__ logits, const float* __restrict__ bias, long long total, int C) {
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x)
-    logits[i] += bias[static_cast<int>(i % C)];
-}
 // dst[r, c] = bias[c] + sum_t src[r, t * ld + c], smallest term (highest t) first
 __global__ void sum_terms_kernel(const float* __restrict__ src, const float* __restrict__ bias,
                                  float* __restrict__ dst, long long rows, int cols, int ld, int terms) {
@@ -762,13 +770,49 @@ __global__ void sum_terms_kernel(const float* __restrict__ src, const float* __r
     dst[i] = bias != nullptr ? acc + bias[c] : acc;
   }
 }
+// partial[chunk][c] = sum over the chunk's rows of the three terms of column c: 32 groups of eight 16-byte pieces
+constexpr int kTermRows = 256;
+__global__ void __launch_bounds__(256)
+term_col_sum_kernel(const __nv_bfloat16* __restrict__ terms, float* __restrict__ partial, int rows, int ld) {
+  __shared__ float red[32][65];
+  const int piece = threadIdx.x & 7, g = threadIdx.x >> 3;
+  const int c = blockIdx.x * 64 + piece * 8, r0 = blockIdx.y * kTermRows;
+  float acc[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+  if (c < ld) {
+#pragma unroll 4
+    for (int r = r0 + g; r < min(rows, r0 + kTermRows); r += 32) {
+#pragma unroll
+      for (int t = 2; t >= 0; --t) {
+        const uint4 v = *reinterpret_cast<const uint4*>(terms + (static_cast<long long>(t) * rows + r) * ld + c);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          acc[2 * j] += __uint_as_float(w[j] << 16);
+          acc[2 * j + 1] += __uint_as_float(w[j] & 0xFFFF0000u);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) red[g][piece * 8 + j] = acc[j];
+  __syncthreads();
+  const int col = blockIdx.x * 64 + threadIdx.x;
+  if (threadIdx.x < 64 && col < ld) {
+    float t = 0.f;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) t += red[i][threadIdx.x];
+    partial[static_cast<long long>(blockIdx.y) * ld + col] = t;
+  }
+}
 // out[c] = sum_r x[r, c]: one CTA per 32 columns, 8 row groups, fixed-order sums
-__global__ void col_sum_kernel(const float* __restrict__ x, float* __restrict__ out, long long rows, int cols) {
+__global__ void col_sum_kernel(const float* __restrict__ x, float* __restrict__ out, long long rows, int cols, int ld) {
   __shared__ float part[8][32];
   const int c = blockIdx.x * 32 + (threadIdx.x & 31), g = threadIdx.x >> 5;
   float acc = 0.f;
   if (c < cols)
-    for (long long r = g; r < rows; r += 8) acc += x[r * cols + c];
+    for (long long r = g; r < rows; r += 8) acc += x[r * ld + c];
   part[g][threadIdx.x & 31] = acc;
   __syncthreads();
   if (g == 0 && c < cols) {
@@ -781,12 +825,17 @@ __global__ void col_sum_kernel(const float* __restrict__ x, float* __restrict__ 
 
 // ---- backward --------------------------------------------------------------------------------
 // One CTA per batch row: gradient of everything downstream of the logits.
-__global__ void __launch_bounds__(kSelectThreads)
+// One CTA per row; terms != nullptr: the gradient leaves as three bf16 terms ([3][B][ld], zeros behind column C), what the
+// products that follow on the tensor cores read.
+// NV > 0: the row's probabilities stay in registers (rows of up to TH NV chapters), all loads in flight together.  8,192 rows
+// of 4,097: 227 us with TH 1,024, a pad copy of 93 us and a pass of 133 us into the terms -> 147 us in all.
+template <int NV, int TH>
+__global__ void __launch_bounds__(TH)
 dlogits_kernel(const float* __restrict__ probs, const long long* __restrict__ idx,
                const float* __restrict__ weights, const float* __restrict__ comb_w,
                const float* __restrict__ row_stats, const float* __restrict__ chapter_stats,
                const float* __restrict__ d_weights, const float* __restrict__ d_comb_w,
-               const float* __restrict__ d_losses, float* __restrict__ d_logits,
+               const float* __restrict__ d_losses, float* __restrict__ d_logits, __nv_bfloat16* __restrict__ terms, int ld,
                int B, int C, int k_sel, int S, float rho) {
   extern __shared__ float dp[];   // [C]
   __shared__ float red[33];
@@ -800,6 +849,16 @@ dlogits_kernel(const float* __restrict__ probs, const long long* __restrict__ id
   const float g_z = d_losses ? d_losses[2] : 0.f, g_ent = d_losses ? d_losses[3] : 0.f;
   const int kc = S + k_sel;
 
+  float pr[NV > 0 ? NV : 1];
+  // terms go out in pairs of columns, so a thread owns pairs; single columns otherwise
+  constexpr int kN = NV > 0 ? NV : 1;
+  auto col = [&](int i) {
+    return terms != nullptr ? 2 * static_cast<int>(threadIdx.x) + (i & 1) + (i >> 1) * 2 * TH : static_cast<int>(threadIdx.x) + i * TH;
+  };
+  if constexpr (NV > 0) {
+#pragma unroll
+    for (int i = 0; i < kN; ++i) pr[i] = p[min(col(i), C - 1)];
+  }
   // (a)+(b): gradients of the k selected (unnormalised) masked probabilities v_j
   __shared__ float s_w[1024];
   float dotu_p = 0.f;
@@ -835,13 +894,20 @@ dlogits_kernel(const float* __restrict__ probs, const long long* __restrict__ id
   const float inv_s = renorm ? ((s_mass >= 1e-12f) ? 1.f / s_mass : 1e12f) : 1.f;
   const float dense = (renorm && s_mass >= 1e-12f) ? -A * inv_s : 0.f;
   const float invB = 1.f / static_cast<float>(B), invC = 1.f / static_cast<float>(C);
-  for (int c = threadIdx.x; c < C; c += blockDim.x) {
-    const float pv = p[c];
+  auto dense_grad = [&](int c, float pv) {
     float g = (c >= S) ? dense : 0.f;
-    g += g_lb * static_cast<float>(C) * chapter_stats[c] * invB;
-    g += g_aux * (2.f * invC) * (chapter_stats[C + c] - invC) * (2.f * pv * invB);
-    g += g_ent * (-invB) * (logf(fmaxf(pv, 1e-12f)) + (pv > 1e-12f ? 1.f : 0.f));
-    dp[c] = g;
+    // (a loss without a gradient costs nothing, and its statistics may not have been computed)
+    if (g_lb != 0.f) g += g_lb * static_cast<float>(C) * chapter_stats[c] * invB;
+    if (g_aux != 0.f) g += g_aux * (2.f * invC) * (chapter_stats[C + c] - invC) * (2.f * pv * invB);
+    if (g_ent != 0.f) g += g_ent * (-invB) * (logf(fmaxf(pv, 1e-12f)) + (pv > 1e-12f ? 1.f : 0.f));
+    return g;
+  };
+  if constexpr (NV > 0) {
+#pragma unroll
+    for (int i = 0; i < kN; ++i)
+      if (col(i) < C) dp[col(i)] = dense_grad(col(i), pr[i]);
+  } else {
+    for (int c = threadIdx.x; c < C; c += blockDim.x) dp[c] = dense_grad(c, p[c]);
   }
   __syncthreads();
   for (int j = threadIdx.x; j < k_sel; j += blockDim.x) {
@@ -850,11 +916,45 @@ dlogits_kernel(const float* __restrict__ probs, const long long* __restrict__ id
   }
   __syncthreads();
   float dot = 0.f;
-  for (int c = threadIdx.x; c < C; c += blockDim.x) dot += dp[c] * p[c];
+  if constexpr (NV > 0) {
+#pragma unroll
+    for (int i = 0; i < kN; ++i)
+      if (col(i) < C) dot += dp[col(i)] * pr[i];
+  } else {
+    for (int c = threadIdx.x; c < C; c += blockDim.x) dot += dp[c] * p[c];
+  }
   dot = block_sum(dot, red);
   const float zc = g_z * 2.f * lse * invB;
-  for (int c = threadIdx.x; c < C; c += blockDim.x)
-    d_logits[static_cast<long long>(b) * C + c] = p[c] * (dp[c] - dot + zc);
+  if (terms != nullptr) {
+    const long long stride = static_cast<long long>(B) * ld;
+    __nv_bfloat162* t0 = reinterpret_cast<__nv_bfloat162*>(terms + static_cast<long long>(b) * ld);
+    auto emit = [&](int c, float x, float y) {
+#pragma unroll
+      for (int t = 0; t < 3; ++t) {
+        const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+        t0[(t * stride + c) / 2] = v;
+        x -= __low2float(v); y -= __high2float(v);
+      }
+    };
+    auto grad = [&](int c, float pv) { return c < C ? pv * (dp[c] - dot + zc) : 0.f; };
+    if constexpr (NV > 0) {
+#pragma unroll
+      for (int i = 0; i + 1 < kN; i += 2)
+        if (col(i) < ld) emit(col(i), grad(col(i), pr[i]), grad(col(i + 1), pr[i + 1]));
+    } else {
+      for (int c = 2 * threadIdx.x; c < ld; c += 2 * TH)
+        emit(c, grad(c, p[min(c, C - 1)]), grad(c + 1, p[min(c + 1, C - 1)]));
+    }
+    return;
+  }
+  if constexpr (NV > 0) {
+#pragma unroll
+    for (int i = 0; i < kN; ++i)
+      if (col(i) < C) d_logits[static_cast<long long>(b) * C + col(i)] = pr[i] * (dp[col(i)] - dot + zc);
+  } else {
+    for (int c = threadIdx.x; c < C; c += blockDim.x)
+      d_logits[static_cast<long long>(b) * C + c] = p[c] * (dp[c] - dot + zc);
+  }
 }
 
 // d_w[c,:] = sum_b d_logits[b,c] * pooled[b,:]; d_bias[c] = sum_b d_logits[b,c]; one warp per chapter, 8 batch rows of
@@ -1008,6 +1108,41 @@ __global__ void dh_broadcast_kernel(const float* __restrict__ d_pooled, T* __res
   }
 }
 
+// kManyRows rows are enough to fill the chip with CTAs of 1,024 threads twice over; from there on smaller ones win
+constexpr int kManyRows = 2 * 296;
+int launch_select(const float* logits, long long ld, const float* bias, float* probs, int64_t* idx, float* weights,
+                  int* comb_idx, float* comb_w, float* row_stats, int B, int C, int k_sel, int S, float rho,
+                  cudaStream_t stream) {
+  const size_t sm = (static_cast<size_t>(C) + 2 * static_cast<size_t>(k_sel > 0 ? k_sel : 1)) * 4;
+  // The row's values stay in registers: up to 9 a thread of 1,024 (64 registers leave room for no more), 17 of 256; the
+  // steps are a power of two of routed chapters and a few shared ones.
+  const bool small = B >= kManyRows && C <= 17 * 256;
+  auto kern = small ? (C <= 5 * 256 ? select_kernel<5, 256> : select_kernel<17, 256>)
+              : C <= 2 * 1024 ? select_kernel<2, 1024> : C <= 5 * 1024 ? select_kernel<5, 1024>
+              : C <= 9 * 1024 ? select_kernel<9, 1024> : select_kernel<0, 1024>;
+  MOC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm)));
+  kern<<<B, small ? 256 : 1024, sm, stream>>>(logits, ld, bias, probs, reinterpret_cast<long long*>(idx), weights, comb_idx,
+                                              comb_w, row_stats, C, k_sel, S, rho);
+  MOC_CUDA_OK(cudaGetLastError());
+  return MOC_OK;
+}
+
+int launch_dlogits(const float* probs, const int64_t* idx, const float* weights, const float* comb_w, const float* row_stats,
+                   const float* chapter_stats, const float* d_weights, const float* d_comb_w, const float* d_losses,
+                   float* d_logits, __nv_bfloat16* terms, int ld, int B, int C, int k_sel, int S, float rho,
+                   cudaStream_t stream) {
+  const size_t sm = static_cast<size_t>(C) * 4;
+  const int cols = terms != nullptr ? ld : C;
+  const bool small = B >= kManyRows && cols <= 18 * 256;
+  auto kern = small ? dlogits_kernel<18, 256> : cols <= 6 * 1024 ? dlogits_kernel<6, 1024> : dlogits_kernel<0, 1024>;
+  MOC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm)));
+  kern<<<B, small ? 256 : 1024, sm, stream>>>(probs, reinterpret_cast<const long long*>(idx), weights, comb_w, row_stats,
+                                              chapter_stats, d_weights, d_comb_w, d_losses, d_logits, terms, ld, B, C, k_sel, S,
+                                              rho);
+  MOC_CUDA_OK(cudaGetLastError());
+  return MOC_OK;
+}
+
 inline int k_selected(const moc_router_shape* s) {
   int k = s->top_k;
   const int avail = s->num_chapters - s->num_shared;
@@ -1044,10 +1179,119 @@ inline int check_shape(const moc_router_shape* s) {
   return MOC_OK;
 }
 
+void launch_losses(const moc_router_shape* s, const float* probs, const int64_t* idx, const float* row_stats,
+                   float* chapter_stats, float* losses, float* loss_partial, cudaStream_t stream) {
+  const int B = s->batch, C = s->num_chapters, k_sel = k_selected(s);
+  const int nblk = ceil_div(C, kLossChunk);
+  const int splits = loss_row_splits(s);
+  if (splits > 1) {
+    float* rows_part = reinterpret_cast<float*>(
+        (reinterpret_cast<uintptr_t>(loss_partial + static_cast<size_t>(nblk) * 3) + 15) & ~uintptr_t(15));
+    const int rows_per_split = ceil_div(B, splits);
+    loss_rows_partial_kernel<<<dim3(nblk, splits), kLossChunk, 0, stream>>>(
+        probs, reinterpret_cast<const long long*>(idx), rows_part, B, C, k_sel, rows_per_split);
+    loss_rows_finish_kernel<<<nblk, kLossChunk, 0, stream>>>(rows_part, chapter_stats, loss_partial, B, C, splits);
+  } else {
+    loss_partial_kernel<<<nblk, kLossChunk, 0, stream>>>(probs, reinterpret_cast<const long long*>(idx),
+                                                         chapter_stats, loss_partial, B, C, k_sel);
+  }
+  loss_finish_kernel<<<1, 32, 0, stream>>>(loss_partial, row_stats, losses, nblk, B, C);
+}
+
+struct TokenSaved { __nv_bfloat16* w_terms; float *probs, *row_stats, *chapter_stats, *loss_ws; };
+moc_router_shape token_shape(const moc_token_route_desc* s) {
+  return moc_router_shape{s->rows, 1, s->hidden_dim, s->num_chapters, s->top_k, s->num_shared, 1.f, MOC_BF16};
+}
+int64_t carve(const moc_token_route_desc* s, TokenSaved* a) {
+  const moc_router_shape r = token_shape(s);
+  Carver c{static_cast<char*>(s->arena), 0};
+  const int64_t C = s->num_chapters;
+  a->w_terms = c.take<__nv_bfloat16>(3 * C * s->hidden_dim + 8 * s->hidden_dim);   // (a padded K reads a few rows further)
+  a->probs = c.take<float>(s->rows * C);
+  a->row_stats = c.take<float>(4 * static_cast<int64_t>(s->rows));
+  a->chapter_stats = c.take<float>(2 * C);
+  a->loss_ws = c.take<float>(static_cast<int64_t>(loss_floats(&r)));
+  return c.off;
+}
+inline int64_t padded(int n) { return (n + 7) / 8 * 8; }
+
 }  // namespace
 }  // namespace moc
 
 using namespace moc;
+
+extern "C" int64_t moc_token_route_arena_bytes(const moc_token_route_desc* s) {
+  TokenSaved a;
+  return s ? carve(s, &a) : -1;
+}
+extern "C" int64_t moc_token_route_scratch_bytes(const moc_token_route_desc* s, int32_t backward) {
+  if (!s) return -1;
+  const int64_t cp = padded(s->num_chapters);
+  return backward ? 3 * s->rows * cp * 2 + ceil_div(s->rows, kTermRows) * cp * 4 : s->rows * cp * 4;
+}
+
+extern "C" int moc_token_route_fwd(const moc_token_route_desc* s, void* scratch) {
+  MOC_REQUIRE(s && s->h && s->w && s->weights && s->arena && scratch && s->status, "NULL token-router buffer");
+  const moc_router_shape r = token_shape(s);
+  int rc = check_shape(&r);
+  if (rc != MOC_OK) return rc;
+  MOC_REQUIRE(r.hidden_dim % 8 == 0, "the bf16 token router takes a width of a multiple of 8");
+  TokenSaved a;
+  carve(s, &a);
+  cudaStream_t stream = static_cast<cudaStream_t>(s->stream);
+  const int C = s->num_chapters, d = s->hidden_dim;
+  const int64_t cp = padded(C);
+  // bf16 activations are exact bf16 numbers: h (w0 + w1 + w2)^T as one product over three times the width, smallest term
+  // first, carries the fp32 weight's 24 mantissa bits; nothing is added up outside the accumulator
+  MOC_TRY(moc_split_bf16(s->w, a.w_terms, static_cast<int64_t>(C) * d, 3, stream));
+  float* logits = static_cast<float*>(scratch);
+  Gemm g(MOC_BF16, s->rows, C, d, true, true, MOC_F32);
+  g.ldc = cp;
+  g.terms = 3; g.b_term_rows = C;
+  MOC_TRY(moc_gemm(&g, s->h, a.w_terms, logits, nullptr, nullptr, s->status, stream));
+  MOC_TRY(launch_select(logits, cp, s->bias, a.probs, s->idx, s->weights, nullptr, nullptr, a.row_stats, s->rows, C,
+                        k_selected(&r), s->num_shared, 1.f, stream));
+  if (s->losses != nullptr)
+    launch_losses(&r, a.probs, s->idx, a.row_stats, a.chapter_stats, s->losses, a.loss_ws, stream);
+  MOC_CUDA_OK(cudaGetLastError());
+  return MOC_OK;
+}
+
+extern "C" int moc_token_route_bwd(const moc_token_route_desc* s, const float* g_weights, const float* g_losses, void* d_h,
+                                   float* d_w, float* d_bias, void* scratch) {
+  MOC_REQUIRE(s && s->h && s->weights && s->arena && scratch && s->status, "NULL token-router buffer");
+  const moc_router_shape r = token_shape(s);
+  int rc = check_shape(&r);
+  if (rc != MOC_OK) return rc;
+  MOC_REQUIRE(d_w == nullptr || s->rows % 8 == 0, "a bf16 weight gradient takes the tokens in multiples of 8");
+  TokenSaved a;
+  carve(s, &a);
+  cudaStream_t stream = static_cast<cudaStream_t>(s->stream);
+  const int C = s->num_chapters, d = s->hidden_dim, rows = s->rows, k_sel = k_selected(&r);
+  const int64_t cp = padded(C);
+  __nv_bfloat16* terms = static_cast<__nv_bfloat16*>(scratch);
+  float* partial = reinterpret_cast<float*>(terms + 3 * rows * cp);
+  MOC_TRY(launch_dlogits(a.probs, s->idx, s->weights, nullptr, a.row_stats, a.chapter_stats, g_weights, nullptr, g_losses,
+                         nullptr, terms, static_cast<int>(cp), rows, C, k_sel, s->num_shared, 1.f, stream));
+  if (d_h != nullptr) {        // leaves in bf16: one product of the leading terms
+    Gemm g(MOC_BF16, rows, d, cp, true, false, MOC_BF16);
+    MOC_TRY(moc_gemm(&g, terms, a.w_terms, d_h, nullptr, nullptr, s->status, stream));
+  }
+  if (d_w != nullptr) {
+    Gemm g(MOC_BF16, C, d, rows, false, false, MOC_F32);
+    g.lda = cp;
+    g.terms = 3; g.a_term_rows = rows;
+    MOC_TRY(moc_gemm(&g, terms, s->h, d_w, nullptr, nullptr, s->status, stream));
+  }
+  if (d_bias != nullptr) {
+    const int chunks = ceil_div(rows, kTermRows);
+    term_col_sum_kernel<<<dim3(ceil_div(static_cast<int>(cp), 64), chunks), 256, 0, stream>>>(terms, partial, rows,
+                                                                                            static_cast<int>(cp));
+    col_sum_kernel<<<ceil_div(C, 32), 256, 0, stream>>>(partial, d_bias, chunks, C, static_cast<int>(cp));
+  }
+  MOC_CUDA_OK(cudaGetLastError());
+  return MOC_OK;
+}
 
 extern "C" size_t moc_router_workspace_bytes(const moc_router_shape* s) { return s ? ws_bytes(s) : 0; }
 extern "C" size_t moc_router_workspace_bytes_parts(const moc_router_shape* s, int32_t fwd_parts, int32_t bwd_parts) {
@@ -1092,14 +1336,9 @@ extern "C" int moc_router_fwd_parts(const moc_router_shape* s, const void* h, co
     pool_partial_kernel<__nv_bfloat16><<<pg, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(h), ws, L, d);
   if (!one) pool_finish_kernel<<<ceil_div(B * d, 256), 256, 0, stream>>>(ws, pooled, L, d, B * d);
   }
-  if (parts & 16) {        // bit 16: `logits` already holds pooled x W^T (a projection kernel ran); only the bias is missing
-    if (bias != nullptr) {
-      const long long total = static_cast<long long>(B) * C;
-      long long blocks = (total + 255) / 256;
-      if (blocks > 148LL * 16) blocks = 148LL * 16;
-      add_bias_kernel<<<static_cast<int>(blocks), 256, 0, stream>>>(logits, bias, total, C);
-    }
-  } else {
+  // bit 16: `logits` already holds pooled x W^T (a projection kernel ran); only the bias is missing
+  const float* bias_left = (parts & 16) ? bias : nullptr;
+  if (!(parts & 16)) {
     const size_t sm = static_cast<size_t>(8) * d * sizeof(float);
     if (d % 4 == 0 && d <= 1024 && ((reinterpret_cast<uintptr_t>(pooled) | reinterpret_cast<uintptr_t>(w)) & 15) == 0) {
       const bool few = B <= 8;
@@ -1115,33 +1354,12 @@ extern "C" int moc_router_fwd_parts(const moc_router_shape* s, const void* h, co
       logits_kernel<<<ceil_div(C, 8), 256, sm, stream>>>(pooled, w, bias, logits, B, d, C);
     }
   }
-  {
-    const size_t sm = (static_cast<size_t>(C) + 2 * static_cast<size_t>(k_sel > 0 ? k_sel : 1)) * 4;
-    // The row's values stay in registers up to 9 a thread (64 registers a thread leave room for no more); the steps are a
-    // power of two of routed chapters and a few shared ones.
-    auto kern = C <= 2 * kSelectThreads ? select_kernel<2>
-                : C <= 5 * kSelectThreads ? select_kernel<5> : C <= 9 * kSelectThreads ? select_kernel<9> : select_kernel<0>;
-    MOC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm)));
-    kern<<<B, kSelectThreads, sm, stream>>>(logits, probs, reinterpret_cast<long long*>(idx), weights, comb_idx, comb_w,
-                                            row_stats, C, k_sel, S, s->routed_scale);
-  }
+  if ((rc = launch_select(logits, C, bias_left, probs, idx, weights, comb_idx, comb_w, row_stats, B, C, k_sel, S,
+                          s->routed_scale, stream)) != MOC_OK) return rc;
   }
   if ((parts & 2) && losses != nullptr) {
     MOC_REQUIRE(chapter_stats != nullptr, "chapter_stats is NULL");
-    const int nblk = ceil_div(C, kLossChunk);
-    const int splits = loss_row_splits(s);
-    if (splits > 1) {
-      float* rows_part = reinterpret_cast<float*>(
-          (reinterpret_cast<uintptr_t>(loss_partial + static_cast<size_t>(nblk) * 3) + 15) & ~uintptr_t(15));
-      const int rows_per_split = ceil_div(B, splits);
-      loss_rows_partial_kernel<<<dim3(nblk, splits), kLossChunk, 0, stream>>>(
-          probs, reinterpret_cast<const long long*>(idx), rows_part, B, C, k_sel, rows_per_split);
-      loss_rows_finish_kernel<<<nblk, kLossChunk, 0, stream>>>(rows_part, chapter_stats, loss_partial, B, C, splits);
-    } else {
-      loss_partial_kernel<<<nblk, kLossChunk, 0, stream>>>(probs, reinterpret_cast<const long long*>(idx),
-                                                           chapter_stats, loss_partial, B, C, k_sel);
-    }
-    loss_finish_kernel<<<1, 32, 0, stream>>>(loss_partial, row_stats, losses, nblk, B, C);
+    launch_losses(s, probs, idx, row_stats, chapter_stats, losses, loss_partial, stream);
   }
   MOC_CUDA_OK(cudaGetLastError());
   return MOC_OK;
@@ -1174,11 +1392,8 @@ extern "C" int moc_router_bwd_parts(const moc_router_shape* s, const float* w, c
   const int k_sel = k_selected(s);
   float* ws = static_cast<float*>(workspace);
   if (parts & 1) {
-    const size_t sm = static_cast<size_t>(C) * 4;
-    MOC_CUDA_OK(cudaFuncSetAttribute(dlogits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm)));
-    dlogits_kernel<<<B, kSelectThreads, sm, stream>>>(probs, reinterpret_cast<const long long*>(idx), weights,
-                                                      comb_w, row_stats, chapter_stats, d_weights, d_comb_w,
-                                                      d_losses, d_logits, B, C, k_sel, S, s->routed_scale);
+    if ((rc = launch_dlogits(probs, idx, weights, comb_w, row_stats, chapter_stats, d_weights, d_comb_w, d_losses, d_logits,
+                             nullptr, 0, B, C, k_sel, S, s->routed_scale, stream)) != MOC_OK) return rc;
   }
   if (parts & 2) {
     const size_t sm = static_cast<size_t>(8) * d * sizeof(float);
@@ -1283,7 +1498,7 @@ extern "C" int moc_loss_total(const float* losses, const float* grad, float c0, 
 
 extern "C" int moc_col_sum(const float* x, float* out, int64_t rows, int32_t cols, void* stream_) {
   MOC_REQUIRE(x && out && rows > 0 && cols > 0, "bad column-sum arguments");
-  col_sum_kernel<<<ceil_div(cols, 32), 256, 0, static_cast<cudaStream_t>(stream_)>>>(x, out, rows, cols);
+  col_sum_kernel<<<ceil_div(cols, 32), 256, 0, static_cast<cudaStream_t>(stream_)>>>(x, out, rows, cols, cols);
   MOC_CUDA_OK(cudaGetLastError());
   return MOC_OK;
 }

@@ -582,26 +582,24 @@ class _RouteTokens(torch.autograd.Function):
         b, l, d = h.shape
         rows = b * l
         h2 = h.reshape(rows, d).contiguous()
-        h32 = ops.cast(h2, torch.float32)
         w32 = weight.float().contiguous()
         c = w32.shape[0]
-        split = None
-        if h.dtype == torch.bfloat16 and d % 8 == 0 and rows * c * d >= _SPLIT_ROUTER_MIN_WORK:
-            # bf16 activations are exact bf16 numbers: logits = h (w0 + w1 + w2)^T as three tensor-core products
-            # accumulated in fp32 (smallest term first) carry the fp32 weight's 24 mantissa bits
-            cp = -(-c // 8) * 8
-            w_terms = ops.split_bf16(w32 if cp == c else torch.nn.functional.pad(w32, (0, 0, 0, cp - c)), 3)
-            parts = ops.gemm(h2, w_terms.view(3 * cp, d), out_dtype=torch.float32, tag="token_router_logits")
-            logits = ops.sum_terms(parts, c, 3, bias=None if bias is None else bias.float())
-            del parts
-            split = (h2, w_terms, cp)
-        else:
-            logits = ops.gemm(h32, w32, tag="token_router_logits")                 # [rows, C] fp32, no bias yet
-        ctx.split = split
-        r = ops.router_fwd(h32.view(rows, 1, d), w32, None if split is not None else bias, top_k, num_shared, 1.0,
-                           with_losses, pooled=h32, logits=logits)      # (the split path has added the bias)
-        k = r["idx"].shape[1]
         ctx.cfg = ((b, l, d), h.dtype, int(top_k), int(num_shared), bias is not None)
+        ctx.desc = None
+        if h.dtype == torch.bfloat16 and d % 8 == 0 and rows * c * d >= _SPLIT_ROUTER_MIN_WORK:
+            desc, idx, weights, losses, arena = ops.token_route_fwd(h2, w32, None if bias is None else bias.float(), top_k,
+                                                                    num_shared, with_losses)
+            if any(ctx.needs_input_grad[:3]):
+                ctx.desc = desc
+                ctx.save_for_backward(h2, arena, idx, weights)
+            idx = idx.view(b, l, -1)
+            ctx.mark_non_differentiable(idx)
+            return (idx, weights.view(b, l, -1),
+                    losses if with_losses else torch.zeros(4, dtype=torch.float32, device=h.device))
+        h32 = ops.cast(h2, torch.float32)
+        logits = ops.gemm(h32, w32, tag="token_router_logits")                 # [rows, C] fp32, no bias yet
+        r = ops.router_fwd(h32.view(rows, 1, d), w32, bias, top_k, num_shared, 1.0, with_losses, pooled=h32, logits=logits)
+        k = r["idx"].shape[1]
         ctx.internals = {n: r[n] for n in ("pooled", "probs", "idx", "row_stats", "chapter_stats", "_ws", "comb_w")}
         ctx.save_for_backward(w32, r["weights"])
         idx = r["idx"].view(b, l, k)
@@ -611,9 +609,17 @@ class _RouteTokens(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, _g_idx, g_w, g_losses):
-        w32, weights = ctx.saved_tensors
         (b, l, d), h_dtype, top_k, num_shared, has_bias = ctx.cfg
         rows = b * l
+        if ctx.desc is not None:
+            h2, arena, idx, weights = ctx.saved_tensors
+            d_h, d_w, d_b = ops.token_route_bwd(ctx.desc, h2, arena, idx, weights,
+                                                None if g_w is None else g_w.reshape(rows, -1).float().contiguous(),
+                                                None if g_losses is None else g_losses.float().contiguous(),
+                                                ctx.needs_input_grad[0], ctx.needs_input_grad[1],
+                                                has_bias and ctx.needs_input_grad[2])
+            return None if d_h is None else d_h.view(b, l, d), d_w, d_b, None, None, None
+        w32, weights = ctx.saved_tensors
         saved = dict(ctx.internals, weights=weights)
         g_w = None if g_w is None else g_w.reshape(rows, -1).float().contiguous()
         g_losses = None if g_losses is None else g_losses.float()
@@ -622,24 +628,10 @@ class _RouteTokens(torch.autograd.Function):
         d_logits = r["d_logits"]
         h32 = saved["pooled"]
         d_h = d_w = d_b = None
-        if ctx.split is not None:
-            h2, w_terms, cp = ctx.split
-            c = w32.shape[0]
-            dl = d_logits if cp == c else torch.nn.functional.pad(d_logits, (0, cp - c))
-            dl_terms = ops.split_bf16(dl, 3)                                       # [3, rows, cp]
-            if ctx.needs_input_grad[0]:
-                # the gradient leaves in bf16: one product of the leading terms
-                d_h = ops.gemm(dl_terms[0], w_terms[0], b_kmajor=False, tag="token_router_dh").view(b, l, d)
-            if ctx.needs_input_grad[1]:
-                for t in (2, 1, 0):
-                    d_w = ops.gemm(dl_terms[t], h2, a_kmajor=False, b_kmajor=False, out=d_w, out_dtype=torch.float32,
-                                   accumulate=d_w is not None, tag="token_router_dw")
-                d_w = d_w[:c]
-        else:
-            if ctx.needs_input_grad[0]:
-                d_h = ops.gemm(d_logits, w32, b_kmajor=False, tag="token_router_dh").view(b, l, d).to(h_dtype)
-            if ctx.needs_input_grad[1]:
-                d_w = ops.gemm(d_logits, h32, a_kmajor=False, b_kmajor=False, tag="token_router_dw")
+        if ctx.needs_input_grad[0]:
+            d_h = ops.gemm(d_logits, w32, b_kmajor=False, tag="token_router_dh").view(b, l, d).to(h_dtype)
+        if ctx.needs_input_grad[1]:
+            d_w = ops.gemm(d_logits, h32, a_kmajor=False, b_kmajor=False, tag="token_router_dw")
         if has_bias and ctx.needs_input_grad[2]:
             d_b = ops.col_sum(d_logits)
         return d_h, d_w, d_b, None, None, None

@@ -1267,3 +1267,44 @@ def decode_step(hidden: torch.Tensor, routing_states: torch.Tensor, router_w: to
     _report(5 + int(window <= 1024) + 2 * int(window > 1024) + int(h.dtype == f32), lambda: (
         "router_fwd:" + _TAG_OF_CODE[s.router.h_dtype], "gemm:bf16", "decode_attn:bf16", "gemm:bf16"))
     return out, idx, weights, comb_idx, comb_w
+
+
+# --------------------------------------------------------------------------------------------
+# token-level routing of bf16 states
+# --------------------------------------------------------------------------------------------
+def token_route_fwd(h: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], top_k: int, num_shared: int,
+                    with_losses: bool):
+    """``moc_token_route_fwd`` on h [rows, d] bf16 and the fp32 weight [C, d].  Returns (descriptor, idx int64 [rows, k'],
+    weights, losses or None, arena); descriptor and arena go to :func:`token_route_bwd`."""
+    L.require_cuda(h, weight, bias)
+    rows, d = h.shape
+    c, dev = weight.shape[0], h.device
+    k = router_selected_k(c, top_k, num_shared)
+    idx = torch.empty(rows, k, dtype=torch.int64, device=dev)
+    weights = torch.empty(rows, k, dtype=torch.float32, device=dev)
+    losses = torch.empty(4, dtype=torch.float32, device=dev) if with_losses else None
+    bias = _contig(bias)
+    p = L.ptr
+    s = L.TokenRouteDesc(rows, d, c, top_k, num_shared, p(h), p(weight), p(bias), p(idx), p(weights), p(losses), None,
+                         p(L.status_word(dev)), L.stream_ptr(dev))
+    arena = torch.empty(_size("moc_token_route_arena_bytes", s), dtype=torch.uint8, device=dev)
+    s.arena = p(arena)
+    scratch = torch.empty(L.lib().moc_token_route_scratch_bytes(C.byref(s), 0), dtype=torch.uint8, device=dev)
+    L.check(_timed("token_route_fwd", lambda: L.lib().moc_token_route_fwd(C.byref(s), p(scratch))), "moc_token_route_fwd")
+    _report(3 + 3 * int(bool(with_losses)), lambda: ("split_bf16:f32", "gemm:bf16", "router_fwd:f32"))
+    return s, idx, weights, losses, arena
+
+
+def token_route_bwd(s, h, arena, idx, weights, g_weights, g_losses, want_dh: bool, want_dw: bool, want_db: bool):
+    """``moc_token_route_bwd`` on the forward call's descriptor; returns (d_h bf16 or None, d_w, d_bias)."""
+    dev, p = h.device, L.ptr
+    s.h, s.arena, s.idx, s.weights, s.stream = p(h), p(arena), p(idx), p(weights), L.stream_ptr(dev)
+    d_h = torch.empty_like(h) if want_dh else None
+    d_w = torch.empty(s.num_chapters, s.hidden_dim, dtype=torch.float32, device=dev) if want_dw else None
+    d_b = torch.empty(s.num_chapters, dtype=torch.float32, device=dev) if want_db else None
+    scratch = torch.empty(L.lib().moc_token_route_scratch_bytes(C.byref(s), 1), dtype=torch.uint8, device=dev)
+    L.check(_timed("token_route_bwd", lambda: L.lib().moc_token_route_bwd(
+        C.byref(s), p(g_weights), p(g_losses), p(d_h), p(d_w), p(d_b), p(scratch))), "moc_token_route_bwd")
+    _report(1 + int(want_dh) + int(want_dw) + 2 * int(want_db),
+            lambda: ("router_bwd:f32",) + ("gemm:bf16",) * (int(want_dh) + int(want_dw)))
+    return d_h, d_w, d_b

@@ -80,3 +80,34 @@ def test_routing_window_is_the_sliced_concatenation(dev, dtype, d):
     for n in (1, 2, 3):
         want = torch.cat([want, prompt[:, :n]], 1)[:, -6:]
         assert torch.equal(window.step(prompt[:, :n]), want)
+
+
+@pytest.mark.parametrize("rows,c,d,k,s", [(136, 4097, 256, 16, 1), (592, 1280, 256, 300, 0), (600, 1283, 200, 8, 2), (608, 4352, 64, 5, 1),
+                                          (616, 4355, 72, 5, 1)])
+def test_token_router_shapes(dev, rows, c, d, k, s):
+    """Both CTA widths of the selection, chapter counts and widths that fill no tile, the terms of weight and gradient."""
+    import memory_b200 as M
+    torch.manual_seed(rows + c)
+    h = torch.randn(1, rows, d, device=dev).bfloat16().requires_grad_(True)
+    w = (torch.randn(c, d, device=dev) * 0.05).requires_grad_(True)
+    bias = (torch.randn(c, device=dev) * 0.1).requires_grad_(True)
+    idx, wt, losses = M.route_tokens(h, w, bias, k, s, True)
+    g = torch.randn_like(wt)
+    coef = {"load_balance": 0.3, "z_loss": 0.2, "entropy": 0.1}
+    (sum(coef[n] * losses[n] for n in coef) + (wt * g).sum()).backward()
+    h64, w64, b64 = (t.detach().double().requires_grad_(True) for t in (h, w, bias))
+    z = h64[0] @ w64.t() + b64
+    p = z.softmax(-1)
+    masked = torch.cat([torch.zeros_like(p[:, :s]), p[:, s:]], 1)
+    top = masked.gather(1, idx[0])
+    assert (top.min(1).values >= masked.detach().topk(k, 1).values[:, -1] * (1 - 1e-5)).all()
+    w_ref = top / top.sum(1, keepdim=True)
+    f = torch.zeros_like(p).scatter_(1, idx[0], 1.0).mean(0)
+    lb = c * (f * p.mean(0)).sum()
+    zl = torch.logsumexp(z, 1).square().mean()
+    ent = -(p * p.clamp_min(1e-12).log()).sum(1).mean()
+    for name, ref in (("load_balance", lb), ("z_loss", zl), ("entropy", ent)):
+        assert abs(float(losses[name]) - float(ref)) < 2e-5 * abs(float(ref)), name
+    (0.3 * lb + 0.2 * zl + 0.1 * ent + (w_ref * g[0].double()).sum()).backward()
+    assert _rel(wt[0], w_ref) < 1e-5
+    assert _rel(w.grad, w64.grad) < 1e-4 and _rel(bias.grad, b64.grad) < 1e-4 and _rel(h.grad, h64.grad) < 1e-2
