@@ -303,7 +303,11 @@ int moc_scatter_bank_grad(const float* bank_grad, const int32_t* uniq, const int
  * C = row_scale * (A B) + residual -- the residual add that follows the output projection in the
  * reference's block (memory_block.py:558) done in the projection's epilogue.
  * terms > 1 (bf16 kernel): C = sum over t of op(A_t) op(B_t), all in one accumulator, the last term first; A_t / B_t start
- * t * a_term_rows / b_term_rows stored rows behind A / B (0: the same operand in every term). */
+ * t * a_term_rows / b_term_rows stored rows behind A / B (0: the same operand in every term).
+ * limit (device, bf16 kernel, may be NULL): only the first *limit * limit_block of the M rows (limit_k != 0: of the K range,
+ * limit_block a multiple of 64) exist; what lies behind is neither read into a stored result nor, for M, defined in C.
+ * c_row_blocks (device, bf16 kernel, may be NULL): block i of c_block_rows (a multiple of 32) rows of C is stored as block
+ * c_row_blocks[i] of a matrix of c_stored_rows rows. */
 typedef struct {
   int32_t dtype, c_dtype;
   int32_t m, n, k;
@@ -316,6 +320,9 @@ typedef struct {
   const float* residual;
   int64_t ldr;
   int32_t terms, a_term_rows, b_term_rows;
+  int32_t limit_block, limit_k, c_block_rows;
+  int64_t c_stored_rows;
+  const int32_t *limit, *c_row_blocks;
 } moc_gemm_desc;
 
 int moc_gemm(const moc_gemm_desc* g, const void* a, const void* b, void* c, const float* row_scale,
@@ -453,6 +460,36 @@ typedef struct {
 } moc_decode_step_desc;
 int64_t moc_decode_step_arena_bytes(const moc_decode_step_desc* s);
 int moc_decode_step(const moc_decode_step_desc* s);
+
+/* Token-routed memory attention with per-token chapter weights, projections included, in one call per pass (bf16 arithmetic,
+ * head_dim 64, 64-row chapters): h [rows, hidden_dim], shared [shared_rows, hidden_dim] (shared_rows 0: none), routed
+ * [routed_rows, hidden_dim], idx [rows, n_select] int32 chapter ids local to routed, weights [rows, n_select] fp32.
+ * arena holds what the backward pass reads; for_backward 0: it may be dropped after the call.  d_routed (the dtype of routed)
+ * is dense; d_shared / d_routed NULL: not wanted; d_wkv: K rows then V rows; the weight gradients are fp32. */
+typedef struct {
+  int32_t rows, hidden_dim, num_heads, num_kv_heads, n_select, shared_rows, routed_rows;
+  int32_t h_dtype, shared_dtype, routed_dtype, weight_dtype, out_dtype, for_backward;
+  float routed_scale;
+  const void *h, *shared, *routed;
+  const int32_t* idx;
+  const float* weights;
+  const void *wq, *wk, *wv, *wo;
+  void *out, *arena;
+  int32_t* status;
+  void* stream;
+} moc_token_attn_desc;
+typedef struct {
+  int32_t g_dtype;
+  const void* g;
+  void *d_h, *d_shared, *d_routed;
+  float *d_weights, *d_wq, *d_wkv, *d_wo;
+  void* scratch;
+} moc_token_attn_bwd_desc;
+int64_t moc_token_attn_arena_bytes(const moc_token_attn_desc* s);
+int64_t moc_token_attn_fwd_scratch_bytes(const moc_token_attn_desc* s);
+int64_t moc_token_attn_bwd_scratch_bytes(const moc_token_attn_desc* s, const moc_token_attn_bwd_desc* b);
+int moc_token_attn_fwd(const moc_token_attn_desc* s, void* scratch);
+int moc_token_attn_bwd(const moc_token_attn_desc* s, const moc_token_attn_bwd_desc* b);
 
 /* ------------------------------------------------------------------------------------------------
  * Per-token chapter-sparse attention: the contract of memory_cross_attn(q, k, v, block_indices,

@@ -35,7 +35,9 @@ class GemmDesc(C.Structure):
                 ("accumulate", C.c_int32), ("split_k", C.c_int32), ("scale_block_rows", C.c_int32),
                 ("a_block_rows", C.c_int32), ("a_stored_rows", C.c_int64),
                 ("residual", C.c_void_p), ("ldr", C.c_int64),
-                ("terms", C.c_int32), ("a_term_rows", C.c_int32), ("b_term_rows", C.c_int32)]
+                ("terms", C.c_int32), ("a_term_rows", C.c_int32), ("b_term_rows", C.c_int32),
+                ("limit_block", C.c_int32), ("limit_k", C.c_int32), ("c_block_rows", C.c_int32),
+                ("c_stored_rows", C.c_int64), ("limit", C.c_void_p), ("c_row_blocks", C.c_void_p)]
 
 
 class AttnShape(C.Structure):
@@ -73,6 +75,17 @@ class RouteDesc(C.Structure):
 
 class TokenRouteDesc(C.Structure):
     _fields_ = _fields("i: rows hidden_dim num_chapters top_k num_shared; p: h w bias idx weights losses arena status stream")
+
+
+class TokenAttnDesc(C.Structure):
+    _fields_ = _fields(
+        "i: rows hidden_dim num_heads num_kv_heads n_select shared_rows routed_rows h_dtype shared_dtype routed_dtype"
+        " weight_dtype out_dtype for_backward; f: routed_scale;"
+        "p: h shared routed idx weights wq wk wv wo out arena status stream")
+
+
+class TokenAttnBwdDesc(C.Structure):
+    _fields_ = _fields("i: g_dtype; p: g d_h d_shared d_routed d_weights d_wq d_wkv d_wo scratch")
 
 
 class DecodeStepDesc(C.Structure):
@@ -170,6 +183,11 @@ _PROTOTYPES = {
     "moc_token_route_scratch_bytes": (C.c_int64, [C.POINTER(TokenRouteDesc), C.c_int32]),
     "moc_token_route_fwd": (C.c_int, [C.POINTER(TokenRouteDesc), P]),
     "moc_token_route_bwd": (C.c_int, [C.POINTER(TokenRouteDesc), P, P, P, P, P, P]),
+    "moc_token_attn_arena_bytes": (C.c_int64, [C.POINTER(TokenAttnDesc)]),
+    "moc_token_attn_fwd_scratch_bytes": (C.c_int64, [C.POINTER(TokenAttnDesc)]),
+    "moc_token_attn_bwd_scratch_bytes": (C.c_int64, [C.POINTER(TokenAttnDesc), C.POINTER(TokenAttnBwdDesc)]),
+    "moc_token_attn_fwd": (C.c_int, [C.POINTER(TokenAttnDesc), P]),
+    "moc_token_attn_bwd": (C.c_int, [C.POINTER(TokenAttnDesc), C.POINTER(TokenAttnBwdDesc)]),
     "moc_chapter_lists": (C.c_int, [P, C.c_int32, C.c_int32, C.c_int32, P, P, P]),
     "moc_loss_total": (C.c_int, [P, P, C.c_float, C.c_float, C.c_float, C.c_float, P, P]),
     "moc_sparse_attn_tc_sizes": (C.c_int, [C.POINTER(SparseAttnShape), P, P, P]),

@@ -29,7 +29,7 @@ extern "C" int moc_gemm(const moc_gemm_desc* g, const void* a, const void* b, vo
   MOC_REQUIRE(g->m > 0 && g->n > 0 && g->k > 0, "empty projection");
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (g->dtype == MOC_F32) {
-    MOC_REQUIRE(g->terms <= 1, "operands in terms are bf16");
+    MOC_REQUIRE(g->terms <= 1 && !g->limit && !g->c_row_blocks, "operand terms, limits and scattered rows are bf16 only");
     MOC_REQUIRE(a_row_blocks == nullptr, "the fp32 projection takes gathered rows, not a gather list");
     return launch_sgemm(g, static_cast<const float*>(a), static_cast<const float*>(b), static_cast<float*>(c),
                         row_scale, stream);

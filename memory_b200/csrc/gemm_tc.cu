@@ -59,6 +59,11 @@ struct GemmTcParams {
   int k_tiles_total;
   int k_tiles_per_term, terms; // the K range of one term and the number of terms (see moc_gemm_desc)
   int a_term_rows, b_term_rows;
+  const int* limit;        // device: rows of C (limit_k: of the K range) that exist, in blocks
+  int limit_block, limit_k;
+  const int* c_row_blocks; // where blocks of c_block_rows rows of C are stored, or nullptr
+  int c_block_rows;
+  long long c_stored_rows;
   int k_tiles_per_split;
   int splits;
   int m_tiles, n_tiles;
@@ -89,6 +94,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   const int lane = threadIdx.x & 31;
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
 
+  int m_rows = p.m, num_items = p.num_items, k_tiles_total = p.k_tiles_total, k_tiles_per_split = p.k_tiles_per_split;
+  if (p.limit != nullptr) {
+    const int n = *p.limit * p.limit_block;
+    if (p.limit_k) {
+      k_tiles_total = min(k_tiles_total, n / BK);
+      k_tiles_per_split = (k_tiles_total + p.splits - 1) / p.splits;
+    } else {
+      m_rows = min(m_rows, n);
+      num_items = (m_rows + BM * MT - 1) / (BM * MT) * p.n_tiles * p.splits;
+    }
+  }
+
   if (threadIdx.x == 0) {
     abort_flag = 0;
     for (int s = 0; s < C::kStages; ++s) {
@@ -116,14 +133,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     if (lane == 0) {
       uint32_t it = 0;
       bool ok = true;
-      for (int item = blockIdx.x; item < p.num_items && ok; item += gridDim.x) {
+      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
         const int split = item % p.splits;
         const int tile = item / p.splits;
         const int n0 = (tile % p.n_tiles) * BN;
         const int m0 = (tile / p.n_tiles) * (BM * MT);
-        const int kt_begin = split * p.k_tiles_per_split;
-        int kt_count = p.k_tiles_total - kt_begin;
-        if (kt_count > p.k_tiles_per_split) kt_count = p.k_tiles_per_split;
+        const int kt_begin = split * k_tiles_per_split;
+        int kt_count = k_tiles_total - kt_begin;
+        if (kt_count > k_tiles_per_split) kt_count = k_tiles_per_split;
         // Gathered A: the stored rows of this tile's boxes depend on the tile only, so the list is read once per
         // item (up to 32 boxes: 256 rows of 8), not once per K step -- a dependent global load in front of every
         // copy would pace the whole pipeline.
@@ -236,11 +253,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       const uint64_t b_step = p.b_kmajor ? (32 >> 4) : (2048 >> 4);
       uint32_t it = 0, t = 0;
       bool ok = true;
-      for (int item = blockIdx.x; item < p.num_items && ok; item += gridDim.x, ++t) {
+      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x, ++t) {
         const int split = item % p.splits;
-        const int kt_begin = split * p.k_tiles_per_split;
-        int kt_count = p.k_tiles_total - kt_begin;
-        if (kt_count > p.k_tiles_per_split) kt_count = p.k_tiles_per_split;
+        const int kt_begin = split * k_tiles_per_split;
+        int kt_count = k_tiles_total - kt_begin;
+        if (kt_count > k_tiles_per_split) kt_count = k_tiles_per_split;
         const uint32_t buf = (MT == 1) ? (t & 1) : 0;
         ok = mbar_wait_w(&acc_empty[buf], (MT == 1 ? ((t >> 1) & 1) : (t & 1)) ^ 1, &abort_flag, p.status);
         if (!ok) break;
@@ -283,21 +300,31 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     uint8_t* stage_c = tiles + C::kStages * C::kStageBytes + (warp - 2) * C::kStoreBytes;
     const uint32_t stage_row = smem_u32(stage_c) + lane * 128;
     uint32_t t = 0;
-    for (int item = blockIdx.x; item < p.num_items; item += gridDim.x, ++t) {
+    for (int item = blockIdx.x; item < num_items; item += gridDim.x, ++t) {
       const int split = item % p.splits;
       const int tile = item / p.splits;
       const int n0 = (tile % p.n_tiles) * BN;
       const int m0 = (tile / p.n_tiles) * (BM * MT) + sub * BM;
-      const int kt_begin = split * p.k_tiles_per_split;
-      const bool has_k = kt_begin < p.k_tiles_total;
+      const int kt_begin = split * k_tiles_per_split;
+      const bool has_k = kt_begin < k_tiles_total;
       const uint32_t buf = (MT == 1) ? (t & 1) : 0;
       bool have_acc = mbar_wait_w(&acc_full[buf], MT == 1 ? ((t >> 1) & 1) : (t & 1), &abort_flag, p.status);
       if (!have_acc) break;
       tc_fence_after();
       const uint32_t tmem_acc = tmem_base + (MT == 1 ? buf : static_cast<uint32_t>(sub)) * 256;
       const int row = m0 + lane_group + lane;
+      long long c_row0 = m0 + lane_group;          // where this warp's 32 rows are stored (< 0: nowhere)
+      if (p.c_row_blocks != nullptr) {
+        const int blk = (m0 + lane_group) / p.c_block_rows;
+        const int to = m0 + lane_group < m_rows ? p.c_row_blocks[blk] : -1;
+        c_row0 = static_cast<long long>(to) * p.c_block_rows + (m0 + lane_group - blk * p.c_block_rows);
+        if (to < 0 || c_row0 >= p.c_stored_rows) {
+          if (m0 + lane_group < m_rows && lane == 0) atomicMax(p.status, MOC_DEV_BAD_INDEX);
+          c_row0 = -1;
+        }
+      }
       float rs = 1.0f;
-      if (p.row_scale != nullptr && row < p.m) rs = p.row_scale[row / p.scale_block_rows];
+      if (p.row_scale != nullptr && row < m_rows) rs = p.row_scale[row / p.scale_block_rows];
 #pragma unroll 1
       for (int c = 0; c < BN / 32; ++c) {
         uint32_t r[32];
@@ -315,7 +342,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             if (lane == 0) bulk_wait_read_all();
             __syncwarp();
           }
-          if (p.residual != nullptr && row < p.m) {
+          if (p.residual != nullptr && row < m_rows) {
             const float* res = p.residual + static_cast<long long>(row) * p.ldr + col0;
 #pragma unroll
             for (int j = 0; j < 32; ++j)
@@ -337,14 +364,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           if ((c & 1) || col0 + 32 >= p.n) {
             fence_proxy_async();
             __syncwarp();
-            if (lane == 0) {
-              tma_store_2d(&tmap_c, stage_c, n0 + (c & ~1) * 32, m0 + lane_group);
+            if (lane == 0 && c_row0 >= 0) {
+              tma_store_2d(&tmap_c, stage_c, n0 + (c & ~1) * 32, static_cast<int>(c_row0));
               bulk_commit_group();
             }
           }
           continue;
         }
-        if (row >= p.m) continue;
+        if (row >= m_rows || c_row0 < 0) continue;
         if (p.residual != nullptr && split == 0) {
           // fold the row scale and the residual into the registers; the stores below then see rs = 1
           const float* res = p.residual + static_cast<long long>(row) * p.ldr + col0;
@@ -369,7 +396,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         }
         const float rs_store = (p.residual != nullptr && split == 0) ? 1.0f : rs;
         if (p.c_bf16) {
-          __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.c) + static_cast<long long>(row) * p.ldc + col0;
+          __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.c) + (c_row0 + lane) * p.ldc + col0;
           const bool vec = ((p.ldc & 7) == 0) && (col0 + 32 <= p.n) &&
                            ((reinterpret_cast<uintptr_t>(p.c) & 15) == 0);
           if (vec) {
@@ -387,7 +414,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
               if (col0 + j < p.n) dst[j] = __float2bfloat16(__uint_as_float(r[j]) * rs_store);
           }
         } else {
-          float* dst = reinterpret_cast<float*>(p.c) + static_cast<long long>(row) * p.ldc + col0;
+          float* dst = reinterpret_cast<float*>(p.c) + (c_row0 + lane) * p.ldc + col0;
           if (p.atomic) {
             const bool vec4 = ((p.ldc & 3) == 0) && (col0 + 32 <= p.n) &&
                               ((reinterpret_cast<uintptr_t>(p.c) & 15) == 0);
@@ -501,6 +528,12 @@ int launch_gemm_tc(const moc_gemm_desc* g, const void* a, const void* b, void* c
   const uint64_t a_more = static_cast<uint64_t>(terms - 1) * static_cast<uint64_t>(terms > 1 ? g->a_term_rows : 0);
   const uint64_t b_more = static_cast<uint64_t>(terms - 1) * static_cast<uint64_t>(terms > 1 ? g->b_term_rows : 0);
 
+  MOC_REQUIRE(g->limit == nullptr || (g->limit_block > 0 && (!g->limit_k || (g->limit_block % BK == 0 && terms == 1))),
+              "a K limit counts blocks of a multiple of 64");
+  MOC_REQUIRE(g->c_row_blocks == nullptr || (g->c_block_rows > 0 && g->c_block_rows % 32 == 0 && g->c_stored_rows > 0 &&
+                                             !g->accumulate && split == 1 && g->residual == nullptr),
+              "scattered rows of C come in blocks of a multiple of 32, stored once");
+
   // Tile width.  The kernel is fed from L2 (~8.4 TB/s measured over all SMs), so a tile's time goes with the
   // bytes it loads per K step, (BM + BN) * 128: the cost of a width is rounds-of-items times that.
   const int sms = sm_count();
@@ -545,7 +578,7 @@ int launch_gemm_tc(const moc_gemm_desc* g, const void* a, const void* b, void* c
   const bool c_tma = g->c_dtype == MOC_BF16 && (g->ldc % 8) == 0 && (reinterpret_cast<uintptr_t>(c) & 15) == 0;
   CUtensorMap tmap_c = tmap_a;      // placeholder when the TMA-store epilogue is not used
   if (c_tma) {
-    rc = make_tmap_bf16_2d(&tmap_c, c, static_cast<uint64_t>(g->m), static_cast<uint64_t>(g->n),
+    rc = make_tmap_bf16_2d(&tmap_c, c, static_cast<uint64_t>(g->c_row_blocks ? g->c_stored_rows : g->m), static_cast<uint64_t>(g->n),
                            static_cast<uint64_t>(g->ldc), 32, 64);
     if (rc != MOC_OK) return rc;
   }
@@ -562,6 +595,8 @@ int launch_gemm_tc(const moc_gemm_desc* g, const void* a, const void* b, void* c
   p.a_stored_rows = a_stored_rows;
   p.b_row_blocks = b_row_blocks; p.b_block_rows = b_block_rows; p.b_box_rows = b_box_rows;
   p.b_num_blocks = b_num_blocks; p.b_stored_rows = b_stored_rows;
+  p.limit = g->limit; p.limit_block = g->limit_block; p.limit_k = g->limit_k;
+  p.c_row_blocks = g->c_row_blocks; p.c_block_rows = g->c_block_rows; p.c_stored_rows = g->c_stored_rows;
   p.terms = terms; p.k_tiles_per_term = ceil_div(g->k, BK);
   p.a_term_rows = g->a_term_rows; p.b_term_rows = g->b_term_rows;
   p.k_tiles_total = terms * p.k_tiles_per_term;

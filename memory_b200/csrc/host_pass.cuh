@@ -43,6 +43,7 @@ struct Gemm : moc_gemm_desc {
     a_stored_rows = a_k ? m : k;
     residual = nullptr; ldr = 0;
     terms = 1; a_term_rows = b_term_rows = 0;
+    limit_block = limit_k = c_block_rows = 0; c_stored_rows = 0; limit = c_row_blocks = nullptr;
   }
 };
 // K-splits of a weight gradient [out_rows, out_cols] over `rows`: enough (tile, split) items to fill the SMs once

@@ -654,10 +654,31 @@ class _TokenRoutedAttention(torch.autograd.Function):
     dense attention kernel over the S*T shared rows with all B*L tokens as one sequence."""
 
     @staticmethod
+    def _native(h, shared_mem, routed_mem, idx_local, wq, wk, wv, wo, num_heads, num_kv_heads, t, cd) -> bool:
+        """Whether ``moc_token_attn_fwd`` takes the call: bf16 arithmetic, head_dim 64, whole 64-row chapters."""
+        ok = (torch.float32, torch.bfloat16)
+        return (cd == torch.bfloat16 and t == 64 and h.shape[-1] == num_heads * 64 and wk.shape[0] == num_kv_heads * 64
+                and num_heads % num_kv_heads == 0 and wq.shape == wo.shape == (h.shape[-1], h.shape[-1])
+                and wk.dtype == wq.dtype == wv.dtype == wo.dtype and wq.dtype in ok and h.dtype in ok and h.numel() > 0
+                and idx_local.shape[-1] > 0 and routed_mem is not None and routed_mem.numel() > 0
+                and routed_mem.shape[0] % 64 == 0 and routed_mem.dtype in ok
+                and (shared_mem is None or shared_mem.dtype in ok))
+
+    @staticmethod
     def forward(ctx, h, shared_mem, routed_mem, idx_local, weights, wq, wk, wv, wo, cfg):
         num_heads, num_kv_heads, t, rho, cd = cfg
         b, l, d = h.shape
         rows = b * l
+        ctx.desc = None
+        if _TokenRoutedAttention._native(h, shared_mem, routed_mem, idx_local, wq, wk, wv, wo, num_heads, num_kv_heads, t, cd):
+            need_grad = any(ctx.needs_input_grad)
+            desc, out, keep = ops.token_attn_fwd(h.reshape(rows, d), shared_mem, routed_mem, idx_local, weights, wq, wk, wv, wo,
+                                                 num_heads, num_kv_heads, rho, need_grad)
+            if need_grad:
+                ctx.desc = desc
+                ctx.meta = (tuple(h.shape), weights.dtype, tuple(weights.shape))
+                ctx.save_for_backward(*keep)
+            return out.view(b, l, -1)
         dkv = wk.shape[0]
         head_dim = d // num_heads
         scale = head_dim ** -0.5
@@ -688,17 +709,10 @@ class _TokenRoutedAttention(torch.autograd.Function):
             w2 = weights.reshape(1, rows, k_sel).float().contiguous()
             q4 = q.view(1, rows, num_heads, head_dim)
             base = None if comb is None else comb.contiguous().view(1, rows, num_heads, head_dim)
-            mix_ws = None
-            if ops.token_mix_supported(q4, k4, t, 1):
-                # tensor cores: every chapter's K / V tile stationary under the tokens that selected it
-                bidx = idx_local.reshape(1, rows, 1, k_sel).to(torch.int32).contiguous()
-                comb4, lse_slots, mix_ws = ops.token_mix_fwd(q4, k4, v4, bidx, w2, scale, base=base, out_scale=rho)
-            else:
-                bidx = idx_local.reshape(1, rows, 1, k_sel).expand(1, rows, num_kv_heads, k_sel).to(torch.int32).contiguous()
-                comb4, lse_slots = ops.sparse_attn_weighted_fwd(q4, k4, v4, bidx, w2, t, scale, base=base,
-                                                                out_scale=rho)
+            bidx = idx_local.reshape(1, rows, 1, k_sel).expand(1, rows, num_kv_heads, k_sel).to(torch.int32).contiguous()
+            comb4, lse_slots = ops.sparse_attn_weighted_fwd(q4, k4, v4, bidx, w2, t, scale, base=base, out_scale=rho)
             comb = comb4.view(rows, -1)
-            rt = (rm2, kv_rt, bidx, w2, lse_slots, n_rt, mix_ws)
+            rt = (rm2, kv_rt, bidx, w2, lse_slots, n_rt)
         if comb is None:
             comb = q.new_zeros(rows, d)
         out = ops.gemm(comb.contiguous(), wo_c, out_dtype=h.dtype if h.dtype in (torch.float32, cd) else cd, tag="o_proj")
@@ -712,6 +726,13 @@ class _TokenRoutedAttention(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
+        if ctx.desc is not None:
+            h_shape, w_dtype, w_shape = ctx.meta
+            d_h, d_sh, d_rt, d_w, d_wq, d_wkv, d_wo = ops.token_attn_bwd(ctx.desc, ctx.saved_tensors, g,
+                                                                        ctx.needs_input_grad[1], ctx.needs_input_grad[2])
+            dkv, wd = d_wkv.shape[0] // 2, ctx.saved_tensors[5].dtype
+            return (d_h.view(h_shape), d_sh, d_rt, None, _cast(d_w, w_dtype).view(w_shape), _cast(d_wq, wd),
+                    _cast(d_wkv[:dkv], wd), _cast(d_wkv[dkv:], wd), _cast(d_wo, wd), None)
         h2, q, comb, wq_c, wkv_c, wo_c = ctx.saved_tensors
         num_heads, num_kv_heads, t, rho, cd = ctx.cfg
         b, l, d, dkv, scale, h_dtype, sh_dtype, rt_dtype, w_dtype, wdt = ctx.meta
@@ -737,24 +758,17 @@ class _TokenRoutedAttention(torch.autograd.Function):
             d_wkv = ops.gemm(d_kv_sh2, sm2, a_kmajor=False, b_kmajor=False, out_dtype=f32,
                              split_k=_weight_grad_splits(cd, sm2.shape[0], 2 * dkv, d), tag="d_wkv_shared")
         if ctx.rt is not None:
-            rm2, kv_rt, bidx, w2, lse_slots, n_rt, mix_ws = ctx.rt
+            rm2, kv_rt, bidx, w2, lse_slots, n_rt = ctx.rt
             k4 = kv_rt[:, :dkv].unflatten(1, (num_kv_heads, head_dim)).unsqueeze(0)
             v4 = kv_rt[:, dkv:].unflatten(1, (num_kv_heads, head_dim)).unsqueeze(0)
-            # (the tensor-core mixture writes every row itself; the CUDA-core one adds into zeros)
-            d_kv_rt = (torch.zeros(n_rt, 2 * dkv, dtype=f32, device=q.device) if mix_ws is None
-                       else torch.empty(n_rt, 2 * dkv, dtype=cd, device=q.device))
+            d_kv_rt = torch.zeros(n_rt, 2 * dkv, dtype=f32, device=q.device)
             dk4 = d_kv_rt[:, :dkv].unflatten(1, (num_kv_heads, head_dim)).unsqueeze(0)
             dv4 = d_kv_rt[:, dkv:].unflatten(1, (num_kv_heads, head_dim)).unsqueeze(0)
             q4, dc4 = q.view(1, rows, num_heads, head_dim), d_comb.view(1, rows, num_heads, head_dim)
             d_q4 = None if d_q is None else d_q.view(1, rows, num_heads, head_dim)
-            if mix_ws is not None:
-                d_q, d_w = ops.token_mix_bwd(q4, k4, v4, bidx, w2, lse_slots, dc4, scale, rho, mix_ws, dk4, dv4,
-                                             d_q_base=d_q4)
-                d_kv_c = d_kv_rt
-            else:
-                d_q, d_w = ops.sparse_attn_weighted_bwd(q4, k4, v4, bidx, w2, lse_slots, dc4, t, scale, rho, dk4, dv4,
-                                                        d_q_accum=d_q4)
-                d_kv_c = ops.cast(d_kv_rt, cd)
+            d_q, d_w = ops.sparse_attn_weighted_bwd(q4, k4, v4, bidx, w2, lse_slots, dc4, t, scale, rho, dk4, dv4,
+                                                    d_q_accum=d_q4)
+            d_kv_c = ops.cast(d_kv_rt, cd)
             d_q = d_q.view(rows, -1)
             d_weights = d_w.view(b, l, -1).to(w_dtype)
             # written in the bank's dtype by the projection's epilogue (an fp32 master bank: no conversion pass

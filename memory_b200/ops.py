@@ -1308,3 +1308,64 @@ def token_route_bwd(s, h, arena, idx, weights, g_weights, g_losses, want_dh: boo
     _report(1 + int(want_dh) + int(want_dw) + 2 * int(want_db),
             lambda: ("router_bwd:f32",) + ("gemm:bf16",) * (int(want_dh) + int(want_dw)))
     return d_h, d_w, d_b
+
+
+# --------------------------------------------------------------------------------------------
+# token-routed attention, projections included
+# --------------------------------------------------------------------------------------------
+def token_attn_fwd(h, shared, routed, idx, weights, wq, wk, wv, wo, num_heads: int, num_kv_heads: int, routed_scale: float,
+                   for_backward: bool):
+    """``moc_token_attn_fwd`` on h [rows, d], the bank slices and chapter ids / weights [.., k] local to ``routed``.  Returns
+    (descriptor, out [rows, d] in the dtype of h, tensors to keep for :func:`token_attn_bwd`)."""
+    L.require_cuda(h, shared, routed, idx, weights, wq, wk, wv, wo)
+    rows, d = h.shape
+    k, dev, code, p = idx.shape[-1], h.device, L.dtype_code, L.ptr
+    h, routed = _contig(h), _contig(routed)
+    shared = _contig(shared) if shared is not None and shared.numel() > 0 else None
+    ids = _contig(idx.to(torch.int32))
+    w = _contig(weights.float())
+    wq, wk, wv, wo = (_contig(t) for t in (wq, wk, wv, wo))
+    if ids.numel() != rows * k or w.numel() != rows * k:
+        raise ValueError("chapter ids and weights must be given for every token")
+    for name, t in (("shared_memory", shared), ("routed_memory", routed), ("wk", wk), ("wv", wv)):
+        if t is not None and (t.dim() != 2 or t.shape[1] != d):
+            raise ValueError(f"inner dimensions differ: {name} {tuple(t.shape)} vs {d}")
+    s = L.TokenAttnDesc(rows, d, num_heads, num_kv_heads, k, 0 if shared is None else shared.shape[0], routed.shape[0],
+                        code(h.dtype), code(h.dtype if shared is None else shared.dtype), code(routed.dtype), code(wq.dtype),
+                        code(h.dtype), int(for_backward), routed_scale, p(h), p(shared), p(routed), p(ids), p(w), p(wq), p(wk),
+                        p(wv), p(wo), None, None, p(L.status_word(dev)), L.stream_ptr(dev))
+    out = torch.empty(rows, d, dtype=h.dtype, device=dev)
+    arena = torch.empty(_size("moc_token_attn_arena_bytes", s), dtype=torch.uint8, device=dev)
+    scratch = torch.empty(_size("moc_token_attn_fwd_scratch_bytes", s), dtype=torch.uint8, device=dev)
+    s.out, s.arena = p(out), p(arena)
+    L.check(_timed("token_attn_fwd", lambda: L.lib().moc_token_attn_fwd(C.byref(s), p(scratch))), "moc_token_attn_fwd")
+    parts = ["gemm:bf16"] * 3 + ["token_mix_fwd:bf16"] + (["gemm:bf16", "attn_fwd:bf16"] if shared is not None else [])
+    _report(11 + 2 * int(shared is not None) + int(rows * k < 2 * (routed.shape[0] // 64)) * 4, lambda: parts)
+    return s, out, (h, shared, routed, ids, w, wq, arena)
+
+
+def token_attn_bwd(s, keep, g, want_shared: bool, want_routed: bool):
+    """``moc_token_attn_bwd`` on the forward call's descriptor; returns (d_h, d_shared, d_routed, d_weights [rows, k], d_wq,
+    d_wkv (K rows, then V rows), d_wo), the weight gradients in fp32."""
+    h, shared, routed, ids, w, wq, arena = keep
+    p, dev, f32 = L.ptr, h.device, torch.float32
+    g = _contig(g.reshape(s.rows, s.hidden_dim))
+    s.h, s.shared, s.routed, s.idx, s.weights, s.arena = p(h), p(shared), p(routed), p(ids), p(w), p(arena)
+    s.stream = L.stream_ptr(dev)
+    d = s.hidden_dim
+    d_h = torch.empty_like(h)
+    d_shared = torch.empty_like(shared) if shared is not None and want_shared else None
+    d_routed = torch.empty_like(routed) if want_routed else None
+    d_w = torch.empty(s.rows, s.n_select, dtype=f32, device=dev)
+    d_wq = torch.empty(d, d, dtype=f32, device=dev)
+    d_wkv = torch.empty(2 * s.num_kv_heads * 64, d, dtype=f32, device=dev)
+    d_wo = torch.empty(d, d, dtype=f32, device=dev)
+    b = L.TokenAttnBwdDesc(L.dtype_code(g.dtype), p(g), p(d_h), p(d_shared), p(d_routed), p(d_w), p(d_wq), p(d_wkv), p(d_wo), None)
+    scratch = torch.empty(_size("moc_token_attn_bwd_scratch_bytes", s, b), dtype=torch.uint8, device=dev)
+    b.scratch = p(scratch)
+    L.check(_timed("token_attn_bwd", lambda: L.lib().moc_token_attn_bwd(C.byref(s), C.byref(b))), "moc_token_attn_bwd")
+    parts = ["gemm:bf16"] * (5 + int(want_routed)) + ["token_mix_bwd:bf16"]
+    if shared is not None:
+        parts += ["attn_bwd:bf16"] + ["gemm:bf16"] * (1 + int(want_shared))
+    _report(len(parts) + 3 + 2 * int(shared is not None), lambda: parts)
+    return d_h, d_shared, d_routed, d_w, d_wq, d_wkv, d_wo

@@ -111,3 +111,47 @@ def test_token_router_shapes(dev, rows, c, d, k, s):
     (0.3 * lb + 0.2 * zl + 0.1 * ent + (w_ref * g[0].double()).sum()).backward()
     assert _rel(wt[0], w_ref) < 1e-5
     assert _rel(w.grad, w64.grad) < 1e-4 and _rel(bias.grad, b64.grad) < 1e-4 and _rel(h.grad, h64.grad) < 1e-2
+
+
+@pytest.mark.parametrize("rows,k,m,s,h,hk,bank_dtype", [(8, 1, 300, 2, 4, 2, torch.float32), (136, 3, 205, 0, 2, 2, torch.bfloat16),
+                                                        (72, 5, 180, 1, 3, 1, torch.float32), (72, 5, 181, 1, 3, 1, torch.bfloat16),
+                                                        (600, 2, 7, 1, 2, 1, torch.float32)])
+def test_token_attention_over_listed_chapters(dev, rows, k, m, s, h, hk, bank_dtype):
+    """Few selections (only the chapters somebody selected are projected) and many, on both sides of the line between them."""
+    import memory_b200 as M
+    torch.manual_seed(rows + m)
+    d, dkv = h * 64, hk * 64
+    rnd = lambda *shape, std=1.0, dtype=torch.float32: (torch.randn(*shape, device=dev) * std).to(dtype).requires_grad_(True)
+    x = rnd(1, rows, d, dtype=torch.bfloat16)
+    shared, routed = (rnd(s * 64, d, dtype=bank_dtype) if s else None), rnd(m * 64, d, dtype=bank_dtype)
+    wq, wk, wv, wo = rnd(d, d, std=0.1), rnd(dkv, d, std=0.1), rnd(dkv, d, std=0.1), rnd(d, d, std=0.1)
+    idx = torch.rand(rows, m, device=dev).topk(k, 1).indices.int().view(1, rows, k)
+    u = torch.rand(1, rows, k, device=dev).requires_grad_(True)
+    leaves = [t for t in (x, shared, routed, u, wq, wk, wv, wo) if t is not None]
+    g = torch.randn(1, rows, d, device=dev).bfloat16()
+
+    def grads(out):
+        return [out] + list(torch.autograd.grad(out, leaves, g.to(out.dtype)))
+
+    got = grads(M.token_routed_attention(x, shared, routed, idx, u, wq, wk, wv, wo, num_heads=h, num_kv_heads=hk,
+                                         tokens_per_chapter=64, routed_scale=2.5, compute_dtype=torch.bfloat16))
+    q = (x[0].float() @ wq.t()).view(rows, h, 64)
+
+    def heads(mem):
+        kv = [(mem.float() @ w.t()).view(-1, hk, 64).repeat_interleave(h // hk, 1) for w in (wk, wv)]
+        return kv
+
+    out = torch.zeros(rows, h, 64, device=dev)
+    if s:
+        ks, vs = heads(shared)
+        out = torch.einsum("thn,nhd->thd", (torch.einsum("thd,nhd->thn", q, ks) * 0.125).softmax(-1), vs)
+    kr, vr = (t.view(m, 64, h, 64) for t in heads(routed))
+    for j in range(k):
+        c = idx[0, :, j].long()
+        p = (torch.einsum("thd,tnhd->thn", q, kr[c]) * 0.125).softmax(-1)
+        out = out + 2.5 * u[0, :, j, None, None] * torch.einsum("thn,tnhd->thd", p, vr[c])
+    want = grads((out.reshape(rows, d) @ wo.t()).view(1, rows, d))
+    for i, (a, b) in enumerate(zip(got, want)):
+        assert _rel(a, b) < 2e-2, i
+    from memory_b200 import _lib as L
+    L.check_device_status(dev)
