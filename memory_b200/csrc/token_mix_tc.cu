@@ -204,6 +204,26 @@ __device__ __forceinline__ void gather_row(uint8_t* tile, int r, const __nv_bflo
   for (int j = 0; j < 8; ++j) *reinterpret_cast<uint4*>(tile + r * 128 + ((j ^ (r & 7)) << 4)) = v[j];
 }
 
+// Rows of 128 bytes (64 bf16) that lie scattered in global memory move between it and 128-byte-swizzled tiles by eight
+// lanes a row: the four row-owning warps take 16 rows per pass, whole lines at a time.  kAhead passes (64 rows, more than most
+// chapters have pairs) can be requested into registers before the tile is free.
+constexpr int kAhead = 4;
+__device__ __forceinline__ int move_row(int pass) { return (static_cast<int>(threadIdx.x) >> 3) + 16 * pass; }
+__device__ __forceinline__ uint32_t tile_at(int r, int piece) { return r * 128 + ((piece ^ (r & 7)) << 4); }
+__device__ __forceinline__ uint4 load_piece(const __nv_bfloat16* src, long long row_stride, int col, const int* tok, int r, int cnt) {
+  if (r >= cnt) return make_uint4(0u, 0u, 0u, 0u);
+  return *reinterpret_cast<const uint4*>(src + tok[r] * row_stride + col + (threadIdx.x & 7) * 8);
+}
+__device__ __forceinline__ void put_piece(uint8_t* tile, int r, const uint4& v) {
+  *reinterpret_cast<uint4*>(tile + tile_at(r, threadIdx.x & 7)) = v;
+}
+__device__ __forceinline__ void row_warps_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+// one arrival per warp for what all its lanes have done
+__device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
+  __syncwarp();
+  if (lane == 0) mbar_arrive(bar);
+}
+
 struct MixShape {
   int B, TQ, TK, HQ, HK, HI, S, M;
   float scale, scale_log2, out_scale;
@@ -220,7 +240,7 @@ struct MixFwdParams {
   int* status;
 };
 constexpr int kMixThreads = 160;                       // 4 row-owning warps + 1 control warp (TMA, MMA issue)
-constexpr int kFwdSmem = kTileQ + 2 * kTileKV + 1024;
+constexpr int kFwdSmem = 2 * kTileQ + 2 * kTileKV + 1024;
 
 __global__ void __launch_bounds__(kMixThreads, 4)
 token_mix_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
@@ -229,17 +249,19 @@ token_mix_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
   __shared__ __align__(8) uint64_t kv_bar, q_ready, s_bar, p_bar, o_bar;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
+  __shared__ int tok[2][kTok], slot[2][kTok];        // of a tile's pairs (two tiles: a slow warp may still read the last)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* q_s = base;
   uint8_t* k_s = base + kTileQ;
   uint8_t* v_s = k_s + kTileKV;
+  uint8_t* o_s = v_s + kTileKV;
   const MixShape& x = p.x;
   const int G = x.HQ / x.HK;
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
-    mbar_init(&kv_bar, 1); mbar_init(&q_ready, kTok); mbar_init(&s_bar, 1); mbar_init(&p_bar, kTok);
+    mbar_init(&kv_bar, 1); mbar_init(&q_ready, 4); mbar_init(&s_bar, 1); mbar_init(&p_bar, 4);
     mbar_init(&o_bar, 1);
     fence_mbar_init();
     prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v);
@@ -249,7 +271,7 @@ token_mix_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
   const int n_tiles = p.totals[0];
-  uint32_t it = 0, kvn = 0;
+  uint32_t it = 0, kvn = 0, tile_no = 0;
   bool ok = true;
 
   for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
@@ -288,54 +310,80 @@ token_mix_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
     } else {
       const int r = threadIdx.x;
       const uint32_t lane_sel = static_cast<uint32_t>(warp * 32) << 16;
-      const bool valid = r < cnt;
-      const int pair = valid ? p.entries[first + r] : 0;
-      const int s = pair % x.S;
-      const long long tokrow = (pair / x.S) / x.HI;
-      const float wv = valid ? p.w[tokrow * x.S + s] : 0.f;
+      const bool valid = r < cnt, active = warp * 32 < cnt;      // (a warp without pairs only moves rows)
+      const int rows32 = (cnt + 31) & ~31;
+      int *tk = tok[tile_no & 1], *sl = slot[tile_no & 1];
+      ++tile_no;
+      float wv = 0.f;
+      long long lse_at = 0;
+      if (valid) {
+        const int pair = p.entries[first + r];
+        const int s = pair % x.S, t = (pair / x.S) / x.HI;
+        tk[r] = t; sl[r] = s;
+        wv = p.w[static_cast<long long>(t) * x.S + s];
+        lse_at = static_cast<long long>(t) * x.HQ * x.S + s;
+      }
+      row_warps_sync();
+      uint4 ahead[kAhead];
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) ahead[i] = load_piece(p.q, x.HQ * kD, hq_lo * kD, tk, move_row(i), cnt);
       for (int hq = hq_lo; hq < hq_hi && ok; ++hq, ++it) {
-        gather_row(q_s, r, p.q + tokrow * (x.HQ * kD) + hq * kD, valid);
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i)
+          if (move_row(i) < rows32) put_piece(q_s, move_row(i), ahead[i]);
+        for (int i = kAhead; 16 * i < rows32; ++i)
+          if (move_row(i) < rows32) put_piece(q_s, move_row(i), load_piece(p.q, x.HQ * kD, hq * kD, tk, move_row(i), cnt));
         fence_proxy_async();
-        mbar_arrive(&q_ready);
-        ok = mbar_wait_w(&s_bar, it & 1, &abort_flag, p.status);
-        if (!ok) break;
-        tc_fence_after();
-        float m, l = 0.f;
-        {
-          uint32_t s0[32], s1[32], pk[32];
-          tmem_ld32(tmem + lane_sel, s0);
-          tmem_ld32(tmem + lane_sel + 32, s1);
-          tmem_wait_ld();
-          m = __uint_as_float(s0[0]);
+        warp_arrive(&q_ready, lane);
+        float m = 0.f, l = 1.f;
+        if (active) {
+          ok = mbar_wait_w(&s_bar, it & 1, &abort_flag, p.status);
+          if (!ok) break;
+          tc_fence_after();
+          // S is read twice, half a row at a time: both halves in registers would spill
+          m = -INFINITY;
 #pragma unroll
-          for (int i = 0; i < 32; ++i) m = fmaxf(m, fmaxf(__uint_as_float(s0[i]), __uint_as_float(s1[i])));
-          const float mm = m * x.scale_log2;
+          for (int half = 0; half < 2; ++half) {
+            uint32_t sv[32];
+            tmem_ld32(tmem + lane_sel + half * 32, sv);
+            tmem_wait_ld();
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const float a0 = ex2(fmaf(__uint_as_float(s0[i]), x.scale_log2, -mm));
-            const float a1 = ex2(fmaf(__uint_as_float(s0[i + 1]), x.scale_log2, -mm));
-            const float b0 = ex2(fmaf(__uint_as_float(s1[i]), x.scale_log2, -mm));
-            const float b1 = ex2(fmaf(__uint_as_float(s1[i + 1]), x.scale_log2, -mm));
-            l += (a0 + a1) + (b0 + b1);
-            pk[i / 2] = pack_bf16x2(a0, a1);
-            pk[16 + i / 2] = pack_bf16x2(b0, b1);
+            for (int i = 0; i < 32; ++i) m = fmaxf(m, __uint_as_float(sv[i]));
           }
-          tmem_st32(tmem + lane_sel, pk);          // P over the first half of S's columns (own lanes only)
+          const float mm = m * x.scale_log2;
+          l = 0.f;
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            uint32_t sv[32], pk[16];
+            tmem_ld32(tmem + lane_sel + half * 32, sv);
+            tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) {
+              const float a0 = ex2(fmaf(__uint_as_float(sv[i]), x.scale_log2, -mm));
+              const float a1 = ex2(fmaf(__uint_as_float(sv[i + 1]), x.scale_log2, -mm));
+              l += a0 + a1;
+              pk[i / 2] = pack_bf16x2(a0, a1);
+            }
+            tmem_st16(tmem + lane_sel + half * 16, pk);   // P over the first half of S's columns (own lanes only)
+          }
           tmem_wait_st();
+          tc_fence_before();
         }
-        tc_fence_before();
-        mbar_arrive(&p_bar);
+        warp_arrive(&p_bar, lane);
+        if (hq + 1 < hq_hi) {                      // lands under P V
+#pragma unroll
+          for (int i = 0; i < kAhead; ++i) ahead[i] = load_piece(p.q, x.HQ * kD, (hq + 1) * kD, tk, move_row(i), cnt);
+        }
         ok = mbar_wait_w(&o_bar, it & 1, &abort_flag, p.status);
         if (!ok) break;
-        tc_fence_after();
-        const float f = x.out_scale * wv / l;
-        __nv_bfloat16* dst = p.partial + ((tokrow * x.S + s) * x.HQ + hq) * kD;
+        if (active) {
+          tc_fence_after();
+          const float f = x.out_scale * wv / l;
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          uint32_t o[32];
-          tmem_ld32(tmem + lane_sel + 64 + half * 32, o);
-          tmem_wait_ld();
-          if (valid) {
+          for (int half = 0; half < 2; ++half) {
+            uint32_t o[32];
+            tmem_ld32(tmem + lane_sel + 64 + half * 32, o);
+            tmem_wait_ld();
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               uint4 v;
@@ -343,12 +391,19 @@ token_mix_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
               v.y = pack_bf16x2(__uint_as_float(o[8 * j + 2]) * f, __uint_as_float(o[8 * j + 3]) * f);
               v.z = pack_bf16x2(__uint_as_float(o[8 * j + 4]) * f, __uint_as_float(o[8 * j + 5]) * f);
               v.w = pack_bf16x2(__uint_as_float(o[8 * j + 6]) * f, __uint_as_float(o[8 * j + 7]) * f);
-              *reinterpret_cast<uint4*>(dst + half * 32 + j * 8) = v;
+              *reinterpret_cast<uint4*>(o_s + tile_at(r, half * 4 + j)) = v;
             }
           }
+          if (valid) p.lse_slots[lse_at + static_cast<long long>(hq) * x.S] = fmaf(m, x.scale, __logf(l));
+          tc_fence_before();
         }
-        if (valid) p.lse_slots[(tokrow * x.HQ + hq) * x.S + s] = fmaf(m, x.scale, __logf(l));
-        tc_fence_before();
+        row_warps_sync();
+        for (int i = 0; 16 * i < cnt; ++i) {
+          const int rr = move_row(i), piece = threadIdx.x & 7;
+          if (rr < cnt)
+            *reinterpret_cast<uint4*>(p.partial + ((static_cast<long long>(tk[rr]) * x.S + sl[rr]) * x.HQ + hq) * kD + piece * 8) =
+                *reinterpret_cast<const uint4*>(o_s + tile_at(rr, piece));
+        }
       }
     }
   }
@@ -410,45 +465,43 @@ struct MixBwdParams {
   __nv_bfloat16 *d_k, *d_v;      // rows b*TK + key, row stride dkv_ld elements; head kh at column kh*64
   long long dkv_ld;
   const int *entries, *bucket_off;
-  int n_buckets;
+  int n_items, runs;             // (bucket, run of KV heads), runs per bucket
   MixShape x;
   int* status;
 };
 constexpr int kBwdSmem = 4 * kTileQ + 4 * kTileKV + 1024;
 constexpr uint32_t kColS = 0, kColDP = 64, kColD = 128;      // dQ reuses S's columns
 
-// The (chapter bucket, KV head) groups a CTA works through: buckets blockIdx.x, + gridDim.x, ... that hold pairs,
-// and for each the KV heads that read its index list.  The control warp and the row warps walk the same sequence.
+// The (chapter bucket, KV head) groups a CTA works through: items blockIdx.x, + gridDim.x, ... that hold pairs, an item being
+// a run of at most kRunHeads of the KV heads that read a bucket's list (whole buckets leave the CTAs up to 14 % apart at 32
+// pairs a chapter).  The control warp and the row warps walk the same sequence.
+constexpr int kRunHeads = 4;
 struct GroupIter {
-  int bkt, kh, kh_hi, first, n, kv_row;
-  // first non-empty bucket at or after bkt; with zero_row >= 0 (thread index of a row-owning thread) the dK / dV rows
-  // of the empty buckets passed on the way are zero-filled, so the caller need not clear the buffers
+  int item, kh, kh_hi, first, n, kv_row;
+  // first non-empty item at or after `item`; with zero_row >= 0 (thread index of a row-owning thread) the dK / dV rows
+  // of the empty ones passed on the way are zero-filled, so the caller need not clear the buffers
   __device__ __forceinline__ void seek(const MixBwdParams& p, int zero_row = -1) {
-    for (; bkt < p.n_buckets; bkt += gridDim.x) {
+    const MixShape& x = p.x;
+    for (; item < p.n_items; item += gridDim.x) {
+      const int bkt = item / p.runs, run = item - bkt * p.runs;
+      const int c = bkt % x.M, bh = bkt / x.M, hi = bh % x.HI, b = bh / x.HI;
+      kh = x.HI == 1 ? run * kRunHeads : hi;
+      kh_hi = x.HI == 1 ? min(x.HK, kh + kRunHeads) : hi + 1;
+      kv_row = b * x.TK + c * kKeys;
       first = p.bucket_off[bkt];
       n = p.bucket_off[bkt + 1] - first;
       if (n > 0) break;
       if (zero_row >= 0) {
-        const MixShape& x = p.x;
-        const int c = bkt % x.M, bh = bkt / x.M, hi = bh % x.HI, b = bh / x.HI;
-        const int h0 = x.HI == 1 ? 0 : hi, h1 = x.HI == 1 ? x.HK : hi + 1;
-        __nv_bfloat16* dst = (zero_row >= 64 ? p.d_k : p.d_v) +
-                             (static_cast<long long>(b) * x.TK + c * kKeys + (zero_row & 63)) * p.dkv_ld;
-        for (int e = h0 * (kD / 8); e < h1 * (kD / 8); ++e) reinterpret_cast<uint4*>(dst)[e] = make_uint4(0u, 0u, 0u, 0u);
+        __nv_bfloat16* dst = (zero_row >= 64 ? p.d_k : p.d_v) + (static_cast<long long>(kv_row) + (zero_row & 63)) * p.dkv_ld;
+        for (int e = kh * (kD / 8); e < kh_hi * (kD / 8); ++e) reinterpret_cast<uint4*>(dst)[e] = make_uint4(0u, 0u, 0u, 0u);
       }
     }
-    if (bkt >= p.n_buckets) return;
-    const MixShape& x = p.x;
-    const int c = bkt % x.M, bh = bkt / x.M, hi = bh % x.HI, b = bh / x.HI;
-    kh = x.HI == 1 ? 0 : hi;
-    kh_hi = x.HI == 1 ? x.HK : hi + 1;
-    kv_row = b * x.TK + c * kKeys;
   }
-  __device__ __forceinline__ void start(const MixBwdParams& p, int zero_row = -1) { bkt = blockIdx.x; seek(p, zero_row); }
-  __device__ __forceinline__ bool done(const MixBwdParams& p) const { return bkt >= p.n_buckets; }
+  __device__ __forceinline__ void start(const MixBwdParams& p, int zero_row = -1) { item = blockIdx.x; seek(p, zero_row); }
+  __device__ __forceinline__ bool done(const MixBwdParams& p) const { return item >= p.n_items; }
   __device__ __forceinline__ void next(const MixBwdParams& p, int zero_row = -1) {
     if (++kh < kh_hi) return;
-    bkt += gridDim.x;
+    item += gridDim.x;
     seek(p, zero_row);
   }
 };
@@ -715,7 +768,7 @@ int check_shape(const moc_sparse_attn_shape* s, int index_heads, MixShape* x) {
   MOC_REQUIRE(s->tk % kKeys == 0 && s->n_select > 0, "whole chapters only");
   const long long n_pairs = static_cast<long long>(s->batch) * s->tq * index_heads * s->n_select;
   const long long n_buckets = static_cast<long long>(s->batch) * index_heads * (s->tk / kKeys);
-  MOC_REQUIRE(n_pairs < (1ll << 31) && n_buckets < (1ll << 30), "too many (token, slot) pairs for 32-bit pair ids");
+  MOC_REQUIRE(n_pairs < (1ll << 31) && n_buckets * s->h < (1ll << 30), "too many (token, slot) pairs for 32-bit pair ids");
   x->B = s->batch; x->TQ = s->tq; x->TK = s->tk; x->HQ = s->hq; x->HK = s->h; x->HI = index_heads;
   x->S = s->n_select; x->M = s->tk / kKeys;
   x->scale = s->scale; x->scale_log2 = s->scale * kLog2e; x->out_scale = 1.f;
@@ -821,14 +874,16 @@ extern "C" int moc_token_mix_bwd(const moc_sparse_attn_shape* s, int32_t index_h
   p.w = weights; p.lse_slots = lse_slots;
   p.dq_partial = static_cast<__nv_bfloat16*>(dq_partial); p.d_w_heads = d_w_heads;
   p.d_k = static_cast<__nv_bfloat16*>(d_k); p.d_v = static_cast<__nv_bfloat16*>(d_v); p.dkv_ld = dkv_row_stride;
-  p.entries = ib.entries; p.bucket_off = ib.bucket_off; p.n_buckets = static_cast<int>(n_buckets);
+  p.entries = ib.entries; p.bucket_off = ib.bucket_off;
+  p.runs = x.HI == 1 ? (x.HK + kRunHeads - 1) / kRunHeads : 1;
+  p.n_items = static_cast<int>(n_buckets) * p.runs;
   p.x = x; p.status = status;
   static bool attr_set = false;
   if (!attr_set) {
     MOC_CUDA_OK(cudaFuncSetAttribute(token_mix_bwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem));
     attr_set = true;
   }
-  const long long grid = std::min<long long>(n_buckets, static_cast<long long>(sm_count()) * 2);
+  const long long grid = std::min<long long>(p.n_items, static_cast<long long>(sm_count()) * 2);
   token_mix_bwd_tc_kernel<<<static_cast<int>(grid), kMixThreads, kBwdSmem, st>>>(mk, mv, p);
   const long long rows = static_cast<long long>(x.B) * x.TQ;
   const long long threads = rows * x.HQ * (kD / 8);
