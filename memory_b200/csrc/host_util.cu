@@ -32,19 +32,19 @@ static EncodeTiledFn encode_fn() {
   return fn;
 }
 
-int make_tmap_bf16_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,
-                      uint64_t row_stride_elems, uint32_t box_rows, uint32_t box_cols) {
+static int make_tmap_2d(CUtensorMap* map, CUtensorMapDataType type, uint32_t esize, const void* base, uint64_t rows,
+                        uint64_t cols, uint64_t row_stride_elems, uint32_t box_rows, uint32_t box_cols) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) {
     set_last_error("cuTensorMapEncodeTiled", "driver entry point not found");
     return MOC_ERR_CUDA;
   }
-  MOC_REQUIRE(box_cols * 2 == 128, "tile rows must be 128 bytes for the 128-byte swizzle");
+  MOC_REQUIRE(box_cols * esize == 128, "tile rows must be 128 bytes for the 128-byte swizzle");
   MOC_REQUIRE(box_rows >= 1 && box_rows <= 256, "box rows out of range");
   MOC_REQUIRE((reinterpret_cast<uintptr_t>(base) & 15) == 0, "tensor base must be 16-byte aligned");
-  MOC_REQUIRE((row_stride_elems * 2) % 16 == 0, "row stride must be a multiple of 16 bytes");
+  MOC_REQUIRE((row_stride_elems * esize) % 16 == 0, "row stride must be a multiple of 16 bytes");
   cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {row_stride_elems * 2};
+  cuuint64_t strides[1] = {row_stride_elems * esize};
   cuuint32_t box[2] = {box_cols, box_rows};
   cuuint32_t estr[2] = {1, 1};
   // The encoder is a driver-API call and needs a context current on the calling thread.  A thread that has made no
@@ -57,7 +57,7 @@ int make_tmap_bf16_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_
     if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) cudaFree(nullptr);
     context_bound = true;
   }
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+  CUresult r = fn(map, type, 2, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
@@ -72,6 +72,14 @@ int make_tmap_bf16_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_
     return MOC_ERR_CUDA;
   }
   return MOC_OK;
+}
+int make_tmap_bf16_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,
+                      uint64_t row_stride_elems, uint32_t box_rows, uint32_t box_cols) {
+  return make_tmap_2d(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, rows, cols, row_stride_elems, box_rows, box_cols);
+}
+int make_tmap_f32_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,
+                     uint64_t row_stride_elems, uint32_t box_rows, uint32_t box_cols) {
+  return make_tmap_2d(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, rows, cols, row_stride_elems, box_rows, box_cols);
 }
 
 // One CTA whose first warp waits, with the library's bounded wait, on an mbarrier that `arrivals` of the
