@@ -441,7 +441,7 @@ int moc_roll_window(const void* cache, int64_t cache_stride, int32_t cache_rows,
 
 /* One decoding step of a memory layer in one call: router on routing_states, query projection of hidden
  * [batch * n_q, hidden_dim] (hidden_dtype), moc_decode_attn, output projection into out [batch * n_q, out_dim]
- * (hidden_dtype).  wq / wo bf16. */
+ * (hidden_dtype).  wq / wo bf16.  The query projection runs on side_stream beside the router where it is long enough. */
 typedef struct {
   moc_router_shape router;
   moc_decode_shape attn;
@@ -456,7 +456,7 @@ typedef struct {
   float* comb_w;
   void *out, *arena;
   int32_t* status;
-  void* stream;
+  void *stream, *side_stream;
 } moc_decode_step_desc;
 int64_t moc_decode_step_arena_bytes(const moc_decode_step_desc* s);
 int moc_decode_step(const moc_decode_step_desc* s);

@@ -91,7 +91,8 @@ class TokenAttnBwdDesc(C.Structure):
 class DecodeStepDesc(C.Structure):
     _fields_ = [("router", RouterShape), ("attn", DecodeShape)] + _fields(
         "i: hidden_dtype out_dim; l: bank_rows;"
-        "p: routing_states hidden router_w router_b wq wo kv_bank idx weights comb_idx comb_w out arena status stream")
+        "p: routing_states hidden router_w router_b wq wo kv_bank idx weights comb_idx comb_w out arena status stream"
+        " side_stream")
 
 
 class LayerDesc(C.Structure):

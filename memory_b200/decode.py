@@ -100,6 +100,7 @@ class MemoryDecoder:
         cd = torch.bfloat16
         self.wq_c, self.wo_c = ops.cast(wq.contiguous(), cd), ops.cast(wo.contiguous(), cd)
         self.scale = (wq.shape[0] // self.num_heads) ** -0.5
+        self._plans: dict = {}
 
     def step(self, hidden_states: torch.Tensor, routing_states: torch.Tensor) -> Tuple[torch.Tensor, dict]:
         """``hidden_states`` [B, n_q, d]: the tokens being decoded (input of the cross attention);
@@ -108,5 +109,6 @@ class MemoryDecoder:
         out, idx, w, cidx, cw = ops.decode_step(
             hidden_states, routing_states, self.router_weight, self.router_bias, self.wq_c, self.wo_c, self.cache.kv_bank,
             num_heads=self.num_heads, num_kv_heads=self.num_kv_heads, tokens_per_chapter=self.cache.tokens_per_chapter,
-            top_k=self.top_k, num_shared=self.num_shared, routed_scale=self.routed_scale, scale=self.scale)
+            top_k=self.top_k, num_shared=self.num_shared, routed_scale=self.routed_scale, scale=self.scale,
+            plans=self._plans)
         return out, {"indices": idx, "weights": w, "combined_indices": cidx, "combined_weights": cw}

@@ -1209,63 +1209,86 @@ def roll_window(cache: torch.Tensor, h: torch.Tensor, rows: int) -> Optional[tor
     """The last ``rows`` positions of ``cat([cache, h], dim=1)`` as a new [B, rows, d] tensor, or None where the rows are
     no whole 16-byte pieces of CUDA memory (the caller concatenates)."""
     b, d = h.shape[0], h.shape[2]
-    size = h.element_size()
-    if (not h.is_cuda or h.device != cache.device or h.dtype != cache.dtype or cache.shape[0] != b or cache.shape[2] != d
-            or d * size % 16 or b == 0 or b > 65535):
+    size, dev = h.element_size(), h.device
+    cb, n, cd = cache.shape
+    if not h.is_cuda or dev != cache.device or h.dtype != cache.dtype or cb != b or cd != d or d * size % 16 or b == 0 or b > 65535:
         return None
-    for t in (cache, h):
-        sb, st, sd = t.stride()
-        if (sd != 1 and d > 1) or (st != d and t.shape[1] > 1) or sb * size % 16 or t.data_ptr() % 16:
-            return None
-    out = torch.empty(b, rows, d, dtype=h.dtype, device=h.device)
-    rc = _timed("roll_window", lambda: L.lib().moc_roll_window(
-        cache.data_ptr(), cache.stride(0) * size, cache.shape[1], h.data_ptr(), h.stride(0) * size, h.shape[1], out.data_ptr(),
-        rows, b, d * size, L.stream_ptr(h.device)))
-    L.check(rc, "moc_roll_window")
+    (c0, c1, c2), (h0, h1, h2), h_rows = cache.stride(), h.stride(), h.shape[1]
+    cp, hp = cache.data_ptr(), h.data_ptr()
+    if (((c2 != 1 or h2 != 1) and d > 1) or (c1 != d and n > 1) or (h1 != d and h_rows > 1)
+            or (c0 * size | h0 * size | cp | hp) % 16):
+        return None
+    out = torch.empty((b, rows, d), dtype=h.dtype, device=dev)
+    args = (cp, c0 * size, n, hp, h0 * size, h_rows, out.data_ptr(), rows, b, d * size, L.stream_ptr(dev))
+    rc = L.lib().moc_roll_window(*args) if TIMER is None else _timed("roll_window", lambda: L.lib().moc_roll_window(*args))
+    if rc:
+        L.check(rc, "moc_roll_window")
     _report(1, lambda: ("roll_window:" + _DTYPE_TAG.get(h.dtype, str(h.dtype)),))
     return out
+
+
+_DECODE_PLANS_MAX = 32
 
 
 def decode_step(hidden: torch.Tensor, routing_states: torch.Tensor, router_w: torch.Tensor,
                 router_b: Optional[torch.Tensor], wq: torch.Tensor, wo: torch.Tensor, kv_bank: torch.Tensor, *,
                 num_heads: int, num_kv_heads: int, tokens_per_chapter: int, top_k: int, num_shared: int,
-                routed_scale: float, scale: float):
+                routed_scale: float, scale: float, plans: Optional[dict] = None):
     """One decoding step (``moc_decode_step``): out [B, n_q, d] in the dtype of ``hidden``, then indices int64, weights,
-    combined indices int32 and combined weights of the router."""
-    L.require_cuda(hidden, routing_states, router_w, router_b, wq, wo, kv_bank)
-    if routing_states.dim() != 3:
-        raise ValueError(f"hidden_states must be 3D (B, T, D), got shape {tuple(routing_states.shape)}")
-    b, n_q, d = hidden.shape
-    rb, window, rd = routing_states.shape
-    c, head_dim, dev = router_w.shape[0], wq.shape[0] // num_heads, hidden.device
-    if wq.shape[1] != d or wo.shape[1] != wq.shape[0]:
-        raise ValueError(f"inner dimensions differ: {d} / {wq.shape[0]} vs {wq.shape[1]} / {wo.shape[1]}")
-    if rd != router_w.shape[1]:
-        raise ValueError(f"inner dimensions differ: {rd} vs {router_w.shape[1]}")
-    if kv_bank.shape[1] != 2 * num_kv_heads * head_dim:
-        raise ValueError("kv_bank must be [rows, 2 * num_kv_heads * head_dim]")
-    if rb != b:
-        raise ValueError("hidden_states and routing_states must share the batch")
-    k = router_selected_k(c, top_k, num_shared)
-    f32 = torch.float32
-    h, states, w = _contig(hidden), _contig(routing_states), _contig(router_w.float())
+    combined indices int32 and combined weights of the router.  ``plans``: a dict the caller keeps; descriptors of calls
+    that agree in shapes, types and weights (by address) are filled once."""
+    w = _contig(router_w.float())
     bias = None if router_b is None else _contig(router_b.float())
-    out = torch.empty(b, n_q, wo.shape[0], dtype=h.dtype, device=dev)
-    idx = torch.empty(b, k, dtype=torch.int64, device=dev)
-    weights = torch.empty(b, k, dtype=f32, device=dev)
-    comb_idx = torch.empty(b, num_shared + k, dtype=torch.int32, device=dev)
-    comb_w = torch.empty(b, num_shared + k, dtype=f32, device=dev)
-    p = L.ptr
-    s = L.DecodeStepDesc(
-        L.RouterShape(b, window, rd, c, top_k, num_shared, routed_scale, L.dtype_code(states.dtype)),
-        L.DecodeShape(b, n_q, num_heads, num_kv_heads, head_dim, num_shared + k, tokens_per_chapter, scale),
-        L.dtype_code(h.dtype), wo.shape[0], kv_bank.shape[0], p(states), p(h), p(w), p(bias), p(wq), p(wo), p(kv_bank), p(idx),
-        p(weights), p(comb_idx), p(comb_w), p(out), None, p(L.status_word(dev)), L.stream_ptr(dev))
-    arena = torch.empty(_size("moc_decode_step_arena_bytes", s), dtype=torch.uint8, device=dev)
-    s.arena = p(arena)
-    L.check(_timed("decode_step", lambda: L.lib().moc_decode_step(C.byref(s))), "moc_decode_step")
-    _report(5 + int(window <= 1024) + 2 * int(window > 1024) + int(h.dtype == f32), lambda: (
-        "router_fwd:" + _TAG_OF_CODE[s.router.h_dtype], "gemm:bf16", "decode_attn:bf16", "gemm:bf16"))
+    h, states = _contig(hidden), _contig(routing_states)
+    dev, p = h.device, L.ptr
+    stream = L.stream_ptr(dev)
+    key = (h.shape, states.shape, w.shape, kv_bank.shape, h.dtype, states.dtype, dev, w.data_ptr(), p(bias), wq.data_ptr(),
+           wo.data_ptr(), kv_bank.data_ptr(), top_k, stream)
+    plan = None if plans is None else plans.get(key)
+    if plan is None:
+        L.require_cuda(h, states, w, bias, wq, wo, kv_bank)
+        if states.dim() != 3:
+            raise ValueError(f"hidden_states must be 3D (B, T, D), got shape {tuple(states.shape)}")
+        b, n_q, d = h.shape
+        rb, window, rd = states.shape
+        c, head_dim = w.shape[0], wq.shape[0] // num_heads
+        if wq.shape[1] != d or wo.shape[1] != wq.shape[0]:
+            raise ValueError(f"inner dimensions differ: {d} / {wq.shape[0]} vs {wq.shape[1]} / {wo.shape[1]}")
+        if rd != w.shape[1]:
+            raise ValueError(f"inner dimensions differ: {rd} vs {w.shape[1]}")
+        if kv_bank.shape[1] != 2 * num_kv_heads * head_dim:
+            raise ValueError("kv_bank must be [rows, 2 * num_kv_heads * head_dim]")
+        if rb != b:
+            raise ValueError("hidden_states and routing_states must share the batch")
+        k = router_selected_k(c, top_k, num_shared)
+        from .functional import _side_stream
+        s = L.DecodeStepDesc(
+            L.RouterShape(b, window, rd, c, top_k, num_shared, routed_scale, L.dtype_code(states.dtype)),
+            L.DecodeShape(b, n_q, num_heads, num_kv_heads, head_dim, num_shared + k, tokens_per_chapter, scale),
+            L.dtype_code(h.dtype), wo.shape[0], kv_bank.shape[0], None, None, p(w), p(bias), p(wq), p(wo), p(kv_bank), None,
+            None, None, None, None, None, p(L.status_word(dev)), stream, _side_stream(L.device_index(dev), stream))
+        plan = (bytes(s), _size("moc_decode_step_arena_bytes", s), (b, k), (b, num_shared + k), (b, n_q, wo.shape[0]),
+                5 + int(window <= 1024) + 2 * int(window > 1024) + int(h.dtype == torch.float32))
+        if plans is not None:
+            if len(plans) >= _DECODE_PLANS_MAX:
+                plans.clear()
+            plans[key] = plan
+    image, arena_bytes, routed, joint, out_shape, launches = plan
+    f32 = torch.float32
+    out = torch.empty(out_shape, dtype=h.dtype, device=dev)
+    idx = torch.empty(routed, dtype=torch.int64, device=dev)
+    weights = torch.empty(routed, dtype=f32, device=dev)
+    comb_idx = torch.empty(joint, dtype=torch.int32, device=dev)
+    comb_w = torch.empty(joint, dtype=f32, device=dev)
+    arena = torch.empty(arena_bytes, dtype=torch.uint8, device=dev)
+    s = L.DecodeStepDesc.from_buffer_copy(image)
+    s.routing_states, s.hidden, s.out, s.arena = states.data_ptr(), h.data_ptr(), out.data_ptr(), arena.data_ptr()
+    s.idx, s.weights, s.comb_idx, s.comb_w = idx.data_ptr(), weights.data_ptr(), comb_idx.data_ptr(), comb_w.data_ptr()
+    rc = (L.lib().moc_decode_step(C.byref(s)) if TIMER is None
+          else _timed("decode_step", lambda: L.lib().moc_decode_step(C.byref(s))))
+    if rc:
+        L.check(rc, "moc_decode_step")
+    _report(launches, lambda: ("router_fwd:" + _TAG_OF_CODE[s.router.h_dtype], "gemm:bf16", "decode_attn:bf16", "gemm:bf16"))
     return out, idx, weights, comb_idx, comb_w
 
 
