@@ -129,6 +129,7 @@ def _side_stream(dev_index: int, main_handle: int) -> int:
 class _Route(torch.autograd.Function):
     @staticmethod
     def forward(ctx, h, weight, bias, top_k, num_shared, routed_scale, with_losses, pos_weight):
+        ctx.set_materialize_grads(False)
         L.require_cuda(h, weight, bias)
         if h.dim() != 3:
             raise ValueError(f"hidden_states must be 3D (B, T, D), got shape {tuple(h.shape)}")
@@ -366,6 +367,7 @@ class _MemoryLayerTwoStream(torch.autograd.Function):
     @staticmethod
     def forward(ctx, h_router, h_attn, bank, router_w, router_b, wq, wk, wv, wo, norm_w, norm_b, cfg, sink,
                 fused=None):
+        ctx.set_materialize_grads(False)       # an output nobody used has no gradient: no zeros to fill and add
         (num_heads, num_kv_heads, t, top_k, num_shared, routed_scale, row_norm, row_eps, with_losses,
          pre_norm, pre_eps, add_residual, grad_on) = cfg
         L.require_cuda(h_router, h_attn, bank, router_w)
@@ -455,7 +457,7 @@ class _MemoryLayerTwoStream(torch.autograd.Function):
         s.stream = L.stream_ptr(dev)
         s.side_stream = _side_stream(L.device_index(dev), s.stream)
 
-        g = ops._contig(g if g.dtype == attn_dtype else g.to(attn_dtype))
+        g = torch.zeros(b, l, d, dtype=attn_dtype, device=dev) if g is None else ops._contig(g.to(attn_dtype))
         as_f32 = lambda v: None if v is None else ops._contig(v.float())     # noqa: E731
         g_w, g_cw, g_losses = as_f32(g_w), as_f32(g_cw), as_f32(g_losses)
         fuse_dh = ctx.same_h and need[0] and hr_dtype == in_dtype and in_dtype == attn_dtype
@@ -579,6 +581,7 @@ class _RouteTokens(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, h, weight, bias, top_k, num_shared, with_losses):
+        ctx.set_materialize_grads(False)
         b, l, d = h.shape
         rows = b * l
         h2 = h.reshape(rows, d).contiguous()
