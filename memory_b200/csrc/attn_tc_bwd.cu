@@ -413,6 +413,7 @@ struct DkvParams {
   const uint4* statb;
   int L, n_sel, H, HK;
   float scale, scale_log2;
+  int split;               // CTAs of a cluster that share a key tile, a run of the query tiles each
   int* status;
 };
 
@@ -430,6 +431,8 @@ __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, u
 //   row owners: P^T_j = exp2(S^T_j c - lse c) -> shared memory;  dS^T_j = P^T_j (dP^T_j - delta) -> tensor memory
 // so the exponentials of tile j run while the tensor pipe computes S^T_{j+1}, dV_{j-1}... and neither side
 // waits for the other in steady state.  P^T lives in shared memory so that S^T's columns are free early.
+// Few key tiles leave most of the chip idle: a cluster of p.split CTAs then shares one, each with a run of the query tiles,
+// and the first adds the others' parts through distributed shared memory.
 __global__ void __launch_bounds__(kThreads, 2)
 attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_do,
                        const __grid_constant__ CUtensorMap tmap_kv, const __grid_constant__ CUtensorMap tmap_dkv,
@@ -449,11 +452,16 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
   uint8_t* sel_s = stats + kStages * kStatBytes;     // 128 rows (1,1,1,0,0,0,0,0): picks the -lse terms
   uint8_t* sel_d = sel_s + kOnesBytes;               // 128 rows (0,0,0,1,1,1,0,0): picks the -delta terms
   uint8_t* zeros = sel_d + kOnesBytes;               // second half of every rank-16 operand
-  const int key0 = blockIdx.x * kKeysB, kh = blockIdx.y, b = blockIdx.z;
+  const int rank = p.split > 1 ? static_cast<int>(cluster_rank()) : 0;
+  const int key0 = static_cast<int>(blockIdx.x) / p.split * kKeysB, kh = blockIdx.y, b = blockIdx.z;
   const int G = p.H / p.HK;
   const int q_tiles = p.L / kQB;
-  const int n_iter = G * q_tiles;
+  const int it_first = static_cast<int>(static_cast<long long>(G) * q_tiles * rank / p.split);
+  const int n_iter = static_cast<int>(static_cast<long long>(G) * q_tiles * (rank + 1) / p.split) - it_first;
 
+  auto part_at = [&](int which, int row, int chunk) {      // 16 bytes of an exported fp32 row
+    return smem_u32(base) + which * 32768 + row * 256 + ((chunk ^ (row & 15)) << 4);
+  };
   if (threadIdx.x == 0) {
     abort_flag = 0;
     mbar_init(&k_bar, 1);
@@ -478,6 +486,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
+  bool ok = true;                                    // (of the row-owning warps)
 
   if (warp == 8) {
     if (lane == 0) {
@@ -490,7 +499,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
       for (int it = 0; it < n_iter; ++it) {
         const int s = it % kStages;
         if (!mbar_wait(&q_empty[s], ((it / kStages) & 1) ^ 1, &abort_flag, p.status)) break;
-        const int h = kh * G + it / q_tiles, l0 = (it % q_tiles) * kQB;
+        const int h = kh * G + (it_first + it) / q_tiles, l0 = ((it_first + it) % q_tiles) * kQB;
         uint8_t* st = ring + s * kStageB;
         mbar_arrive_expect_tx(&q_full[s], kStageTx);
         tma_load_2d(st, &tmap_q, &q_full[s], h * kD, b * p.L + l0);
@@ -573,7 +582,6 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     const uint32_t pt_row = smem_u32(pt_s) + row * 128;
     const uint32_t sw = static_cast<uint32_t>(row & 7);
     const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2);
-    bool ok = true;
     for (int it = 0; it < n_iter; ++it) {
       ok = mbar_wait_w(&s_full, it & 1, &abort_flag, p.status);
       if (!ok) break;
@@ -632,6 +640,42 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     if (ok) {
       ok = mbar_wait_w(&acc_bar, 0, &abort_flag, p.status);
     }
+    if (ok && rank > 0) {
+      // fp32 rows over the K, V and ring tiles, which nothing reads any more: dK, then dV; chunks rotated against conflicts
+      tc_fence_after();
+#pragma unroll
+      for (int which = 0; which < 2; ++which) {
+        uint32_t r[32];
+        tmem_ld32(tmem + lane_sel + (which ? kColDV : kColDK) + half * 32, r);
+        tmem_wait_ld();
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(part_at(which, row, half * 8 + c)), "r"(r[4 * c]),
+                       "r"(r[4 * c + 1]), "r"(r[4 * c + 2]), "r"(r[4 * c + 3]) : "memory");
+      }
+      tc_fence_before();
+    }
+  }
+  if (p.split > 1) {                                 // the other CTAs' parts are written
+    __syncthreads();
+    cluster_sync();
+  }
+  if (warp < 8 && rank == 0) {
+    const int half = warp >> 2;
+    const uint32_t lane_sel = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const int row = (warp & 3) * 32 + lane;
+    auto add_parts = [&](uint32_t (&r)[32], int which) {
+      for (int i = 1; i < p.split; ++i) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const float4 v = cluster_ld4(cluster_map(part_at(which, row, half * 8 + c), i));
+          r[4 * c + 0] = __float_as_uint(__uint_as_float(r[4 * c + 0]) + v.x);
+          r[4 * c + 1] = __float_as_uint(__uint_as_float(r[4 * c + 1]) + v.y);
+          r[4 * c + 2] = __float_as_uint(__uint_as_float(r[4 * c + 2]) + v.z);
+          r[4 * c + 3] = __float_as_uint(__uint_as_float(r[4 * c + 3]) + v.w);
+        }
+      }
+    };
     float kv_dot_part = 0.f;        // this thread's share of sum_rows (<dK, K> + <dV, V>) for its key row and column half
     if (p.dkv_tma) {
       // One thread owns one key row, so direct stores would scatter 16-byte pieces over 32 rows per instruction.
@@ -645,6 +689,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
           uint32_t r[32];
           tmem_ld32(tmem + lane_sel + (which ? kColDV : kColDK) + half * 32, r);
           tmem_wait_ld();
+          add_parts(r, which);
           const int krow = key0 + quarter * 32 + lane;
           const float rsf = (p.row_scale != nullptr && krow < p.n_sel)
                                 ? p.row_scale[static_cast<long long>(b) * p.n_sel + krow] : 1.f;
@@ -712,6 +757,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         uint32_t r[32];
         tmem_ld32(tmem + lane_sel + (which ? kColDV : kColDK) + half * 32, r);
         tmem_wait_ld();
+        add_parts(r, which);
         const float rsf = (p.row_scale != nullptr && key < p.n_sel)
                               ? p.row_scale[static_cast<long long>(b) * p.n_sel + key] : 1.f;
         const float f = (which ? 1.f : p.scale) * rsf;
@@ -732,6 +778,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     tc_fence_before();
   }
   __syncthreads();
+  if (p.split > 1) cluster_sync();                   // no CTA leaves while its part is read
   if (abort_flag) { for (int i = 0; i < 200; ++i) __nanosleep(1000); }
   if (warp == 9) { tc_fence_after(); tmem_dealloc(tmem, 256); }
 }
@@ -787,8 +834,10 @@ int launch_attn_tc_bwd(const moc_attn_shape* s, const void* q, const void* kv, c
       MOC_REQUIRE(p.dkv_tma && s->n_sel % 64 == 0, "the per-block <dKV, KV> sums need n_sel % 64 == 0 and an aligned d_kv");
     p.L = L; p.n_sel = s->n_sel; p.H = H; p.HK = HK;
     p.scale = s->scale; p.scale_log2 = s->scale * kLog2e; p.status = status;
-    dim3 grid(ceil_div(s->n_sel, kKeysB), HK, B);
-    attn_bwd_dkv_tc_kernel<<<grid, kThreads, kDkvSmem, stream>>>(tq64, tdo64, tkv, tdkv, p);
+    // (the rule for the other kernels' key tiles: an iteration over 64 queries x 128 keys costs what one of theirs does)
+    p.split = attn_key_split(ceil_div(s->n_sel, kKeysB) * HK * B, H / HK * (L / kQB));
+    dim3 grid(ceil_div(s->n_sel, kKeysB) * p.split, HK, B);
+    MOC_CUDA_OK(launch_clustered(attn_bwd_dkv_tc_kernel, grid, kThreads, kDkvSmem, p.split, stream, tq64, tdo64, tkv, tdkv, p));
   }
   MOC_CUDA_OK(cudaGetLastError());
   return MOC_OK;

@@ -759,6 +759,24 @@ def test_backward_entered_first_on_a_fresh_autograd_thread():
     assert r.returncode == 0 and "ok" in r.stdout, r.stderr[-2000:]
 
 
+@pytest.mark.parametrize("B,L,H,HK,N", [(1, 1024, 4, 2, 64), (1, 640, 2, 1, 200), (1, 256, 3, 3, 32), (2, 2048, 12, 12, 128)])
+def test_attention_key_tiles_shared_by_a_cluster(B, L, H, HK, N, dev):
+    """Few key tiles under many queries: a cluster of CTAs shares the query tiles of a dK / dV tile (runs of unequal length,
+    ragged tiles, both ways out of the kernel, the per-block sums of the scaled variant)."""
+    from memory_b200 import ops
+    g = torch.Generator().manual_seed(N + L)
+    q, do = (torch.randn(B, L, H * 64, generator=g).bfloat16().to(dev) for _ in range(2))
+    kv = torch.randn(B, N, 2 * HK * 64, generator=g).bfloat16().to(dev)
+    qr, kr = q.float().requires_grad_(True), kv.float().requires_grad_(True)
+    ref, _ = attn_reference(qr, kr, H, HK, 64)
+    ref.backward(do.float())
+    o, lse = ops.attn_fwd(q, kv, H, HK, 0.125)
+    dq, dkv = ops.attn_bwd(q, kv, o, lse, do, H, HK, 0.125)
+    assert rel_err(dq, qr.grad) < 3e-2 and rel_err(dkv, kr.grad) < 3e-2
+    assert torch.equal(dkv, ops.attn_bwd(q, kv, o, lse, do, H, HK, 0.125)[1])
+    _status_ok(dev)
+
+
 @pytest.mark.parametrize("B,L,H,HK,N", [(1, 64, 2, 2, 257), (1, 320, 3, 1, 512), (2, 128, 2, 2, 2049), (1, 65, 1, 1, 40),
                                         (1, 192, 12, 12, 4160)])
 def test_attention_split_over_clusters_and_large_scores(B, L, H, HK, N, dev):
