@@ -28,34 +28,20 @@ __device__ __forceinline__ float quotient(float x, float d, float r) {
 }
 
 // ---- block reductions (fixed order) ----------------------------------------------------------
+// (one barrier each: every reduction of a kernel has 32 floats of its own)
 __device__ __forceinline__ float block_sum(float v, float* red) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
   v = warp_sum(v);
-  __syncthreads();
   if (lane == 0) red[warp] = v;
   __syncthreads();
-  float t = 0.f;
-  if (warp == 0) {
-    t = lane < nw ? red[lane] : 0.f;
-    t = warp_sum(t);
-    if (lane == 0) red[32] = t;
-  }
-  __syncthreads();
-  return red[32];
+  return warp_sum(lane < nw ? red[lane] : 0.f);
 }
 __device__ __forceinline__ float block_max(float v, float* red) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
   v = warp_max(v);
-  __syncthreads();
   if (lane == 0) red[warp] = v;
   __syncthreads();
-  if (warp == 0) {
-    float t = lane < nw ? red[lane] : -INFINITY;
-    t = warp_max(t);
-    if (lane == 0) red[32] = t;
-  }
-  __syncthreads();
-  return red[32];
+  return warp_max(lane < nw ? red[lane] : -INFINITY);
 }
 
 // ---- forward ---------------------------------------------------------------------------------
@@ -335,7 +321,7 @@ select_kernel(const float* __restrict__ logits, long long ld, const float* __res
   float* pt = sm;                          // p~
   uint32_t* sel_key = reinterpret_cast<uint32_t*>(sm + C);   // [k_sel]
   int* sel_idx = reinterpret_cast<int*>(sel_key + k_sel);    // [k_sel]
-  __shared__ float red[33];
+  __shared__ float red[5][32];
   __shared__ int hist[256];
   __shared__ uint32_t s_prefix;
   __shared__ int s_krem, s_count, s_ties;
@@ -367,7 +353,7 @@ select_kernel(const float* __restrict__ logits, long long ld, const float* __res
   } else {
     for (int c = threadIdx.x; c < C; c += blockDim.x) m = fmaxf(m, logit(c));
   }
-  m = block_max(m, red);
+  m = block_max(m, red[0]);
   float s = 0.f;
   if constexpr (NV > 0) {
 #pragma unroll
@@ -380,7 +366,7 @@ select_kernel(const float* __restrict__ logits, long long ld, const float* __res
       s += e;
     }
   }
-  const float denom = block_sum(s, red);
+  const float denom = block_sum(s, red[1]);
   const float r_denom = 1.f / denom;
   float ms = 0.f;
   if constexpr (NV > 0) {
@@ -403,7 +389,7 @@ select_kernel(const float* __restrict__ logits, long long ld, const float* __res
       ms += pm;
     }
   }
-  const float masked_mass = block_sum(ms, red);
+  const float masked_mass = block_sum(ms, red[2]);
   const float dn0 = fmaxf(masked_mass, 1e-12f);
   if constexpr (NV > 0) {
     if (S > 0) {
@@ -590,7 +576,7 @@ select_kernel(const float* __restrict__ logits, long long ld, const float* __res
     }
     float part = 0.f;
     for (int j = threadIdx.x; j < k_sel; j += blockDim.x) part += srt_w[j];
-    topk_mass = block_sum(part, red);
+    topk_mass = block_sum(part, red[3]);
     const float dn = fmaxf(topk_mass, 1e-12f);
     long long* out_idx = idx + static_cast<long long>(b) * k_sel;
     float* out_w = weights + static_cast<long long>(b) * k_sel;
@@ -602,7 +588,7 @@ select_kernel(const float* __restrict__ logits, long long ld, const float* __res
       out_idx[j] = srt_i[j];
       cpart += wj * rho;
     }
-    comb_mass = static_cast<float>(S) + block_sum(cpart, red);
+    comb_mass = static_cast<float>(S) + block_sum(cpart, red[4]);
   }
   // shared prefix + renormalised combined weights (only meaningful when S > 0; with S == 0 the
   // combined lists are the routed lists unchanged)
@@ -629,7 +615,7 @@ __global__ void loss_partial_kernel(const float* __restrict__ probs, const long 
                                     float* __restrict__ chapter_stats, float* __restrict__ partial,
                                     int B, int C, int k_sel) {
   __shared__ int cnt[kLossChunk];
-  __shared__ float red[33];
+  __shared__ float red[5][32];
   const int c0 = blockIdx.x * kLossChunk;
   for (int i = threadIdx.x; i < kLossChunk; i += blockDim.x) cnt[i] = 0;
   __syncthreads();
@@ -659,9 +645,9 @@ __global__ void loss_partial_kernel(const float* __restrict__ probs, const long 
     aux = dv * dv;
     ent = e;
   }
-  lb = block_sum(lb, red);
-  aux = block_sum(aux, red);
-  ent = block_sum(ent, red);
+  lb = block_sum(lb, red[0]);
+  aux = block_sum(aux, red[1]);
+  ent = block_sum(ent, red[2]);
   if (threadIdx.x == 0) {
     partial[blockIdx.x * 3 + 0] = lb;
     partial[blockIdx.x * 3 + 1] = aux;
@@ -698,7 +684,7 @@ __global__ void loss_rows_partial_kernel(const float* __restrict__ probs, const 
 }
 __global__ void loss_rows_finish_kernel(const float* __restrict__ part, float* __restrict__ chapter_stats,
                                         float* __restrict__ partial, int B, int C, int splits) {
-  __shared__ float red[33];
+  __shared__ float red[5][32];
   const int c = blockIdx.x * kLossChunk + threadIdx.x;
   float lb = 0.f, aux = 0.f, ent = 0.f;
   if (c < C) {
@@ -717,9 +703,9 @@ __global__ void loss_rows_finish_kernel(const float* __restrict__ part, float* _
     aux = dv * dv;
     ent = e;
   }
-  lb = block_sum(lb, red);
-  aux = block_sum(aux, red);
-  ent = block_sum(ent, red);
+  lb = block_sum(lb, red[0]);
+  aux = block_sum(aux, red[1]);
+  ent = block_sum(ent, red[2]);
   if (threadIdx.x == 0) {
     partial[blockIdx.x * 3 + 0] = lb;
     partial[blockIdx.x * 3 + 1] = aux;
@@ -839,9 +825,8 @@ dlogits_kernel(const float* __restrict__ probs, const long long* __restrict__ id
                const float* __restrict__ d_losses, float* __restrict__ d_logits, __nv_bfloat16* __restrict__ terms, int ld,
                int B, int C, int k_sel, int S, float rho) {
   extern __shared__ float dp[];   // [C]
-  __shared__ float red[33];
+  __shared__ float red[5][32];
   __shared__ float s_dv[1024];    // k_sel <= 1024
-  __shared__ float s_scal[2];
   const int b = blockIdx.x;
   const float* p = probs + static_cast<long long>(b) * C;
   const float lse = row_stats[b * 4 + 0], s_mass = row_stats[b * 4 + 1];
@@ -866,7 +851,7 @@ dlogits_kernel(const float* __restrict__ probs, const long long* __restrict__ id
   if (d_comb_w != nullptr && S > 0)
     for (int i = threadIdx.x; i < kc; i += blockDim.x)
       dotu_p += d_comb_w[static_cast<long long>(b) * kc + i] * comb_w[static_cast<long long>(b) * kc + i];
-  const float dotu = block_sum(dotu_p, red);
+  const float dotu = (d_comb_w != nullptr && S > 0) ? block_sum(dotu_p, red[0]) : 0.f;
   float dotw_p = 0.f;
   for (int j = threadIdx.x; j < k_sel; j += blockDim.x) {
     float dw = d_weights ? d_weights[static_cast<long long>(b) * k_sel + j] : 0.f;
@@ -880,17 +865,14 @@ dlogits_kernel(const float* __restrict__ probs, const long long* __restrict__ id
     s_w[j] = wj;
     dotw_p += dw * wj;
   }
-  const float dotw = block_sum(dotw_p, red);
+  const float dotw = block_sum(dotw_p, red[1]);
   float a_p = 0.f;
   for (int j = threadIdx.x; j < k_sel; j += blockDim.x) {
     const float dv = (v_mass >= 1e-12f) ? (s_dv[j] - dotw) / v_mass : s_dv[j] / 1e-12f;
     s_dv[j] = dv;
     a_p += dv * (s_w[j] * fmaxf(v_mass, 1e-12f));   // v_j
   }
-  const float a_tot = block_sum(a_p, red);
-  if (threadIdx.x == 0) s_scal[0] = a_tot;
-  __syncthreads();
-  const float A = s_scal[0];
+  const float A = block_sum(a_p, red[2]);
   const bool renorm = (S > 0);
   const float inv_s = renorm ? ((s_mass >= 1e-12f) ? 1.f / s_mass : 1e12f) : 1.f;
   const float dense = (renorm && s_mass >= 1e-12f) ? -A * inv_s : 0.f;
@@ -903,7 +885,18 @@ dlogits_kernel(const float* __restrict__ probs, const long long* __restrict__ id
     if (g_ent != 0.f) g += g_ent * (-invB) * (logf(fmaxf(pv, 1e-12f)) + (pv > 1e-12f ? 1.f : 0.f));
     return g;
   };
-  if constexpr (NV > 0) {
+  if (NV > 0 && g_aux == 0.f && g_ent == 0.f) {          // the usual losses; all loads first, they are independent
+    float f[kN];
+#pragma unroll
+    for (int i = 0; i < kN; ++i) f[i] = 0.f;
+    if (g_lb != 0.f) {
+#pragma unroll
+      for (int i = 0; i < kN; ++i) f[i] = chapter_stats[min(col(i), C - 1)];
+    }
+#pragma unroll
+    for (int i = 0; i < kN; ++i)
+      if (col(i) < C) dp[col(i)] = (col(i) >= S ? dense : 0.f) + g_lb * static_cast<float>(C) * f[i] * invB;
+  } else if constexpr (NV > 0) {
 #pragma unroll
     for (int i = 0; i < kN; ++i)
       if (col(i) < C) dp[col(i)] = dense_grad(col(i), pr[i]);
@@ -924,7 +917,7 @@ dlogits_kernel(const float* __restrict__ probs, const long long* __restrict__ id
   } else {
     for (int c = threadIdx.x; c < C; c += blockDim.x) dot += dp[c] * p[c];
   }
-  dot = block_sum(dot, red);
+  dot = block_sum(dot, red[3]);
   const float zc = g_z * 2.f * lse * invB;
   if (terms != nullptr) {
     const long long stride = static_cast<long long>(B) * ld;
