@@ -233,7 +233,7 @@ logits_rows_kernel(const float* __restrict__ pooled, const float* __restrict__ w
       if (lane + 32 * i < d4) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          if (b0 + j >= B) break;
+          if (CH == 1 && b0 + j >= B) break;      // (four chapters: the branch costs more than the last rows)
           const float4 pv = sp4[(buf * 8 + j) * d4 + lane + 32 * i];
 #pragma unroll
           for (int ch = 0; ch < CH; ++ch)
