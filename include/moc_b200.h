@@ -301,13 +301,7 @@ int moc_scatter_bank_grad(const float* bank_grad, const int32_t* uniq, const int
  * (fp32 C only, C must be pre-zeroed or accumulate set).
  * residual (device fp32 [M,N], row stride ldr, may be NULL): added to the product before it is stored,
  * C = row_scale * (A B) + residual -- the residual add that follows the output projection in the
- * reference's block (memory_block.py:558) done in the projection's epilogue.
- * terms > 1 (bf16 kernel): C = sum over t of op(A_t) op(B_t), all in one accumulator, the last term first; A_t / B_t start
- * t * a_term_rows / b_term_rows stored rows behind A / B (0: the same operand in every term).
- * limit (device, bf16 kernel, may be NULL): only the first *limit * limit_block of the M rows (limit_k != 0: of the K range,
- * limit_block a multiple of 64) exist; what lies behind is neither read into a stored result nor, for M, defined in C.
- * c_row_blocks (device, bf16 kernel, may be NULL): block i of c_block_rows (a multiple of 32) rows of C is stored as block
- * c_row_blocks[i] of a matrix of c_stored_rows rows. */
+ * reference's block (memory_block.py:558) done in the projection's epilogue. */
 typedef struct {
   int32_t dtype, c_dtype;
   int32_t m, n, k;
@@ -319,10 +313,6 @@ typedef struct {
   int64_t a_stored_rows;   /* rows of the stored A when a gather list is used */
   const float* residual;
   int64_t ldr;
-  int32_t terms, a_term_rows, b_term_rows;
-  int32_t limit_block, limit_k, c_block_rows;
-  int64_t c_stored_rows;
-  const int32_t *limit, *c_row_blocks;
 } moc_gemm_desc;
 
 int moc_gemm(const moc_gemm_desc* g, const void* a, const void* b, void* c, const float* row_scale,

@@ -34,10 +34,7 @@ class GemmDesc(C.Structure):
                 ("lda", C.c_int64), ("ldb", C.c_int64), ("ldc", C.c_int64),
                 ("accumulate", C.c_int32), ("split_k", C.c_int32), ("scale_block_rows", C.c_int32),
                 ("a_block_rows", C.c_int32), ("a_stored_rows", C.c_int64),
-                ("residual", C.c_void_p), ("ldr", C.c_int64),
-                ("terms", C.c_int32), ("a_term_rows", C.c_int32), ("b_term_rows", C.c_int32),
-                ("limit_block", C.c_int32), ("limit_k", C.c_int32), ("c_block_rows", C.c_int32),
-                ("c_stored_rows", C.c_int64), ("limit", C.c_void_p), ("c_row_blocks", C.c_void_p)]
+                ("residual", C.c_void_p), ("ldr", C.c_int64)]
 
 
 class AttnShape(C.Structure):

@@ -3,9 +3,11 @@
 #include "moc_common.cuh"
 
 namespace moc {
+struct GemmExtra;
 int launch_gemm_tc(const moc_gemm_desc* g, const void* a, const void* b, void* c, const float* row_scale,
                    const int32_t* a_row_blocks, int32_t* status, cudaStream_t stream,
-                   const int32_t* b_row_blocks = nullptr, int32_t b_block_rows = 0, int64_t b_stored_rows = 0);
+                   const int32_t* b_row_blocks = nullptr, int32_t b_block_rows = 0, int64_t b_stored_rows = 0,
+                   const GemmExtra* extra = nullptr);
 int launch_sgemm(const moc_gemm_desc* g, const float* a, const float* b, float* c, const float* row_scale,
                  cudaStream_t stream);
 int launch_delta(int dtype, const void* o, const void* d_o, float* delta, int B, int L, int H, int D,
@@ -29,7 +31,6 @@ extern "C" int moc_gemm(const moc_gemm_desc* g, const void* a, const void* b, vo
   MOC_REQUIRE(g->m > 0 && g->n > 0 && g->k > 0, "empty projection");
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (g->dtype == MOC_F32) {
-    MOC_REQUIRE(g->terms <= 1 && !g->limit && !g->c_row_blocks, "operand terms, limits and scattered rows are bf16 only");
     MOC_REQUIRE(a_row_blocks == nullptr, "the fp32 projection takes gathered rows, not a gather list");
     return launch_sgemm(g, static_cast<const float*>(a), static_cast<const float*>(b), static_cast<float*>(c),
                         row_scale, stream);

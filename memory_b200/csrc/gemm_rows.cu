@@ -88,7 +88,7 @@ gemm_rows_kernel(const __nv_bfloat16* __restrict__ a, long long lda, const __nv_
 // fills the chip (64 x 1,536: 16 us here, 10 there).
 bool gemm_rows_supported(const moc_gemm_desc* g, const float* row_scale, const int32_t* a_row_blocks,
                          const int32_t* b_row_blocks) {
-  return g->m <= 64 && static_cast<long long>(g->m) * g->n <= 64 * 1024 && g->k <= 1024 && g->a_kmajor && g->b_kmajor && !g->accumulate && g->split_k <= 1 && g->terms <= 1 && g->limit == nullptr && g->c_row_blocks == nullptr &&
+  return g->m <= 64 && static_cast<long long>(g->m) * g->n <= 64 * 1024 && g->k <= 1024 && g->a_kmajor && g->b_kmajor && !g->accumulate && g->split_k <= 1 &&
          g->residual == nullptr && row_scale == nullptr && a_row_blocks == nullptr && b_row_blocks == nullptr;
 }
 int launch_gemm_rows(const moc_gemm_desc* g, const void* a, const void* b, void* c, cudaStream_t stream) {

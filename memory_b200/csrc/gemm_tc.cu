@@ -10,7 +10,7 @@
 // main loop of the next.  The A operand can be fetched through a row-block gather
 // list, which is how selected chapters are read straight out of the memory bank.
 #define MOC_KERNEL_TAG 1
-#include "moc_common.cuh"
+#include "host_pass.cuh"
 
 namespace moc {
 
@@ -61,7 +61,7 @@ struct GemmTcParams {
   int b_num_blocks;
   long long b_stored_rows;
   int k_tiles_total;
-  int k_tiles_per_term, terms; // the K range of one term and the number of terms (see moc_gemm_desc)
+  int k_tiles_per_term, terms; // the K range of one term and the number of terms (see GemmExtra)
   int a_term_rows, b_term_rows;
   const int* limit;        // device: rows of C (limit_k: of the K range) that exist, in blocks
   int limit_block, limit_k;
@@ -520,7 +520,8 @@ int launch_gemm_rows(const moc_gemm_desc* g, const void* a, const void* b, void*
 
 int launch_gemm_tc(const moc_gemm_desc* g, const void* a, const void* b, void* c, const float* row_scale,
                    const int32_t* a_row_blocks, int32_t* status, cudaStream_t stream,
-                   const int32_t* b_row_blocks, int32_t b_block_rows, int64_t b_stored_rows) {
+                   const int32_t* b_row_blocks, int32_t b_block_rows, int64_t b_stored_rows, const GemmExtra* extra) {
+  const GemmExtra x = extra ? *extra : GemmExtra{};
   MOC_REQUIRE(g->k % 8 == 0, "bf16 projection needs K % 8 == 0");
   MOC_REQUIRE(g->lda % 8 == 0 && g->ldb % 8 == 0, "bf16 projection needs 16-byte aligned operand rows");
   MOC_REQUIRE((reinterpret_cast<uintptr_t>(a) & 15) == 0 && (reinterpret_cast<uintptr_t>(b) & 15) == 0,
@@ -528,7 +529,8 @@ int launch_gemm_tc(const moc_gemm_desc* g, const void* a, const void* b, void* c
   MOC_REQUIRE(g->c_dtype == MOC_BF16 || g->c_dtype == MOC_F32, "bad c_dtype");
   const int split = g->split_k > 1 ? g->split_k : 1;
   if (split > 1 || g->accumulate) MOC_REQUIRE(g->c_dtype == MOC_F32, "accumulate / split_k need an fp32 C");
-  if (gemm_rows_supported(g, row_scale, a_row_blocks, b_row_blocks)) return launch_gemm_rows(g, a, b, c, stream);
+  if (x.terms <= 1 && !x.limit && !x.c_row_blocks && gemm_rows_supported(g, row_scale, a_row_blocks, b_row_blocks))
+    return launch_gemm_rows(g, a, b, c, stream);
   int a_box_rows = 64;
   int a_num_blocks = 0;
   long long a_stored_rows = g->a_kmajor ? g->m : g->k;
@@ -554,15 +556,15 @@ int launch_gemm_tc(const moc_gemm_desc* g, const void* a, const void* b, void* c
     b_num_blocks = g->k / b_block_rows;
   }
 
-  const int terms = g->terms > 1 ? g->terms : 1;
-  MOC_REQUIRE(terms == 1 || (a_row_blocks == nullptr && b_row_blocks == nullptr && g->a_term_rows >= 0 && g->b_term_rows >= 0),
+  const int terms = x.terms > 1 ? x.terms : 1;
+  MOC_REQUIRE(terms == 1 || (a_row_blocks == nullptr && b_row_blocks == nullptr && x.a_term_rows >= 0 && x.b_term_rows >= 0),
               "operands in terms take no gather list");
-  const uint64_t a_more = static_cast<uint64_t>(terms - 1) * static_cast<uint64_t>(terms > 1 ? g->a_term_rows : 0);
-  const uint64_t b_more = static_cast<uint64_t>(terms - 1) * static_cast<uint64_t>(terms > 1 ? g->b_term_rows : 0);
+  const uint64_t a_more = static_cast<uint64_t>(terms - 1) * static_cast<uint64_t>(terms > 1 ? x.a_term_rows : 0);
+  const uint64_t b_more = static_cast<uint64_t>(terms - 1) * static_cast<uint64_t>(terms > 1 ? x.b_term_rows : 0);
 
-  MOC_REQUIRE(g->limit == nullptr || (g->limit_block > 0 && (!g->limit_k || (g->limit_block % BK == 0 && terms == 1))),
+  MOC_REQUIRE(x.limit == nullptr || (x.limit_block > 0 && (!x.limit_k || (x.limit_block % BK == 0 && terms == 1))),
               "a K limit counts blocks of a multiple of 64");
-  MOC_REQUIRE(g->c_row_blocks == nullptr || (g->c_block_rows > 0 && g->c_block_rows % 32 == 0 && g->c_stored_rows > 0 &&
+  MOC_REQUIRE(x.c_row_blocks == nullptr || (x.c_block_rows > 0 && x.c_block_rows % 32 == 0 && x.c_stored_rows > 0 &&
                                              !g->accumulate && split == 1 && g->residual == nullptr),
               "scattered rows of C come in blocks of a multiple of 32, stored once");
 
@@ -611,7 +613,7 @@ int launch_gemm_tc(const moc_gemm_desc* g, const void* a, const void* b, void* c
   const bool c_tma = g->ldc % (c_f32 ? 4 : 8) == 0 && (reinterpret_cast<uintptr_t>(c) & 15) == 0;
   CUtensorMap tmap_c = tmap_a;      // placeholder when the TMA-store epilogue is not used
   if (c_tma) {
-    const uint64_t c_rows = static_cast<uint64_t>(g->c_row_blocks ? g->c_stored_rows : g->m);
+    const uint64_t c_rows = static_cast<uint64_t>(x.c_row_blocks ? x.c_stored_rows : g->m);
     rc = c_f32 ? make_tmap_f32_2d(&tmap_c, c, c_rows, static_cast<uint64_t>(g->n), static_cast<uint64_t>(g->ldc), 32, 32)
                : make_tmap_bf16_2d(&tmap_c, c, c_rows, static_cast<uint64_t>(g->n), static_cast<uint64_t>(g->ldc), 32, 64);
     if (rc != MOC_OK) return rc;
@@ -629,10 +631,10 @@ int launch_gemm_tc(const moc_gemm_desc* g, const void* a, const void* b, void* c
   p.a_stored_rows = a_stored_rows;
   p.b_row_blocks = b_row_blocks; p.b_block_rows = b_block_rows; p.b_box_rows = b_box_rows;
   p.b_num_blocks = b_num_blocks; p.b_stored_rows = b_stored_rows;
-  p.limit = g->limit; p.limit_block = g->limit_block; p.limit_k = g->limit_k;
-  p.c_row_blocks = g->c_row_blocks; p.c_block_rows = g->c_block_rows; p.c_stored_rows = g->c_stored_rows;
+  p.limit = x.limit; p.limit_block = x.limit_block; p.limit_k = x.limit_k;
+  p.c_row_blocks = x.c_row_blocks; p.c_block_rows = x.c_block_rows; p.c_stored_rows = x.c_stored_rows;
   p.terms = terms; p.k_tiles_per_term = ceil_div(g->k, BK);
-  p.a_term_rows = g->a_term_rows; p.b_term_rows = g->b_term_rows;
+  p.a_term_rows = x.a_term_rows; p.b_term_rows = x.b_term_rows;
   p.k_tiles_total = terms * p.k_tiles_per_term;
   p.k_tiles_per_split = ceil_div(p.k_tiles_total, split);
   p.splits = ceil_div(p.k_tiles_total, p.k_tiles_per_split);   // no empty splits

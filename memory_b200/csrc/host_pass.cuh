@@ -32,8 +32,26 @@ int fork_event(cudaStream_t from, cudaEvent_t* out);
 // `after` continues behind what `before` holds now.
 int order(cudaStream_t before, cudaStream_t after);
 
+// What the bf16 projection kernel can do beside moc_gemm_desc:
+// terms > 1: C = sum over t of op(A_t) op(B_t), all in one accumulator, the last term first; A_t / B_t start
+//   t * a_term_rows / b_term_rows stored rows behind A / B (0: the same operand in every term).
+// limit (device): only the first *limit * limit_block of the M rows (limit_k: of the K range, limit_block a multiple of 64)
+//   exist; what lies behind is not read into a stored result nor, for M, defined in C.
+// c_row_blocks (device): block i of c_block_rows (a multiple of 32) rows of C is stored as block c_row_blocks[i] of a matrix
+//   of c_stored_rows rows.
+struct GemmExtra {
+  int terms = 1, a_term_rows = 0, b_term_rows = 0;
+  int limit_block = 0, limit_k = 0, c_block_rows = 0;
+  int64_t c_stored_rows = 0;
+  const int32_t *limit = nullptr, *c_row_blocks = nullptr;
+};
+int launch_gemm_tc(const moc_gemm_desc* g, const void* a, const void* b, void* c, const float* row_scale,
+                   const int32_t* a_row_blocks, int32_t* status, cudaStream_t stream,
+                   const int32_t* b_row_blocks, int32_t b_block_rows, int64_t b_stored_rows, const GemmExtra* extra);
+
 // C [m, n] = op(A) op(B), dense operands
 struct Gemm : moc_gemm_desc {
+  GemmExtra extra;
   Gemm(int dt, int64_t m_, int64_t n_, int64_t k_, bool a_k, bool b_k, int c_dt) {
     dtype = dt; c_dtype = c_dt;
     m = static_cast<int>(m_); n = static_cast<int>(n_); k = static_cast<int>(k_);
@@ -42,10 +60,12 @@ struct Gemm : moc_gemm_desc {
     accumulate = 0; split_k = 1; scale_block_rows = 1; a_block_rows = 0;
     a_stored_rows = a_k ? m : k;
     residual = nullptr; ldr = 0;
-    terms = 1; a_term_rows = b_term_rows = 0;
-    limit_block = limit_k = c_block_rows = 0; c_stored_rows = 0; limit = c_row_blocks = nullptr;
   }
 };
+// with its extras (bf16 operands)
+inline int gemm_extra(const Gemm& g, const void* a, const void* b, void* c, int32_t* status, cudaStream_t stream) {
+  return launch_gemm_tc(&g, a, b, c, nullptr, nullptr, status, stream, nullptr, 0, 0, &g.extra);
+}
 // K-splits of a weight gradient [out_rows, out_cols] over `rows`: enough (tile, split) items to fill the SMs once
 inline int splits(int64_t rows, int64_t out_rows, int64_t out_cols) {
   const int64_t tiles = ((out_rows + 127) / 128) * ((out_cols + 255) / 256);

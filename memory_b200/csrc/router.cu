@@ -1241,8 +1241,8 @@ extern "C" int moc_token_route_fwd(const moc_token_route_desc* s, void* scratch)
   float* logits = static_cast<float*>(scratch);
   Gemm g(MOC_BF16, s->rows, C, d, true, true, MOC_F32);
   g.ldc = cp;
-  g.terms = 3; g.b_term_rows = C;
-  MOC_TRY(moc_gemm(&g, s->h, a.w_terms, logits, nullptr, nullptr, s->status, stream));
+  g.extra.terms = 3; g.extra.b_term_rows = C;
+  MOC_TRY(gemm_extra(g, s->h, a.w_terms, logits, s->status, stream));
   MOC_TRY(launch_select(logits, cp, s->bias, a.probs, s->idx, s->weights, nullptr, nullptr, a.row_stats, s->rows, C,
                         k_selected(&r), s->num_shared, 1.f, stream));
   if (s->losses != nullptr)
@@ -1274,8 +1274,8 @@ extern "C" int moc_token_route_bwd(const moc_token_route_desc* s, const float* g
   if (d_w != nullptr) {
     Gemm g(MOC_BF16, C, d, rows, false, false, MOC_F32);
     g.lda = cp;
-    g.terms = 3; g.a_term_rows = rows;
-    MOC_TRY(moc_gemm(&g, terms, s->h, d_w, nullptr, nullptr, s->status, stream));
+    g.extra.terms = 3; g.extra.a_term_rows = rows;
+    MOC_TRY(gemm_extra(g, terms, s->h, d_w, s->status, stream));
   }
   if (d_bias != nullptr) {
     const int chunks = ceil_div(rows, kTermRows);

@@ -229,11 +229,11 @@ extern "C" int moc_token_attn_fwd(const moc_token_attn_desc* s, void* scratch) {
     MOC_CUDA_OK(cudaGetLastError());
     bidx = a.bidx;
     rm2 = a.rm2;
-    gkv.limit = a.count; gkv.limit_block = kT;
+    gkv.extra.limit = a.count; gkv.extra.limit_block = kT;
   } else {
     MOC_TRY(as_dtype(s->routed, s->routed_dtype, a.rm2, MOC_BF16, x.M * kT * d, st, &rm2));
   }
-  MOC_TRY(moc_gemm(&gkv, rm2, a.wkv, a.kv, nullptr, nullptr, s->status, st));
+  MOC_TRY(gemm_extra(gkv, rm2, a.wkv, a.kv, s->status, st));
   const moc_sparse_attn_shape ms = mix_shape(s, x);
   MOC_TRY(moc_token_mix_index(&ms, 1, bidx, a.index, s->status, st));
   MOC_TRY(moc_token_mix_fwd(&ms, 1, a.q, a.kv, a.kv + x.dkv, 2 * x.dkv, bidx, s->weights, a.o_sh, s->routed_scale, a.index,
@@ -266,8 +266,8 @@ extern "C" int moc_token_attn_bwd(const moc_token_attn_desc* s, const moc_token_
     Gemm g(MOC_BF16, 2 * x.dkv, d, rows, false, false, MOC_F32);
     g.accumulate = 1;
     g.split_k = splits(rows, 2 * x.dkv, d);
-    g.limit = limit; g.limit_block = kT; g.limit_k = 1;
-    return moc_gemm(&g, d_kv, mem, b->d_wkv, nullptr, nullptr, s->status, st);
+    g.extra.limit = limit; g.extra.limit_block = kT; g.extra.limit_k = 1;
+    return gemm_extra(g, d_kv, mem, b->d_wkv, s->status, st);
   };
   if (x.shared) {
     if (x.rows_pad > x.rows)
@@ -291,10 +291,10 @@ extern "C" int moc_token_attn_bwd(const moc_token_attn_desc* s, const moc_token_
     Gemm g(MOC_BF16, x.U * kT, d, 2 * x.dkv, true, true, s->routed_dtype);
     if (x.listed) {
       MOC_CUDA_OK(cudaMemsetAsync(b->d_routed, 0, static_cast<size_t>(x.M * kT * d) * (s->routed_dtype == MOC_F32 ? 4 : 2), st));
-      g.limit = a.count; g.limit_block = kT;
-      g.c_row_blocks = a.uniq; g.c_block_rows = kT; g.c_stored_rows = x.M * kT;
+      g.extra.limit = a.count; g.extra.limit_block = kT;
+      g.extra.c_row_blocks = a.uniq; g.extra.c_block_rows = kT; g.extra.c_stored_rows = x.M * kT;
     }
-    MOC_TRY(moc_gemm(&g, t.d_kv, a.wkv_t, b->d_routed, nullptr, nullptr, s->status, st));
+    MOC_TRY(gemm_extra(g, t.d_kv, a.wkv_t, b->d_routed, s->status, st));
   }
   MOC_TRY(wkv_grad(x.U * kT, t.d_kv, rm2, x.listed ? a.count : nullptr));
   const Gemm gh(MOC_BF16, x.rows, d, x.hd, true, true, s->h_dtype);
