@@ -155,3 +155,22 @@ def test_token_attention_over_listed_chapters(dev, rows, k, m, s, h, hk, bank_dt
         assert _rel(a, b) < 2e-2, i
     from memory_b200 import _lib as L
     L.check_device_status(dev)
+
+
+@pytest.mark.parametrize("rows,d", [(1, 4), (17, 256), (33, 260), (100, 768), (16, 772), (31, 1024), (9, 1028)])
+@pytest.mark.parametrize("kind", ["rms", "layernorm"])
+def test_norm_backward_widths(dev, rows, d, kind):
+    """Rows in registers (every width class and its edge) and in two passes."""
+    from memory_b200 import ops
+    torch.manual_seed(rows + d)
+    x, dy, res = (torch.randn(rows, d, device=dev) for _ in range(3))
+    w, b = torch.rand(d, device=dev) + 0.5, torch.randn(d, device=dev)
+    x64, w64, b64 = (t.double().requires_grad_(True) for t in (x, w, b))
+    mu = x64.mean(-1, keepdim=True) if kind == "layernorm" else 0.0
+    y = (x64 - mu) / ((x64 - mu).square().mean(-1, keepdim=True) + 1e-5).sqrt() * w64
+    (y + b64 if kind == "layernorm" else y).backward(dy.double())
+    _, stats = ops.norm_fwd(x, w, b if kind == "layernorm" else None, kind, 1e-5, torch.float32)
+    dx, dw, db = ops.norm_bwd(dy, x, w, stats, res, kind, kind == "layernorm")
+    assert _rel(dx, x64.grad + res.double()) < 1e-5 and _rel(dw, w64.grad) < 1e-5
+    if kind == "layernorm":
+        assert _rel(db, b64.grad) < 1e-5
