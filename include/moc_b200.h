@@ -657,6 +657,7 @@ typedef struct {
   void *out, *arena;
   int32_t* status;
   void *stream, *side_stream;
+  int32_t attn_dim, out_dim;   /* rows of wq (columns of wo) and rows of wo; 0: hidden_dim */
 } moc_xattn_desc;
 
 int64_t moc_xattn_arena_bytes(const moc_xattn_desc* s);

@@ -113,7 +113,7 @@ class XattnDesc(C.Structure):
     _fields_ = _fields(
         "i: batch seq n_sel hidden_dim mem_dim num_heads num_kv_heads mem_shared h_dtype mem_dtype weight_dtype"
         " compute_dtype out_dtype pre_norm add_residual for_backward; f: pre_eps;"
-        "p: h memory wq wk wv wo norm_w norm_b out arena status stream side_stream")
+        "p: h memory wq wk wv wo norm_w norm_b out arena status stream side_stream; i: attn_dim out_dim")
 
 
 class XattnBwdDesc(C.Structure):

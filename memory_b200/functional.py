@@ -31,6 +31,28 @@ def _cast(v, dtype):
     return v if v is None or v.dtype == dtype else v.to(dtype)
 
 
+# A pass that is one native call takes raw pointers and the sizes of its descriptor; what a tensor's shape says against
+# those sizes is refused here, before the descriptor is filled.
+def _check_width(name: str, t: torch.Tensor, width: int) -> None:
+    if t.dim() != 2 or t.shape[1] != width:
+        raise ValueError(f"inner dimensions differ: {name} {tuple(t.shape)} vs {width}")
+
+
+def _check_numel(name: str, t: Optional[torch.Tensor], n: int) -> None:
+    if t is not None and t.numel() != n:
+        raise ValueError(f"{name} must have {n} elements, got shape {tuple(t.shape)}")
+
+
+def _check_projections(d: int, mem_dim: int, wq, wk, wv, wo, num_heads: int, num_kv_heads: int) -> None:
+    for name, w, width in (("wq", wq, d), ("wk", wk, mem_dim), ("wv", wv, mem_dim), ("wo", wo, wq.shape[0])):
+        _check_width(name, w, width)
+    if num_heads <= 0 or num_kv_heads <= 0 or wq.shape[0] % num_heads != 0:
+        raise ValueError(f"wq {tuple(wq.shape)} does not hold {num_heads} heads")
+    dkv = num_kv_heads * (wq.shape[0] // num_heads)
+    if wk.shape[0] != dkv or wv.shape[0] != dkv:
+        raise ValueError(f"wk {tuple(wk.shape)} and wv {tuple(wv.shape)} must have num_kv_heads * head_dim = {dkv} rows")
+
+
 class _LossDict(dict):
     """Router loss dict (same keys as the reference) that also carries the raw 4-vector as ``.vector`` (order of
     LOSS_KEYS), for a single backward seed and a single-kernel weighted sum.  A dict somebody has changed no longer
@@ -234,40 +256,46 @@ class _CrossAttention(torch.autograd.Function):
     @staticmethod
     def forward(ctx, h, memory, wq, wk, wv, wo, norm_w, norm_b, num_heads, num_kv_heads, compute_dtype,
                 norm_kind, norm_eps, add_residual, grad_on):
-        L.require_cuda(h, memory, wq, wk, wv, wo)
         b, l, d = h.shape
         cd = compute_dtype
         dev = h.device
         mem_shared = memory.dim() == 2
-        in_dtype, mem_dtype = h.dtype, memory.dtype
+        in_dtype, mem_dtype, mem_shape = h.dtype, memory.dtype, memory.shape
+        if not mem_shared and (memory.dim() < 3 or mem_shape[:-2].numel() != b):
+            raise ValueError("memory must be (N, d) or (B, N, d) with the batch size of the hidden states")
+        _check_projections(d, mem_shape[-1], wq, wk, wv, wo, num_heads, num_kv_heads)
+        attn_dim, out_dim = wq.shape[0], wo.shape[0]
+        if add_residual and out_dim != d:
+            raise ValueError(f"the residual has {d} columns, the result {out_dim}")
+        _check_numel("norm_weight", norm_w, d)
+        _check_numel("norm_bias", norm_b, d)
+        L.require_cuda(h, memory, wq, wk, wv, wo, norm_w, norm_b)
         # the kernels take fp32 or bf16; anything else goes through the compute dtype
         hc = ops._contig(h if in_dtype in _KERNEL_DTYPES else h.to(cd))
         mc = ops._contig(memory if mem_dtype in _KERNEL_DTYPES else memory.to(cd))
-        if mc.dim() == 3 and mc.shape[0] != b:
-            raise ValueError("memory must be (N, d) or (B, N, d) with the batch size of the hidden states")
         w_dtypes = (wq.dtype, wk.dtype, wv.dtype, wo.dtype)
         same = len(set(w_dtypes)) == 1 and wq.dtype in _KERNEL_DTYPES
         ws = [ops._contig(w if same else w.float()) for w in (wq, wk, wv, wo)]
         nw = None if norm_w is None else ops._contig(norm_w.float())
         nb = None if norm_b is None else ops._contig(norm_b.float())
         need_grad = grad_on and any(ctx.needs_input_grad[:8])
-        out = torch.empty(b, l, d, dtype=in_dtype if in_dtype in (torch.float32, cd) else cd, device=dev)
+        out = torch.empty(b, l, out_dim, dtype=in_dtype if in_dtype in (torch.float32, cd) else cd, device=dev)
         if cd == torch.float32 and out.dtype != cd:
-            out = torch.empty(b, l, d, dtype=cd, device=dev)
+            out = torch.empty(b, l, out_dim, dtype=cd, device=dev)
         main = L.stream_ptr(dev)
         code, p = L.dtype_code, L.ptr
         s = L.XattnDesc(b, l, mc.shape[-2], d, mc.shape[-1], num_heads, num_kv_heads, int(mem_shared), code(hc.dtype),
                         code(mc.dtype), code(ws[0].dtype), code(cd), code(out.dtype),
                         ops.NORM_KINDS[norm_kind] if norm_kind is not None else 0, int(add_residual), int(need_grad),
                         norm_eps, p(hc), p(mc), p(ws[0]), p(ws[1]), p(ws[2]), p(ws[3]), p(nw), p(nb), p(out), None,
-                        p(L.status_word(dev)), main, _side_stream(L.device_index(dev), main))
+                        p(L.status_word(dev)), main, _side_stream(L.device_index(dev), main), attn_dim, out_dim)
         arena = torch.empty(ops.xattn_arena_bytes(s), dtype=torch.uint8, device=dev)
         s.arena = p(arena)
         ops.xattn_fwd(s)
         if need_grad:
             ctx.desc = s
             ctx.dtypes = (in_dtype, mem_dtype, w_dtypes, None if norm_w is None else norm_w.dtype,
-                          None if norm_b is None else norm_b.dtype, wk.shape[0])
+                          None if norm_b is None else norm_b.dtype, wk.shape[0], mem_shape)
             # inputs the backward pass reads itself: as projection operands, or for the normalisation
             keep_h = hc if (norm_kind is not None or hc.dtype == cd) else None
             keep_m = mc if mc.dtype == cd else None
@@ -279,7 +307,7 @@ class _CrossAttention(torch.autograd.Function):
     def backward(ctx, g):
         arena, hc, mc, wq, wo, nw = ctx.saved_tensors
         s = ctx.desc
-        in_dtype, mem_dtype, wdt, nw_dtype, nb_dtype, dkv = ctx.dtypes
+        in_dtype, mem_dtype, wdt, nw_dtype, nb_dtype, dkv, mem_shape = ctx.dtypes
         dev, f32, p = arena.device, torch.float32, L.ptr
         need = ctx.needs_input_grad
         cd = f32 if s.compute_dtype == L.MOC_F32 else torch.bfloat16
@@ -293,13 +321,10 @@ class _CrossAttention(torch.autograd.Function):
         if nw is not None and cd == torch.bfloat16 and in_dtype not in _KERNEL_DTYPES:
             dh_dtype = f32
         d_h = torch.empty(b, l, d, dtype=dh_dtype if cd != f32 else f32, device=dev) if (need[0] or nw is not None) else None
-        d_mem = None
-        if need[1]:
-            shape = (s.n_sel, md) if s.mem_shared else (b, s.n_sel, md)
-            d_mem = torch.empty(shape, dtype=dm_dtype if cd != f32 else f32, device=dev)
-        d_wq = torch.empty(d, d, dtype=f32, device=dev)
+        d_mem = torch.empty(mem_shape, dtype=dm_dtype if cd != f32 else f32, device=dev) if need[1] else None
+        d_wq = torch.empty(s.attn_dim, d, dtype=f32, device=dev)
         d_wkv = torch.empty(2 * dkv, md, dtype=f32, device=dev)
-        d_wo = torch.empty(d, d, dtype=f32, device=dev)
+        d_wo = torch.empty(s.out_dim, s.attn_dim, dtype=f32, device=dev)
         d_nw = torch.empty(d, dtype=f32, device=dev) if nw is not None else None
         d_nb = torch.empty(d, dtype=f32, device=dev) if nb_dtype is not None else None
         q = L.XattnBwdDesc(p(g), L.dtype_code(g.dtype), L.dtype_code(d_h.dtype) if d_h is not None else 0,

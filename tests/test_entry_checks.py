@@ -1,0 +1,75 @@
+"""What the entry points refuse before a native pass gets raw pointers: shapes that contradict the sizes of its descriptor.
+The refusals come ahead of the look at the device, so CPU tensors show them; the accepted odd shapes are compared on the GPU."""
+import pytest
+import torch
+
+D, HEADS = 128, 2
+
+
+def _attn_args(**over):
+    a = dict(h=torch.zeros(2, 8, D), memory=torch.zeros(2, 24, D), wq=torch.zeros(D, D), wk=torch.zeros(D, D),
+             wv=torch.zeros(D, D), wo=torch.zeros(D, D), num_heads=HEADS, num_kv_heads=None)
+    a.update(over)
+    return a
+
+
+@pytest.mark.parametrize("over, message", [
+    # grouped weights with the group count left out: the likeliest mistake
+    (dict(wk=torch.zeros(64, D), wv=torch.zeros(64, D)), "num_kv_heads"),
+    (dict(wv=torch.zeros(64, D)), "num_kv_heads"),
+    (dict(num_kv_heads=1), "num_kv_heads"),
+    (dict(wq=torch.zeros(D, 64)), "inner dimensions differ: wq"),
+    (dict(wk=torch.zeros(D, 64)), "inner dimensions differ: wk"),
+    (dict(wv=torch.zeros(D, 64)), "inner dimensions differ: wv"),
+    (dict(wo=torch.zeros(D, 64)), "inner dimensions differ: wo"),
+    (dict(memory=torch.zeros(2, 24, 64)), "inner dimensions differ: wk"),
+    (dict(memory=torch.zeros(3, 24, D)), "batch size"),
+    (dict(num_heads=3), "heads"),
+    (dict(wo=torch.zeros(64, D), add_residual=True), "residual"),
+    (dict(pre_norm="rms", norm_weight=torch.ones(64)), "norm_weight"),
+    (dict(pre_norm="layernorm", norm_weight=torch.ones(D), norm_bias=torch.ones(64)), "norm_bias"),
+    ({}, "CUDA"),
+])
+def test_cross_attention_refuses(over, message):
+    from memory_b200 import functional as F
+    with pytest.raises(ValueError, match=message):
+        F.cross_attention(**_attn_args(**over))
+
+
+def _dense_attention(h, memory, wq, wk, wv, wo, heads, kv_heads):
+    """Plain fp64 form; the softmax scale is that of the hidden width."""
+    b, l, d = h.shape
+    q = (h @ wq.T).view(b, l, heads, -1).transpose(1, 2)
+    k, v = ((memory @ w.T).view(b, -1, kv_heads, q.shape[-1]).transpose(1, 2).repeat_interleave(heads // kv_heads, dim=1)
+            for w in (wk, wv))
+    p = torch.softmax(q @ k.transpose(-1, -2) * (d // heads) ** -0.5, dim=-1)
+    return (p @ v).transpose(1, 2).reshape(b, l, -1) @ wo.T
+
+
+# widths of Q and of the result that are not the hidden width; d_model, attention width, result width, heads, KV heads
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype, dims", [
+    (torch.float32, (96, 64, 96, 4, 2)), (torch.float32, (96, 128, 40, 2, 1)), (torch.float32, (96, 96, 64, 3, 3)),
+    (torch.bfloat16, (192, 128, 64, 2, 1)), (torch.bfloat16, (128, 256, 128, 4, 2)),
+])
+def test_cross_attention_takes_rectangular_projections(dtype, dims):
+    from memory_b200 import _lib as L, functional as F
+    d, hd, od, heads, kv = dims
+    dkv, g = kv * (hd // heads), torch.Generator().manual_seed(3)
+    shapes = {"h": (2, 64, d), "memory": (2, 76, 72), "wq": (hd, d), "wk": (dkv, 72), "wv": (dkv, 72), "wo": (od, hd)}
+    x = {n: (torch.randn(*s, generator=g) * (1.0 if n in ("h", "memory") else s[-1] ** -0.5)).to(dtype)
+         for n, s in shapes.items()}
+    ref = {n: t.double().requires_grad_(True) for n, t in x.items()}
+    want = _dense_attention(*ref.values(), heads, kv)
+    grad = torch.randn(want.shape, generator=g)
+    want.backward(grad.to(dtype).double())
+    mine = {n: t.cuda().requires_grad_(True) for n, t in x.items()}
+    out = F.cross_attention(*mine.values(), heads, kv)
+    out.backward(grad.to(dtype).cuda())
+    L.check_device_status(out.device)
+    # fp32: sums of at most a few hundred fp32 products; bf16: a handful of bf16 roundings (2^-9 each) on the way
+    tol = 2e-5 if dtype == torch.float32 else 2e-2
+    for name, a, b in [("out", out, want)] + [(n, mine[n].grad, ref[n].grad) for n in x]:
+        assert a.shape == b.shape, name
+        err = (a.detach().double().cpu() - b.detach()).norm() / b.detach().norm()
+        assert float(err) < tol, (name, float(err))
