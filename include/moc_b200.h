@@ -616,6 +616,7 @@ typedef struct {
   void* arena;
   int32_t* status;
   void *stream, *side_stream;
+  int32_t router_dim;      /* width of h_router and of the router's weight; 0: hidden_dim */
 } moc_layer_desc;
 
 int64_t moc_layer_arena_bytes(const moc_layer_desc* s);

@@ -98,7 +98,7 @@ class LayerDesc(C.Structure):
         " router_dtype attn_dtype bank_dtype weight_dtype row_norm pre_norm add_residual with_losses fused for_backward;"
         "f: routed_scale row_eps pre_eps; l: bank_rows;"
         "p: h_router h_attn bank bank_shadow bank_inv_rms router_w router_b wq wk wv wo norm_w norm_b"
-        " out idx weights comb_idx comb_w losses uniq num_unique arena status stream side_stream")
+        " out idx weights comb_idx comb_w losses uniq num_unique arena status stream side_stream; i: router_dim")
 
 
 class LayerBwdDesc(C.Structure):

@@ -25,13 +25,14 @@ __global__ void add_kernel(float* __restrict__ a, const float* __restrict__ b, i
 }
 
 struct Dims {
-  int64_t rows, n_sel, sel_rows, pairs, d, dkv;
+  int64_t rows, n_sel, sel_rows, pairs, d, dkv, rd;   // rd: width of the router's states
   int k_sel;
 };
 Dims dims_of(const moc_layer_desc* s) {
   Dims x;
   x.k_sel = std::max(0, std::min(s->top_k, s->num_chapters - s->num_shared));
   x.d = s->hidden_dim;
+  x.rd = s->router_dim ? s->router_dim : s->hidden_dim;
   x.dkv = static_cast<int64_t>(s->num_kv_heads) * (s->hidden_dim / s->num_heads);
   x.rows = static_cast<int64_t>(s->batch) * s->seq;
   x.pairs = static_cast<int64_t>(s->batch) * (s->num_shared + x.k_sel);
@@ -40,7 +41,7 @@ Dims dims_of(const moc_layer_desc* s) {
   return x;
 }
 moc_router_shape router_shape(const moc_layer_desc* s) {
-  return {s->batch, s->router_seq, s->hidden_dim, s->num_chapters, s->top_k, s->num_shared, s->routed_scale, s->router_dtype};
+  return {s->batch, s->router_seq, s->router_dim ? s->router_dim : s->hidden_dim, s->num_chapters, s->top_k, s->num_shared, s->routed_scale, s->router_dtype};
 }
 
 // what the forward pass leaves for the backward pass
@@ -59,7 +60,7 @@ int64_t carve(const moc_layer_desc* s, const Dims& x, void* arena, Saved* a) {
   Carver c{static_cast<char*>(arena), 0};
   const moc_router_shape rs = router_shape(s);
   const int64_t B = s->batch, C = s->num_chapters;
-  a->pooled = c.take<float>(B * x.d); a->logits = c.take<float>(B * C); a->probs = c.take<float>(B * C);
+  a->pooled = c.take<float>(B * x.rd); a->logits = c.take<float>(B * C); a->probs = c.take<float>(B * C);
   a->row_stats = c.take<float>(B * 4); a->chapter_stats = c.take<float>(2 * C);
   a->router_ws = c.take<char>(static_cast<int64_t>(moc_router_workspace_bytes(&rs)));
   a->seg_off = c.take<int>(x.pairs + 1); a->seg_pairs = c.take<int>(x.pairs); a->pair_to_uniq = c.take<int>(x.pairs);
@@ -87,6 +88,7 @@ int check(const moc_layer_desc* s) {
   MOC_REQUIRE(s->batch > 0 && s->seq > 0 && s->hidden_dim > 0 && s->num_heads > 0 && s->num_kv_heads > 0 &&
                   s->tokens_per_chapter > 0 && s->num_chapters > 0 && s->bank_rows >= s->tokens_per_chapter, "empty layer problem");
   MOC_REQUIRE(s->hidden_dim % s->num_heads == 0, "hidden_dim must be divisible by num_heads");
+  MOC_REQUIRE(s->router_dim >= 0, "bad router_dim");
   MOC_REQUIRE(s->attn_dtype == MOC_F32 || s->attn_dtype == MOC_BF16, "bad attn_dtype");
   MOC_REQUIRE(!s->fused || (s->bank_shadow && (s->row_norm == MOC_NORM_NONE ||
                                                (s->row_norm == MOC_NORM_RMS && s->bank_inv_rms))),
@@ -243,7 +245,7 @@ int64_t carve_bwd(const moc_layer_desc* s, const moc_layer_bwd_desc* b, const Di
   t->kv_dot = s->fused && s->tokens_per_chapter == 64 ? c.take<float>(x.pairs * s->num_kv_heads) : nullptr;
   t->d_comb_w = c.take<float>(x.pairs);
   t->d_logits = c.take<float>(static_cast<int64_t>(s->batch) * s->num_chapters);
-  t->d_pooled = c.take<float>(static_cast<int64_t>(s->batch) * x.d);
+  t->d_pooled = c.take<float>(static_cast<int64_t>(s->batch) * x.rd);
   t->dummy_b = c.take<float>(s->num_chapters);
   t->router_ws = c.take<char>(static_cast<int64_t>(moc_router_workspace_bytes(&rs)));
   return c.off;
@@ -263,6 +265,8 @@ extern "C" int moc_layer_bwd(const moc_layer_desc* s, const moc_layer_bwd_desc* 
   MOC_REQUIRE(s->for_backward && b && b->g && b->d_h_attn && b->d_wq && b->d_wkv && b->d_wo && b->scratch && s->arena &&
                   s->uniq && s->num_unique && s->status, "NULL layer gradient buffer");
   MOC_REQUIRE(!b->want_router_w || b->d_router_w, "NULL router gradient buffer");
+  MOC_REQUIRE(!b->want_dh_router || b->d_h_router || s->router_dim == 0 || s->router_dim == s->hidden_dim,
+              "router states of another width have a gradient of their own");
   const Dims x = dims_of(s);
   Saved a;
   Scratch t;

@@ -395,12 +395,19 @@ class _MemoryLayerTwoStream(torch.autograd.Function):
         ctx.set_materialize_grads(False)       # an output nobody used has no gradient: no zeros to fill and add
         (num_heads, num_kv_heads, t, top_k, num_shared, routed_scale, row_norm, row_eps, with_losses,
          pre_norm, pre_eps, add_residual, grad_on) = cfg
-        L.require_cuda(h_router, h_attn, bank, router_w)
         if h_router.dim() != 3:
             raise ValueError(f"hidden_states must be 3D (B, T, D), got shape {tuple(h_router.shape)}")
         dev = h_attn.device
         b, l, d = h_attn.shape
         rows, c = bank.shape[0], router_w.shape[0]
+        if h_router.shape[0] != b:
+            raise ValueError(f"h_router and h_attn must share the batch: {h_router.shape[0]} vs {b}")
+        # (the router may look at states of another width than the attention's)
+        _check_width("router_weight", router_w, h_router.shape[2])
+        _check_numel("router_bias", router_b, c)
+        _check_numel("pre_norm_weight", norm_w, d)
+        _check_numel("pre_norm_bias", norm_b, d)
+        L.require_cuda(h_router, h_attn, bank, router_w, router_b, wq, wk, wv, wo, norm_w, norm_b)
         # the kernels take fp32 or bf16 activations; anything else computes in bf16 and is cast back
         in_dtype = h_attn.dtype
         ha = ops._contig(h_attn if in_dtype in (torch.float32, torch.bfloat16) else h_attn.to(torch.bfloat16))
@@ -413,7 +420,9 @@ class _MemoryLayerTwoStream(torch.autograd.Function):
         shadow = None if fused is None else ops._contig(fused["shadow"])
         if shadow is not None and (shadow.dtype != torch.bfloat16 or shadow.shape != bank.shape):
             raise TypeError("bank_shadow must be a bf16 tensor shaped like the bank")
-        inv_rms = ops._contig(fused["inv_rms"]) if (fused is not None and norm == "rms") else None
+        inv_rms = ops._contig(fused["inv_rms"].float()) if (fused is not None and norm == "rms") else None
+        _check_numel("bank_inv_rms", inv_rms, rows)
+        L.require_cuda(shadow, inv_rms)
         bank_c = ops._contig(bank)
         rw = ops._contig(router_w.float())
         rb = None if router_b is None else ops._contig(router_b.float())
@@ -442,7 +451,7 @@ class _MemoryLayerTwoStream(torch.autograd.Function):
             ws[1].data_ptr(), ws[2].data_ptr(), ws[3].data_ptr(), L.ptr(nw), L.ptr(nb), out.data_ptr(), idx.data_ptr(),
             weights.data_ptr(), comb_idx.data_ptr(), comb_w.data_ptr(), losses.data_ptr(), L.ptr(touched),
             None if touched is None else touched.data_ptr() + 4 * n_pairs, None, L.status_word(dev).data_ptr(), main,
-            _side_stream(index, main))
+            _side_stream(index, main), hr.shape[2])
         arena = torch.empty(ops.layer_arena_bytes(s), dtype=torch.uint8, device=dev)
         s.arena = arena.data_ptr()
         ops.layer_fwd(s)
@@ -553,9 +562,10 @@ def memory_layer(h_router: torch.Tensor, h_attn: torch.Tensor, bank: torch.Tenso
     gradient read the bank through a gather list as well instead of copying the raw selected rows out on the side
     stream first (no gathered copy at all, but slower at the paper shape).
     """
-    cd = compute_dtype or h_attn.dtype
+    cd, d = compute_dtype or h_attn.dtype, h_attn.shape[-1]
+    _check_projections(d, bank.shape[1], wq, wk, wv, wo, int(num_heads), int(num_kv_heads or num_heads))
     if (cd == torch.bfloat16 and two_stream and wq.dtype == wk.dtype == wv.dtype == wo.dtype
-            and bank.shape[1] == h_attn.shape[-1]):
+            and bank.shape[1] == wq.shape[0] == wo.shape[0] == d):
         cfg = (int(num_heads), int(num_kv_heads or num_heads), int(tokens_per_chapter), int(top_k),
                int(num_shared_chapters), float(routed_scaling_factor), norm_type, float(norm_eps), bool(with_losses),
                pre_norm, float(pre_norm_eps), bool(add_residual), torch.is_grad_enabled())

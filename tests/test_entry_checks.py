@@ -73,3 +73,65 @@ def test_cross_attention_takes_rectangular_projections(dtype, dims):
         assert a.shape == b.shape, name
         err = (a.detach().double().cpu() - b.detach()).norm() / b.detach().norm()
         assert float(err) < tol, (name, float(err))
+
+
+# ---- the whole layer ---------------------------------------------------------------------------------------------
+def _layer_args(**over):
+    a = dict(h_router=torch.zeros(2, 8, D, dtype=torch.bfloat16), h_attn=torch.zeros(2, 8, D, dtype=torch.bfloat16),
+             bank=torch.zeros(9 * 64, D), router_weight=torch.zeros(9, D), router_bias=torch.zeros(9), wq=torch.zeros(D, D),
+             wk=torch.zeros(D, D), wv=torch.zeros(D, D), wo=torch.zeros(D, D), num_heads=HEADS, num_kv_heads=None,
+             tokens_per_chapter=64, top_k=2)
+    a.update(over)
+    return a
+
+
+@pytest.mark.parametrize("over, message", [
+    (dict(wk=torch.zeros(64, D), wv=torch.zeros(64, D)), "num_kv_heads"),
+    (dict(wv=torch.zeros(64, D)), "num_kv_heads"),
+    (dict(wq=torch.zeros(D, 64)), "inner dimensions differ: wq"),
+    (dict(wk=torch.zeros(D, 64)), "inner dimensions differ: wk"),
+    (dict(wo=torch.zeros(D, 64)), "inner dimensions differ: wo"),
+    (dict(h_router=torch.zeros(1, 8, D, dtype=torch.bfloat16)), "share the batch"),
+    (dict(h_router=torch.zeros(2, 8, 64, dtype=torch.bfloat16)), "inner dimensions differ: router_weight"),
+    (dict(router_weight=torch.zeros(9, 64)), "inner dimensions differ: router_weight"),
+    (dict(router_bias=torch.zeros(8)), "router_bias"),
+    (dict(pre_norm="rms", pre_norm_weight=torch.ones(64)), "pre_norm_weight"),
+    (dict(pre_norm="layernorm", pre_norm_weight=torch.ones(D), pre_norm_bias=torch.ones(64)), "pre_norm_bias"),
+    ({}, "CUDA"),
+])
+def test_memory_layer_refuses(over, message):
+    from memory_b200 import functional as F
+    with pytest.raises(ValueError, match=message):
+        F.memory_layer(**_layer_args(**over))
+
+
+def _layer_run(two_stream, h_router, h_attn, seed=7):
+    """(outputs, gradients) of a small layer; router and attention may look at different states."""
+    from memory_b200 import _lib as L, functional as F
+    g = torch.Generator().manual_seed(seed)
+    dr = h_router.shape[2]
+    p = {"bank": torch.randn(9 * 64, D, generator=g), "router_w": torch.randn(9, dr, generator=g) * 0.3,
+         "router_b": torch.randn(9, generator=g) * 0.1, **{n: torch.randn(D, D, generator=g) * D ** -0.5
+                                                          for n in ("wq", "wk", "wv", "wo")}}
+    p = {n: t.cuda().requires_grad_(True) for n, t in p.items()}
+    same = h_router is h_attn
+    ha = h_attn.cuda().requires_grad_(True)
+    hr = ha if same else h_router.cuda().requires_grad_(True)
+    out, losses, info = F.memory_layer(hr, ha, *p.values(), num_heads=HEADS, num_kv_heads=None, tokens_per_chapter=64,
+                                       top_k=3, two_stream=two_stream, compute_dtype=torch.bfloat16)
+    torch.autograd.backward([out, losses.vector], [torch.randn(out.shape, generator=g).to(out.dtype).cuda(),
+                                                   torch.tensor([1.0, 0.5, 0.1, 0.2], device="cuda")])
+    L.check_device_status(out.device)
+    return {"out": out, "idx": info["indices"], "h_attn": ha.grad, "h_router": hr.grad, **{n: t.grad for n, t in p.items()}}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width, seq", [(64, 50), (200, 64), (72, 1500)])
+def test_router_states_of_another_width_than_the_attention(width, seq):
+    g = torch.Generator().manual_seed(1)
+    h_router, h_attn = (torch.randn(2, n, w, generator=g).bfloat16() for n, w in ((seq, width), (64, D)))
+    one, chain = (_layer_run(two, h_router, h_attn) for two in (True, False))
+    assert torch.equal(one.pop("idx"), chain.pop("idx"))
+    for n in one:        # the same bf16 operators in one call or in three; gradients may round once more between nodes
+        err = (one[n].detach().float() - chain[n].detach().float()).norm() / chain[n].detach().float().norm()
+        assert one[n].dtype == chain[n].dtype and float(err) < 2e-2, (n, float(err))
