@@ -496,7 +496,8 @@ class _MemoryLayerTwoStream(torch.autograd.Function):
         g_w, g_cw, g_losses = as_f32(g_w), as_f32(g_cw), as_f32(g_losses)
         fuse_dh = ctx.same_h and need[0] and hr_dtype == in_dtype and in_dtype == attn_dtype
         d_ha = torch.empty(b, l, d, dtype=attn_dtype, device=dev)
-        d_hr = None if fuse_dh or not need[0] else torch.empty(hr_shape, dtype=hr_dtype, device=dev)
+        r_dtype = f32 if s.router_dtype == L.MOC_F32 else torch.bfloat16      # what the router's kernels write
+        d_hr = None if fuse_dh or not need[0] else torch.empty(hr_shape, dtype=r_dtype, device=dev)
         rows = wire = dense = None
         if need[2]:
             n_rows = n_pairs * t
@@ -524,7 +525,7 @@ class _MemoryLayerTwoStream(torch.autograd.Function):
         if rows is not None or wire is not None:
             sink.add(touched[:n_pairs], touched[n_pairs:], wire if rows is None else rows, t, wire=wire)
 
-        d_ha = _cast(d_ha, in_dtype)
+        d_ha, d_hr = _cast(d_ha, in_dtype), _cast(d_hr, hr_dtype)
         if fuse_dh:
             d_hr, d_ha = d_ha, None
         return (d_hr, d_ha, _cast(dense, bank.dtype), _cast(d_rw, rw.dtype) if need[3] else None, d_rb, _cast(d_wq, wdt[0]),

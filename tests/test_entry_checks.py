@@ -135,3 +135,13 @@ def test_router_states_of_another_width_than_the_attention(width, seq):
     for n in one:        # the same bf16 operators in one call or in three; gradients may round once more between nodes
         err = (one[n].detach().float() - chain[n].detach().float()).norm() / chain[n].detach().float().norm()
         assert one[n].dtype == chain[n].dtype and float(err) < 2e-2, (n, float(err))
+
+
+@pytest.mark.gpu
+def test_fp16_states_get_fp16_gradients():
+    """States the kernels do not take themselves go through bf16, and so do their gradients."""
+    h = torch.randn(2, 64, D, generator=torch.Generator().manual_seed(2)).bfloat16()
+    want, got = (_layer_run(True, x, x) for x in (h, h.half()))
+    assert got["h_attn"].dtype == torch.float16
+    err = (got["h_attn"].float() - want["h_attn"].float()).norm() / want["h_attn"].float().norm()
+    assert float(err) < 1e-2, float(err)      # two bf16 roundings (2^-9) of the sum of both branches against one
