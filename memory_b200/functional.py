@@ -152,9 +152,12 @@ class _Route(torch.autograd.Function):
     @staticmethod
     def forward(ctx, h, weight, bias, top_k, num_shared, routed_scale, with_losses, pos_weight):
         ctx.set_materialize_grads(False)
-        L.require_cuda(h, weight, bias)
         if h.dim() != 3:
             raise ValueError(f"hidden_states must be 3D (B, T, D), got shape {tuple(h.shape)}")
+        _check_width("router weight", weight, h.shape[2])
+        _check_numel("router bias", bias, weight.shape[0])
+        _check_numel("pos_weight", pos_weight, h.shape[1])
+        L.require_cuda(h, weight, bias, pos_weight)
         dev, f32 = h.device, torch.float32
         hc, w = ops._contig(h), ops._contig(weight.float())
         bc = None if bias is None else ops._contig(bias.float())
@@ -619,6 +622,9 @@ class _RouteTokens(torch.autograd.Function):
     def forward(ctx, h, weight, bias, top_k, num_shared, with_losses):
         ctx.set_materialize_grads(False)
         b, l, d = h.shape
+        _check_width("router weight", weight, d)
+        _check_numel("router bias", bias, weight.shape[0])
+        L.require_cuda(h, weight, bias)
         rows = b * l
         h2 = h.reshape(rows, d).contiguous()
         w32 = weight.float().contiguous()

@@ -1299,9 +1299,13 @@ def token_route_fwd(h: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.
                     with_losses: bool):
     """``moc_token_route_fwd`` on h [rows, d] bf16 and the fp32 weight [C, d].  Returns (descriptor, idx int64 [rows, k'],
     weights, losses or None, arena); descriptor and arena go to :func:`token_route_bwd`."""
-    L.require_cuda(h, weight, bias)
     rows, d = h.shape
     c, dev = weight.shape[0], h.device
+    if weight.dim() != 2 or weight.shape[1] != d:
+        raise ValueError(f"inner dimensions differ: {d} vs {tuple(weight.shape)}")
+    if bias is not None and bias.numel() != c:
+        raise ValueError(f"the router's bias must have {c} elements, got {bias.numel()}")
+    L.require_cuda(h, weight, bias)
     k = router_selected_k(c, top_k, num_shared)
     idx = torch.empty(rows, k, dtype=torch.int64, device=dev)
     weights = torch.empty(rows, k, dtype=torch.float32, device=dev)

@@ -145,3 +145,28 @@ def test_fp16_states_get_fp16_gradients():
     assert got["h_attn"].dtype == torch.float16
     err = (got["h_attn"].float() - want["h_attn"].float()).norm() / want["h_attn"].float().norm()
     assert float(err) < 1e-2, float(err)      # two bf16 roundings (2^-9) of the sum of both branches against one
+
+
+# ---- routers -----------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("over, message", [
+    (dict(weight=torch.zeros(9, 64)), "inner dimensions differ"),
+    (dict(weight=torch.zeros(9, 256)), "inner dimensions differ"),
+    (dict(bias=torch.zeros(8)), "bias"),
+    ({}, "CUDA"),
+])
+def test_routers_refuse(over, message):
+    from memory_b200 import functional as F, ops
+    a = dict(dict(weight=torch.zeros(9, D), bias=torch.zeros(9)), **over)
+    h = torch.zeros(2, 8, D, dtype=torch.bfloat16)
+    with pytest.raises(ValueError, match=message):
+        F.route(h, a["weight"], a["bias"], 2, 1)
+    with pytest.raises(ValueError, match=message):
+        F.route_tokens(h, a["weight"], a["bias"], 2, 1)
+    with pytest.raises(ValueError, match=message):
+        ops.token_route_fwd(h.view(16, D), a["weight"], a["bias"], 2, 1, True)
+
+
+def test_route_refuses_pooling_coefficients_of_another_length():
+    from memory_b200 import functional as F
+    with pytest.raises(ValueError, match="pos_weight"):
+        F.route(torch.zeros(2, 8, D), torch.zeros(9, D), torch.zeros(9), 2, 1, pos_weight=torch.zeros(7))
