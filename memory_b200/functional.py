@@ -703,7 +703,7 @@ class _TokenRoutedAttention(torch.autograd.Function):
         """Whether ``moc_token_attn_fwd`` takes the call: bf16 arithmetic, head_dim 64, whole 64-row chapters."""
         ok = (torch.float32, torch.bfloat16)
         return (cd == torch.bfloat16 and t == 64 and h.shape[-1] == num_heads * 64 and wk.shape[0] == num_kv_heads * 64
-                and num_heads % num_kv_heads == 0 and wq.shape == wo.shape == (h.shape[-1], h.shape[-1])
+                and wv.shape == wk.shape and num_heads % num_kv_heads == 0 and wq.shape == wo.shape == (h.shape[-1], h.shape[-1])
                 and wk.dtype == wq.dtype == wv.dtype == wo.dtype and wq.dtype in ok and h.dtype in ok and h.numel() > 0
                 and idx_local.shape[-1] > 0 and routed_mem is not None and routed_mem.numel() > 0
                 and routed_mem.shape[0] % 64 == 0 and routed_mem.dtype in ok

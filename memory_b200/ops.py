@@ -1344,8 +1344,11 @@ def token_attn_fwd(h, shared, routed, idx, weights, wq, wk, wv, wo, num_heads: i
                    for_backward: bool):
     """``moc_token_attn_fwd`` on h [rows, d], the bank slices and chapter ids / weights [.., k] local to ``routed``.  Returns
     (descriptor, out [rows, d] in the dtype of h, tensors to keep for :func:`token_attn_bwd`)."""
-    L.require_cuda(h, shared, routed, idx, weights, wq, wk, wv, wo)
     rows, d = h.shape
+    for name, t, n in (("wq", wq, num_heads * 64), ("wk", wk, num_kv_heads * 64), ("wv", wv, num_kv_heads * 64), ("wo", wo, d)):
+        if tuple(t.shape) != (n, d):
+            raise ValueError(f"inner dimensions differ: {name} {tuple(t.shape)} vs {(n, d)}")
+    L.require_cuda(h, shared, routed, idx, weights, wq, wk, wv, wo)
     k, dev, code, p = idx.shape[-1], h.device, L.dtype_code, L.ptr
     h, routed = _contig(h), _contig(routed)
     shared = _contig(shared) if shared is not None and shared.numel() > 0 else None
@@ -1354,7 +1357,7 @@ def token_attn_fwd(h, shared, routed, idx, weights, wq, wk, wv, wo, num_heads: i
     wq, wk, wv, wo = (_contig(t) for t in (wq, wk, wv, wo))
     if ids.numel() != rows * k or w.numel() != rows * k:
         raise ValueError("chapter ids and weights must be given for every token")
-    for name, t in (("shared_memory", shared), ("routed_memory", routed), ("wk", wk), ("wv", wv)):
+    for name, t in (("shared_memory", shared), ("routed_memory", routed)):
         if t is not None and (t.dim() != 2 or t.shape[1] != d):
             raise ValueError(f"inner dimensions differ: {name} {tuple(t.shape)} vs {d}")
     s = L.TokenAttnDesc(rows, d, num_heads, num_kv_heads, k, 0 if shared is None else shared.shape[0], routed.shape[0],

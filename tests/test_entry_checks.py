@@ -170,3 +170,21 @@ def test_route_refuses_pooling_coefficients_of_another_length():
     from memory_b200 import functional as F
     with pytest.raises(ValueError, match="pos_weight"):
         F.route(torch.zeros(2, 8, D), torch.zeros(9, D), torch.zeros(9), 2, 1, pos_weight=torch.zeros(7))
+
+
+# ---- token-routed attention --------------------------------------------------------------------------------------
+def test_token_attention_refuses_projections_of_another_size():
+    from memory_b200 import functional as F, ops
+    h, routed = torch.zeros(1, 8, D, dtype=torch.bfloat16), torch.zeros(4 * 64, D)
+    idx, w = torch.zeros(1, 8, 2, dtype=torch.int32), torch.zeros(1, 8, 2)
+    good = {"wq": (D, D), "wk": (64, D), "wv": (64, D), "wo": (D, D)}
+
+    def native(**over):
+        return F._TokenRoutedAttention._native(h, None, routed, idx, *(torch.zeros(*s) for s in dict(good, **over).values()),
+                                               HEADS, 1, 64, torch.bfloat16)
+    assert native()
+    for name, shape in (("wv", (128, D)), ("wv", (64, 64)), ("wk", (128, D)), ("wo", (D, 64)), ("wq", (64, D))):
+        assert not native(**{name: shape}), (name, shape)
+        ws = [torch.zeros(*s) for s in dict(good, **{name: shape}).values()]
+        with pytest.raises(ValueError, match="inner dimensions differ"):
+            ops.token_attn_fwd(h.view(8, D), None, routed, idx, w, *ws, HEADS, 1, 1.0, False)
