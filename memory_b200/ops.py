@@ -1239,16 +1239,23 @@ def decode_step(hidden: torch.Tensor, routing_states: torch.Tensor, router_w: to
     that agree in shapes, types and weights (by address) are filled once."""
     w = _contig(router_w.float())
     bias = None if router_b is None else _contig(router_b.float())
-    h, states = _contig(hidden), _contig(routing_states)
+    h, states, wq, wo, kv_bank = (_contig(t) for t in (hidden, routing_states, wq, wo, kv_bank))
     dev, p = h.device, L.ptr
     stream = L.stream_ptr(dev)
-    key = (h.shape, states.shape, w.shape, kv_bank.shape, h.dtype, states.dtype, dev, w.data_ptr(), p(bias), wq.data_ptr(),
-           wo.data_ptr(), kv_bank.data_ptr(), top_k, stream)
+    # everything the descriptor holds or a check looked at; the per-step buffers are filled in below
+    key = (h.shape, states.shape, w.shape, wq.shape, wo.shape, kv_bank.shape, h.dtype, states.dtype, wq.dtype, wo.dtype,
+           kv_bank.dtype, dev, w.data_ptr(), p(bias), None if bias is None else bias.shape, wq.data_ptr(),
+           wo.data_ptr(), kv_bank.data_ptr(), num_heads, num_kv_heads, tokens_per_chapter, top_k, num_shared, routed_scale,
+           scale, stream)
     plan = None if plans is None else plans.get(key)
     if plan is None:
         L.require_cuda(h, states, w, bias, wq, wo, kv_bank)
         if states.dim() != 3:
             raise ValueError(f"hidden_states must be 3D (B, T, D), got shape {tuple(states.shape)}")
+        if not wq.dtype == wo.dtype == kv_bank.dtype == torch.bfloat16:
+            raise TypeError("decoding runs on bf16 projections and a bf16 K/V cache")
+        if bias is not None and bias.numel() != w.shape[0]:
+            raise ValueError(f"the router's bias must have {w.shape[0]} elements, got {bias.numel()}")
         b, n_q, d = h.shape
         rb, window, rd = states.shape
         c, head_dim = w.shape[0], wq.shape[0] // num_heads

@@ -188,3 +188,83 @@ def test_token_attention_refuses_projections_of_another_size():
         ws = [torch.zeros(*s) for s in dict(good, **{name: shape}).values()]
         with pytest.raises(ValueError, match="inner dimensions differ"):
             ops.token_attn_fwd(h.view(8, D), None, routed, idx, w, *ws, HEADS, 1, 1.0, False)
+
+
+# ---- decoding ----------------------------------------------------------------------------------------------------
+class _FakeLibrary:
+    """Stands in for the native library: keeps the descriptors it is called with."""
+
+    def __init__(self):
+        self.seen = []
+
+    def moc_decode_step_arena_bytes(self, s):
+        return 16
+
+    def moc_decode_step(self, s):
+        self.seen.append(bytes(s._obj))
+        return 0
+
+
+@pytest.fixture
+def decoder(monkeypatch):
+    """A decoder on CPU tensors over the fake library, and what that was called with."""
+    from types import SimpleNamespace
+    from memory_b200 import MemoryDecoder, _lib as L, functional as F
+    fake, status = _FakeLibrary(), torch.zeros(1, dtype=torch.int32)
+    for name, fn in (("lib", lambda: fake), ("stream_ptr", lambda dev: 1), ("require_cuda", lambda *t: None),
+                     ("status_word", lambda dev: status), ("device_index", lambda dev: 0)):
+        monkeypatch.setattr(L, name, fn)
+    monkeypatch.setattr(F, "_side_stream", lambda dev, main: 2)
+    cache = SimpleNamespace(kv_bank=torch.zeros(9 * 64, 2 * D, dtype=torch.bfloat16), tokens_per_chapter=64)
+    bf = torch.zeros(D, D, dtype=torch.bfloat16)
+    return MemoryDecoder(cache, torch.zeros(9, D), torch.zeros(9), bf, bf.clone(), num_heads=HEADS, top_k=2), fake
+
+
+def _decode_states():
+    return torch.zeros(2, 1, D, dtype=torch.bfloat16), torch.zeros(2, 16, D, dtype=torch.bfloat16)
+
+
+@pytest.mark.parametrize("change, where", [
+    (dict(routed_scale=7.5), ("router", "routed_scale", 7.5)),
+    (dict(num_shared=0), ("router", "num_shared", 0)),
+    (dict(top_k=3), ("router", "top_k", 3)),
+    (dict(scale=0.5), ("attn", "scale", 0.5)),
+    (dict(num_heads=1, num_kv_heads=1), ("attn", "num_heads", 1)),
+    (dict(tokens_per_chapter=32), ("attn", "tokens_per_chapter", 32)),
+])
+def test_a_decoder_changed_between_steps_decodes_with_the_change(decoder, change, where):
+    from memory_b200 import _lib as L
+    dec, fake = decoder
+    dec.step(*_decode_states())
+    dec.step(*_decode_states())
+    for name, value in change.items():
+        setattr(dec.cache if name == "tokens_per_chapter" else dec, name, value)
+    dec.step(*_decode_states())
+    first, _, last = (L.DecodeStepDesc.from_buffer_copy(b) for b in fake.seen)
+    part, field, value = where
+    assert getattr(getattr(last, part), field) == value != getattr(getattr(first, part), field)
+    assert last.attn.n_chapters == last.router.num_shared + last.router.top_k
+
+
+@pytest.mark.parametrize("name, tensor, error", [
+    ("wq_c", torch.zeros(D, D), TypeError), ("wo_c", torch.zeros(D, D), TypeError),
+    ("wq_c", torch.zeros(D, 64, dtype=torch.bfloat16), ValueError),
+    ("wo_c", torch.zeros(D, 64, dtype=torch.bfloat16), ValueError),
+    ("router_bias", torch.zeros(8), ValueError), ("router_weight", torch.zeros(9, 64), ValueError),
+])
+def test_a_decoder_refuses_weights_swapped_in_between_steps(decoder, name, tensor, error):
+    dec, fake = decoder
+    dec.step(*_decode_states())
+    setattr(dec, name, tensor)
+    with pytest.raises(error):
+        dec.step(*_decode_states())
+    assert len(fake.seen) == 1
+
+
+def test_a_decoder_passes_dense_copies_of_strided_weights(decoder):
+    from memory_b200 import _lib as L
+    dec, fake = decoder
+    wide = torch.zeros(D, 2 * D, dtype=torch.bfloat16)
+    dec.wq_c = wide[:, :D]
+    dec.step(*_decode_states())
+    assert L.DecodeStepDesc.from_buffer_copy(fake.seen[0]).wq != wide.data_ptr()
