@@ -447,6 +447,7 @@ typedef struct {
   void *out, *arena;
   int32_t* status;
   void *stream, *side_stream;
+  int32_t hidden_dim;      /* width of hidden; 0: that of the routing states */
 } moc_decode_step_desc;
 int64_t moc_decode_step_arena_bytes(const moc_decode_step_desc* s);
 int moc_decode_step(const moc_decode_step_desc* s);

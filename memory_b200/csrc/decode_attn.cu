@@ -216,12 +216,13 @@ struct StepArena {
   __nv_bfloat16 *x, *q, *o;
   char* route_arena;
 };
+int64_t width_of(const moc_decode_step_desc* s) { return s->hidden_dim ? s->hidden_dim : s->router.hidden_dim; }
 int64_t carve(const moc_decode_step_desc* s, StepArena* a) {
   a->route = moc_route_desc{};
   a->route.shape = s->router;
   Carver c{static_cast<char*>(s->arena), 0};
   const int64_t rows = static_cast<int64_t>(s->attn.batch) * s->attn.n_q, width = static_cast<int64_t>(s->attn.num_heads) * kDD;
-  a->x = c.take<__nv_bfloat16>(rows * s->router.hidden_dim);
+  a->x = c.take<__nv_bfloat16>(rows * width_of(s));
   a->q = c.take<__nv_bfloat16>(rows * width);
   a->o = c.take<__nv_bfloat16>(rows * width);
   a->route_arena = c.take<char>(moc_route_arena_bytes(&a->route));
@@ -294,14 +295,14 @@ extern "C" int moc_decode_step(const moc_decode_step_desc* s) {
   MOC_REQUIRE(s && s->routing_states && s->hidden && s->router_w && s->wq && s->wo && s->kv_bank && s->out && s->arena &&
               s->status, "NULL decode-step buffer");
   MOC_REQUIRE(s->attn.head_dim == kDD, "decode attention needs head_dim 64");
-  MOC_REQUIRE(s->router.batch == s->attn.batch && s->out_dim > 0, "bad decode-step shape");
+  MOC_REQUIRE(s->router.batch == s->attn.batch && s->out_dim > 0 && s->hidden_dim >= 0, "bad decode-step shape");
   StepArena a;
   carve(s, &a);
   moc_route_desc* r = &a.route;
   r->h = s->routing_states; r->w = s->router_w; r->bias = s->router_b;
   r->idx = s->idx; r->weights = s->weights; r->comb_idx = s->comb_idx; r->comb_w = s->comb_w;
   r->arena = a.route_arena; r->status = s->status; r->stream = s->stream;
-  const int64_t rows = static_cast<int64_t>(s->attn.batch) * s->attn.n_q, d = s->router.hidden_dim;
+  const int64_t rows = static_cast<int64_t>(s->attn.batch) * s->attn.n_q, d = width_of(s);
   const int64_t width = static_cast<int64_t>(s->attn.num_heads) * kDD;
   // the query projection needs nothing of the router; beside it from a dozen rows on, where it takes longer than the events
   cudaStream_t main = static_cast<cudaStream_t>(s->stream);

@@ -1261,6 +1261,8 @@ def decode_step(hidden: torch.Tensor, routing_states: torch.Tensor, router_w: to
         c, head_dim = w.shape[0], wq.shape[0] // num_heads
         if wq.shape[1] != d or wo.shape[1] != wq.shape[0]:
             raise ValueError(f"inner dimensions differ: {d} / {wq.shape[0]} vs {wq.shape[1]} / {wo.shape[1]}")
+        if wq.shape[0] % num_heads != 0:
+            raise ValueError(f"wq {tuple(wq.shape)} does not hold {num_heads} heads")
         if rd != w.shape[1]:
             raise ValueError(f"inner dimensions differ: {rd} vs {w.shape[1]}")
         if kv_bank.shape[1] != 2 * num_kv_heads * head_dim:
@@ -1273,7 +1275,7 @@ def decode_step(hidden: torch.Tensor, routing_states: torch.Tensor, router_w: to
             L.RouterShape(b, window, rd, c, top_k, num_shared, routed_scale, L.dtype_code(states.dtype)),
             L.DecodeShape(b, n_q, num_heads, num_kv_heads, head_dim, num_shared + k, tokens_per_chapter, scale),
             L.dtype_code(h.dtype), wo.shape[0], kv_bank.shape[0], None, None, p(w), p(bias), p(wq), p(wo), p(kv_bank), None,
-            None, None, None, None, None, p(L.status_word(dev)), stream, _side_stream(L.device_index(dev), stream))
+            None, None, None, None, None, p(L.status_word(dev)), stream, _side_stream(L.device_index(dev), stream), d)
         plan = (bytes(s), _size("moc_decode_step_arena_bytes", s), (b, k), (b, num_shared + k), (b, n_q, wo.shape[0]),
                 5 + int(window <= 1024) + 2 * int(window > 1024) + int(h.dtype == torch.float32))
         if plans is not None:

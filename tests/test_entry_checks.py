@@ -268,3 +268,31 @@ def test_a_decoder_passes_dense_copies_of_strided_weights(decoder):
     dec.wq_c = wide[:, :D]
     dec.step(*_decode_states())
     assert L.DecodeStepDesc.from_buffer_copy(fake.seen[0]).wq != wide.data_ptr()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width", [64, 200])
+def test_decoding_with_routing_states_of_another_width(width):
+    import memory_b200 as M
+    from memory_b200 import _lib as L, ops
+    g = torch.Generator().manual_seed(11)
+    rnd = lambda *s, scale=1.0: (torch.randn(*s, generator=g) * scale).cuda()      # noqa: E731
+    cache = M.ProjectedBankCache(rnd(9 * 64, D), rnd(D, D, scale=0.1), rnd(D, D, scale=0.1), 64)
+    dec = M.MemoryDecoder(cache, rnd(9, width), rnd(9), rnd(D, D, scale=0.1), rnd(D, D, scale=0.1), num_heads=HEADS, top_k=3)
+    hidden, states = rnd(20, 1, D).bfloat16(), rnd(20, 16, width).bfloat16()
+    out, info = dec.step(hidden, states)
+    idx, _, cidx, cw, _ = M.route(states, dec.router_weight, dec.router_bias, 3, 1, 2.5, False)
+    q = ops.gemm(hidden.view(20, D), dec.wq_c)
+    o = ops.decode_attn(q.view(20, 1, D), cache.kv_bank, cidx, cw, HEADS, HEADS, 64, dec.scale)
+    want = ops.gemm(o.view(20, D), dec.wo_c).view(20, 1, D)
+    L.check_device_status(out.device)
+    assert torch.equal(info["indices"], idx) and torch.equal(out, want)            # the same operators, issued singly
+
+
+def test_the_descriptor_of_a_decoding_step_has_both_widths(decoder):
+    from memory_b200 import _lib as L
+    dec, fake = decoder
+    dec.router_weight = torch.zeros(9, 64)
+    dec.step(_decode_states()[0], torch.zeros(2, 16, 64, dtype=torch.bfloat16))
+    s = L.DecodeStepDesc.from_buffer_copy(fake.seen[0])
+    assert (s.router.hidden_dim, s.hidden_dim) == (64, D)
