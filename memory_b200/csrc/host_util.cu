@@ -103,6 +103,24 @@ __global__ void wait_probe_kernel(int expected, int arrivals, uint32_t poll_limi
   }
 }
 
+// Four warps, each waiting for a barrier of its own that is complete except in the warps of `late`: what each then hears
+// from the barrier at which they agree.
+__global__ void agree_probe_kernel(uint32_t late, uint32_t poll_limit, int* status, int* out) {
+  __shared__ __align__(8) uint64_t bars[4];
+  __shared__ int abort_flag[4];
+  const int warp = threadIdx.x >> 5;
+  if (threadIdx.x < 4) {
+    abort_flag[threadIdx.x] = 0;
+    mbar_init(&bars[threadIdx.x], 1);
+    fence_mbar_init();
+    if (!((late >> threadIdx.x) & 1u)) mbar_arrive(&bars[threadIdx.x]);
+  }
+  __syncthreads();
+  const bool mine = __all_sync(0xffffffffu, mbar_wait_limited(&bars[warp], 0, &abort_flag[warp], status, poll_limit));
+  const bool all = warps_agree<1, 128>(mine);
+  if ((threadIdx.x & 31) == 0) { out[warp] = mine ? 1 : 0; out[4 + warp] = all ? 1 : 0; }
+}
+
 // Barrier between the ranks of one node over flag words in each other's memory (plain peer stores and loads, one
 // thread per peer, no SM held while nothing is due).  Rank r's flag array lives in r's own memory; word q of it is
 // written by rank q only.  An arrival stores the epoch (a counter that only grows) with release semantics at system
@@ -149,6 +167,16 @@ extern "C" int moc_wait_probe(int32_t expected, int32_t arrivals, uint32_t poll_
   MOC_REQUIRE(expected >= 1 && expected <= 96 && arrivals >= 0 && arrivals <= expected, "bad arrival counts");
   MOC_REQUIRE(poll_limit >= 1 && poll_limit <= (1u << 20), "poll_limit must be in [1, 2^20]");
   wait_probe_kernel<<<1, 128, 0, static_cast<cudaStream_t>(stream_)>>>(expected, arrivals, poll_limit, status, out);
+  MOC_CUDA_OK(cudaGetLastError());
+  return MOC_OK;
+}
+
+extern "C" int moc_agree_probe(uint32_t late_warps, uint32_t poll_limit, int32_t* status, int32_t* out, void* stream_) {
+  using namespace moc;
+  MOC_REQUIRE(status && out, "NULL buffer");
+  MOC_REQUIRE(late_warps < 16, "four warps");
+  MOC_REQUIRE(poll_limit >= 1 && poll_limit <= (1u << 20), "poll_limit must be in [1, 2^20]");
+  agree_probe_kernel<<<1, 128, 0, static_cast<cudaStream_t>(stream_)>>>(late_warps, poll_limit, status, out);
   MOC_CUDA_OK(cudaGetLastError());
   return MOC_OK;
 }

@@ -123,6 +123,17 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
   if (__all_sync(0xffffffffu, ok)) return true;
   return __all_sync(0xffffffffu, ok || mbar_wait_slow(bar, parity, abort_flag, status, kWaitPollLimit, where));
 }
+// Barrier ID of N threads (whole warps) that tells each whether all of them came with `ok`
+template <int ID, int N> __device__ __forceinline__ bool warps_agree(bool ok) {
+  uint32_t all;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "bar.red.and.pred q, %2, %3, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(all) : "r"(ok ? 1u : 0u), "n"(ID), "n"(N) : "memory");
+  return all != 0;
+}
 #define mbar_wait(bar, parity, abort_flag, status) \
   mbar_wait_limited(bar, parity, abort_flag, status, kWaitPollLimit, __LINE__)
 

@@ -250,6 +250,16 @@ def wait_probe(device, expected: int, arrivals: int, poll_limit: int):
     return tuple(int(v) for v in out.tolist())
 
 
+def agree_probe(device, late_warps: int, poll_limit: int):
+    """Runs the self-test of the agreement barrier; returns (each warp's own wait, what each warp hears)."""
+    out = torch.zeros(8, dtype=torch.int32, device=device)
+    rc = L.lib().moc_agree_probe(int(late_warps), int(poll_limit), L.ptr(L.status_word(device)), L.ptr(out),
+                                 L.stream_ptr(device))
+    L.check(rc, "moc_agree_probe")
+    got = out.tolist()
+    return got[:4], got[4:]
+
+
 # --------------------------------------------------------------------------------------------
 # gather
 # --------------------------------------------------------------------------------------------

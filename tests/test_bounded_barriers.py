@@ -1,0 +1,33 @@
+"""Waits of the kernels give up after a limit, in one warp and not in another; a barrier between such waits has no limit.  So
+warps that share one must all reach it, and leave their loops on what it tells all of them."""
+import os
+import re
+
+import pytest
+import torch
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "memory_b200", "csrc")
+
+
+def test_row_warps_of_the_token_mixture_leave_their_loop_at_the_barrier_only():
+    text = open(os.path.join(CSRC, "token_mix_tc.cu")).read()
+    kernel = text[text.index("token_mix_fwd_tc_kernel("):text.index("__global__ void slot_reduce_kernel")]
+    rows = kernel[kernel.index("const int r = threadIdx.x;"):]          # what the row-owning warps run
+    lines = [ln.strip() for ln in rows.splitlines()]
+    meets = [i for i, ln in enumerate(lines) if "row_warps_agree(" in ln]
+    exits = [i for i, ln in enumerate(lines) if re.search(r"\b(break|return|continue|goto)\b", ln)]
+    assert len(meets) == 2 and "bar.sync" not in rows
+    assert [i - 1 for i in exits] == meets[1:], "a way out that another warp need not take"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("late", [0, 1, 8, 6, 15])
+def test_warps_agree_about_their_waits(late):
+    from memory_b200 import _lib as L, ops
+    dev = torch.device("cuda:0")
+    own, heard = ops.agree_probe(dev, late, 2000)
+    assert own == [1 - ((late >> w) & 1) for w in range(4)] and heard == [int(late == 0)] * 4
+    if late:
+        with pytest.raises(RuntimeError, match="timed out"):
+            L.check_device_status(dev)
+    L.check_device_status(dev)
