@@ -508,8 +508,9 @@ int moc_sparse_attn_bwd(const moc_sparse_attn_shape* s, const void* q, const voi
  * KV head): an inverted index key unit -> (token, slot) pairs is built on the device, every unit's K / V tile is
  * multiplied with the gathered query rows that selected it, and a token's partial results are merged.  d_k / d_v are
  * bf16 like k / v, written in full.  `index` (index_bytes) is filled by the forward call; the backward call reads it
- * when have_index != 0 and fills it from block_indices otherwise.  `scratch`: fwd_bytes / bwd_bytes.  All three are
- * 16-byte aligned.  Chapter ids outside [0, TK / block_size) raise MOC_DEV_BAD_INDEX and contribute nothing. */
+ * when have_index != 0 and fills it from block_indices otherwise.  `scratch`: fwd_bytes / bwd_bytes, at most 1 GiB (and
+ * fp32 dK / dV of one batch item): larger problems run in slices of batch items or tokens, one after the other, and
+ * build the index of each anew.  All three are 16-byte aligned.  Chapter ids outside [0, TK / block_size) raise MOC_DEV_BAD_INDEX and contribute nothing. */
 int moc_sparse_attn_tc_sizes(const moc_sparse_attn_shape* s, int64_t* index_bytes, int64_t* fwd_bytes,
                              int64_t* bwd_bytes);
 int moc_sparse_attn_tc_fwd(const moc_sparse_attn_shape* s, const void* q, const void* k, const void* v,

@@ -274,6 +274,7 @@ struct BwdParams {
   const float* delta;        // [B * TQ, HQ]
   float* dq_partial;         // [KU / 64][n_pairs * G, 64], in entry order
   __nv_bfloat16 *d_k, *d_v;  // [B, TK, H, 64]
+  float *acc_k, *acc_v;      // the same in fp32, added to in their place: a slice of a batch item's tokens; else NULL
   float* part;               // [parts][KU / 64][128, 64]: dV rows, then dK rows, of buckets cut into several items
   int* status;
 };
@@ -406,11 +407,11 @@ sparse_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   } else {
     const int r = threadIdx.x;
     const uint32_t t_row = tmem + (static_cast<uint32_t>(warp * 32) << 16);
-    // a key row of an item's dK (threads 64..127) or dV
-    auto out_row = [&](const TileIter& i) {
+    // where a key row of an item's dK (threads 64..127) or dV starts
+    auto out_at = [&](const TileIter& i) {
       int h;
       const long long row = i.key_row(p, &h);
-      return (r >= 64 ? p.d_k : p.d_v) + ((row + (r & 63)) * x.H + h) * kD;
+      return ((row + (r & 63)) * x.H + h) * kD;
     };
     auto advance = [&](TileIter& i) {               // as above; the dK / dV rows of empty items are zero-filled
       if (i.t + 1 < i.nt) { ++i.t; return; }
@@ -419,7 +420,8 @@ sparse_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         if (i.w >= n_work) return;
         i.open(p);
         if (i.nt > 0) return;
-        uint4* dst = reinterpret_cast<uint4*>(out_row(i));
+        if (p.acc_k != nullptr) continue;
+        uint4* dst = reinterpret_cast<uint4*>((r >= 64 ? p.d_k : p.d_v) + out_at(i));
 #pragma unroll
         for (int e = 0; e < 8; ++e) dst[e] = make_uint4(0u, 0u, 0u, 0u);
       }
@@ -501,8 +503,20 @@ sparse_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         tmem_wait_ld();
         tc_fence_before();
         mbar_arrive(d_read);
-        if (cur.part < 0) {
-          uint4* dst = reinterpret_cast<uint4*>(out_row(cur));
+        if (cur.part < 0 && p.acc_k != nullptr) {      // (these rows are this item's alone)
+          float* dst = (r >= 64 ? p.acc_k : p.acc_v) + out_at(cur);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float4 a0 = reinterpret_cast<const float4*>(dst + j * 8)[0], a1 = reinterpret_cast<const float4*>(dst + j * 8)[1];
+            const uint32_t* o = j < 4 ? o0 + 8 * j : o1 + 8 * (j - 4);
+            const float v[8] = {fmaf(__uint_as_float(o[0]), f, a0.x), fmaf(__uint_as_float(o[1]), f, a0.y),
+                                fmaf(__uint_as_float(o[2]), f, a0.z), fmaf(__uint_as_float(o[3]), f, a0.w),
+                                fmaf(__uint_as_float(o[4]), f, a1.x), fmaf(__uint_as_float(o[5]), f, a1.y),
+                                fmaf(__uint_as_float(o[6]), f, a1.z), fmaf(__uint_as_float(o[7]), f, a1.w)};
+            st_v8(dst + j * 8, v);
+          }
+        } else if (cur.part < 0) {
+          uint4* dst = reinterpret_cast<uint4*>((r >= 64 ? p.d_k : p.d_v) + out_at(cur));
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const uint32_t* o = j < 4 ? o0 + 8 * j : o1 + 8 * (j - 4);
@@ -534,7 +548,7 @@ sparse_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 
 // dK / dV of the buckets that were cut into several items: their fp32 partials in item order.  One CTA per bucket.
 __global__ void part_sum_kernel(Shape x, Index ib, const float* __restrict__ part, __nv_bfloat16* __restrict__ d_k,
-                                __nv_bfloat16* __restrict__ d_v) {
+                                __nv_bfloat16* __restrict__ d_v, float* __restrict__ acc_k, float* __restrict__ acc_v) {
   const int bkt = blockIdx.x;
   const int p0 = ib.part_off[bkt], n = ib.part_off[bkt + 1] - p0;
   if (n == 0) return;
@@ -547,8 +561,13 @@ __global__ void part_sum_kernel(Shape x, Index ib, const float* __restrict__ par
       const float4 v = reinterpret_cast<const float4*>(part + ((static_cast<long long>(p0 + k) * halves + half) * 128 + r) * kD)[c4];
       acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
     }
-    __nv_bfloat16* dst = (r >= 64 ? d_k : d_v) + ((row0 + half * 64 + (r & 63)) * x.H + h) * kD;
-    reinterpret_cast<uint2*>(dst)[c4] = make_uint2(pack_bf16x2(acc.x, acc.y), pack_bf16x2(acc.z, acc.w));
+    const long long at = ((row0 + half * 64 + (r & 63)) * x.H + h) * kD;
+    if (acc_k != nullptr) {
+      float4* dst = reinterpret_cast<float4*>((r >= 64 ? acc_k : acc_v) + at) + c4;
+      *dst = make_float4(dst->x + acc.x, dst->y + acc.y, dst->z + acc.z, dst->w + acc.w);
+    } else {
+      reinterpret_cast<uint2*>((r >= 64 ? d_k : d_v) + at)[c4] = make_uint2(pack_bf16x2(acc.x, acc.y), pack_bf16x2(acc.z, acc.w));
+    }
   }
 }
 
@@ -599,13 +618,76 @@ static int make_shape(const moc_sparse_attn_shape* s, Shape* x) {
   x->ppt = kRows / x->G;
   x->n_pairs = static_cast<long long>(s->batch) * s->tq * s->h * s->n_select * x->U;
   x->n_buckets = static_cast<long long>(s->batch) * s->h * x->M;
-  MOC_REQUIRE(x->n_pairs < (1ll << 30) && x->n_buckets < (1ll << 28) &&
-                  static_cast<long long>(s->batch) * s->tq * s->hq < (1ll << 31) &&
-                  static_cast<long long>(s->batch) * s->tk < (1ll << 31), "problem too large for 32-bit row ids");
   // backward items: about three per resident CTA when the buckets are too few or too uneven to fill the chip
   x->chunk = 1;
   x->chunk = static_cast<int>(std::max<long long>(1, max_tiles(*x) * (x->KU / 64) / (sm_count() * 2 * 3)));
   x->scale = s->scale; x->scale_log2 = s->scale * kLog2e;
+  return MOC_OK;
+}
+
+// Fixed-size pieces of a problem.  Its scratch grows with the listed (token, slot) pairs: 512 bytes a pair and query head
+// with 128-key units, 0.54 GB for 8,192 tokens x 8 blocks x 16 heads on one KV head.  What needs more than kScratchLimit
+// runs in slices that share one scratch: whole batch items where one fits, else runs of one item's tokens, whose dK / dV
+// add up in fp32.  The limit keeps problems of the size measured whole, and a slice fills the chip many times over.
+constexpr int64_t kScratchLimit = int64_t{1} << 30;
+struct Sizes { int64_t index, fwd, bwd; };
+static bool sizes_of(const Shape& x, Sizes* z) {          // false: beyond 32-bit row and pair ids
+  Index ib;
+  z->index = static_cast<int64_t>(carve(x, nullptr, &ib));
+  const int64_t rows = x.n_pairs * x.G, toks = static_cast<int64_t>(x.B) * x.TQ * x.HQ;
+  z->fwd = rows * (kD + 1) * 4 + 64;
+  z->bwd = rows * (x.KU / 64) * kD * 4 + max_parts(x) * (x.KU / 64) * 128 * kD * 4 + toks * 4 + 64;
+  return x.n_pairs < (1ll << 30) && x.n_buckets < (1ll << 28) && toks < (1ll << 31) &&
+         static_cast<long long>(x.B) * x.TK < (1ll << 31);
+}
+struct Slices { int items, tokens; };                     // batch items and tokens of a slice (the last may have fewer)
+static int slice(const moc_sparse_attn_shape* s, Slices* p, Sizes* z) {
+  MOC_REQUIRE(s != nullptr, "shape is NULL");
+  p->items = s->batch; p->tokens = s->tq;
+  bool ids = false;
+  auto size = [&](int items, int tokens, Sizes* out) -> int {
+    moc_sparse_attn_shape part = *s;
+    part.batch = items; part.tq = tokens;
+    Shape x;
+    const int rc = make_shape(&part, &x);
+    if (rc == MOC_OK) ids = sizes_of(x, out);
+    return rc;
+  };
+  for (;;) {
+    const int rc = size(p->items, p->tokens, z);
+    if (rc != MOC_OK) return rc;
+    const int64_t bytes = std::max(z->fwd, z->bwd);
+    if ((ids && bytes <= kScratchLimit) || (p->items == 1 && p->tokens == 1)) break;
+    int& n = p->items > 1 ? p->items : p->tokens;         // equal shares of as many pieces as the bytes ask for
+    const int64_t total = p->items > 1 ? s->batch : s->tq, now = (total + n - 1) / n;
+    const int64_t pieces = std::max(now + 1, now * ((bytes + kScratchLimit - 1) / kScratchLimit));
+    n = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(n - 1, (total + pieces - 1) / pieces)));
+  }
+  MOC_REQUIRE(ids, "problem too large for 32-bit row ids");
+  // the tail can need more than a full slice: its buckets may be cut finer
+  const int tail_items = s->batch % p->items, tail_tokens = s->tq % p->tokens;
+  if (tail_items || tail_tokens) {
+    Sizes t;
+    const int rc = size(tail_items ? tail_items : p->items, tail_tokens ? tail_tokens : p->tokens, &t);
+    if (rc != MOC_OK) return rc;
+    z->index = std::max(z->index, t.index); z->fwd = std::max(z->fwd, t.fwd); z->bwd = std::max(z->bwd, t.bwd);
+  }
+  if (p->tokens < s->tq) z->bwd += 2 * static_cast<int64_t>(s->tk) * s->h * kD * 4;       // fp32 dK / dV of one item
+  return MOC_OK;
+}
+// what a slice starts with: its shape, its first (batch item, token) and (batch item, key row)
+template <typename Fn> static int for_slices(const moc_sparse_attn_shape* s, const Slices& p, Fn fn) {
+  for (int b0 = 0; b0 < s->batch; b0 += p.items) {
+    for (int t0 = 0; t0 < s->tq; t0 += p.tokens) {
+      moc_sparse_attn_shape part = *s;
+      part.batch = std::min(p.items, s->batch - b0); part.tq = std::min(p.tokens, s->tq - t0);
+      Shape x;
+      int rc = make_shape(&part, &x);
+      if (rc != MOC_OK) return rc;
+      rc = fn(x, static_cast<int64_t>(b0) * s->tq + t0, static_cast<int64_t>(b0) * s->tk, t0 == 0, t0 + part.tq == s->tq);
+      if (rc != MOC_OK) return rc;
+    }
+  }
   return MOC_OK;
 }
 static int kv_maps(const Shape& x, const void* k, const void* v, int rows, CUtensorMap* mk, CUtensorMap* mv) {
@@ -636,75 +718,101 @@ using namespace moc::sparse_tc;
 
 extern "C" int moc_sparse_attn_tc_sizes(const moc_sparse_attn_shape* s, int64_t* index_bytes, int64_t* fwd_bytes,
                                         int64_t* bwd_bytes) {
-  Shape x;
-  const int rc = make_shape(s, &x);
+  Slices p;
+  Sizes z;
+  const int rc = slice(s, &p, &z);
   if (rc != MOC_OK) return rc;
   MOC_REQUIRE(index_bytes && fwd_bytes && bwd_bytes, "NULL argument");
-  Index ib;
-  *index_bytes = static_cast<int64_t>(carve(x, nullptr, &ib));
-  const int64_t rows = x.n_pairs * x.G;
-  *fwd_bytes = rows * (kD + 1) * 4 + 64;
-  *bwd_bytes = rows * (x.KU / 64) * kD * 4 + max_parts(x) * (x.KU / 64) * 128 * kD * 4 +
-               static_cast<int64_t>(x.B) * x.TQ * x.HQ * 4 + 64;
+  *index_bytes = z.index; *fwd_bytes = z.fwd; *bwd_bytes = z.bwd;
   return MOC_OK;
 }
 
-extern "C" int moc_sparse_attn_tc_fwd(const moc_sparse_attn_shape* s, const void* q, const void* k, const void* v,
-                                      const int32_t* block_indices, void* index, void* scratch, void* o, float* lse,
+extern "C" int moc_sparse_attn_tc_fwd(const moc_sparse_attn_shape* s, const void* q_, const void* k_, const void* v_,
+                                      const int32_t* block_indices, void* index, void* scratch, void* o_, float* lse,
                                       int32_t* status, void* stream) {
-  FwdParams p;
-  int rc = make_shape(s, &p.x);
+  Slices sl;
+  Sizes z;
+  const int rc = slice(s, &sl, &z);
   if (rc != MOC_OK) return rc;
-  const Shape& x = p.x;
-  MOC_REQUIRE(q && k && v && block_indices && index && scratch && o && lse && status, "NULL buffer");
+  MOC_REQUIRE(q_ && k_ && v_ && block_indices && index && scratch && o_ && lse && status, "NULL buffer");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  CUtensorMap mq, mk, mv;
-  if ((rc = row_map(x, q, &mq)) != MOC_OK || (rc = kv_maps(x, k, v, x.KU, &mk, &mv)) != MOC_OK) return rc;
-  carve(x, static_cast<int*>(index), &p.ib);
-  if ((rc = build_index(block_indices, x, p.ib, status, st)) != MOC_OK) return rc;
-  p.partial = static_cast<float*>(scratch);
-  p.lse_rows = p.partial + x.n_pairs * x.G * kD;
-  p.status = status;
-  rc = x.KU == 128 ? launch_fwd<128>(mq, mk, mv, p, st) : launch_fwd<64>(mq, mk, mv, p, st);
-  if (rc != MOC_OK) return rc;
-  const long long threads = static_cast<long long>(x.B) * x.TQ * x.HQ * 16;
-  merge_kernel<<<static_cast<int>((threads + 255) / 256), 256, 0, st>>>(x, p.ib.pos, p.partial, p.lse_rows,
-                                                                        static_cast<__nv_bfloat16*>(o), lse);
-  MOC_CUDA_OK(cudaGetLastError());
-  return MOC_OK;
+  using bf16 = __nv_bfloat16;
+  return for_slices(s, sl, [&](const Shape& x, int64_t tok, int64_t key, bool, bool) -> int {
+    const bf16 *q = static_cast<const bf16*>(q_) + tok * x.HQ * kD, *k = static_cast<const bf16*>(k_) + key * x.H * kD,
+               *v = static_cast<const bf16*>(v_) + key * x.H * kD;
+    FwdParams p;
+    p.x = x;
+    int rc;
+    CUtensorMap mq, mk, mv;
+    if ((rc = row_map(x, q, &mq)) != MOC_OK || (rc = kv_maps(x, k, v, x.KU, &mk, &mv)) != MOC_OK) return rc;
+    carve(x, static_cast<int*>(index), &p.ib);
+    if ((rc = build_index(block_indices + tok * x.H * x.S, x, p.ib, status, st)) != MOC_OK) return rc;
+    p.partial = static_cast<float*>(scratch);
+    p.lse_rows = p.partial + x.n_pairs * x.G * kD;
+    p.status = status;
+    rc = x.KU == 128 ? launch_fwd<128>(mq, mk, mv, p, st) : launch_fwd<64>(mq, mk, mv, p, st);
+    if (rc != MOC_OK) return rc;
+    const long long threads = static_cast<long long>(x.B) * x.TQ * x.HQ * 16;
+    merge_kernel<<<static_cast<int>((threads + 255) / 256), 256, 0, st>>>(
+        x, p.ib.pos, p.partial, p.lse_rows, static_cast<bf16*>(o_) + tok * x.HQ * kD, lse + tok * x.HQ);
+    MOC_CUDA_OK(cudaGetLastError());
+    return MOC_OK;
+  });
 }
 
-extern "C" int moc_sparse_attn_tc_bwd(const moc_sparse_attn_shape* s, const void* q, const void* k, const void* v,
+extern "C" int moc_sparse_attn_tc_bwd(const moc_sparse_attn_shape* s, const void* q_, const void* k_, const void* v_,
                                       const int32_t* block_indices, void* index, int32_t have_index, void* scratch,
-                                      const void* o, const float* lse, const void* d_o, void* d_q, void* d_k, void* d_v,
+                                      const void* o_, const float* lse, const void* d_o_, void* d_q, void* d_k, void* d_v,
                                       int32_t* status, void* stream) {
-  BwdParams p;
-  int rc = make_shape(s, &p.x);
+  Slices sl;
+  Sizes z;
+  const int rc = slice(s, &sl, &z);
   if (rc != MOC_OK) return rc;
-  const Shape& x = p.x;
-  MOC_REQUIRE(q && k && v && block_indices && index && scratch && o && lse && d_o && d_q && d_k && d_v && status,
+  MOC_REQUIRE(q_ && k_ && v_ && block_indices && index && scratch && o_ && lse && d_o_ && d_q && d_k && d_v && status,
               "NULL buffer");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  CUtensorMap mq, mdo, mk, mv;
-  if ((rc = row_map(x, q, &mq)) != MOC_OK || (rc = row_map(x, d_o, &mdo)) != MOC_OK ||
-      (rc = kv_maps(x, k, v, 64, &mk, &mv)) != MOC_OK) return rc;
-  carve(x, static_cast<int*>(index), &p.ib);
-  if (!have_index && (rc = build_index(block_indices, x, p.ib, status, st)) != MOC_OK) return rc;
-  const int halves = x.KU / 64;
-  p.dq_partial = static_cast<float*>(scratch);
-  p.part = p.dq_partial + x.n_pairs * x.G * halves * kD;
-  float* delta = p.part + max_parts(x) * halves * 128 * kD;
-  p.lse = lse; p.delta = delta; p.d_k = static_cast<__nv_bfloat16*>(d_k); p.d_v = static_cast<__nv_bfloat16*>(d_v);
-  p.status = status;
-  rc = moc_row_dot(o, d_o, MOC_BF16, delta, static_cast<int64_t>(x.B) * x.TQ * x.HQ, kD, stream);
-  if (rc != MOC_OK) return rc;
-  MOC_CUDA_OK(cudaFuncSetAttribute(sparse_bwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem));
-  const long long grid = std::min<long long>(max_items(x) * halves, static_cast<long long>(sm_count()) * 2);
-  sparse_bwd_tc_kernel<<<static_cast<int>(grid), kThreads, kBwdSmem, st>>>(mq, mdo, mk, mv, p);
-  part_sum_kernel<<<static_cast<int>(x.n_buckets), 256, 0, st>>>(x, p.ib, p.part, p.d_k, p.d_v);
-  const long long threads = static_cast<long long>(x.B) * x.TQ * x.HQ * 16;
-  dq_sum_kernel<<<static_cast<int>((threads + 255) / 256), 256, 0, st>>>(x, p.ib.pos, p.dq_partial,
-                                                                         static_cast<__nv_bfloat16*>(d_q));
-  MOC_CUDA_OK(cudaGetLastError());
-  return MOC_OK;
+  using bf16 = __nv_bfloat16;
+  const bool whole = sl.items == s->batch && sl.tokens == s->tq, add = sl.tokens < s->tq;
+  return for_slices(s, sl, [&](const Shape& x, int64_t tok, int64_t key, bool first, bool last) -> int {
+    const int64_t row = tok * x.HQ, kv = key * x.H * kD, n_kv = static_cast<int64_t>(x.B) * x.TK * x.H * kD;
+    const bf16 *q = static_cast<const bf16*>(q_) + row * kD, *k = static_cast<const bf16*>(k_) + kv,
+               *v = static_cast<const bf16*>(v_) + kv, *o = static_cast<const bf16*>(o_) + row * kD,
+               *d_o = static_cast<const bf16*>(d_o_) + row * kD;
+    BwdParams p;
+    p.x = x;
+    int rc;
+    CUtensorMap mq, mdo, mk, mv;
+    if ((rc = row_map(x, q, &mq)) != MOC_OK || (rc = row_map(x, d_o, &mdo)) != MOC_OK ||
+        (rc = kv_maps(x, k, v, 64, &mk, &mv)) != MOC_OK) return rc;
+    carve(x, static_cast<int*>(index), &p.ib);
+    if (!(have_index && whole) && (rc = build_index(block_indices + tok * x.H * x.S, x, p.ib, status, st)) != MOC_OK) return rc;
+    const int halves = x.KU / 64;
+    p.acc_k = p.acc_v = nullptr;
+    p.dq_partial = static_cast<float*>(scratch);
+    if (add) {                                  // a slice is part of one item, whose sums stand before the rest
+      p.acc_k = p.dq_partial; p.acc_v = p.acc_k + n_kv;
+      p.dq_partial = p.acc_v + n_kv;
+      if (first) MOC_CUDA_OK(cudaMemsetAsync(p.acc_k, 0, static_cast<size_t>(2 * n_kv) * 4, st));
+    }
+    p.part = p.dq_partial + x.n_pairs * x.G * halves * kD;
+    float* delta = p.part + max_parts(x) * halves * 128 * kD;
+    p.d_k = static_cast<bf16*>(d_k) + kv; p.d_v = static_cast<bf16*>(d_v) + kv;
+    p.lse = lse + row; p.delta = delta;
+    p.status = status;
+    rc = moc_row_dot(o, d_o, MOC_BF16, delta, static_cast<int64_t>(x.B) * x.TQ * x.HQ, kD, stream);
+    if (rc != MOC_OK) return rc;
+    MOC_CUDA_OK(cudaFuncSetAttribute(sparse_bwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem));
+    const long long grid = std::min<long long>(max_items(x) * halves, static_cast<long long>(sm_count()) * 2);
+    sparse_bwd_tc_kernel<<<static_cast<int>(grid), kThreads, kBwdSmem, st>>>(mq, mdo, mk, mv, p);
+    part_sum_kernel<<<static_cast<int>(x.n_buckets), 256, 0, st>>>(x, p.ib, p.part, p.d_k, p.d_v, p.acc_k, p.acc_v);
+    const long long threads = static_cast<long long>(x.B) * x.TQ * x.HQ * 16;
+    dq_sum_kernel<<<static_cast<int>((threads + 255) / 256), 256, 0, st>>>(x, p.ib.pos, p.dq_partial,
+                                                                           static_cast<bf16*>(d_q) + row * kD);
+    MOC_CUDA_OK(cudaGetLastError());
+    if (add && last) {
+      if ((rc = moc_cast_f32_to_bf16(p.acc_k, p.d_k, n_kv, stream)) != MOC_OK) return rc;
+      return moc_cast_f32_to_bf16(p.acc_v, p.d_v, n_kv, stream);
+    }
+    return MOC_OK;
+  });
 }
