@@ -34,15 +34,16 @@ def _same_dtype(q, k, v):
 
 def _forward(q, k, v, bi, block_size, scale):
     """(o, lse, index or None): the tensor-core kernels where they apply, else a warp per (token, head)."""
-    if _same_dtype(q, k, v) and ops.sparse_attn_tc_supported(q, k, block_size):
+    if _same_dtype(q, k, v) and ops.sparse_attn_tc_supported(q, k, block_size, v):
         return ops.sparse_attn_tc_fwd(q, k, v, bi, block_size, scale)
     return (*ops.sparse_attn_fwd(q, k, v, bi, block_size, scale), None)
 
 
 def _backward(q, k, v, bi, o, lse, do, block_size, scale, index=None):
-    if _same_dtype(q, k, v) and do.dtype == q.dtype and ops.sparse_attn_tc_supported(q, k, block_size):
-        return ops.sparse_attn_tc_bwd(q, k, v, bi, o, lse, do.contiguous(), block_size, scale, index)
-    dq, dk, dv = ops.sparse_attn_bwd(q, k, v, bi, o, lse, do.contiguous(), block_size, scale)
+    do = do.contiguous()
+    if _same_dtype(q, k, v) and do.dtype == q.dtype and ops.sparse_attn_tc_supported(q, k, block_size, v, o, do):
+        return ops.sparse_attn_tc_bwd(q, k, v, bi, o, lse, do, block_size, scale, index)
+    dq, dk, dv = ops.sparse_attn_bwd(q, k, v, bi, o, lse, do, block_size, scale)
     return dq, dk.to(k.dtype), dv.to(v.dtype)
 
 

@@ -844,11 +844,14 @@ def sparse_attn_bwd(q, k, v, block_indices, o, lse, d_o, block_size: int, scale:
     return d_q, d_k, d_v
 
 
-def sparse_attn_tc_supported(q: torch.Tensor, k: torch.Tensor, block_size: int) -> bool:
+def sparse_attn_tc_supported(q: torch.Tensor, k: torch.Tensor, block_size: int, *others: torch.Tensor) -> bool:
     """Whether the tensor-core kernels take this joint-softmax problem: bf16, head_dim 64, chapters of a multiple of 64
-    rows.  They are the faster ones at every size measured (100 tokens up), so nothing else decides."""
+    rows, and tensors (``others``: V, and the result and its gradient in the backward pass) that start on 16 bytes, as
+    their tiled loads need.  They are the faster ones at every size measured, so size does not decide: 1 to 160 tokens, 1
+    to 8 KV heads, 24 to 4,096 chapters take 31 to 295 us forward against 76 to 1,352 a warp per (token, head), and 25 to
+    686 against 162 to 3,036 backward."""
     return (q.dtype == torch.bfloat16 and k.dtype == torch.bfloat16 and q.shape[-1] == 64 and int(block_size) % 64 == 0
-            and q.shape[2] // k.shape[2] <= 128)
+            and q.shape[2] // k.shape[2] <= 128 and all(t.data_ptr() % 16 == 0 for t in (q, k, *others)))
 
 
 def _sparse_tc_sizes(s):

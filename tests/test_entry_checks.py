@@ -296,3 +296,39 @@ def test_the_descriptor_of_a_decoding_step_has_both_widths(decoder):
     dec.step(_decode_states()[0], torch.zeros(2, 16, 64, dtype=torch.bfloat16))
     s = L.DecodeStepDesc.from_buffer_copy(fake.seen[0])
     assert (s.router.hidden_dim, s.hidden_dim) == (64, D)
+
+
+# ---- sparse attention --------------------------------------------------------------------------------------------
+def _off_by(t, n):
+    """The same numbers, contiguous, starting ``n`` elements into a buffer."""
+    buf = torch.empty(t.numel() + n, dtype=t.dtype, device=t.device)
+    return buf[n:].copy_(t.reshape(-1)).view(t.shape)
+
+
+def test_unaligned_tensors_stay_with_the_kernels_that_take_them():
+    from memory_b200 import ops
+    q, k = torch.zeros(1, 5, 2, 64, dtype=torch.bfloat16), torch.zeros(1, 128, 2, 64, dtype=torch.bfloat16)
+    assert ops.sparse_attn_tc_supported(q, k, 64, k, q)
+    for bad in ((_off_by(q, 1), k, k), (q, _off_by(k, 4), k), (q, k, _off_by(k, 7))):
+        assert not ops.sparse_attn_tc_supported(bad[0], bad[1], 64, bad[2])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("which", ["q", "k", "v", "do"])
+def test_unaligned_tensors_give_the_same_attention(which):
+    import memory_b200 as M
+    from memory_b200 import _lib as L
+    g = torch.Generator().manual_seed(4)
+    x = {n: torch.randn(1, r, h, 64, generator=g).bfloat16().cuda() for n, r, h in
+         (("q", 33, 4), ("k", 5 * 64, 2), ("v", 5 * 64, 2), ("do", 33, 4))}
+    bi = torch.rand(33 * 2, 5, generator=g).topk(2, dim=1).indices.view(1, 33, 2, 2).int().cuda()
+
+    def run(x):
+        leaves = [x[n].detach().requires_grad_(True) for n in ("q", "k", "v")]
+        o = M.memory_cross_attn(*leaves, bi, 64)
+        o.backward(x["do"])
+        return [o.detach()] + [t.grad for t in leaves]
+    want, got = run(x), run(dict(x, **{which: _off_by(x[which], 3)}))
+    L.check_device_status(torch.device("cuda:0"))
+    for a, b in zip(got, want):          # bf16 results of two kernels: probabilities rounded to bf16 in one, not in the other
+        assert float((a.float() - b.float()).norm() / b.float().norm()) < 1e-2
