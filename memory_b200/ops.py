@@ -1373,6 +1373,8 @@ def token_attn_fwd(h, shared, routed, idx, weights, wq, wk, wv, wo, num_heads: i
     L.require_cuda(h, shared, routed, idx, weights, wq, wk, wv, wo)
     k, dev, code, p = idx.shape[-1], h.device, L.dtype_code, L.ptr
     h, routed = _contig(h), _contig(routed)
+    if routed.data_ptr() % 16:           # the listed chapters' rows are read in 16-byte pieces
+        routed = routed.clone()
     shared = _contig(shared) if shared is not None and shared.numel() > 0 else None
     ids = _contig(idx.to(torch.int32))
     w = _contig(weights.float())

@@ -190,6 +190,24 @@ def test_token_attention_refuses_projections_of_another_size():
             ops.token_attn_fwd(h.view(8, D), None, routed, idx, w, *ws, HEADS, 1, 1.0, False)
 
 
+def test_listed_chapters_are_read_from_16_byte_rows(monkeypatch):
+    """A bank slice that starts anywhere is copied: its rows are converted with 16-byte loads."""
+    from types import SimpleNamespace
+    from memory_b200 import _lib as L, ops
+    seen = []
+    fake = SimpleNamespace(moc_token_attn_arena_bytes=lambda s: 16, moc_token_attn_fwd_scratch_bytes=lambda s: 16,
+                           moc_token_attn_fwd=lambda s, scratch: seen.append(s._obj.routed) or 0)
+    for name, fn in (("lib", lambda: fake), ("stream_ptr", lambda dev: 1), ("require_cuda", lambda *t: None),
+                     ("status_word", lambda dev: torch.zeros(1, dtype=torch.int32))):
+        monkeypatch.setattr(L, name, fn)
+    h, idx, w = torch.zeros(8, D, dtype=torch.bfloat16), torch.zeros(1, 8, 2, dtype=torch.int32), torch.zeros(1, 8, 2)
+    ws = [torch.zeros(n, D) for n in (D, 64, 64, D)]
+    for bank in (_off_by(torch.zeros(4 * 64, D), 1), _off_by(torch.zeros(4 * 64, D).bfloat16(), 3), torch.zeros(4 * 64, D)):
+        _, _, keep = ops.token_attn_fwd(h, None, bank, idx, w, *ws, HEADS, 1, 1.0, False)
+        assert seen[-1] == keep[2].data_ptr() and seen[-1] % 16 == 0 and torch.equal(keep[2], bank)
+    assert seen[-1] == bank.data_ptr()          # (an aligned one is read where it is)
+
+
 # ---- decoding ----------------------------------------------------------------------------------------------------
 class _FakeLibrary:
     """Stands in for the native library: keeps the descriptors it is called with."""
