@@ -58,11 +58,14 @@ __device__ __forceinline__ float ex2(float x) {
 
 // 2^x for two values on the FMA pipe: x = n + f with |f| <= 1/2 (Cody-Waite with the round-to-nearest addition of
 // 1.5 * 2^23), a degree-5 polynomial fitted to 2^f for least relative error (2.3e-7 in fp32, that of the hardware
-// instruction), n added to the exponent.  Arguments below -126 count as -126.
+// instruction), times 2^n.  As the instruction does, it gives 0 for -inf (a masked column) and NaN for NaN; arguments count
+// as no less than -127, for which 2^n is 0.
 __device__ __forceinline__ void ex2_poly2(uint64_t x, float& y0, float& y1) {
   float x0, x1;
   f2_unpack(x, x0, x1);
-  x = f2_pack(fmaxf(x0, -126.f), fmaxf(x1, -126.f));
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x0) : "f"(-127.f));
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x1) : "f"(-127.f));
+  x = f2_pack(x0, x1);
   const uint64_t magic = f2_pack(12582912.f, 12582912.f), nmagic = f2_pack(-12582912.f, -12582912.f);
   const uint64_t t = f2_add(x, magic);
   const uint64_t n = f2_add(t, nmagic);
@@ -73,11 +76,16 @@ __device__ __forceinline__ void ex2_poly2(uint64_t x, float& y0, float& y1) {
   p = f2_fma(p, f, f2_pack(0.24022120237350464f, 0.24022120237350464f));
   p = f2_fma(p, f, f2_pack(0.6931469440460205f, 0.6931469440460205f));
   p = f2_fma(p, f, f2_pack(1.0000001192092896f, 1.0000001192092896f));
-  float p0, p1, t0, t1;
-  f2_unpack(p, p0, p1);
+  float t0, t1;
   f2_unpack(t, t0, t1);
-  y0 = __int_as_float(__float_as_int(p0) + (__float_as_int(t0) << 23));
-  y1 = __int_as_float(__float_as_int(p1) + (__float_as_int(t1) << 23));
+  const float s0 = __int_as_float((__float_as_int(t0) << 23) + 0x3F800000), s1 = __int_as_float((__float_as_int(t1) << 23) + 0x3F800000);
+  f2_unpack(f2_mul(p, f2_pack(s0, s1)), y0, y1);
+}
+
+__global__ void exp2_probe_kernel(const float* __restrict__ x, float* __restrict__ y, int pairs) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= pairs) return;
+  ex2_poly2(f2_pack(x[2 * i], x[2 * i + 1]), y[2 * i], y[2 * i + 1]);
 }
 
 // MMA groups issued as one instruction block by one elected lane (~3 instructions per MMA): the MMA warp
@@ -428,3 +436,11 @@ int launch_attn_tc_fwd(const moc_attn_shape* s, const void* q, const void* kv, v
 }
 
 }  // namespace moc
+
+extern "C" int moc_exp2_probe(const float* x, float* y, int32_t n, void* stream) {
+  using namespace moc;
+  MOC_REQUIRE(x && y && n > 0 && n % 2 == 0, "bad exponential probe");
+  exp2_probe_kernel<<<ceil_div(n / 2, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(x, y, n / 2);
+  MOC_CUDA_OK(cudaGetLastError());
+  return MOC_OK;
+}

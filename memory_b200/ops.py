@@ -250,6 +250,14 @@ def wait_probe(device, expected: int, arrivals: int, poll_limit: int):
     return tuple(int(v) for v in out.tolist())
 
 
+def exp2_probe(x: torch.Tensor) -> torch.Tensor:
+    """2^x of an even number of fp32 values by the attention's polynomial."""
+    L.require_cuda(x)
+    y = torch.empty_like(x)
+    L.check(L.lib().moc_exp2_probe(L.ptr(x), L.ptr(y), x.numel(), L.stream_ptr(x.device)), "moc_exp2_probe")
+    return y
+
+
 def agree_probe(device, late_warps: int, poll_limit: int):
     """Runs the self-test of the agreement barrier; returns (each warp's own wait, what each warp hears)."""
     out = torch.zeros(8, dtype=torch.int32, device=device)

@@ -1,0 +1,55 @@
+"""The kernels' own arithmetic over its whole range, against what it stands in for."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def test_polynomial_exponential():
+    from memory_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(1)
+    x = torch.cat([torch.empty(1 << 22, device=DEV).uniform_(-126, 12, generator=g),
+                   torch.empty(1 << 20, device=DEV).uniform_(-1, 1, generator=g),
+                   torch.arange(-126, 13, device=DEV).float(), torch.arange(-251, 25, device=DEV).float() / 2,
+                   torch.zeros(1, device=DEV)])
+    y, want = ops.exp2_probe(x).double(), x.double().exp2()
+    # 2.1e-7 is the polynomial's own error; six fp32 roundings, the last two at full weight, add up to 1e-7
+    assert float(((y - want) / want)[x >= -125.5].abs().max()) < 3.2e-7
+    assert float((y - want)[x < -125.5].abs().max()) < 2.0 ** -126        # (the exponential unit flushes these to zero)
+    small = torch.cat([torch.empty(1 << 16, device=DEV).uniform_(-300, -126, generator=g),
+                       torch.tensor([-126.5, -127.0, -127.5, -1e4, -3e38, -math.inf], device=DEV)])
+    y = ops.exp2_probe(small)
+    assert float(y.min()) >= 0.0 and float(y.max()) <= 2.0 ** -126 and not y[small <= -127].any()
+    nan = ops.exp2_probe(torch.tensor([math.nan, 0.0, 1.0, math.nan], device=DEV))
+    assert nan.isnan().tolist() == [True, False, False, True] and float(nan[2]) == pytest.approx(2.0, rel=3e-7)
+
+
+def test_a_nan_score_makes_its_row_nan_in_every_column():
+    from memory_b200 import _lib as L, ops
+    g = torch.Generator(device=DEV).manual_seed(2)
+    n_sel, heads = 128, 2
+    q = torch.randn(n_sel, 5, heads * 64, generator=g, device=DEV).bfloat16()
+    kv = torch.randn(n_sel, n_sel, 2 * heads * 64, generator=g, device=DEV).bfloat16()
+    for i in range(n_sel):
+        kv[i, i, 3] = math.nan                         # one key of head 0, another one in every item
+    o, lse = ops.attn_fwd(q, kv, heads, heads, 0.125)
+    L.check_device_status(o.device)
+    assert o[..., :64].isnan().all() and lse[:, 0].isnan().all()
+    assert o[..., 64:].isfinite().all() and lse[:, 1].isfinite().all()
+
+
+@pytest.mark.parametrize("n_sel", [70, 97, 200])
+def test_columns_past_the_end_add_nothing(n_sel):
+    """What lies behind an item's last key is the next item's, whatever its size."""
+    from memory_b200 import _lib as L, ops
+    g = torch.Generator(device=DEV).manual_seed(3)
+    q = torch.randn(2, 40, 64, generator=g, device=DEV).bfloat16()
+    kv = torch.randn(2, n_sel, 128, generator=g, device=DEV).bfloat16()
+    want, want_lse = ops.attn_fwd(q[:1].contiguous(), kv[:1].contiguous(), 1, 1, 0.125)
+    kv[1, :, 64:] = 1e38
+    o, lse = ops.attn_fwd(q, kv, 1, 1, 0.125)
+    L.check_device_status(o.device)
+    assert torch.equal(o[:1], want) and torch.equal(lse[:1], want_lse)
