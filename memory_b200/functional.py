@@ -44,13 +44,15 @@ def _check_numel(name: str, t: Optional[torch.Tensor], n: int) -> None:
 
 
 def _check_projections(d: int, mem_dim: int, wq, wk, wv, wo, num_heads: int, num_kv_heads: int) -> None:
-    for name, w, width in (("wq", wq, d), ("wk", wk, mem_dim), ("wv", wv, mem_dim), ("wo", wo, wq.shape[0])):
-        _check_width(name, w, width)
-    if num_heads <= 0 or num_kv_heads <= 0 or wq.shape[0] % num_heads != 0:
-        raise ValueError(f"wq {tuple(wq.shape)} does not hold {num_heads} heads")
-    dkv = num_kv_heads * (wq.shape[0] // num_heads)
-    if wk.shape[0] != dkv or wv.shape[0] != dkv:
-        raise ValueError(f"wk {tuple(wk.shape)} and wv {tuple(wv.shape)} must have num_kv_heads * head_dim = {dkv} rows")
+    q, k, v, o = wq.shape, wk.shape, wv.shape, wo.shape
+    for name, shape, width in (("wq", q, d), ("wk", k, mem_dim), ("wv", v, mem_dim), ("wo", o, q[0])):
+        if len(shape) != 2 or shape[1] != width:
+            raise ValueError(f"inner dimensions differ: {name} {tuple(shape)} vs {width}")
+    if num_heads <= 0 or num_kv_heads <= 0 or q[0] % num_heads != 0:
+        raise ValueError(f"wq {tuple(q)} does not hold {num_heads} heads")
+    dkv = num_kv_heads * (q[0] // num_heads)
+    if k[0] != dkv or v[0] != dkv:
+        raise ValueError(f"wk {tuple(k)} and wv {tuple(v)} must have num_kv_heads * head_dim = {dkv} rows")
 
 
 class _LossDict(dict):

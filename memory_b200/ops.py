@@ -1260,7 +1260,8 @@ def decode_step(hidden: torch.Tensor, routing_states: torch.Tensor, router_w: to
     that agree in shapes, types and weights (by address) are filled once."""
     w = _contig(router_w.float())
     bias = None if router_b is None else _contig(router_b.float())
-    h, states, wq, wo, kv_bank = (_contig(t) for t in (hidden, routing_states, wq, wo, kv_bank))
+    h, states = _contig(hidden), _contig(routing_states)
+    wq, wo, kv_bank = _contig(wq), _contig(wo), _contig(kv_bank)
     dev, p = h.device, L.ptr
     stream = L.stream_ptr(dev)
     # everything the descriptor holds or a check looked at; the per-step buffers are filled in below
