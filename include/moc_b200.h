@@ -56,6 +56,8 @@ int moc_wait_probe(int32_t expected, int32_t arrivals, uint32_t poll_limit, int3
 int moc_agree_probe(uint32_t late_warps, uint32_t poll_limit, int32_t* status, int32_t* out, void* stream);
 /* y[i] = 2^x[i] by the polynomial that takes a share of the attention's exponentials (n even). */
 int moc_exp2_probe(const float* x, float* y, int32_t n, void* stream);
+/* y[i] = x[i] / d[i] as the router's softmax forms it (x >= 0, d > 0). */
+int moc_quotient_probe(const float* x, const float* d, float* y, int32_t n, void* stream);
 
 /* Barrier between the ranks of one node through flag words in each other's memory (peer-mapped device pointers,
  * e.g. views of one symmetric-memory allocation): flag_arrays[r] points at rank r's array of `world` uint32 words,

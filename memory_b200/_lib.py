@@ -136,6 +136,7 @@ _PROTOTYPES = {
     "moc_pool_weighted_bwd": (C.c_int, [P, P, P, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32, P]),
     "moc_wait_probe": (C.c_int, [C.c_int32, C.c_int32, C.c_uint32, P, P, P]),
     "moc_exp2_probe": (C.c_int, [P, P, C.c_int32, P]),
+    "moc_quotient_probe": (C.c_int, [P, P, P, C.c_int32, P]),
     "moc_agree_probe": (C.c_int, [C.c_uint32, C.c_uint32, P, P, P]),
     "moc_gather_rows_fwd": (C.c_int, [P, C.c_int32, C.c_int64, C.c_int32, C.c_int32, P, P, C.c_int32,
                                       C.c_int32, C.c_int32, C.c_float, P, C.c_int32, P, P, P]),

@@ -21,10 +21,16 @@ template <typename T> __device__ __forceinline__ float to_f32(T v);
 template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 
-// x / d for many x and one d, r = 1 / d: the quotient of the rounded reciprocal, corrected by its remainder (Markstein)
+// x / d for many x and one d, r = 1 / d: the quotient of the rounded reciprocal, corrected by its remainder (Markstein).
+// Equal to the division for x = 0 and x >= 2^-100.  The remainder is a multiple of about 2^-47 x: from 2^-102 down fp32
+// cannot hold it, and the last bit is off in one of a hundred quotients.
 __device__ __forceinline__ float quotient(float x, float d, float r) {
   const float q = x * r;
   return fmaf(fmaf(-q, d, x), r, q);
+}
+__global__ void quotient_probe_kernel(const float* __restrict__ x, const float* __restrict__ d, float* __restrict__ y, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) y[i] = quotient(x[i], d[i], 1.f / d[i]);
 }
 
 // ---- block reductions (fixed order) ----------------------------------------------------------
@@ -311,9 +317,10 @@ __global__ void logits_kernel(const float* __restrict__ pooled, const float* __r
 // (rows of up to TH NV chapters), 0 for longer rows.  Bound by its chain of block-wide steps: at 4,097 chapters, k 64, 16 ->
 // 10 us for a few rows with TH 1,024 against four radix passes over shared memory.  Thousands of rows take CTAs of 256
 // threads, whose barriers are shorter and chains more: 8,192 rows, k 16: 252 us with TH 1,024 -> 152.
+// (The resident CTAs are what the registers allow without the divisions of wide rows, which would take more.)
 constexpr int kBins = 512, kBinBits = 9, kCand = 512;
 template <int NV, int TH>
-__global__ void __launch_bounds__(TH)
+__global__ void __launch_bounds__(TH, TH == 256 ? (NV > 5 ? 3 : 6) : (NV > 5 ? 1 : 2))
 select_kernel(const float* __restrict__ logits, long long ld, const float* __restrict__ bias, float* __restrict__ probs, long long* __restrict__ idx,
               float* __restrict__ weights, int* __restrict__ comb_idx, float* __restrict__ comb_w,
               float* __restrict__ row_stats, int C, int k_sel, int S, float rho) {
@@ -337,7 +344,7 @@ select_kernel(const float* __restrict__ logits, long long ld, const float* __res
   // is only made for the radix select.  Sums run in the same order either way.
   constexpr int kN = NV > 0 ? NV : 1;
   float v[kN];
-  float m = -INFINITY;
+  float m = -INFINITY, lo = INFINITY;
   if constexpr (NV > 0) {
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -349,11 +356,27 @@ select_kernel(const float* __restrict__ logits, long long ld, const float* __res
       for (int i = 0; i < NV; ++i) v[i] += bias[min(static_cast<int>(threadIdx.x) + i * TH, C - 1)];
     }
 #pragma unroll
-    for (int i = 0; i < NV; ++i) m = fmaxf(m, v[i]);       // (a repeated last entry changes no maximum)
+    for (int i = 0; i < NV; ++i) { m = fmaxf(m, v[i]); lo = fminf(lo, v[i]); }       // (a repeated last entry changes neither)
   } else {
     for (int c = threadIdx.x; c < C; c += blockDim.x) m = fmaxf(m, logit(c));
   }
   m = block_max(m, red[0]);
+  // A thread whose smallest exponential may lie below 2^-83 divides.  Both quotients below stay within what `quotient` is
+  // exact for otherwise: the exponentials, and those over a sum of at most 2^14.  (8,192 rows of 4,097 chapters: 157 us
+  // without the test, 161 with it, 184 with a test of every value on its own.)
+  const bool wide = lo - m < -57.5f;
+  auto divide = [&](float d) {             // v[i] = v[i] / d
+    if constexpr (NV > 0) {
+      if (wide) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) v[i] = v[i] / d;
+      } else {
+        const float r = 1.f / d;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) v[i] = quotient(v[i], d, r);
+      }
+    }
+  };
   float s = 0.f;
   if constexpr (NV > 0) {
 #pragma unroll
@@ -367,16 +390,15 @@ select_kernel(const float* __restrict__ logits, long long ld, const float* __res
     }
   }
   const float denom = block_sum(s, red[1]);
-  const float r_denom = 1.f / denom;
   float ms = 0.f;
   if constexpr (NV > 0) {
+    divide(denom);
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int c = threadIdx.x + i * TH;
       if (c < C) {
-        const float pv = quotient(v[i], denom, r_denom);
-        p[c] = pv;
-        v[i] = (c < S) ? 0.f : pv;
+        p[c] = v[i];
+        if (c < S) v[i] = 0.f;
         ms += v[i];
       }
     }
@@ -392,11 +414,7 @@ select_kernel(const float* __restrict__ logits, long long ld, const float* __res
   const float masked_mass = block_sum(ms, red[2]);
   const float dn0 = fmaxf(masked_mass, 1e-12f);
   if constexpr (NV > 0) {
-    if (S > 0) {
-      const float r_dn0 = 1.f / dn0;
-#pragma unroll
-      for (int i = 0; i < NV; ++i) v[i] = quotient(v[i], dn0, r_dn0);
-    }
+    if (S > 0) divide(dn0);
   } else {
     if (S > 0)
       for (int c = threadIdx.x; c < C; c += blockDim.x) pt[c] = pt[c] / dn0;
@@ -1493,6 +1511,13 @@ extern "C" int moc_loss_total(const float* losses, const float* grad, float c0, 
 extern "C" int moc_col_sum(const float* x, float* out, int64_t rows, int32_t cols, void* stream_) {
   MOC_REQUIRE(x && out && rows > 0 && cols > 0, "bad column-sum arguments");
   col_sum_kernel<<<ceil_div(cols, 32), 256, 0, static_cast<cudaStream_t>(stream_)>>>(x, out, rows, cols, cols);
+  MOC_CUDA_OK(cudaGetLastError());
+  return MOC_OK;
+}
+
+extern "C" int moc_quotient_probe(const float* x, const float* d, float* y, int32_t n, void* stream) {
+  MOC_REQUIRE(x && d && y && n > 0, "bad quotient probe");
+  quotient_probe_kernel<<<ceil_div(n, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(x, d, y, n);
   MOC_CUDA_OK(cudaGetLastError());
   return MOC_OK;
 }

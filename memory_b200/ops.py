@@ -258,6 +258,14 @@ def exp2_probe(x: torch.Tensor) -> torch.Tensor:
     return y
 
 
+def quotient_probe(x: torch.Tensor, d: torch.Tensor) -> torch.Tensor:
+    """x / d of fp32 values as the router's softmax forms it."""
+    L.require_cuda(x, d)
+    y = torch.empty_like(x)
+    L.check(L.lib().moc_quotient_probe(L.ptr(x), L.ptr(d), L.ptr(y), x.numel(), L.stream_ptr(x.device)), "moc_quotient_probe")
+    return y
+
+
 def agree_probe(device, late_warps: int, poll_limit: int):
     """Runs the self-test of the agreement barrier; returns (each warp's own wait, what each warp hears)."""
     out = torch.zeros(8, dtype=torch.int32, device=device)

@@ -53,3 +53,40 @@ def test_columns_past_the_end_add_nothing(n_sel):
     o, lse = ops.attn_fwd(q, kv, 1, 1, 0.125)
     L.check_device_status(o.device)
     assert torch.equal(o[:1], want) and torch.equal(lse[:1], want_lse)
+
+
+def test_router_quotient_is_the_division():
+    """Exponentials from 1 down to 2^-100, over sums from the floor of a masked row to a few thousand."""
+    from memory_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(4)
+    n = 1 << 24
+    x = torch.empty(n, device=DEV).uniform_(1, 2, generator=g) * torch.empty(n, device=DEV).uniform_(-100, 0, generator=g).exp2()
+    x[: n // 8] = torch.empty(n // 8, device=DEV).uniform_(2.0 ** -20, 1, generator=g)
+    d = torch.empty(n, device=DEV).uniform_(-40, 14, generator=g).exp2()
+    # (divisors that are all ones but for the last bits are the hard ones for a corrected reciprocal)
+    d[::3] = (d[::3].view(torch.int32) | 0x7FFFF8).view(torch.float32)
+    x[:3], d[:3] = torch.tensor([0.0, 1.0, 2.0 ** -100], device=DEV), torch.tensor([3.0, 3.0, 7.0], device=DEV)
+    want = (x.double() / d.double()).float()         # (all normal numbers: twice rounded is once rounded)
+    got = ops.quotient_probe(x, d)
+    assert torch.equal(got, want), float((got != want).float().mean())
+    assert ops.quotient_probe(torch.tensor([math.nan], device=DEV), torch.ones(1, device=DEV)).isnan().all()
+
+
+@pytest.mark.parametrize("rows", [2, 4096])
+@pytest.mark.parametrize("chapters", [200, 1025, 2000, 4097, 5000, 9000])
+def test_router_probabilities_of_rows_with_a_wide_range_are_divided(rows, chapters):
+    """Two rows with the same tiny rest under one large value and under two.  The first row's sum is 1, so its
+    probabilities are the exponentials themselves; the second's must be those divided by its sum, to the last bit."""
+    from memory_b200 import _lib as L, ops
+    g = torch.Generator(device=DEV).manual_seed(chapters)
+    logits = torch.empty(chapters, device=DEV).uniform_(-104, -30, generator=g).repeat(rows, 1)
+    logits[:, 0], logits[0::2, 1], logits[1::2, 1] = 0.0, -104.0, -0.3
+    total = 1.0 + torch.full((1,), -0.3, device=DEV).exp()
+    h = torch.zeros(rows, 1, 8, device=DEV)
+    r = ops.router_fwd(h, torch.zeros(chapters, 8, device=DEV), None, 4, 1, 1.0, False, pooled=h.view(rows, 8), logits=logits)
+    L.check_device_status(h.device)
+    e, p = r["probs"][0].cpu().numpy(), r["probs"].cpu().numpy()
+    assert e[2:].min() < 1e-44 and e[0] == 1.0
+    for row in (1, rows - 1):
+        assert p[row, 0] == 1.0 / total.cpu().numpy()[0]
+        assert (p[row, 2:] == e[2:] / total.cpu().numpy()[0]).all()
