@@ -249,13 +249,17 @@ extern "C" int moc_decode_attn(const moc_decode_shape* s, const void* q, const v
   // query heads that share a KV head go together: their rows are fetched once
   const int per_kv = s->num_heads / s->num_kv_heads;
   const int group = per_kv % 4 == 0 ? 4 : per_kv % 3 == 0 ? 3 : per_kv % 2 == 0 ? 2 : 1;
-  // a cluster per group while the chip (two CTAs an SM) has room and every warp has rows to take
-  const long long ctas = static_cast<long long>(s->num_heads / group) * s->n_q * s->batch;
-  const int units = s->n_chapters * ceil_div(s->tokens_per_chapter, kDecRows);
-  int split = 1;
-  while (split < 8 && ctas * split * 2 <= 296 && split * kDecWarps < units) split *= 2;
   auto kern = group == 4 ? decode_attn_kernel<4> : group == 3 ? decode_attn_kernel<3>
               : group == 2 ? decode_attn_kernel<2> : decode_attn_kernel<1>;
+  // A cluster per group while all of them are resident at once and every warp has rows to take.  How many are depends on
+  // the registers (an SM holds two CTAs of one head, one of a group) and on what is left of each GPC beside whole clusters:
+  // 33 clusters of eight single-head CTAs, 15 of grouped ones.  With 296 slots counted for either, 12 heads on 4 KV heads
+  // and 65 chapters took 14.8 us for 4 sequences, 22.0 for 8, 19.9 for 12, now 10.3, 10.8, 16.1; 12 heads of their own
+  // 13.6 us for 3 sequences and 18.0 for 6, now 10.8 and 14.2.
+  const long long groups = static_cast<long long>(s->num_heads / group) * s->n_q * s->batch;
+  const int units = s->n_chapters * ceil_div(s->tokens_per_chapter, kDecRows);
+  int split = 1;
+  while (split < 8 && split * kDecWarps < units && groups <= resident_clusters(kern, kDecThreads, 0, split * 2)) split *= 2;
   dim3 grid(s->num_heads / group * split, s->n_q, s->batch);
   MOC_CUDA_OK(launch_clustered(kern, grid, kDecThreads, 0, split, static_cast<cudaStream_t>(stream_),
                                static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(kv_bank),

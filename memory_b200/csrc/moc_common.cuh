@@ -429,6 +429,23 @@ inline int attn_key_split(int ctas, int key_tiles) {
   }
   return best;
 }
+// How many clusters of `cluster` CTAs of a kernel the device holds at once (0.2 us to ask).
+template <typename... Params>
+inline int resident_clusters(void (*kernel)(Params...), int threads, int smem, int cluster) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cluster);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = cluster; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess) return n;
+  cudaGetLastError();
+  return 0;
+}
 // Launch on clusters of `cluster` CTAs along x (1: a plain launch).
 template <typename... Params, typename... Args>
 inline cudaError_t launch_clustered(void (*kernel)(Params...), dim3 grid, int threads, int smem, int cluster,
