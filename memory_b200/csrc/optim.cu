@@ -44,6 +44,7 @@ bank_adamw_kernel(float4* __restrict__ param, float4* __restrict__ exp_avg, floa
   const float decay = 1.f - h.lr * h.weight_decay, w1 = 1.f - h.beta1, w2 = 1.f - h.beta2;
   for (I first = static_cast<I>(blockIdx.x) * 256 + threadIdx.x; first < total4; first += kAdamAhead * stride) {
     float4 p[kAdamAhead], m[kAdamAhead], v[kAdamAhead], g[kAdamAhead];
+    float gs[kAdamAhead];         // (no gradient is none at any scale, infinite and NaN ones included)
 #pragma unroll
     for (int u = 0; u < kAdamAhead; ++u) {
       const I i = first + u * stride;
@@ -52,6 +53,7 @@ bank_adamw_kernel(float4* __restrict__ param, float4* __restrict__ exp_avg, floa
       const I row = i / dim4, chapter = row / T;
       const int slot = slot_of[chapter];
       g[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      gs[u] = slot >= 0 ? h.grad_scale : 1.f;
       if (slot >= 0)
         g[u] = __ldcs(grad_rows + (static_cast<long long>(slot) * T + (row - chapter * T)) * dim4 + (i - row * dim4));
     }
@@ -60,7 +62,7 @@ bank_adamw_kernel(float4* __restrict__ param, float4* __restrict__ exp_avg, floa
       const I i = first + u * stride;
       if (u > 0 && i >= total4) break;
 #define MOC_ADAMW_ONE(X)                                                     \
-      g[u].X *= h.grad_scale;                                                \
+      g[u].X *= gs[u];                                                       \
       p[u].X *= decay;                                                       \
       m[u].X = m[u].X + w1 * (g[u].X - m[u].X);           /* lerp */         \
       v[u].X = v[u].X * h.beta2 + w2 * g[u].X * g[u].X;                      \
