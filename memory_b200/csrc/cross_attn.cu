@@ -204,6 +204,7 @@ extern "C" int moc_xattn_bwd(const moc_xattn_desc* s, const moc_xattn_bwd_desc* 
   const void* g2;
   MOC_TRY(as_dtype(b->g, b->g_dtype, t.g2, cd, x.rows * od, main, &g2));
   MOC_TRY(order(main, side));
+  Join join(side, main);
   MOC_TRY(weight_grad(cd, od, hd, x.rows, g2, a.o, b->d_wo, status, side));
   MOC_TRY(grad_in(x.rows, hd, od, g2, wo, a.wo_t, t.d_o, cd, nullptr, main));
   const moc_attn_shape as = attn_shape(s);
@@ -253,5 +254,5 @@ extern "C" int moc_xattn_bwd(const moc_xattn_desc* s, const moc_xattn_bwd_desc* 
   MOC_TRY(weight_grad(cd, 2 * x.dkv, md, x.mem_rows, d_kv, m2, b->d_wkv, status, side));
   if (b->d_memory)
     MOC_TRY(grad_in(x.mem_rows, md, 2 * x.dkv, d_kv, a.wkv, a.wkv_t, b->d_memory, b->d_mem_dtype, nullptr, main));
-  return order(side, main);
+  return join.done();
 }

@@ -312,12 +312,13 @@ extern "C" int moc_decode_step(const moc_decode_step_desc* s) {
   cudaStream_t main = static_cast<cudaStream_t>(s->stream);
   cudaStream_t side = rows > 8 && s->side_stream ? static_cast<cudaStream_t>(s->side_stream) : main;
   if (side != main) MOC_TRY(order(main, side));
+  Join join(side, main);
   const void* x;
   MOC_TRY(as_dtype(s->hidden, s->hidden_dtype, a.x, MOC_BF16, rows * d, side, &x));
   Gemm gq(MOC_BF16, rows, width, d, true, true, MOC_BF16);
   MOC_TRY(moc_gemm(&gq, x, s->wq, a.q, nullptr, nullptr, s->status, side));
   MOC_TRY(moc_route_fwd(r));
-  if (side != main) MOC_TRY(order(side, main));
+  MOC_TRY(join.done());
   MOC_TRY(moc_decode_attn(&s->attn, a.q, s->kv_bank, s->bank_rows, s->comb_idx, s->comb_w, a.o, nullptr, s->status, s->stream));
   Gemm go(MOC_BF16, rows, s->out_dim, width, true, true, s->hidden_dtype);
   return moc_gemm(&go, a.o, s->wo, s->out, nullptr, nullptr, s->status, s->stream);

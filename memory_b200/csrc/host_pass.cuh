@@ -32,6 +32,21 @@ int fork_event(cudaStream_t from, cudaEvent_t* out);
 // `after` continues behind what `before` holds now.
 int order(cudaStream_t before, cudaStream_t after);
 
+// A pass that forked `side` off `main` joins it again on every way out.  On an error too: the caller then gives the pass's
+// buffers back, and their next use is ordered behind `main` alone.
+struct Join {
+  cudaStream_t side, main;
+  bool open;
+  Join(cudaStream_t side_, cudaStream_t main_) : side(side_), main(main_), open(side_ != main_) {}
+  Join(const Join&) = delete;
+  ~Join() { done(); }
+  int done() {
+    const bool was = open;
+    open = false;
+    return was ? order(side, main) : MOC_OK;
+  }
+};
+
 // What the bf16 projection kernel can do beside moc_gemm_desc:
 // terms > 1: C = sum over t of op(A_t) op(B_t), all in one accumulator, the last term first; A_t / B_t start
 //   t * a_term_rows / b_term_rows stored rows behind A / B (0: the same operand in every term).

@@ -160,6 +160,7 @@ extern "C" int moc_layer_fwd(const moc_layer_desc* s) {
 
   // side stream: routing; then what nothing before the join reads (loss terms, touched-chapter lists)
   MOC_TRY(order(main, side));
+  Join join(side, main);
   auto router = [&](int parts) {
     return moc_router_fwd_parts(&rs, s->h_router, s->router_w, s->router_b, a.pooled, a.logits, a.probs, s->idx, s->weights,
                                 s->comb_idx, s->comb_w, a.row_stats, a.chapter_stats, s->losses, a.router_ws, ws_bytes,
@@ -217,7 +218,7 @@ extern "C" int moc_layer_fwd(const moc_layer_desc* s) {
   Gemm go(MOC_BF16, x.rows, d, d, true, true, s->attn_dtype);
   if (s->add_residual) { go.residual = x2; go.ldr = d; }
   MOC_TRY(moc_gemm(&go, a.o, a.wo, s->out, nullptr, nullptr, s->status, main));
-  return order(side, main);
+  return join.done();
 }
 
 namespace moc {
@@ -285,6 +286,7 @@ extern "C" int moc_layer_bwd(const moc_layer_desc* s, const moc_layer_bwd_desc* 
     g2 = t.g2;
   }
   MOC_TRY(order(main, side));
+  Join join(side, main);
   MOC_TRY(weight_grad(MOC_BF16, d, d, x.rows, g2, a.o, b->d_wo, st, side));
   {
     const Gemm g(MOC_BF16, x.rows, d, d, true, true, MOC_BF16);
@@ -403,5 +405,5 @@ extern "C" int moc_layer_bwd(const moc_layer_desc* s, const moc_layer_bwd_desc* 
     if (!b->d_h_router) MOC_CUDA_OK(cudaStreamWaitEvent(main, dh_done, 0));
     MOC_TRY(router(4, main));
   }
-  return order(side, main);
+  return join.done();
 }
