@@ -105,6 +105,10 @@ struct EventRing {
   cudaEvent_t ev[kMax];
   bool made = false;
   int next = 0;
+  ~EventRing() {                 // a thread that ends gives its events back
+    if (made)
+      for (cudaEvent_t e : ev) cudaEventDestroy(e);
+  }
 };
 int fork_event(cudaStream_t from, cudaEvent_t* out) {
   thread_local EventRing ring[16];

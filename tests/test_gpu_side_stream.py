@@ -47,6 +47,8 @@ def _decode():
 def test_a_refused_pass_leaves_the_second_stream_joined(prepare):
     from memory_b200 import _lib as L, functional as F
     dev = torch.device("cuda:0")
+    with pytest.raises((ValueError, RuntimeError)):
+        prepare()()                                               # (kernels are loaded on their first launch, which waits)
     run = prepare()
     torch.cuda.synchronize()
     side = torch.cuda.ExternalStream(F._side_stream(0, L.stream_ptr(dev)))
@@ -60,3 +62,22 @@ def test_a_refused_pass_leaves_the_second_stream_joined(prepare):
     assert not done.query()
     torch.cuda.synchronize()
     L.check_device_status(dev)
+
+
+def test_passes_from_threads_that_come_and_go():
+    """Each thread has events of its own and gives them back; streams and results stay as they are."""
+    import threading
+    want, got = _layer(128, 2, 64).detach(), []
+
+    def work(stream):
+        with torch.cuda.stream(stream):
+            got.append(_layer(128, 2, 64).detach())
+    for _ in range(3):
+        threads = [threading.Thread(target=work, args=(torch.cuda.Stream(),)) for _ in range(4)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    torch.cuda.synchronize()
+    assert len(got) == 12 and all(torch.equal(g, want) for g in got)
+    assert torch.equal(_layer(128, 2, 64).detach(), want)
