@@ -9,8 +9,8 @@
 //   s_r = scale * u_c * <q, K_bank[r]>,   out = sum_r softmax(s)_r * u_c * V_bank[r].
 // The kernel is bound by HBM (a full batch) or by latency (a few sequences).  A cluster of CTAs takes the selected rows of
 // one (sequence, query token, group of G query heads on one KV head) in turns of 32 rows per warp; parts merge through
-// shared memory, then distributed shared memory.  One sequence, 12 heads, 4,160 rows: 34 us with a CTA per head -> 9 with a
-// cluster of eight; 64 sequences: 162 us -> 131.
+// shared memory, then distributed shared memory.  One sequence, 12 heads, 4,160 rows: 34 us with a CTA per head -> 7.4 with
+// a cluster of eight; 64 sequences: 162 us -> 120.
 #include "host_pass.cuh"
 
 namespace moc {
@@ -258,8 +258,8 @@ extern "C" int moc_decode_attn(const moc_decode_shape* s, const void* q, const v
   // 13.6 us for 3 sequences and 18.0 for 6, now 10.8 and 14.2.
   const long long groups = static_cast<long long>(s->num_heads / group) * s->n_q * s->batch;
   const int units = s->n_chapters * ceil_div(s->tokens_per_chapter, kDecRows);
-  int split = 1;
-  while (split < 8 && split * kDecWarps < units && groups <= resident_clusters(kern, kDecThreads, 0, split * 2)) split *= 2;
+  int split = 8;
+  while (split > 1 && (split / 2 * kDecWarps >= units || groups > resident_clusters(kern, kDecThreads, 0, split))) split /= 2;
   dim3 grid(s->num_heads / group * split, s->n_q, s->batch);
   MOC_CUDA_OK(launch_clustered(kern, grid, kDecThreads, 0, split, static_cast<cudaStream_t>(stream_),
                                static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(kv_bank),

@@ -1,7 +1,7 @@
 // Projection of a few rows, C [M <= 64, N] = A [M, K] W [N, K]^T with bf16 operands and fp32 accumulation: the query and
 // output projections of a decoding step.  A 128-row tensor-core tile would leave all but a few SMs idle behind one serial
 // chain of K steps (10 us at K 768 whatever M is); bound by latency, the work goes to a warp per column and eight rows, with
-// the weight row in registers and the sums of the eight rows reduced together.  768 x 768: 9.5 -> 2.5 us for one row, 11 -> 10
+// the weight row in registers and the sums of the eight rows reduced together.  768 x 768: 9.5 -> 2.8 us for one row, 11 -> 10
 // for 64.
 #include "moc_common.cuh"
 

@@ -1126,8 +1126,9 @@ int launch_select(const float* logits, long long ld, const float* bias, float* p
                   int* comb_idx, float* comb_w, float* row_stats, int B, int C, int k_sel, int S, float rho,
                   cudaStream_t stream) {
   const size_t sm = (static_cast<size_t>(C) + 2 * static_cast<size_t>(k_sel > 0 ? k_sel : 1)) * 4;
-  // The row's values stay in registers: up to 9 a thread of 1,024 (64 registers leave room for no more), 17 of 256; the
-  // steps are a power of two of routed chapters and a few shared ones.
+  // The row's values stay in registers: up to 9 a thread of 1,024 (64 registers leave room for no more), 17 of 256 (where
+  // more would leave two CTAs an SM).  The steps take a few shared chapters beside 1,024 and 4,096 routed ones and, with
+  // 1,024 threads, beside 1,024 (2), 4,096 (5) and 8,192 (9); longer rows go through shared memory.
   const bool small = B >= kManyRows && C <= 17 * 256;
   auto kern = small ? (C <= 5 * 256 ? select_kernel<5, 256> : select_kernel<17, 256>)
               : C <= 2 * 1024 ? select_kernel<2, 1024> : C <= 5 * 1024 ? select_kernel<5, 1024>
