@@ -320,7 +320,7 @@ __global__ void logits_kernel(const float* __restrict__ pooled, const float* __r
 // (The resident CTAs are what the registers allow without the divisions of wide rows, which would take more.)
 constexpr int kBins = 512, kBinBits = 9, kCand = 512;
 template <int NV, int TH>
-__global__ void __launch_bounds__(TH, TH == 256 ? (NV > 5 ? 3 : 6) : (NV > 5 ? 1 : 2))
+__global__ void __launch_bounds__(TH, TH == 256 ? (NV > 17 ? 2 : NV > 5 ? 3 : 6) : (NV > 5 ? 1 : 2))
 select_kernel(const float* __restrict__ logits, long long ld, const float* __restrict__ bias, float* __restrict__ probs, long long* __restrict__ idx,
               float* __restrict__ weights, int* __restrict__ comb_idx, float* __restrict__ comb_w,
               float* __restrict__ row_stats, int C, int k_sel, int S, float rho) {
@@ -1126,11 +1126,11 @@ int launch_select(const float* logits, long long ld, const float* bias, float* p
                   int* comb_idx, float* comb_w, float* row_stats, int B, int C, int k_sel, int S, float rho,
                   cudaStream_t stream) {
   const size_t sm = (static_cast<size_t>(C) + 2 * static_cast<size_t>(k_sel > 0 ? k_sel : 1)) * 4;
-  // The row's values stay in registers: up to 9 a thread of 1,024 (64 registers leave room for no more), 17 of 256 (where
-  // more would leave two CTAs an SM).  The steps take a few shared chapters beside 1,024 and 4,096 routed ones and, with
-  // 1,024 threads, beside 1,024 (2), 4,096 (5) and 8,192 (9); longer rows go through shared memory.
-  const bool small = B >= kManyRows && C <= 17 * 256;
-  auto kern = small ? (C <= 5 * 256 ? select_kernel<5, 256> : select_kernel<17, 256>)
+  // The row's values stay in registers: up to 9 a thread of 1,024 (64 registers leave room for no more), 33 of 256.  The
+  // steps are a power of two of routed chapters and a few shared ones; rows beyond 8,192 and some go through shared memory.
+  // 8,192 rows of 8,193 chapters: 435 us with 1,024 threads, 305 with 256 (1,024 rows: 62 and 50).
+  const bool small = B >= kManyRows && C <= 33 * 256;
+  auto kern = small ? (C <= 5 * 256 ? select_kernel<5, 256> : C <= 17 * 256 ? select_kernel<17, 256> : select_kernel<33, 256>)
               : C <= 2 * 1024 ? select_kernel<2, 1024> : C <= 5 * 1024 ? select_kernel<5, 1024>
               : C <= 9 * 1024 ? select_kernel<9, 1024> : select_kernel<0, 1024>;
   MOC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm)));
@@ -1146,6 +1146,9 @@ int launch_dlogits(const float* probs, const int64_t* idx, const float* weights,
                    cudaStream_t stream) {
   const size_t sm = static_cast<size_t>(C) * 4;
   const int cols = terms != nullptr ? ld : C;
+  // In registers up to 18 values a thread of 256, 6 of 1,024.  More is no gain: with 34 of 256 the two CTAs an SM take as long
+  // as the general kernel (8,192 rows of 8,193 chapters: 493 and 494 us; 1,024 rows: 61 and 49), with 9 of 1,024 too (8 rows:
+  // 23 us either way).
   const bool small = B >= kManyRows && cols <= 18 * 256;
   auto kern = small ? dlogits_kernel<18, 256> : cols <= 6 * 1024 ? dlogits_kernel<6, 1024> : dlogits_kernel<0, 1024>;
   MOC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm)));

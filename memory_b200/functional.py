@@ -45,6 +45,8 @@ def _check_numel(name: str, t: Optional[torch.Tensor], n: int) -> None:
 
 def _check_projections(d: int, mem_dim: int, wq, wk, wv, wo, num_heads: int, num_kv_heads: int) -> None:
     q, k, v, o = wq.shape, wk.shape, wv.shape, wo.shape
+    if num_heads > 0 and d % num_heads == 0 and q == o == (d, d) and k == v == (num_kv_heads * (d // num_heads), mem_dim):
+        return
     for name, shape, width in (("wq", q, d), ("wk", k, mem_dim), ("wv", v, mem_dim), ("wo", o, q[0])):
         if len(shape) != 2 or shape[1] != width:
             raise ValueError(f"inner dimensions differ: {name} {tuple(shape)} vs {width}")

@@ -73,7 +73,7 @@ def test_router_quotient_is_the_division():
 
 
 @pytest.mark.parametrize("rows", [2, 4096])
-@pytest.mark.parametrize("chapters", [200, 1025, 2000, 4097, 5000, 9000])
+@pytest.mark.parametrize("chapters", [200, 1025, 2000, 4097, 5000, 8193, 9000])
 def test_router_probabilities_of_rows_with_a_wide_range_are_divided(rows, chapters):
     """Two rows with the same tiny rest under one large value and under two.  The first row's sum is 1, so its
     probabilities are the exponentials themselves; the second's must be those divided by its sum, to the last bit."""
