@@ -63,9 +63,7 @@ __device__ __forceinline__ float ex2(float x) {
 __device__ __forceinline__ void ex2_poly2(uint64_t x, float& y0, float& y1) {
   float x0, x1;
   f2_unpack(x, x0, x1);
-  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x0) : "f"(-127.f));
-  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x1) : "f"(-127.f));
-  x = f2_pack(x0, x1);
+  x = f2_pack(max_nan(x0, -127.f), max_nan(x1, -127.f));
   const uint64_t magic = f2_pack(12582912.f, 12582912.f), nmagic = f2_pack(-12582912.f, -12582912.f);
   const uint64_t t = f2_add(x, magic);
   const uint64_t n = f2_add(t, nmagic);

@@ -247,8 +247,8 @@ __global__ void merge_kernel(Shape x, const int* __restrict__ pos, const float* 
       ls[i] = e < 0 ? -INFINITY : lse_rows[row] * kLog2e;
       v[i] = e < 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : reinterpret_cast<const float4*>(partial + row * kD)[lane];
     }
-    const float mn = fmaxf(fmaxf(fmaxf(ls[0], ls[1]), fmaxf(ls[2], ls[3])), m);
-    if (mn == -INFINITY) continue;
+    const float mn = max_nan(max_nan(max_nan(ls[0], ls[1]), max_nan(ls[2], ls[3])), m);
+    if (mn == -INFINITY) continue;             // no listed block exists so far (a NaN sum is no reason to skip)
     const float a = ex2(m - mn);
     den *= a; acc.x *= a; acc.y *= a; acc.z *= a; acc.w *= a;
 #pragma unroll

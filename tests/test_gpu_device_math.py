@@ -90,3 +90,24 @@ def test_router_probabilities_of_rows_with_a_wide_range_are_divided(rows, chapte
     for row in (1, rows - 1):
         assert p[row, 0] == 1.0 / total.cpu().numpy()[0]
         assert (p[row, 2:] == e[2:] / total.cpu().numpy()[0]).all()
+
+
+@pytest.mark.parametrize("block", [64, 128])
+def test_a_nan_query_stays_nan_in_the_sparse_attention(block):
+    """Every listed block of such a token has a NaN sum; a token none of whose blocks exists still gets zeros."""
+    import memory_b200 as M
+    from memory_b200 import _lib as L
+    g = torch.Generator(device=DEV).manual_seed(5)
+    q = torch.randn(1, 20, 4, 64, generator=g, device=DEV).bfloat16()
+    k, v = (torch.randn(1, 6 * block, 2, 64, generator=g, device=DEV).bfloat16() for _ in range(2))
+    bi = torch.rand(40, 6, generator=g, device=DEV).topk(3, dim=1).indices.view(1, 20, 2, 3).int()
+    want, want_lse = M.memory_cross_attn_forward(q, k, v, bi, block)
+    q[0, 7, 2], bi[0, 11] = math.nan, 6
+    o, lse = M.memory_cross_attn_forward(q, k, v, bi, block)
+    with pytest.raises(RuntimeError, match="out of range"):
+        L.check_device_status(o.device)
+    assert o[0, 7, 2].isnan().all() and lse[0, 7, 2].isnan()
+    assert not o[0, 11].any() and (lse[0, 11] == -math.inf).all()
+    rest = torch.ones(20, 4, dtype=torch.bool, device=DEV)
+    rest[7, 2], rest[11] = False, False
+    assert torch.equal(o[0][rest], want[0][rest]) and torch.equal(lse[0][rest], want_lse[0][rest])
