@@ -8,6 +8,7 @@ import ctypes as C
 from typing import Dict, Optional, Tuple
 
 import torch
+from torch.autograd import forward_ad
 
 from . import _lib as L
 
@@ -1236,14 +1237,20 @@ def decode_attn(q: torch.Tensor, kv_bank: torch.Tensor, comb_idx: torch.Tensor, 
 
 def roll_window(cache: torch.Tensor, h: torch.Tensor, rows: int) -> Optional[torch.Tensor]:
     """The last ``rows`` positions of ``cat([cache, h], dim=1)`` as a new [B, rows, d] tensor, or None where the rows are
-    no whole 16-byte pieces of CUDA memory (the caller concatenates)."""
+    no whole 16-byte pieces of CUDA memory, or where torch has to see the operation (a trace, forward-mode gradients,
+    tensors without memory of their own such as those of ``vmap``): the caller then concatenates."""
+    if torch._C._get_tracing_state() is not None or forward_ad._current_level >= 0:
+        return None
     b, d = h.shape[0], h.shape[2]
     size, dev = h.element_size(), h.device
     cb, n, cd = cache.shape
     if not h.is_cuda or dev != cache.device or h.dtype != cache.dtype or cb != b or cd != d or d * size % 16 or b == 0 or b > 65535:
         return None
     (c0, c1, c2), (h0, h1, h2), h_rows = cache.stride(), h.stride(), h.shape[1]
-    cp, hp = cache.data_ptr(), h.data_ptr()
+    try:
+        cp, hp = cache.data_ptr(), h.data_ptr()
+    except RuntimeError:
+        return None
     if (((c2 != 1 or h2 != 1) and d > 1) or (c1 != d and n > 1) or (h1 != d and h_rows > 1)
             or (c0 * size | h0 * size | cp | hp) % 16):
         return None
