@@ -58,12 +58,13 @@ __device__ __forceinline__ float ex2(float x) {
 
 // 2^x for two values on the FMA pipe: x = n + f with |f| <= 1/2 (Cody-Waite with the round-to-nearest addition of
 // 1.5 * 2^23), a degree-5 polynomial fitted to 2^f for least relative error (2.3e-7 in fp32, that of the hardware
-// instruction), times 2^n.  As the instruction does, it gives 0 for -inf (a masked column) and NaN for NaN; arguments count
-// as no less than -127, for which 2^n is 0.
+// instruction), n added to the exponent.  Arguments count as no less than -127, whose 2^n comes out as the smallest
+// subnormal: 0 as bf16, and nothing beside the row's largest term, so a masked column (-inf) adds nothing.  NaN is not
+// kept; the row maximum sees it.
 __device__ __forceinline__ void ex2_poly2(uint64_t x, float& y0, float& y1) {
   float x0, x1;
   f2_unpack(x, x0, x1);
-  x = f2_pack(max_nan(x0, -127.f), max_nan(x1, -127.f));
+  x = f2_pack(fmaxf(x0, -127.f), fmaxf(x1, -127.f));
   const uint64_t magic = f2_pack(12582912.f, 12582912.f), nmagic = f2_pack(-12582912.f, -12582912.f);
   const uint64_t t = f2_add(x, magic);
   const uint64_t n = f2_add(t, nmagic);
@@ -74,10 +75,11 @@ __device__ __forceinline__ void ex2_poly2(uint64_t x, float& y0, float& y1) {
   p = f2_fma(p, f, f2_pack(0.24022120237350464f, 0.24022120237350464f));
   p = f2_fma(p, f, f2_pack(0.6931469440460205f, 0.6931469440460205f));
   p = f2_fma(p, f, f2_pack(1.0000001192092896f, 1.0000001192092896f));
-  float t0, t1;
+  float p0, p1, t0, t1;
+  f2_unpack(p, p0, p1);
   f2_unpack(t, t0, t1);
-  const float s0 = __int_as_float((__float_as_int(t0) << 23) + 0x3F800000), s1 = __int_as_float((__float_as_int(t1) << 23) + 0x3F800000);
-  f2_unpack(f2_mul(p, f2_pack(s0, s1)), y0, y1);
+  y0 = __int_as_float(__float_as_int(p0) + (__float_as_int(t0) << 23));
+  y1 = __int_as_float(__float_as_int(p1) + (__float_as_int(t1) << 23));
 }
 
 __global__ void exp2_probe_kernel(const float* __restrict__ x, float* __restrict__ y, int pairs) {
@@ -284,15 +286,15 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 #pragma unroll
         for (int c = 0; c < 32; c += 4)
 #pragma unroll
-          for (int i = 0; i < 4; ++i) t[i] = max3(t[i], __uint_as_float(r0[c + i]), __uint_as_float(r1[c + i]));
-        return fmaxf(max3(t[0], t[1], t[2]), t[3]);
+          for (int i = 0; i < 4; ++i) t[i] = max3_nan(t[i], __uint_as_float(r0[c + i]), __uint_as_float(r1[c + i]));
+        return max_nan(max3_nan(t[0], t[1], t[2]), t[3]);
       };
       // The maximum is off the critical path: from the second tile on the exponentials are taken against the running
       // maximum at once, and only a tile that exceeds it by more than 2^8 (P would leave bf16's accurate range) is taken
-      // again after the rescale.
+      // again after the rescale.  A NaN score, seen here for all columns, takes that way too and makes the row NaN.
       if (j > 0) exps();
-      const float m_new = fmaxf(m_used, row_max() * p.scale_log2);
-      const bool need = (j == 0) || (m_new - m_used > kRescaleThreshold);
+      const float m_new = max_nan(m_used, row_max() * p.scale_log2);
+      const bool need = (j == 0) || !(m_new - m_used <= kRescaleThreshold);
       if (__any_sync(0xffffffffu, need)) {
         if (j > 0) {
           const int pb = buf == 0 ? kBufs - 1 : buf - 1;      // O is complete up to tile j-1
@@ -359,8 +361,8 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       }
       if (p.split > 1)
         reinterpret_cast<float2*>(q_s)[row] = make_float2(m_used, l_sum);
-      else if (l < p.L)
-        p.lse[(static_cast<long long>(b) * p.H + h) * p.L + l] = (m_used + log2f(l_sum)) * 0.6931471805599453f;
+      else if (l < p.L)             // (an infinite maximum is NaN against itself, as its row is: 0 over a sum of next to 0)
+        p.lse[(static_cast<long long>(b) * p.H + h) * p.L + l] = (m_used + log2f(l_sum) + (m_used - m_used)) * 0.6931471805599453f;
     }
     tc_fence_before();
   }

@@ -367,6 +367,11 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
 }
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {     // NaN where any is
+  float r;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 // the larger, or NaN where either is
 __device__ __forceinline__ float max_nan(float a, float b) {
   float r;
