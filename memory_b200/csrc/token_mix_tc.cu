@@ -219,6 +219,7 @@ __device__ __forceinline__ void put_piece(uint8_t* tile, int r, const uint4& v) 
 }
 // The row-owning warps meet, and agree whether the waits of all of them were met.  A wait can run out in one warp and be met
 // in the next, and the barrier has no limit of its own: every warp comes here, and the loops are left on its answer alone.
+// A warp whose wait ran out works on with what stands in its buffers; nothing of it reaches the partial results.
 __device__ __forceinline__ bool row_warps_agree(bool ok) { return warps_agree<1, kTok>(ok); }
 // one arrival per warp for what all its lanes have done
 __device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
@@ -338,8 +339,8 @@ token_mix_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
         fence_proxy_async();
         warp_arrive(&q_ready, lane);
         float m = 0.f, l = 1.f;
-        if (active) ok = mbar_wait_w(&s_bar, it & 1, &abort_flag, p.status);
-        if (active && ok) {
+        if (active) {
+          ok = mbar_wait_w(&s_bar, it & 1, &abort_flag, p.status);
           tc_fence_after();
           // S is read twice, half a row at a time: both halves in registers would spill
           m = -INFINITY;
@@ -370,13 +371,13 @@ token_mix_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
           tmem_wait_st();
           tc_fence_before();
         }
-        if (ok) warp_arrive(&p_bar, lane);
+        warp_arrive(&p_bar, lane);
         if (hq + 1 < hq_hi) {                      // lands under P V
 #pragma unroll
           for (int i = 0; i < kAhead; ++i) ahead[i] = load_piece(p.q, x.HQ * kD, (hq + 1) * kD, tk, move_row(i), cnt);
         }
-        ok = ok && mbar_wait_w(&o_bar, it & 1, &abort_flag, p.status);
-        if (active && ok) {
+        ok &= mbar_wait_w(&o_bar, it & 1, &abort_flag, p.status);
+        if (active) {
           tc_fence_after();
           const float f = x.out_scale * wv / l;
 #pragma unroll
@@ -397,8 +398,7 @@ token_mix_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
           if (valid) p.lse_slots[lse_at + static_cast<long long>(hq) * x.S] = fmaf(m, x.scale, __logf(l));
           tc_fence_before();
         }
-        ok = row_warps_agree(ok);
-        if (!ok) break;
+        if (!row_warps_agree(ok)) { ok = false; break; }
         for (int i = 0; 16 * i < cnt; ++i) {
           const int rr = move_row(i), piece = threadIdx.x & 7;
           if (rr < cnt)
