@@ -34,16 +34,6 @@ __device__ __forceinline__ float ex2(float x) {
   asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// four rows of a [rows, 64] bf16 tensor into 512 contiguous bytes of a 128-byte-swizzled tile
-__device__ __forceinline__ void tma_gather4(void* dst, const CUtensorMap* map, uint64_t* bar, int r0, int r1, int r2,
-                                            int r3) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes [%0], "
-      "[%1, {%3, %4, %5, %6, %7}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(0), "r"(r0), "r"(r1),
-      "r"(r2), "r"(r3)
-      : "memory");
-}
 // 32 bytes per thread: one full sector
 __device__ __forceinline__ void st_v8(float* dst, const float (&v)[8]) {
   asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
@@ -78,8 +68,8 @@ __device__ __forceinline__ void gather_tile(const Shape& x, const int* entries, 
     const RowRef rr = row_ref(x, entries, first, cnt, lane * 4 + i);
     row[i] = static_cast<int>(rr.tok) * x.HQ + rr.hq;
   }
-  tma_gather4(dst_a + lane * 512, map_a, bar, row[0], row[1], row[2], row[3]);
-  if (dst_b != nullptr) tma_gather4(dst_b + lane * 512, map_b, bar, row[0], row[1], row[2], row[3]);
+  tma_gather4(dst_a + lane * 512, map_a, bar, 0, row[0], row[1], row[2], row[3]);
+  if (dst_b != nullptr) tma_gather4(dst_b + lane * 512, map_b, bar, 0, row[0], row[1], row[2], row[3]);
 }
 
 // ---- forward -------------------------------------------------------------------------------------------------

@@ -14,10 +14,12 @@
 // leaves as per-pair partials, and dK_c / dV_c accumulate in tensor memory over all pairs (and query heads) of the
 // chapter through one 128 x 128 product  [Pw | dS]^T [dO | Q]  whose diagonal blocks are dV_c and dK_c (the
 // off-diagonal blocks are not used: 64-row chapters would otherwise need 64-row MMA tiles).
+//
+// Chapters with few pairs leave these tiles mostly empty: they have kernels of their own (token_mix_rows.cuh).
 #define MOC_KERNEL_TAG 5
 #include <algorithm>
 
-#include "moc_common.cuh"
+#include "host_pass.cuh"
 
 namespace moc {
 namespace {
@@ -751,6 +753,12 @@ token_mix_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
   if (warp == 4) { tc_fence_after(); tmem_dealloc(tmem, 256); }
 }
 
+}  // namespace
+}  // namespace moc
+#include "token_mix_rows.cuh"
+namespace moc {
+namespace {
+
 int sm_count() {
   static int n = 0;
   if (n == 0) {
@@ -760,6 +768,13 @@ int sm_count() {
   }
   return n;
 }
+
+// Below these the kernels of token_mix_rows.cuh are the faster ones.  8,192 tokens x 16 chapters of as many as the figure says, 12
+// heads, us before (128-row tiles) and with them.  Forward, by pairs a chapter: 32: 268 -> 232, 64: 97 -> 104 (8 slots), 128: 208 -> 179,
+// 256: 195 and 206, 512: 131 and 202; with the uneven buckets that a router gives 32: 357 -> 270.  Backward, by rows (pairs x
+// query heads of a KV head) a chapter: 32: 1,064 -> 569, 128: 505 -> 391, 256: 442 -> 367, 384: 501 -> 382, 512: 406 and 397, 1,536: 387 and 466;
+// uneven, 32: 1,196 -> 607.
+constexpr long long kRowFwdPairs = 256, kRowBwdRowsMax = 512;
 
 int check_shape(const moc_sparse_attn_shape* s, int index_heads, MixShape* x) {
   MOC_REQUIRE(s != nullptr, "shape is NULL");
@@ -830,13 +845,19 @@ extern "C" int moc_token_mix_fwd(const moc_sparse_attn_shape* s, int32_t index_h
   p.partial = static_cast<__nv_bfloat16*>(partial); p.lse_slots = lse_slots;
   p.entries = ib.entries; p.tile_bucket = ib.tile_bucket; p.tile_first = ib.tile_first; p.tile_cnt = ib.tile_cnt;
   p.totals = ib.totals; p.x = x; p.status = status;
-  static bool attr_set = false;
-  if (!attr_set) {
+  if (n_pairs < kRowFwdPairs * n_buckets && n_buckets * x.HQ < (1ll << 30)) {
+    CUtensorMap mq;                                              // rows of one head, gathered four at a time
+    const uint64_t q_cols = static_cast<uint64_t>(x.HQ) * kD;
+    MOC_TRY(make_tmap_bf16_2d(&mq, q, static_cast<uint64_t>(x.B) * x.TQ, q_cols, q_cols, 1, kD));
+    const RowItems items{ib.bucket_off, static_cast<int>(n_buckets) * (x.HQ / x.HI), {fast_div(x.S), fast_div(x.HI)}};
+    MOC_CUDA_OK(cudaFuncSetAttribute(token_mix_rows_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowFwdSmem));
+    const int grid = std::min((items.n + kRowFwdWarps - 1) / kRowFwdWarps, sm_count() * kRowFwdCtas);
+    token_mix_rows_fwd_kernel<<<grid, kRowFwdWarps * 32, kRowFwdSmem, st>>>(mk, mv, mq, p, items);
+  } else {
     MOC_CUDA_OK(cudaFuncSetAttribute(token_mix_fwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem));
-    attr_set = true;
+    const long long grid = std::min<long long>(max_tiles(n_pairs, n_buckets), static_cast<long long>(sm_count()) * 4);
+    token_mix_fwd_tc_kernel<<<static_cast<int>(grid), kMixThreads, kFwdSmem, st>>>(mk, mv, p);
   }
-  const long long grid = std::min<long long>(max_tiles(n_pairs, n_buckets), static_cast<long long>(sm_count()) * 4);
-  token_mix_fwd_tc_kernel<<<static_cast<int>(grid), kMixThreads, kFwdSmem, st>>>(mk, mv, p);
   const long long rows = static_cast<long long>(x.B) * x.TQ;
   const long long threads = rows * x.HQ * (kD / 8);
   slot_reduce_kernel<<<static_cast<int>((threads + 255) / 256), 256, 0, st>>>(
@@ -876,16 +897,23 @@ extern "C" int moc_token_mix_bwd(const moc_sparse_attn_shape* s, int32_t index_h
   p.dq_partial = static_cast<__nv_bfloat16*>(dq_partial); p.d_w_heads = d_w_heads;
   p.d_k = static_cast<__nv_bfloat16*>(d_k); p.d_v = static_cast<__nv_bfloat16*>(d_v); p.dkv_ld = dkv_row_stride;
   p.entries = ib.entries; p.bucket_off = ib.bucket_off;
-  p.runs = x.HI == 1 ? (x.HK + kRunHeads - 1) / kRunHeads : 1;
-  p.n_items = static_cast<int>(n_buckets) * p.runs;
   p.x = x; p.status = status;
-  static bool attr_set = false;
-  if (!attr_set) {
+  if (n_pairs * (x.HQ / x.HK) < kRowBwdRowsMax * n_buckets) {
+    CUtensorMap mq, md;                                          // rows of one head, gathered four at a time
+    const uint64_t q_rows = static_cast<uint64_t>(x.B) * x.TQ, q_cols = static_cast<uint64_t>(x.HQ) * kD;
+    MOC_TRY(make_tmap_bf16_2d(&mq, q, q_rows, q_cols, q_cols, 1, kD));
+    MOC_TRY(make_tmap_bf16_2d(&md, d_o, q_rows, q_cols, q_cols, 1, kD));
+    const RowItems items{ib.bucket_off, static_cast<int>(n_buckets) * (x.HK / x.HI), {fast_div(x.S), fast_div(x.HI)}};
+    MOC_CUDA_OK(cudaFuncSetAttribute(token_mix_rows_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowBwdSmem));
+    const int grid = std::min(items.n, sm_count() * kRowBwdCtas);
+    token_mix_rows_bwd_kernel<<<grid, kRowBwdThreads, kRowBwdSmem, st>>>(mk, mv, mq, md, p, items);
+  } else {
+    p.runs = x.HI == 1 ? (x.HK + kRunHeads - 1) / kRunHeads : 1;
+    p.n_items = static_cast<int>(n_buckets) * p.runs;
     MOC_CUDA_OK(cudaFuncSetAttribute(token_mix_bwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem));
-    attr_set = true;
+    const int grid = std::min(p.n_items, sm_count() * 2);
+    token_mix_bwd_tc_kernel<<<grid, kMixThreads, kBwdSmem, st>>>(mk, mv, p);
   }
-  const long long grid = std::min<long long>(p.n_items, static_cast<long long>(sm_count()) * 2);
-  token_mix_bwd_tc_kernel<<<static_cast<int>(grid), kMixThreads, kBwdSmem, st>>>(mk, mv, p);
   const long long rows = static_cast<long long>(x.B) * x.TQ;
   const long long threads = rows * x.HQ * (kD / 8);
   slot_reduce_kernel<<<static_cast<int>((threads + 255) / 256), 256, 0, st>>>(
