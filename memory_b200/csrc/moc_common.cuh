@@ -123,6 +123,14 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
   if (__all_sync(0xffffffffu, ok)) return true;
   return __all_sync(0xffffffffu, ok || mbar_wait_slow(bar, parity, abort_flag, status, kWaitPollLimit, where));
 }
+// One arrival for what all lanes of a converged warp have done: 32 arrivals on one barrier are taken one after the other.
+__device__ __forceinline__ void mbar_arrive_warp(uint64_t* bar) {
+  __syncwarp();
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "@q mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(smem_u32(bar)) : "memory");
+}
 // Barrier ID of N threads (whole warps) that tells each whether all of them came with `ok`
 template <int ID, int N> __device__ __forceinline__ bool warps_agree(bool ok) {
   uint32_t all;
