@@ -308,16 +308,24 @@ extern "C" int moc_decode_step(const moc_decode_step_desc* s) {
   r->arena = a.route_arena; r->status = s->status; r->stream = s->stream;
   const int64_t rows = static_cast<int64_t>(s->attn.batch) * s->attn.n_q, d = width_of(s);
   const int64_t width = static_cast<int64_t>(s->attn.num_heads) * kDD;
-  // the query projection needs nothing of the router; beside it from a dozen rows on, where it takes longer than the events
+  // The query projection needs nothing of the router: for a row or two in the router's launch, beside it from a dozen rows on, where
+  // it takes longer than the events.
   cudaStream_t main = static_cast<cudaStream_t>(s->stream);
   cudaStream_t side = rows > 8 && s->side_stream ? static_cast<cudaStream_t>(s->side_stream) : main;
   if (side != main) MOC_TRY(order(main, side));
   Join join(side, main);
   const void* x;
   MOC_TRY(as_dtype(s->hidden, s->hidden_dtype, a.x, MOC_BF16, rows * d, side, &x));
-  Gemm gq(MOC_BF16, rows, width, d, true, true, MOC_BF16);
-  MOC_TRY(moc_gemm(&gq, x, s->wq, a.q, nullptr, nullptr, s->status, side));
-  MOC_TRY(moc_route_fwd(r));
+  const bool few = rows <= 2 && d % 8 == 0 && d <= 1024 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(s->wq)) & 15) == 0;
+  const RowsProduct q{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(s->wq), a.q, d, d, width,
+                      static_cast<int>(rows), static_cast<int>(width), static_cast<int>(d)};
+  bool q_done = false;
+  if (few) MOC_TRY(route_fwd_impl(r, &q, &q_done));
+  if (!q_done) {
+    Gemm gq(MOC_BF16, rows, width, d, true, true, MOC_BF16);
+    MOC_TRY(moc_gemm(&gq, x, s->wq, a.q, nullptr, nullptr, s->status, side));
+  }
+  if (!few) MOC_TRY(moc_route_fwd(r));
   MOC_TRY(join.done());
   MOC_TRY(moc_decode_attn(&s->attn, a.q, s->kv_bank, s->bank_rows, s->comb_idx, s->comb_w, a.o, nullptr, s->status, s->stream));
   Gemm go(MOC_BF16, rows, s->out_dim, width, true, true, s->hidden_dtype);

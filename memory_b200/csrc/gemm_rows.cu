@@ -3,19 +3,10 @@
 // chain of K steps (10 us at K 768 whatever M is); bound by latency, the work goes to a warp per column and eight rows, with
 // the weight row in registers and the sums of the eight rows reduced together.  768 x 768: 9.5 -> 2.8 us for one row, 11 -> 10
 // for 64.
-#include "moc_common.cuh"
+#include "rows_product.cuh"
 
 namespace moc {
 namespace {
-
-__device__ __forceinline__ void unpack8(const uint4& v, float* f) {
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    f[2 * i] = __uint_as_float(w[i] << 16);
-    f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-  }
-}
 
 constexpr int kRows = 8, kCols = 8;
 // NV: 16-byte pieces of a row per lane (K <= 256 NV)

@@ -44,7 +44,7 @@ extern "C" int64_t moc_route_bwd_scratch_bytes(const moc_route_desc* s) {
   return s ? carve_bwd(&s->shape, nullptr, &t) : -1;
 }
 
-extern "C" int moc_route_fwd(const moc_route_desc* s) {
+int moc::route_fwd_impl(const moc_route_desc* s, const RowsProduct* q, bool* q_done) {
   MOC_REQUIRE(s && s->h && s->w && s->comb_idx && s->comb_w && s->arena && s->status, "NULL router buffer");
   const moc_router_shape* r = &s->shape;
   Saved a;
@@ -56,10 +56,11 @@ extern "C" int moc_route_fwd(const moc_route_desc* s) {
                                   s->stream));
     parts |= 8;
   }
-  return moc_router_fwd_parts(r, s->h, s->w, s->bias, a.pooled, a.logits, a.probs, s->idx, s->weights, s->comb_idx,
-                              s->comb_w, a.row_stats, a.chapter_stats, s->losses, a.ws, ws_bytes, parts, s->status,
-                              s->stream);
+  return router_fwd_parts_impl(r, s->h, s->w, s->bias, a.pooled, a.logits, a.probs, s->idx, s->weights, s->comb_idx,
+                               s->comb_w, a.row_stats, a.chapter_stats, s->losses, a.ws, ws_bytes, parts, q, q_done, s->status,
+                               s->stream);
 }
+extern "C" int moc_route_fwd(const moc_route_desc* s) { return route_fwd_impl(s, nullptr, nullptr); }
 
 extern "C" int moc_route_bwd(const moc_route_desc* s, const float* g_weights, const float* g_comb_w, const float* g_losses,
                              void* d_h, float* d_w, float* d_bias, void* scratch) {

@@ -8,7 +8,7 @@
 
 #include <type_traits>
 
-#include "host_pass.cuh"
+#include "rows_product.cuh"
 
 namespace moc {
 namespace {
@@ -319,12 +319,11 @@ __global__ void logits_kernel(const float* __restrict__ pooled, const float* __r
 // threads, whose barriers are shorter and chains more: 8,192 rows, k 16: 252 us with TH 1,024 -> 152.
 // (The resident CTAs are what the registers allow without the divisions of wide rows, which would take more.)
 constexpr int kBins = 512, kBinBits = 9, kCand = 512;
+// (sm: [C] masked probabilities, then [2 k_sel] selection scratch.  Plain pointers: a kernel may have written the logits itself.)
 template <int NV, int TH>
-__global__ void __launch_bounds__(TH, TH == 256 ? (NV > 17 ? 2 : NV > 5 ? 3 : 6) : (NV > 5 ? 1 : 2))
-select_kernel(const float* __restrict__ logits, long long ld, const float* __restrict__ bias, float* __restrict__ probs, long long* __restrict__ idx,
-              float* __restrict__ weights, int* __restrict__ comb_idx, float* __restrict__ comb_w,
-              float* __restrict__ row_stats, int C, int k_sel, int S, float rho) {
-  extern __shared__ float sm[];            // [C] masked probabilities, then selection scratch
+__device__ __forceinline__ void select_row(const int b, const float* logits, long long ld, const float* bias, float* probs,
+                                           long long* idx, float* weights, int* comb_idx, float* comb_w, float* row_stats,
+                                           int C, int k_sel, int S, float rho, float* sm) {
   float* pt = sm;                          // p~
   uint32_t* sel_key = reinterpret_cast<uint32_t*>(sm + C);   // [k_sel]
   int* sel_idx = reinterpret_cast<int*>(sel_key + k_sel);    // [k_sel]
@@ -335,7 +334,6 @@ select_kernel(const float* __restrict__ logits, long long ld, const float* __res
   __shared__ int bins[NV > 0 ? kBins : 1], wsum[32], cand_idx[NV > 0 ? kCand : 1];
   __shared__ uint32_t mm[64], cand_key[NV > 0 ? kCand : 1];
 
-  const int b = blockIdx.x;
   const float* z = logits + b * ld;       // (bias: not yet in the logits, or nullptr)
   auto logit = [&](int c) { return bias != nullptr ? z[c] + bias[c] : z[c]; };
   float* p = probs + static_cast<long long>(b) * C;
@@ -626,6 +624,120 @@ select_kernel(const float* __restrict__ logits, long long ld, const float* __res
     rs[2] = topk_mass;
     rs[3] = comb_mass;
   }
+}
+template <int NV, int TH>
+__global__ void __launch_bounds__(TH, TH == 256 ? (NV > 17 ? 2 : NV > 5 ? 3 : 6) : (NV > 5 ? 1 : 2))
+select_kernel(const float* __restrict__ logits, long long ld, const float* __restrict__ bias, float* __restrict__ probs, long long* __restrict__ idx,
+              float* __restrict__ weights, int* __restrict__ comb_idx, float* __restrict__ comb_w,
+              float* __restrict__ row_stats, int C, int k_sel, int S, float rho) {
+  extern __shared__ float sm[];
+  select_row<NV, TH>(blockIdx.x, logits, ld, bias, probs, idx, weights, comb_idx, comb_w, row_stats, C, k_sel, S, rho, sm);
+}
+
+// One or two sequences: pooling, logits and selection in one launch, by one cluster of 16 CTAs that meets at its hardware barrier
+// between them (the same sums in the same order as the kernels above).  16 SMs read the router's weights in 6 us where all of
+// them take 3, but what such a call waits for is the host, where three launches are some 10 us.  From three sequences on the products
+// are bound by shared memory and want the whole chip.  The remaining CTAs, clusters of their own, are a projection of as many
+// rows that needs nothing of the routing: the queries of a decoding step, one warp a column.
+// One sequence, window 128, 4,097 chapters, with the queries: 22 us in one launch, 18 in four and the gaps between them; a decoding
+// step 54 -> 46 us, host and device overlapped.
+constexpr int kFrontCtas = 16, kFrontRows = 2;
+struct FrontParams {
+  float *pooled, *logits, *probs;
+  long long* idx;
+  float* weights;
+  int* comb_idx;
+  float *comb_w, *row_stats;
+  int B, L, d, C, k_sel, S;
+  float rho;
+  RowsProduct q;
+};
+// ND: float4 of a weight row per lane
+template <typename T, int NV, int ND>
+__global__ void __launch_bounds__(1024, 1)
+route_front_kernel(const T* __restrict__ h, const float* __restrict__ w, const float* __restrict__ bias, FrontParams p) {
+  extern __shared__ float4 front_smem[];
+  float* sm = reinterpret_cast<float*>(front_smem);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (blockIdx.x >= kFrontCtas) {
+    const int col = (static_cast<int>(blockIdx.x) - kFrontCtas) * 32 + warp;
+    if (col < p.q.n) rows_product_column<kFrontRows>(p.q, col, lane);
+    return;
+  }
+  const int rank = static_cast<int>(blockIdx.x);
+  const int B = p.B, L = p.L, d = p.d, C = p.C;
+  {
+    // mean over the positions: warp = split of the sequence, lane = (sequence, 16-byte piece of columns)
+    constexpr int kV = 16 / sizeof(T), kPart = 32 * kV + 4;
+    const int pieces = d / kV, p0 = rank * pieces / kFrontCtas, np = (rank + 1) * pieces / kFrontCtas - p0, items = B * np;
+    const int rows_per = (L + kPoolSplits - 1) / kPoolSplits, t0 = warp * rows_per, t1 = min(L, t0 + rows_per);
+    for (int i0 = 0; i0 < items; i0 += 32) {
+      float acc[kV];
+#pragma unroll
+      for (int j = 0; j < kV; ++j) acc[j] = 0.f;
+      if (i0 + lane < items) {
+        const int b = (i0 + lane) / np, piece = p0 + (i0 + lane) - b * np;
+        const T* src = h + static_cast<long long>(b) * L * d + piece * kV;
+#pragma unroll 4
+        for (int t = t0; t < t1; ++t) {
+          const uint4 v = *reinterpret_cast<const uint4*>(src + static_cast<long long>(t) * d);
+          const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if constexpr (sizeof(T) == 2) {
+              acc[2 * j] += __uint_as_float(x[j] << 16);
+              acc[2 * j + 1] += __uint_as_float(x[j] & 0xFFFF0000u);
+            } else {
+              acc[j] += __uint_as_float(x[j]);
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < kV; ++j) sm[warp * kPart + lane * kV + j] = acc[j];
+      __syncthreads();
+      const int n = min(32, items - i0) * kV;
+      if (static_cast<int>(threadIdx.x) < n) {
+        const int item = i0 + static_cast<int>(threadIdx.x) / kV, b = item / np;
+        float t = 0.f;
+#pragma unroll 8
+        for (int i = 0; i < kPoolSplits; ++i) t += sm[i * kPart + threadIdx.x];
+        p.pooled[static_cast<long long>(b) * d + (p0 + item - b * np) * kV + threadIdx.x % kV] = t / static_cast<float>(L);
+      }
+      __syncthreads();
+    }
+  }
+  cluster_sync();
+  {
+    const int d4 = d >> 2;
+    float4* sp4 = front_smem;
+    for (int i = threadIdx.x; i < B * d4; i += 1024) sp4[i] = __ldcg(reinterpret_cast<const float4*>(p.pooled) + i);
+    __syncthreads();
+    const int c_hi = static_cast<int>(static_cast<long long>(rank + 1) * C / kFrontCtas);
+    for (int c = static_cast<int>(static_cast<long long>(rank) * C / kFrontCtas) + warp; c < c_hi; c += 32) {
+      const float4* w4 = reinterpret_cast<const float4*>(w + static_cast<long long>(c) * d);
+      float4 wv[ND];
+#pragma unroll
+      for (int i = 0; i < ND; ++i) wv[i] = lane + 32 * i < d4 ? w4[lane + 32 * i] : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float bc = bias != nullptr ? bias[c] : 0.f;
+      for (int b = 0; b < B; ++b) {
+        float a = 0.f;
+#pragma unroll
+        for (int i = 0; i < ND; ++i) {
+          if (lane + 32 * i < d4) {
+            const float4 pv = sp4[b * d4 + lane + 32 * i];
+            a = fmaf(wv[i].x, pv.x, fmaf(wv[i].y, pv.y, fmaf(wv[i].z, pv.z, fmaf(wv[i].w, pv.w, a))));
+          }
+        }
+        a = warp_sum(a);
+        if (lane == 0) p.logits[static_cast<long long>(b) * C + c] = a + bc;
+      }
+    }
+  }
+  cluster_sync();
+  if (rank < B)
+    select_row<NV, 1024>(rank, p.logits, C, nullptr, p.probs, p.idx, p.weights, p.comb_idx, p.comb_w, p.row_stats, C, p.k_sel, p.S,
+                         p.rho, sm);
 }
 
 // Per chapter chunk: f, mean p^2, and partial sums of the three chapter-separable loss terms.
@@ -1159,6 +1271,33 @@ int launch_dlogits(const float* probs, const int64_t* idx, const float* weights,
   return MOC_OK;
 }
 
+// Whether the one launch takes this call (see route_front_kernel), and that launch.
+bool front_takes(const moc_router_shape* s, const void* h, const float* w, const float* pooled) {
+  const int piece = s->h_dtype == MOC_F32 ? 4 : 8;
+  return s->batch <= kFrontRows && s->seq <= kPoolSplits * kPoolOneMaxRows && s->hidden_dim % piece == 0 && s->hidden_dim % 4 == 0 &&
+         s->hidden_dim <= 1024 && s->num_chapters <= 9 * 1024 &&
+         ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(pooled)) & 15) == 0;
+}
+template <typename T>
+int launch_front(const T* h, const float* w, const float* bias, const FrontParams& p, cudaStream_t stream) {
+  const int nd = p.d <= 256 ? 0 : p.d <= 768 ? 1 : 2, nv = p.C <= 2 * 1024 ? 0 : p.C <= 5 * 1024 ? 1 : 2;
+  using Kern = void (*)(const T*, const float*, const float*, FrontParams);
+  static constexpr Kern kerns[3][3] = {
+      {route_front_kernel<T, 2, 2>, route_front_kernel<T, 5, 2>, route_front_kernel<T, 9, 2>},
+      {route_front_kernel<T, 2, 6>, route_front_kernel<T, 5, 6>, route_front_kernel<T, 9, 6>},
+      {route_front_kernel<T, 2, 8>, route_front_kernel<T, 5, 8>, route_front_kernel<T, 9, 8>}};
+  const Kern kern = kerns[nd][nv];
+  const size_t part = static_cast<size_t>(kPoolSplits) * (32 * (16 / sizeof(T)) + 4) * 4;
+  const size_t sel = (static_cast<size_t>(p.C) + 2 * static_cast<size_t>(p.k_sel > 0 ? p.k_sel : 1)) * 4;
+  const size_t bytes = std::max(std::max(part, sel), static_cast<size_t>(p.B) * p.d * 4);
+  if (bytes > 48 * 1024 - 9 * 1024)              // (9 KiB: the selection's static arrays)
+    MOC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+  MOC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  const int more = ceil_div(ceil_div(p.q.n, 32), kFrontCtas);        // clusters for the projection
+  MOC_CUDA_OK(launch_clustered(kern, dim3(kFrontCtas * (1 + more)), 1024, static_cast<int>(bytes), kFrontCtas, stream, h, w, bias, p));
+  return MOC_OK;
+}
+
 inline int k_selected(const moc_router_shape* s) {
   int k = s->top_k;
   const int avail = s->num_chapters - s->num_shared;
@@ -1316,11 +1455,11 @@ extern "C" size_t moc_router_workspace_bytes_parts(const moc_router_shape* s, in
   return (ws_floats(s, pool, (bwd_parts & 4) != 0) + loss_floats(s)) * sizeof(float);
 }
 
-extern "C" int moc_router_fwd_parts(const moc_router_shape* s, const void* h, const float* w, const float* bias,
-                                    float* pooled, float* logits, float* probs, int64_t* idx, float* weights,
-                                    int32_t* comb_idx, float* comb_w, float* row_stats, float* chapter_stats,
-                                    float* losses, void* workspace, size_t workspace_bytes, int32_t parts,
-                                    int32_t* status, void* stream_) {
+namespace moc {
+int router_fwd_parts_impl(const moc_router_shape* s, const void* h, const float* w, const float* bias, float* pooled, float* logits,
+                          float* probs, int64_t* idx, float* weights, int32_t* comb_idx, float* comb_w, float* row_stats,
+                          float* chapter_stats, float* losses, void* workspace, size_t workspace_bytes, int32_t parts,
+                          const RowsProduct* q, bool* q_done, int32_t* status, void* stream_) {
   int rc = check_shape(s);
   if (rc != MOC_OK) return rc;
   const size_t front = ws_floats(s, (parts & 1) && !(parts & 8), false);
@@ -1337,7 +1476,15 @@ extern "C" int moc_router_fwd_parts(const moc_router_shape* s, const void* h, co
   float* loss_partial = ws + (workspace_bytes / sizeof(float) - loss_floats(s));
 
   dim3 pg(B, kPoolSplits);
-  if (parts & 1) {
+  const bool one_launch = (parts & 1) && !(parts & (8 | 16)) && front_takes(s, h, w, pooled);
+  if (one_launch) {
+    FrontParams p{pooled, logits, probs, reinterpret_cast<long long*>(idx), weights, comb_idx, comb_w, row_stats, B, L, d, C, k_sel,
+                  S, s->routed_scale, RowsProduct{}};
+    if (q != nullptr) { p.q = *q; *q_done = true; }
+    MOC_TRY(s->h_dtype == MOC_F32 ? launch_front(static_cast<const float*>(h), w, bias, p, stream)
+                                  : launch_front(static_cast<const __nv_bfloat16*>(h), w, bias, p, stream));
+  }
+  if ((parts & 1) && !one_launch) {
   if (!(parts & 8)) {      // bit 8: `pooled` already holds the pooled states (another pooling rule ran first)
   const int piece = s->h_dtype == MOC_F32 ? 4 : 8;
   const bool one = L <= kPoolSplits * kPoolOneMaxRows && d % piece == 0 && (reinterpret_cast<uintptr_t>(h) & 15) == 0;
@@ -1379,6 +1526,17 @@ extern "C" int moc_router_fwd_parts(const moc_router_shape* s, const void* h, co
   }
   MOC_CUDA_OK(cudaGetLastError());
   return MOC_OK;
+}
+
+}  // namespace moc
+
+extern "C" int moc_router_fwd_parts(const moc_router_shape* s, const void* h, const float* w, const float* bias,
+                                    float* pooled, float* logits, float* probs, int64_t* idx, float* weights,
+                                    int32_t* comb_idx, float* comb_w, float* row_stats, float* chapter_stats,
+                                    float* losses, void* workspace, size_t workspace_bytes, int32_t parts,
+                                    int32_t* status, void* stream) {
+  return router_fwd_parts_impl(s, h, w, bias, pooled, logits, probs, idx, weights, comb_idx, comb_w, row_stats, chapter_stats,
+                               losses, workspace, workspace_bytes, parts, nullptr, nullptr, status, stream);
 }
 
 extern "C" int moc_router_fwd(const moc_router_shape* s, const void* h, const float* w, const float* bias,
