@@ -1,8 +1,9 @@
-// Projection of a few rows, C [M <= 64, N] = A [M, K] W [N, K]^T with bf16 operands and fp32 accumulation: the query and
+// Projection of a few rows, C [M <= 256, N] = A [M, K] W [N, K]^T with bf16 operands and fp32 accumulation: the query and
 // output projections of a decoding step.  A 128-row tensor-core tile would leave all but a few SMs idle behind one serial
-// chain of K steps (10 us at K 768 whatever M is); bound by latency, the work goes to a warp per column and eight rows, with
-// the weight row in registers and the sums of the eight rows reduced together.  768 x 768: 9.5 -> 2.8 us for one row, 11 -> 10
-// for 64.
+// chain of K steps (10 us at K 768 whatever M is).  Bound by latency: up to eight rows the work goes to a warp per column, with
+// the weight row in registers and the sums of the eight rows reduced together (768 x 768: 9.5 -> 2.8 us for one row); with more
+// rows and columns, to CTAs of 16 columns and 32 rows on single-warp matrix instructions (64 rows: 7.9 -> 4.8 us, one behind the
+// other; 10.6 -> 6 in a decoding step).
 #include "rows_product.cuh"
 
 namespace moc {
@@ -72,17 +73,92 @@ gemm_rows_kernel(const __nv_bfloat16* __restrict__ a, long long lda, const __nv_
   }
 }
 
+// Both operands come to shared memory whole (rows of K elements and 16 bytes, so that the eight rows of an ldmatrix
+// meet no bank twice); eight warps take every eighth K step and their sums are added in warp order.
+constexpr int kMmaRows = 32, kMmaCols = 16, kMmaWarps = 8;
+__host__ __device__ inline int mma_stride(int k) { return (k + 15) / 16 * 32 + 16; }
+__global__ void __launch_bounds__(32 * kMmaWarps)
+gemm_rows_mma_kernel(const __nv_bfloat16* __restrict__ a, long long lda, const __nv_bfloat16* __restrict__ w, long long ldb,
+                     void* __restrict__ c, long long ldc, int c_bf16, int m, int n, int k) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row0 = blockIdx.y * kMmaRows, col0 = blockIdx.x * kMmaCols, stride = mma_stride(k), steps = (k + 15) / 16;
+  const uint32_t a_s = smem_u32(smem), w_s = a_s + kMmaRows * stride;
+  const int pieces = steps * 2;                       // 16-byte pieces of a row, the last one past K where K is an odd multiple of 8
+  for (int i = threadIdx.x; i < (kMmaRows + kMmaCols) * pieces; i += 32 * kMmaWarps) {
+    const int r = i / pieces, p = i - r * pieces;
+    const bool is_a = r < kMmaRows;
+    const bool valid = p * 8 < k && (is_a ? row0 + r < m : col0 + r - kMmaRows < n);
+    const __nv_bfloat16* src = is_a ? a + (row0 + r) * lda + p * 8 : w + (col0 + r - kMmaRows) * ldb + p * 8;
+    cp_async16_or_zero(a_s + r * stride + p * 16, valid ? src : a, valid);
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  float acc[2][2][4];
+#pragma unroll
+  for (int t = 0; t < 8; ++t) acc[t >> 2][(t >> 1) & 1][0 + 2 * (t & 1)] = acc[t >> 2][(t >> 1) & 1][1 + 2 * (t & 1)] = 0.f;
+  const uint32_t a_at = a_s + (lane & 15) * stride + (lane >> 4) * 16;
+  const uint32_t w_at = w_s + ((lane & 7) + ((lane >> 4) << 3)) * stride + ((lane >> 3) & 1) * 16;
+#pragma unroll 2
+  for (int ks = warp; ks < steps; ks += kMmaWarps) {
+    uint32_t b[4], x[4], y[4];
+    ldsm4(b, w_at + ks * 32);
+    ldsm4(x, a_at + ks * 32);
+    ldsm4(y, a_at + 16 * stride + ks * 32);
+    mma_16816(acc[0][0], x, b[0], b[1]); mma_16816(acc[0][1], x, b[2], b[3]);
+    mma_16816(acc[1][0], y, b[0], b[1]); mma_16816(acc[1][1], y, b[2], b[3]);
+  }
+  __syncthreads();                                    // the operands are read; their place takes the warps' sums
+  float* red = reinterpret_cast<float*>(smem);        // [warp][row][col]
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; e += 2)
+        *reinterpret_cast<float2*>(red + (warp * kMmaRows + 16 * i + (lane >> 2) + 4 * e) * kMmaCols + 8 * j + (lane & 3) * 2) =
+            make_float2(acc[i][j][e], acc[i][j][e + 1]);
+  __syncthreads();
+  for (int i = threadIdx.x; i < kMmaRows * kMmaCols; i += 32 * kMmaWarps) {
+    const int r = i / kMmaCols, j = i % kMmaCols;
+    float t = 0.f;
+#pragma unroll
+    for (int q = 0; q < kMmaWarps; ++q) t += red[q * kMmaRows * kMmaCols + i];
+    if (row0 + r < m && col0 + j < n) {
+      const long long at = (row0 + r) * ldc + col0 + j;
+      if (c_bf16) static_cast<__nv_bfloat16*>(c)[at] = __float2bfloat16(t);
+      else static_cast<float*>(c)[at] = t;
+    }
+  }
+}
+
 }  // namespace
 
-// Whether the kernel takes this projection: plain operands, rows of at most 1,024 (32 registers of operands a lane and row),
-// and few enough of them: the work grows with M N while the tensor-core tiles stay at the length of their K chain until N
-// fills the chip (64 x 1,536: 16 us here, 10 there).
+// From here on the matrix instructions: 32 x 768 5.3 -> 4.8 us, 24 x 1,536 4.4 -> 3.9; below, the warps a column are faster (24 x 768:
+// 3.5 and 4.8, 64 x 256 over K 1,024: 5.2 and 5.6).
+constexpr long long kMmaFrom = 24 * 1024;
+
+// Whether the kernels take this projection: plain operands, rows of at most 1,024 (32 registers of operands a lane and row),
+// and few enough of them: their work grows with M N while the tensor-core tiles stay at the length of their K chain until N
+// fills the chip.  Here and there, us: 250 x 768 over K 768 7.3 and 10.0, 320 x 768 10.2 and 9.9; 128 x 1,536 over 512 5.9 and 8.1,
+// 250 x 1,536 9.5 and 8.2; 96 x 2,048 over 768 7.9 and 9.7, 128 x 2,048 10.9 and 10.0.
 bool gemm_rows_supported(const moc_gemm_desc* g, const float* row_scale, const int32_t* a_row_blocks,
                          const int32_t* b_row_blocks) {
-  return g->m <= 64 && static_cast<long long>(g->m) * g->n <= 64 * 1024 && g->k <= 1024 && g->a_kmajor && g->b_kmajor && !g->accumulate && g->split_k <= 1 &&
+  return g->m <= 256 && static_cast<long long>(g->m) * g->n <= 192 * 1024 && g->k <= 1024 && g->a_kmajor && g->b_kmajor && !g->accumulate && g->split_k <= 1 &&
          g->residual == nullptr && row_scale == nullptr && a_row_blocks == nullptr && b_row_blocks == nullptr;
 }
 int launch_gemm_rows(const moc_gemm_desc* g, const void* a, const void* b, void* c, cudaStream_t stream) {
+  if (static_cast<long long>(g->m) * g->n >= kMmaFrom) {
+    const int sums = kMmaWarps * kMmaRows * kMmaCols * 4;
+    const int bytes = std::max((kMmaRows + kMmaCols) * mma_stride(g->k), sums);
+    MOC_CUDA_OK(cudaFuncSetAttribute(gemm_rows_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    gemm_rows_mma_kernel<<<dim3(ceil_div(g->n, kMmaCols), ceil_div(g->m, kMmaRows)), 32 * kMmaWarps, bytes, stream>>>(
+        static_cast<const __nv_bfloat16*>(a), g->lda, static_cast<const __nv_bfloat16*>(b), g->ldb, c, g->ldc,
+        g->c_dtype == MOC_BF16, g->m, g->n, g->k);
+    MOC_CUDA_OK(cudaGetLastError());
+    return MOC_OK;
+  }
   auto kern = g->k <= 256 ? gemm_rows_kernel<1> : g->k <= 512 ? gemm_rows_kernel<2>
               : g->k <= 768 ? gemm_rows_kernel<3> : gemm_rows_kernel<4>;
   kern<<<dim3(ceil_div(g->n, kCols), ceil_div(g->m, kRows)), 32 * kCols, 0, stream>>>(
