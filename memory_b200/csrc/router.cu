@@ -634,13 +634,13 @@ select_kernel(const float* __restrict__ logits, long long ld, const float* __res
   select_row<NV, TH>(blockIdx.x, logits, ld, bias, probs, idx, weights, comb_idx, comb_w, row_stats, C, k_sel, S, rho, sm);
 }
 
-// One or two sequences: pooling, logits and selection in one launch, by one cluster of 16 CTAs that meets at its hardware barrier
-// between them (the same sums in the same order as the kernels above).  16 SMs read the router's weights in 6 us where all of
-// them take 3, but what such a call waits for is the host, where three launches are some 10 us.  From three sequences on the products
-// are bound by shared memory and want the whole chip.  The remaining CTAs, clusters of their own, are a projection of as many
-// rows that needs nothing of the routing: the queries of a decoding step, one warp a column.
-// One sequence, window 128, 4,097 chapters, with the queries: 22 us in one launch, 18 in four and the gaps between them; a decoding
-// step 54 -> 46 us, host and device overlapped.
+// A decoding step of one or two sequences, issued by the host: pooling, logits and selection in one launch, by one cluster of 16 CTAs
+// that meets at its hardware barrier between them (the same sums in the same order as the kernels above).  Such a step waits for the
+// host, which needs some 4 us for each launch; on the device 16 SMs take longer than all of them (23 us against 15 for one sequence,
+// 27 against 15 for two, of a window of 128 and 4,097 chapters), so passes that are captured, whose launches cost nothing when they are
+// replayed, and those with work enough to hide the launches keep the kernels above.  The remaining CTAs, clusters of their own,
+// are a projection of as many rows that needs nothing of the routing: the step's queries, one warp a column.
+// One sequence, host and device overlapped: 52 -> 44 us a step, 7 launches -> 4.
 constexpr int kFrontCtas = 16, kFrontRows = 2;
 struct FrontParams {
   float *pooled, *logits, *probs;
@@ -1476,11 +1476,13 @@ int router_fwd_parts_impl(const moc_router_shape* s, const void* h, const float*
   float* loss_partial = ws + (workspace_bytes / sizeof(float) - loss_floats(s));
 
   dim3 pg(B, kPoolSplits);
-  const bool one_launch = (parts & 1) && !(parts & (8 | 16)) && front_takes(s, h, w, pooled);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  const bool one_launch = q != nullptr && (parts & 1) && !(parts & (8 | 16)) && front_takes(s, h, w, pooled) &&
+                          cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
   if (one_launch) {
     FrontParams p{pooled, logits, probs, reinterpret_cast<long long*>(idx), weights, comb_idx, comb_w, row_stats, B, L, d, C, k_sel,
-                  S, s->routed_scale, RowsProduct{}};
-    if (q != nullptr) { p.q = *q; *q_done = true; }
+                  S, s->routed_scale, *q};
+    *q_done = true;
     MOC_TRY(s->h_dtype == MOC_F32 ? launch_front(static_cast<const float*>(h), w, bias, p, stream)
                                   : launch_front(static_cast<const __nv_bfloat16*>(h), w, bias, p, stream));
   }

@@ -66,20 +66,10 @@ def router_selected_k(num_chapters: int, top_k: int, num_shared: int) -> int:
     return max(0, min(int(top_k), int(num_chapters) - int(num_shared)))
 
 
-def _route_launches(batch: int, seq: int, d: int, chapters: int, h_dtype: int) -> int:
-    """Kernels from the states to the selection: one for one or two sequences, else pooling (two above 1,024 positions),
-    logits, selection."""
-    if batch <= 2 and seq <= 1024 and d <= 1024 and d % (4 if h_dtype == L.MOC_F32 else 8) == 0 and chapters <= 9 * 1024:
-        return 1
-    return 3 + int(seq > 1024)
-
-
 def _router_fwd_launches(*a, **k):
-    parts, h, w = k.get("parts", 3), a[0], a[1]
+    parts = k.get("parts", 3)
     with_losses = a[6] if len(a) > 6 else k.get("with_losses")
-    own = k.get("pooled") is not None or k.get("logits") is not None
-    front = 3 if own else _route_launches(h.shape[0], h.shape[1], h.shape[2], w.shape[0], L.dtype_code(h.dtype))
-    return (front if parts & 1 else 0) + (2 if (parts & 2) and with_losses else 0)
+    return (3 if parts & 1 else 0) + (2 if (parts & 2) and with_losses else 0)
 
 
 @_instrument(lambda *a, **k: "router_fwd" if k.get("parts", 3) == 3 else "router_fwd:parts%d" % k["parts"],
@@ -605,8 +595,7 @@ def layer_fwd(s) -> None:
         yield "chapter_row_scale:i32" if s.fused else "gather_rows_fwd:" + _TAG_OF_CODE[s.bank_dtype]
         yield "attn_fwd:bf16"
     casts = int(norm or f32_in) + int((norm or s.add_residual) and not f32_in)
-    route = _route_launches(s.batch, s.router_seq, s.router_dim or s.hidden_dim, s.num_chapters, s.router_dtype)
-    _report(6 + route + 2 * s.with_losses + s.for_backward + casts, parts)
+    _report(9 + int(s.router_seq > 1024) + 2 * s.with_losses + s.for_backward + casts, parts)
 
 
 def layer_bwd(s, b) -> None:
@@ -642,10 +631,7 @@ def route_bwd_scratch_bytes(s) -> int:
 def route_fwd(s) -> None:
     """``moc_route_fwd`` on a filled ``_lib.RouteDesc``."""
     L.check(_timed("router_fwd", lambda: L.lib().moc_route_fwd(C.byref(s))), "moc_route_fwd")
-    r = s.shape
-    route = (3 + int(r.seq > 1024) if s.pos_weight else
-             _route_launches(r.batch, r.seq, r.hidden_dim, r.num_chapters, r.h_dtype))
-    _report(route + 2 * int(bool(s.losses)), lambda: ("router_fwd:" + _TAG_OF_CODE[s.shape.h_dtype],))
+    _report(3 + int(s.shape.seq > 1024) + 2 * int(bool(s.losses)), lambda: ("router_fwd:" + _TAG_OF_CODE[s.shape.h_dtype],))
 
 
 def route_bwd(s, g_w, g_cw, g_losses, d_h, d_w, d_bias, scratch) -> None:
@@ -1327,9 +1313,11 @@ def decode_step(hidden: torch.Tensor, routing_states: torch.Tensor, router_w: to
             L.DecodeShape(b, n_q, num_heads, num_kv_heads, head_dim, num_shared + k, tokens_per_chapter, scale),
             L.dtype_code(h.dtype), wo.shape[0], kv_bank.shape[0], None, None, p(w), p(bias), p(wq), p(wo), p(kv_bank), None,
             None, None, None, None, None, p(L.status_word(dev)), stream, _side_stream(L.device_index(dev), stream), d)
-        route = _route_launches(b, window, rd, c, L.dtype_code(states.dtype))
+        # one or two rows: pooling, logits, selection and the queries in one launch (outside a capture)
+        one = (b * n_q <= 2 and window <= 1024 and max(d, rd) <= 1024 and d % 8 == 0 and c <= 9 * 1024
+               and rd % (4 if states.dtype == torch.float32 else 8) == 0)
         plan = (bytes(s), _size("moc_decode_step_arena_bytes", s), (b, k), (b, num_shared + k), (b, n_q, wo.shape[0]),
-                2 + route + int(route > 1 or b * n_q > 2) + int(h.dtype == torch.float32))
+                3 if one else 5 + int(window <= 1024) + 2 * int(window > 1024) + int(h.dtype == torch.float32))
         if plans is not None:
             if len(plans) >= _DECODE_PLANS_MAX:
                 plans.clear()
