@@ -314,11 +314,13 @@ __global__ void logits_kernel(const float* __restrict__ pooled, const float* __r
 }
 
 // One CTA per batch row: softmax, prefix mask + renormalise, exact top-k, weights, shared prefix.  NV: values per thread
-// (rows of up to TH NV chapters), 0 for longer rows.  Bound by its chain of block-wide steps: at 4,097 chapters, k 64, 16 ->
-// 10 us for a few rows with TH 1,024 against four radix passes over shared memory.  Thousands of rows take CTAs of 256
-// threads, whose barriers are shorter and chains more: 8,192 rows, k 16: 252 us with TH 1,024 -> 152.
-// (The resident CTAs are what the registers allow without the divisions of wide rows, which would take more.)
-constexpr int kBins = 512, kBinBits = 9, kCand = 512;
+// (rows of up to TH NV chapters), 0 for longer rows.  Bound by its chain of block-wide steps for a few rows: at 4,097 chapters,
+// k 64, 16 -> 10 us with TH 1,024 against four radix passes over shared memory.  Thousands of rows take CTAs of 256 threads, whose
+// barriers are shorter and chains more, and are bound by the instructions they issue (91 a value and lane, 2.3 a cycle and SM):
+// tests of the row's end at the loads and stores alone, addresses that are constants behind one pointer, a fourth CTA an SM that the
+// registers then leave room for, lists finished by one warp, candidates ranked as 64-bit words.  8,192 rows of 4,097, k 16: 252 us
+// with TH 1,024, 153 with 256, 112 with these (41 for the bytes); 1,000 rows, k 8: 21 -> 17.  128 threads of 33 values: 120 and 26.
+constexpr int kBins = 512, kBinBits = 9, kCand = 512, kTailCand = 64;
 // (sm: [C] masked probabilities, then [2 k_sel] selection scratch.  Plain pointers: a kernel may have written the logits itself.)
 template <int NV, int TH>
 __device__ __forceinline__ void select_row(const int b, const float* logits, long long ld, const float* bias, float* probs,
@@ -331,8 +333,9 @@ __device__ __forceinline__ void select_row(const int b, const float* logits, lon
   __shared__ int hist[256];
   __shared__ uint32_t s_prefix;
   __shared__ int s_krem, s_count, s_ties;
-  __shared__ int bins[NV > 0 ? kBins : 1], wsum[32], cand_idx[NV > 0 ? kCand : 1];
-  __shared__ uint32_t mm[64], cand_key[NV > 0 ? kCand : 1];
+  __shared__ int bins[NV > 0 ? kBins : 1], wsum[32];
+  __shared__ uint32_t mm[64];
+  __shared__ unsigned long long cand[NV > 0 ? kCand : 1];       // value, then the id's complement: larger is earlier
 
   const float* z = logits + b * ld;       // (bias: not yet in the logits, or nullptr)
   auto logit = [&](int c) { return bias != nullptr ? z[c] + bias[c] : z[c]; };
@@ -342,30 +345,32 @@ __device__ __forceinline__ void select_row(const int b, const float* logits, lon
   // is only made for the radix select.  Sums run in the same order either way.
   constexpr int kN = NV > 0 ? NV : 1;
   float v[kN];
-  float m = -INFINITY, lo = INFINITY;
+  // Columns past the row hold -inf, whose exponential adds nothing: one comparison at the loads instead of one in every pass.
+  const int left = C - static_cast<int>(threadIdx.x);
+  float m = -INFINITY;
   if constexpr (NV > 0) {
+    const float* zt = z + threadIdx.x;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int c = threadIdx.x + i * TH;     // (all loads first: they are independent)
-      v[i] = z[min(c, C - 1)];
-    }
+    for (int i = 0; i < NV; ++i) v[i] = i * TH < left ? zt[i * TH] : -INFINITY;       // (all loads first: they are independent)
     if (bias != nullptr) {
+      const float* bt = bias + threadIdx.x;
 #pragma unroll
-      for (int i = 0; i < NV; ++i) v[i] += bias[min(static_cast<int>(threadIdx.x) + i * TH, C - 1)];
+      for (int i = 0; i < NV; ++i)
+        if (i * TH < left) v[i] += bt[i * TH];
     }
 #pragma unroll
-    for (int i = 0; i < NV; ++i) { m = fmaxf(m, v[i]); lo = fminf(lo, v[i]); }       // (a repeated last entry changes neither)
+    for (int i = 0; i < NV; ++i) m = fmaxf(m, v[i]);
   } else {
     for (int c = threadIdx.x; c < C; c += blockDim.x) m = fmaxf(m, logit(c));
   }
   m = block_max(m, red[0]);
-  // A thread whose smallest exponential may lie below 2^-83 divides.  Both quotients below stay within what `quotient` is
+  // A thread with an exponential below 2^-83 (other than zero) divides.  Both quotients below stay within what `quotient` is
   // exact for otherwise: the exponentials, and those over a sum of at most 2^14.  (8,192 rows of 4,097 chapters: 157 us
   // without the test, 161 with it, 184 with a test of every value on its own.)
-  const bool wide = lo - m < -57.5f;
+  uint32_t least = 0xFFFFFFFFu;
   auto divide = [&](float d) {             // v[i] = v[i] / d
     if constexpr (NV > 0) {
-      if (wide) {
+      if (least < (static_cast<uint32_t>(127 - 83) << 23) - 1u) {
 #pragma unroll
         for (int i = 0; i < NV; ++i) v[i] = v[i] / d;
       } else {
@@ -378,8 +383,11 @@ __device__ __forceinline__ void select_row(const int b, const float* logits, lon
   float s = 0.f;
   if constexpr (NV > 0) {
 #pragma unroll
-    for (int i = 0; i < NV; ++i)
-      if (threadIdx.x + i * TH < C) { v[i] = expf(v[i] - m); s += v[i]; }
+    for (int i = 0; i < NV; ++i) {
+      v[i] = expf(v[i] - m);
+      s += v[i];
+      least = min(least, __float_as_uint(v[i]) - 1u);       // (zero wraps around)
+    }
   } else {
     for (int c = threadIdx.x; c < C; c += blockDim.x) {
       const float e = expf(logit(c) - m);
@@ -391,15 +399,17 @@ __device__ __forceinline__ void select_row(const int b, const float* logits, lon
   float ms = 0.f;
   if constexpr (NV > 0) {
     divide(denom);
+    float* ptr = p + threadIdx.x;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int c = threadIdx.x + i * TH;
-      if (c < C) {
-        p[c] = v[i];
-        if (c < S) v[i] = 0.f;
-        ms += v[i];
-      }
+    for (int i = 0; i < NV; ++i)
+      if (i * TH < left) ptr[i * TH] = v[i];
+    if (S > 0) {
+#pragma unroll
+      for (int i = 0; i < NV; ++i)
+        if (static_cast<int>(threadIdx.x) + i * TH < S) v[i] = 0.f;
     }
+#pragma unroll
+    for (int i = 0; i < NV; ++i) ms += v[i];
   } else {
     for (int c = threadIdx.x; c < C; c += blockDim.x) {
       const float pv = pt[c] / denom;
@@ -409,17 +419,28 @@ __device__ __forceinline__ void select_row(const int b, const float* logits, lon
       ms += pm;
     }
   }
-  const float masked_mass = block_sum(ms, red[2]);
-  const float dn0 = fmaxf(masked_mass, 1e-12f);
-  if constexpr (NV > 0) {
-    if (S > 0) divide(dn0);
+  // without shared chapters nothing waits for this sum: its second half runs at the end, past the barriers in between
+  const bool late_mass = NV > 0 && S == 0 && k_sel > 0;
+  float masked_mass = 0.f;
+  if (late_mass) {
+    ms = warp_sum(ms);
+    if ((threadIdx.x & 31) == 0) red[2][threadIdx.x >> 5] = ms;
   } else {
-    if (S > 0)
-      for (int c = threadIdx.x; c < C; c += blockDim.x) pt[c] = pt[c] / dn0;
+    masked_mass = block_sum(ms, red[2]);
+    const float dn0 = fmaxf(masked_mass, 1e-12f);
+    if constexpr (NV > 0) {
+      if (S > 0) divide(dn0);
+    } else {
+      if (S > 0)
+        for (int c = threadIdx.x; c < C; c += blockDim.x) pt[c] = pt[c] / dn0;
+    }
+    __syncthreads();
   }
-  __syncthreads();
 
   float topk_mass = 0.f, comb_mass = static_cast<float>(S);
+  // Lists of up to 32 entries are finished by the first warp alone, without barriers (the sums of the other warps are zero).
+  int step = blockDim.x;
+  auto tail_sum = [&](float x, float* r) { return step == 32 ? warp_sum(x) : block_sum(x, r); };
   if (k_sel > 0) {
     float* srt_w = sm;                         // sorted: weight and id, over p~ (no longer needed by then)
     int* srt_i = reinterpret_cast<int*>(sm + k_sel);
@@ -432,10 +453,7 @@ __device__ __forceinline__ void select_row(const int b, const float* logits, lon
       constexpr int kPer = kBins / TH > 2 ? kBins / TH : 2, kOwners = kBins / kPer, kWarps = TH / 32;
       uint32_t top = 0u;
 #pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        const int c = threadIdx.x + i * TH;
-        if (c < C && c >= S) top = max(top, __float_as_uint(v[i]));
-      }
+      for (int i = 0; i < NV; ++i) top = max(top, __float_as_uint(v[i]));       // (zero past the row and for shared chapters)
       uint32_t lo = __reduce_min_sync(0xffffffffu, top), hi = __reduce_max_sync(0xffffffffu, top);
       for (int i = threadIdx.x; i < kBins; i += TH) bins[i] = 0;
       if (lane == 0) { mm[warp] = lo; mm[32 + warp] = hi; }
@@ -474,20 +492,27 @@ __device__ __forceinline__ void select_row(const int b, const float* logits, lon
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
           const int c = threadIdx.x + i * TH;
-          if (c < C && c >= S && __float_as_uint(v[i]) >= edge) {
+          if (__float_as_uint(v[i]) >= edge && c < C && c >= S) {
             const int pos = atomicAdd(&s_count, 1);
-            if (pos < kCand) { cand_key[pos] = __float_as_uint(v[i]); cand_idx[pos] = c; }
+            if (pos < kCand) cand[pos] = static_cast<unsigned long long>(__float_as_uint(v[i])) << 32 | ~static_cast<uint32_t>(c);
           }
         }
         __syncthreads();
         const int n = s_count;
         if (n >= k_sel && n <= kCand) {
-          for (int t = threadIdx.x; t < n; t += TH) {
-            const uint32_t kt = cand_key[t];
-            const int it = cand_idx[t];
+          if (n <= kTailCand && S + k_sel <= 32) {
+            if (warp > 0) return;
+            step = 32;
+          }
+          for (int t = threadIdx.x; t < n; t += step) {
+            const unsigned long long mine = cand[t];
             int rank = 0;
-            for (int j = 0; j < n; ++j) rank += (cand_key[j] > kt) || (cand_key[j] == kt && cand_idx[j] < it);
-            if (rank < k_sel) { srt_w[rank] = __uint_as_float(kt); srt_i[rank] = it; }
+#pragma unroll 4
+            for (int j = 0; j < n; ++j) rank += cand[j] > mine;
+            if (rank < k_sel) {
+              srt_w[rank] = __uint_as_float(static_cast<uint32_t>(mine >> 32));
+              srt_i[rank] = ~static_cast<uint32_t>(mine);
+            }
           }
           selected = true;
         }
@@ -497,7 +522,7 @@ __device__ __forceinline__ void select_row(const int b, const float* logits, lon
         for (int i = 0; i < NV; ++i)
           if (threadIdx.x + i * TH < C) pt[threadIdx.x + i * TH] = v[i];
       }
-      __syncthreads();
+      if (step == 32) __syncwarp(); else __syncthreads();
     }
     if (!selected) {
     // radix select on the fp32 bit pattern (non-negative values order like unsigned integers)
@@ -591,25 +616,27 @@ __device__ __forceinline__ void select_row(const int b, const float* logits, lon
     __syncthreads();
     }
     float part = 0.f;
-    for (int j = threadIdx.x; j < k_sel; j += blockDim.x) part += srt_w[j];
-    topk_mass = block_sum(part, red[3]);
+    for (int j = threadIdx.x; j < k_sel; j += step) part += srt_w[j];
+    topk_mass = tail_sum(part, red[3]);
     const float dn = fmaxf(topk_mass, 1e-12f);
     long long* out_idx = idx + static_cast<long long>(b) * k_sel;
     float* out_w = weights + static_cast<long long>(b) * k_sel;
     float cpart = 0.f;
-    for (int j = threadIdx.x; j < k_sel; j += blockDim.x) {
+    for (int j = threadIdx.x; j < k_sel; j += step) {
       const float wj = srt_w[j] / dn;
       srt_w[j] = wj;
       out_w[j] = wj;
       out_idx[j] = srt_i[j];
       cpart += wj * rho;
     }
-    comb_mass = static_cast<float>(S) + block_sum(cpart, red[4]);
+    comb_mass = static_cast<float>(S) + tail_sum(cpart, red[4]);
+    if (step == 32) __syncwarp();
   }
+  if (late_mass) masked_mass = warp_sum(static_cast<int>(threadIdx.x) < TH / 32 ? red[2][threadIdx.x & 31] : 0.f);   // (read by thread 0)
   // shared prefix + renormalised combined weights (only meaningful when S > 0; with S == 0 the
   // combined lists are the routed lists unchanged)
   const int kc = S + k_sel;
-  for (int j = threadIdx.x; j < kc; j += blockDim.x) {
+  for (int j = threadIdx.x; j < kc; j += step) {
     int ci; float u;
     if (j < S) { ci = j; u = 1.f; }
     else { ci = reinterpret_cast<int*>(sm + k_sel)[j - S]; u = sm[j - S] * (S > 0 ? rho : 1.f); }
@@ -626,7 +653,7 @@ __device__ __forceinline__ void select_row(const int b, const float* logits, lon
   }
 }
 template <int NV, int TH>
-__global__ void __launch_bounds__(TH, TH == 256 ? (NV > 17 ? 2 : NV > 5 ? 3 : 6) : (NV > 5 ? 1 : 2))
+__global__ void __launch_bounds__(TH, TH == 256 ? (NV > 17 ? 2 : NV > 5 ? 4 : 6) : (NV > 5 ? 1 : 2))
 select_kernel(const float* __restrict__ logits, long long ld, const float* __restrict__ bias, float* __restrict__ probs, long long* __restrict__ idx,
               float* __restrict__ weights, int* __restrict__ comb_idx, float* __restrict__ comb_w,
               float* __restrict__ row_stats, int C, int k_sel, int S, float rho) {
@@ -941,20 +968,22 @@ __global__ void col_sum_kernel(const float* __restrict__ x, float* __restrict__ 
 }
 
 // ---- backward --------------------------------------------------------------------------------
-// One CTA per batch row: gradient of everything downstream of the logits.
-// One CTA per row; terms != nullptr: the gradient leaves as three bf16 terms ([3][B][ld], zeros behind column C), what the
-// products that follow on the tensor cores read.
+// One CTA per row: gradient of everything downstream of the logits.  TERMS: the gradient leaves as three bf16 terms ([3][B][ld],
+// zeros behind column C), what the products that follow on the tensor cores read.
 // NV > 0: the row's probabilities stay in registers (rows of up to TH NV chapters), all loads in flight together.  8,192 rows
-// of 4,097: 227 us with TH 1,024, a pad copy of 93 us and a pass of 133 us into the terms -> 147 us in all.
-template <int NV, int TH>
-__global__ void __launch_bounds__(TH)
+// of 4,097: 227 us with TH 1,024, a pad copy of 93 us and a pass of 133 us into the terms -> 138 us in all.  Those issued 89
+// instructions a value and lane: with the layout of the columns known to the compiler, no test of the row's end but at the loads,
+// and the sums over the list left to one warp while the others load, 80 us (52 for the bytes); 1,000 rows, k 8: 23 -> 14.
+template <int NV, int TH, bool TERMS>
+__global__ void __launch_bounds__(TH, TH == 256 ? 4 : 1)
 dlogits_kernel(const float* __restrict__ probs, const long long* __restrict__ idx,
                const float* __restrict__ weights, const float* __restrict__ comb_w,
                const float* __restrict__ row_stats, const float* __restrict__ chapter_stats,
                const float* __restrict__ d_weights, const float* __restrict__ d_comb_w,
                const float* __restrict__ d_losses, float* __restrict__ d_logits, __nv_bfloat16* __restrict__ terms, int ld,
                int B, int C, int k_sel, int S, float rho) {
-  extern __shared__ float dp[];   // [C]
+  extern __shared__ float4 dp_smem[];
+  float* dp = reinterpret_cast<float*>(dp_smem);        // [NV TH], or [C]
   __shared__ float red[5][32];
   __shared__ float s_dv[1024];    // k_sel <= 1024
   const int b = blockIdx.x;
@@ -965,44 +994,57 @@ dlogits_kernel(const float* __restrict__ probs, const long long* __restrict__ id
   const float g_z = d_losses ? d_losses[2] : 0.f, g_ent = d_losses ? d_losses[3] : 0.f;
   const int kc = S + k_sel;
 
-  float pr[NV > 0 ? NV : 1];
-  // terms go out in pairs of columns, so a thread owns pairs; single columns otherwise
+  // A thread's columns: pairs where terms go out in pairs, single ones otherwise.  Past the row the probabilities are zero.
   constexpr int kN = NV > 0 ? NV : 1;
-  auto col = [&](int i) {
-    return terms != nullptr ? 2 * static_cast<int>(threadIdx.x) + (i & 1) + (i >> 1) * 2 * TH : static_cast<int>(threadIdx.x) + i * TH;
-  };
+  float pr[kN], g[kN];
+  const int first = TERMS ? 2 * static_cast<int>(threadIdx.x) : static_cast<int>(threadIdx.x), left = C - first;
+  auto off = [](int i) { return TERMS ? (i & 1) + (i >> 1) * 2 * TH : i * TH; };
   if constexpr (NV > 0) {
+    const float* pt = p + first;
 #pragma unroll
-    for (int i = 0; i < kN; ++i) pr[i] = p[min(col(i), C - 1)];
+    for (int i = 0; i < kN; ++i) pr[i] = off(i) < left ? pt[off(i)] : 0.f;
   }
   // (a)+(b): gradients of the k selected (unnormalised) masked probabilities v_j
   __shared__ float s_w[1024];
-  float dotu_p = 0.f;
-  if (d_comb_w != nullptr && S > 0)
-    for (int i = threadIdx.x; i < kc; i += blockDim.x)
-      dotu_p += d_comb_w[static_cast<long long>(b) * kc + i] * comb_w[static_cast<long long>(b) * kc + i];
-  const float dotu = (d_comb_w != nullptr && S > 0) ? block_sum(dotu_p, red[0]) : 0.f;
-  float dotw_p = 0.f;
-  for (int j = threadIdx.x; j < k_sel; j += blockDim.x) {
-    float dw = d_weights ? d_weights[static_cast<long long>(b) * k_sel + j] : 0.f;
-    if (d_comb_w != nullptr) {
-      const float dcu = d_comb_w[static_cast<long long>(b) * kc + S + j];
-      if (S > 0) dw += rho * ((u_mass >= 1e-12f) ? (dcu - dotu) / u_mass : dcu / 1e-12f);
-      else dw += dcu;
+  const bool one_warp = kc <= 32;        // the first warp takes these sums alone, the others go on
+  float A = 0.f;
+  long long my_idx = 0;
+  if (!one_warp || threadIdx.x < 32) {
+    const int step = one_warp ? 32 : static_cast<int>(blockDim.x);
+    auto list_sum = [&](float x, float* r) { return one_warp ? warp_sum(x) : block_sum(x, r); };
+    if (one_warp && static_cast<int>(threadIdx.x) < k_sel) my_idx = idx[static_cast<long long>(b) * k_sel + threadIdx.x];
+    float dotu_p = 0.f;
+    if (d_comb_w != nullptr && S > 0)
+      for (int i = threadIdx.x; i < kc; i += step)
+        dotu_p += d_comb_w[static_cast<long long>(b) * kc + i] * comb_w[static_cast<long long>(b) * kc + i];
+    const float dotu = (d_comb_w != nullptr && S > 0) ? list_sum(dotu_p, red[0]) : 0.f;
+    float dotw_p = 0.f;
+    for (int j = threadIdx.x; j < k_sel; j += step) {
+      float dw = d_weights ? d_weights[static_cast<long long>(b) * k_sel + j] : 0.f;
+      if (d_comb_w != nullptr) {
+        const float dcu = d_comb_w[static_cast<long long>(b) * kc + S + j];
+        if (S > 0) dw += rho * ((u_mass >= 1e-12f) ? (dcu - dotu) / u_mass : dcu / 1e-12f);
+        else dw += dcu;
+      }
+      const float wj = weights[static_cast<long long>(b) * k_sel + j];
+      s_dv[j] = dw;
+      s_w[j] = wj;
+      dotw_p += dw * wj;
     }
-    const float wj = weights[static_cast<long long>(b) * k_sel + j];
-    s_dv[j] = dw;
-    s_w[j] = wj;
-    dotw_p += dw * wj;
+    const float dotw = list_sum(dotw_p, red[1]);
+    float a_p = 0.f;
+    for (int j = threadIdx.x; j < k_sel; j += step) {
+      const float dv = (v_mass >= 1e-12f) ? (s_dv[j] - dotw) / v_mass : s_dv[j] / 1e-12f;
+      s_dv[j] = dv;
+      a_p += dv * (s_w[j] * fmaxf(v_mass, 1e-12f));   // v_j
+    }
+    A = list_sum(a_p, red[2]);
   }
-  const float dotw = block_sum(dotw_p, red[1]);
-  float a_p = 0.f;
-  for (int j = threadIdx.x; j < k_sel; j += blockDim.x) {
-    const float dv = (v_mass >= 1e-12f) ? (s_dv[j] - dotw) / v_mass : s_dv[j] / 1e-12f;
-    s_dv[j] = dv;
-    a_p += dv * (s_w[j] * fmaxf(v_mass, 1e-12f));   // v_j
+  if (one_warp && S > 0) {               // (only shared chapters make the sum a part of every column)
+    if (threadIdx.x == 0) red[4][0] = A;
+    __syncthreads();
+    A = red[4][0];
   }
-  const float A = block_sum(a_p, red[2]);
   const bool renorm = (S > 0);
   const float inv_s = renorm ? ((s_mass >= 1e-12f) ? 1.f / s_mass : 1e12f) : 1.f;
   const float dense = (renorm && s_mass >= 1e-12f) ? -A * inv_s : 0.f;
@@ -1015,66 +1057,86 @@ dlogits_kernel(const float* __restrict__ probs, const long long* __restrict__ id
     if (g_ent != 0.f) g += g_ent * (-invB) * (logf(fmaxf(pv, 1e-12f)) + (pv > 1e-12f ? 1.f : 0.f));
     return g;
   };
-  if (NV > 0 && g_aux == 0.f && g_ent == 0.f) {          // the usual losses; all loads first, they are independent
-    float f[kN];
+  if constexpr (NV > 0) {
+    if (g_aux == 0.f && g_ent == 0.f) {          // the usual losses; all loads first, they are independent
+      const float* ft = chapter_stats + first;
 #pragma unroll
-    for (int i = 0; i < kN; ++i) f[i] = 0.f;
-    if (g_lb != 0.f) {
+      for (int i = 0; i < kN; ++i) g[i] = 0.f;
+      if (g_lb != 0.f) {
 #pragma unroll
-      for (int i = 0; i < kN; ++i) f[i] = chapter_stats[min(col(i), C - 1)];
+        for (int i = 0; i < kN; ++i) g[i] = off(i) < left ? ft[off(i)] : 0.f;
+#pragma unroll
+        for (int i = 0; i < kN; ++i) g[i] = g_lb * static_cast<float>(C) * g[i] * invB;
+      }
+      if (S > 0) {
+#pragma unroll
+        for (int i = 0; i < kN; ++i) g[i] += first + off(i) >= S && off(i) < left ? dense : 0.f;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < kN; ++i) g[i] = off(i) < left ? dense_grad(first + off(i), pr[i]) : 0.f;
     }
+    if constexpr (TERMS) {
 #pragma unroll
-    for (int i = 0; i < kN; ++i)
-      if (col(i) < C) dp[col(i)] = (col(i) >= S ? dense : 0.f) + g_lb * static_cast<float>(C) * f[i] * invB;
-  } else if constexpr (NV > 0) {
+      for (int i = 0; i < kN; i += 2) *reinterpret_cast<float2*>(dp + first + off(i)) = make_float2(g[i], g[i + 1]);
+    } else {
 #pragma unroll
-    for (int i = 0; i < kN; ++i)
-      if (col(i) < C) dp[col(i)] = dense_grad(col(i), pr[i]);
+      for (int i = 0; i < kN; ++i) dp[first + off(i)] = g[i];
+    }
   } else {
     for (int c = threadIdx.x; c < C; c += blockDim.x) dp[c] = dense_grad(c, p[c]);
   }
   __syncthreads();
   for (int j = threadIdx.x; j < k_sel; j += blockDim.x) {
-    const int c = static_cast<int>(idx[static_cast<long long>(b) * k_sel + j]);
+    const int c = static_cast<int>(one_warp ? my_idx : idx[static_cast<long long>(b) * k_sel + j]);
     dp[c] += s_dv[j] * inv_s;    // chapter ids in one row are distinct
   }
   __syncthreads();
   float dot = 0.f;
   if constexpr (NV > 0) {
+    if constexpr (TERMS) {
 #pragma unroll
-    for (int i = 0; i < kN; ++i)
-      if (col(i) < C) dot += dp[col(i)] * pr[i];
+      for (int i = 0; i < kN; i += 2) {
+        const float2 x = *reinterpret_cast<const float2*>(dp + first + off(i));
+        g[i] = x.x; g[i + 1] = x.y;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < kN; ++i) g[i] = dp[first + off(i)];
+    }
+#pragma unroll
+    for (int i = 0; i < kN; ++i) dot += g[i] * pr[i];
   } else {
     for (int c = threadIdx.x; c < C; c += blockDim.x) dot += dp[c] * p[c];
   }
   dot = block_sum(dot, red[3]);
   const float zc = g_z * 2.f * lse * invB;
-  if (terms != nullptr) {
+  if constexpr (TERMS) {
     const long long stride = static_cast<long long>(B) * ld;
-    __nv_bfloat162* t0 = reinterpret_cast<__nv_bfloat162*>(terms + static_cast<long long>(b) * ld);
-    auto emit = [&](int c, float x, float y) {
-#pragma unroll
-      for (int t = 0; t < 3; ++t) {
-        const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
-        t0[(t * stride + c) / 2] = v;
-        x -= __low2float(v); y -= __high2float(v);
-      }
+    __nv_bfloat16* t0 = terms + static_cast<long long>(b) * ld + first;
+    __nv_bfloat16 *t1 = t0 + stride, *t2 = t1 + stride;
+    auto emit = [&](int o, float x, float y) {            // (o: columns behind the thread's first)
+      const __nv_bfloat162 u = __floats2bfloat162_rn(x, y);
+      x -= __low2float(u); y -= __high2float(u);
+      const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+      x -= __low2float(v); y -= __high2float(v);
+      *reinterpret_cast<__nv_bfloat162*>(t0 + o) = u;
+      *reinterpret_cast<__nv_bfloat162*>(t1 + o) = v;
+      *reinterpret_cast<__nv_bfloat162*>(t2 + o) = __floats2bfloat162_rn(x, y);
     };
-    auto grad = [&](int c, float pv) { return c < C ? pv * (dp[c] - dot + zc) : 0.f; };
     if constexpr (NV > 0) {
 #pragma unroll
-      for (int i = 0; i + 1 < kN; i += 2)
-        if (col(i) < ld) emit(col(i), grad(col(i), pr[i]), grad(col(i + 1), pr[i + 1]));
+      for (int i = 0; i < kN; i += 2)
+        if (off(i) < ld - first) emit(off(i), pr[i] * (g[i] - dot + zc), pr[i + 1] * (g[i + 1] - dot + zc));
     } else {
-      for (int c = 2 * threadIdx.x; c < ld; c += 2 * TH)
-        emit(c, grad(c, p[min(c, C - 1)]), grad(c + 1, p[min(c + 1, C - 1)]));
+      auto grad = [&](int c) { return c < C ? p[c] * (dp[c] - dot + zc) : 0.f; };
+      for (int c = first; c < ld; c += 2 * TH) emit(c - first, grad(c), grad(c + 1));
     }
-    return;
-  }
-  if constexpr (NV > 0) {
+  } else if constexpr (NV > 0) {
+    float* dst = d_logits + static_cast<long long>(b) * C + first;
 #pragma unroll
     for (int i = 0; i < kN; ++i)
-      if (col(i) < C) d_logits[static_cast<long long>(b) * C + col(i)] = pr[i] * (dp[col(i)] - dot + zc);
+      if (off(i) < left) dst[off(i)] = pr[i] * (g[i] - dot + zc);
   } else {
     for (int c = threadIdx.x; c < C; c += blockDim.x)
       d_logits[static_cast<long long>(b) * C + c] = p[c] * (dp[c] - dot + zc);
@@ -1256,13 +1318,16 @@ int launch_dlogits(const float* probs, const int64_t* idx, const float* weights,
                    const float* chapter_stats, const float* d_weights, const float* d_comb_w, const float* d_losses,
                    float* d_logits, __nv_bfloat16* terms, int ld, int B, int C, int k_sel, int S, float rho,
                    cudaStream_t stream) {
-  const size_t sm = static_cast<size_t>(C) * 4;
   const int cols = terms != nullptr ? ld : C;
   // In registers up to 18 values a thread of 256, 6 of 1,024.  More is no gain: with 34 of 256 the two CTAs an SM take as long
   // as the general kernel (8,192 rows of 8,193 chapters: 493 and 494 us; 1,024 rows: 61 and 49), with 9 of 1,024 too (8 rows:
   // 23 us either way).
   const bool small = B >= kManyRows && cols <= 18 * 256;
-  auto kern = small ? dlogits_kernel<18, 256> : cols <= 6 * 1024 ? dlogits_kernel<6, 1024> : dlogits_kernel<0, 1024>;
+  const bool held = small || cols <= 6 * 1024;
+  const size_t sm = (small ? 18 * 256 : held ? 6 * 1024 : static_cast<size_t>(C)) * 4;
+  auto kern = terms != nullptr
+                  ? (small ? dlogits_kernel<18, 256, true> : held ? dlogits_kernel<6, 1024, true> : dlogits_kernel<0, 1024, true>)
+                  : (small ? dlogits_kernel<18, 256, false> : held ? dlogits_kernel<6, 1024, false> : dlogits_kernel<0, 1024, false>);
   MOC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm)));
   kern<<<B, small ? 256 : 1024, sm, stream>>>(probs, reinterpret_cast<const long long*>(idx), weights, comb_w, row_stats,
                                               chapter_stats, d_weights, d_comb_w, d_losses, d_logits, terms, ld, B, C, k_sel, S,
