@@ -417,10 +417,12 @@ token_mix_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
 }
 
 // out[t] = base[t] + sum_s partial[t, s] in slot order, fp32 sums; one thread per 8 elements.  Slots whose chapter
-// id is out of range were never written and are skipped.
+// id is out of range were never written and count as zero.  Bound by HBM (8,192 rows of 16 slots, 12 heads: 31 us for the bytes):
+// 53.5 us with a slot's load behind the one before, 46 with four in flight, 53 with eight (registers).
 __global__ void slot_reduce_kernel(const __nv_bfloat16* __restrict__ partial, const __nv_bfloat16* __restrict__ base,
                                    const int* __restrict__ idx, __nv_bfloat16* __restrict__ out, long long rows,
                                    int S, int HQ, int HK, int HI, int M) {
+  constexpr int kBatch = 4;            // slots whose loads are in flight together
   const int chunks = HQ * (kD / 8);
   const long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   if (t >= rows * chunks) return;
@@ -440,15 +442,23 @@ __global__ void slot_reduce_kernel(const __nv_bfloat16* __restrict__ partial, co
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i] = 0.f;
   }
-  for (int s = 0; s < S; ++s) {
-    const int c = idx[(row * HI + hi) * S + s];
-    if (c < 0 || c >= M) continue;
-    const uint4 v = reinterpret_cast<const uint4*>(partial)[(row * S + s) * chunks + ch];
-    const uint32_t wd[4] = {v.x, v.y, v.z, v.w};
+  const int* ids = idx + (row * HI + hi) * S;
+  const uint4* src = reinterpret_cast<const uint4*>(partial) + row * S * chunks + ch;
+  for (int s0 = 0; s0 < S; s0 += kBatch) {
+    uint4 v[kBatch];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      acc[2 * i] += __uint_as_float(wd[i] << 16);
-      acc[2 * i + 1] += __uint_as_float(wd[i] & 0xFFFF0000u);
+    for (int s = 0; s < kBatch; ++s) {
+      const int c = s0 + s < S ? ids[s0 + s] : -1;
+      v[s] = c >= 0 && c < M ? src[static_cast<long long>(s0 + s) * chunks] : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int s = 0; s < kBatch; ++s) {
+      const uint32_t wd[4] = {v[s].x, v[s].y, v[s].z, v[s].w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        acc[2 * i] += __uint_as_float(wd[i] << 16);
+        acc[2 * i + 1] += __uint_as_float(wd[i] & 0xFFFF0000u);
+      }
     }
   }
   uint4 o;
