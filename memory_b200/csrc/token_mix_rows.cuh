@@ -393,7 +393,9 @@ token_mix_rows_bwd_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
       const uint32_t k_s = kv_s + (n & 1) * 2 * kTileKV;         // (V behind it)
       const uint32_t do_s = rows_s + buf * 2 * kRowBwdBytes;     // (Q behind it)
       const uint32_t pt = pt_s + buf * 2 * kPairBytes;
-      const int halves = st.pairs > 16 ? 2 : 1;                  // 16-pair halves of the step that hold pairs
+      // 16-pair halves of the step that hold pairs.  None where a wait ran out: the step's record and rows may never have been
+      // written, so nothing of them is read or stored on the way to the meeting below, where every warp is awaited.
+      const int halves = !ok ? 0 : st.pairs > 16 ? 2 : 1;
       // S^T and dP^T: 64 keys x 8 pairs a warp; this lane's keys are 16 m + g8 and that + 8, its pairs c2 and the next
       if (warp < 2 * halves) {
         float sc[4][4], dp[4][4];
@@ -461,7 +463,7 @@ token_mix_rows_bwd_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
         }
       }
       // Pw^T and dS^T are complete; the step before last, whose buffers these are, was done with two such barriers ago
-      if (!warps_agree<1, 128>(ok)) break;
+      if (!warps_agree<1, 128>(halves > 0)) break;
       // dQ = dS K: 16 pairs x 32 columns a warp
       if ((warp & 1) < halves) {
         float dq[4][4];

@@ -20,6 +20,28 @@ def test_row_warps_of_the_token_mixture_leave_their_loop_at_the_barrier_only():
     assert exits == meets[1:], "a way out that another warp need not take"
 
 
+def test_a_step_whose_wait_ran_out_is_neither_read_nor_stored():
+    """Backward of chapters with few pairs: the record of a step (where its results go) and its rows are written by another warp, so
+    between the waits for them and the meeting of the warps everything that looks at them is under the outcome of the waits."""
+    text = open(os.path.join(CSRC, "token_mix_rows.cuh")).read()
+    kernel = text[text.index("token_mix_rows_bwd_kernel("):]
+    loop = kernel[kernel.index("bool ok = mbar_wait_w(&full[buf]"):]
+    meeting = "if (!warps_agree<1, 128>(halves > 0)) break;"
+    assert loop.count("warps_agree") == loop.count(meeting) == 1
+    way, behind = loop.split(meeting)
+    assert "const int halves = !ok ? 0 : st.pairs > 16 ? 2 : 1;" in way
+    start = way.index("if (warp < 2 * halves) {")
+    depth = 0
+    for end in range(way.index("{", start), len(way)):
+        depth += {"{": 1, "}": -1}.get(way[end], 0)
+        if depth == 0:
+            break
+    assert "p.d_w_heads[st.dw_at" in way[start:end]
+    rest = re.sub(r"//[^\n]*", "", way[:start] + way[end + 1:]).replace("!ok ? 0 : st.pairs > 16 ? 2 : 1", "")
+    assert not re.search(r"\bst\.|ldsm|stsm|\bp\.(?!status\b|dkv_ld\b)", rest), rest
+    assert not re.search(r"\b(break|continue|goto)\b|\breturn;", way) and "break" not in behind[:behind.index("__syncthreads();")]
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("late", [0, 1, 8, 6, 15])
 def test_warps_agree_about_their_waits(late):
