@@ -445,6 +445,9 @@ token_mix_rows_bwd_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
           if (st.out_at[at + 1] >= 0) p.d_w_heads[st.dw_at[at + 1]] = x.out_scale * d1;
         }
         const uint64_t minus = f2_pack(-d0, -d1);
+        // Columns of the step without a pair are zero whatever their products gave: against an infinite key their zero rows give NaN,
+        // which the sums over the chapter's pairs would spread to all of its keys.
+        const uint32_t keep = (at < st.pairs ? 0xFFFFu : 0u) | (at + 1 < st.pairs ? 0xFFFF0000u : 0u);
 #pragma unroll
         for (int m = 0; m < 4; m += 2) {
           uint32_t a[4], d[4];
@@ -454,9 +457,9 @@ token_mix_rows_bwd_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
             const uint64_t pw = f2_mul(wt, f2_pack(sc[mm][c], sc[mm][c + 1]));
             float v0, v1;
             f2_unpack(pw, v0, v1);
-            a[i] = pack_bf16x2(v0, v1);
+            a[i] = pack_bf16x2(v0, v1) & keep;
             f2_unpack(f2_mul(pw, f2_add(f2_pack(dp[mm][c], dp[mm][c + 1]), minus)), v0, v1);
-            d[i] = pack_bf16x2(v0, v1);
+            d[i] = pack_bf16x2(v0, v1) & keep;
           }
           stsm4(pt + pt_to + m * 1024, a[0], a[1], a[2], a[3]);
           stsm4(pt + kPairBytes + pt_to + m * 1024, d[0], d[1], d[2], d[3]);

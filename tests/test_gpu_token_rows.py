@@ -44,3 +44,31 @@ def test_bucket_sizes(name, lists, heads):
     assert not dk[:, len(counts) * 64:].any() and not dv[:, len(counts) * 64:].any()
     again = ops.token_mix_bwd(*d, lse, do.to(dev), 0.125, 2.5, ws, dk2 := torch.empty_like(dk), dv2 := torch.empty_like(dv))
     assert torch.equal(dq, again[0]) and torch.equal(dw, again[1]) and torch.equal(dk, dk2) and torch.equal(dv, dv2)
+
+
+@pytest.mark.parametrize("pairs", [1, 5, 16, 17, 33, 511, 512, 700])
+@pytest.mark.parametrize("heads", [(2, 2), (6, 2)], ids=["mha", "gqa"])
+def test_an_infinite_key_stays_with_its_own_gradients(pairs, heads):
+    """A key whose score is -inf for every pair has weight 0: forward, dV, dW and the dK of the chapter's other keys are what they are
+    without it, whatever stands in the part of a step or tile that holds no pair.  (dQ is NaN by the product 0 * inf.)"""
+    from memory_b200 import _lib as L, ops
+    dev = torch.device("cuda:0")
+    hq, h = heads
+    g = torch.Generator().manual_seed(pairs)
+    q, do = (torch.randn(1, pairs, hq, 64, generator=g).bfloat16() for _ in range(2))
+    k, v = (torch.randn(1, 64, h, 64, generator=g).bfloat16() for _ in range(2))
+    q[..., 3] = -q[..., 3].abs() - 0.125
+    k[0, 7, :, 3] = float("inf")
+    bi, w = torch.zeros(1, pairs, 1, 1, dtype=torch.int32), torch.rand(1, pairs, 1, generator=g) + 0.1
+    qc, kc, vc, wc = (t.float().requires_grad_(True) for t in (q, k, v, w))
+    ref = O.weighted_chapter_attention(qc, kc, vc, bi.expand(1, pairs, h, 1), wc, 64)
+    ref.backward(do.float())
+    d = [t.to(dev) for t in (q, k, v, bi, w)]
+    o, lse, ws = ops.token_mix_fwd(*d, 0.125)
+    dk, dv = (torch.full_like(t, float("nan")) for t in d[1:3])
+    dq, dw = ops.token_mix_bwd(*d, lse, do.to(dev), 0.125, 1.0, ws, dk, dv)
+    L.check_device_status(dev)
+    assert lse.isfinite().all() and dq.isnan().any()
+    for got, want, what in ((o, ref, "o"), (dk, kc.grad, "dk"), (dv, vc.grad, "dv"), (dw, wc.grad, "dw")):
+        assert want.isfinite().all() and got.isfinite().all(), what
+        assert_close_all_forms(got, want, 2e-2, what)           # (bf16 operands, as above)
