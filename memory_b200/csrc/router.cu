@@ -1336,7 +1336,8 @@ int launch_dlogits(const float* probs, const int64_t* idx, const float* weights,
   return MOC_OK;
 }
 
-// Whether the one launch takes this call (see route_front_kernel), and that launch.
+// Whether the one launch takes calls of this shape (see route_front_kernel), and that launch.  `done` says whether it was made: a
+// device that cannot hold a cluster of 16 CTAs of 1,024 threads (a part of a GPU, say) leaves the call to the other kernels.
 bool front_takes(const moc_router_shape* s, const void* h, const float* w, const float* pooled) {
   const int piece = s->h_dtype == MOC_F32 ? 4 : 8;
   return s->batch <= kFrontRows && s->seq <= kPoolSplits * kPoolOneMaxRows && s->hidden_dim % piece == 0 && s->hidden_dim % 4 == 0 &&
@@ -1344,7 +1345,7 @@ bool front_takes(const moc_router_shape* s, const void* h, const float* w, const
          ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(pooled)) & 15) == 0;
 }
 template <typename T>
-int launch_front(const T* h, const float* w, const float* bias, const FrontParams& p, cudaStream_t stream) {
+int launch_front(const T* h, const float* w, const float* bias, const FrontParams& p, cudaStream_t stream, bool* done) {
   const int nd = p.d <= 256 ? 0 : p.d <= 768 ? 1 : 2, nv = p.C <= 2 * 1024 ? 0 : p.C <= 5 * 1024 ? 1 : 2;
   using Kern = void (*)(const T*, const float*, const float*, FrontParams);
   static constexpr Kern kerns[3][3] = {
@@ -1358,7 +1359,9 @@ int launch_front(const T* h, const float* w, const float* bias, const FrontParam
   if (bytes > 48 * 1024 - 9 * 1024)              // (9 KiB: the selection's static arrays)
     MOC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
   MOC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  const int more = ceil_div(ceil_div(p.q.n, 32), kFrontCtas);        // clusters for the projection
+  *done = resident_clusters(kern, 1024, static_cast<int>(bytes), kFrontCtas) > 0;
+  if (!*done) return MOC_OK;
+  const int more = ceil_div(ceil_div(p.q.n, 32), kFrontCtas);        // clusters for the projection; they wait for nobody
   MOC_CUDA_OK(launch_clustered(kern, dim3(kFrontCtas * (1 + more)), 1024, static_cast<int>(bytes), kFrontCtas, stream, h, w, bias, p));
   return MOC_OK;
 }
@@ -1542,14 +1545,14 @@ int router_fwd_parts_impl(const moc_router_shape* s, const void* h, const float*
 
   dim3 pg(B, kPoolSplits);
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  const bool one_launch = q != nullptr && (parts & 1) && !(parts & (8 | 16)) && front_takes(s, h, w, pooled) &&
-                          cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
-  if (one_launch) {
+  bool one_launch = false;
+  if (q != nullptr && (parts & 1) && !(parts & (8 | 16)) && front_takes(s, h, w, pooled) &&
+      cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
     FrontParams p{pooled, logits, probs, reinterpret_cast<long long*>(idx), weights, comb_idx, comb_w, row_stats, B, L, d, C, k_sel,
                   S, s->routed_scale, *q};
-    *q_done = true;
-    MOC_TRY(s->h_dtype == MOC_F32 ? launch_front(static_cast<const float*>(h), w, bias, p, stream)
-                                  : launch_front(static_cast<const __nv_bfloat16*>(h), w, bias, p, stream));
+    MOC_TRY(s->h_dtype == MOC_F32 ? launch_front(static_cast<const float*>(h), w, bias, p, stream, &one_launch)
+                                  : launch_front(static_cast<const __nv_bfloat16*>(h), w, bias, p, stream, &one_launch));
+    *q_done = one_launch;
   }
   if ((parts & 1) && !one_launch) {
   if (!(parts & 8)) {      // bit 8: `pooled` already holds the pooled states (another pooling rule ran first)

@@ -106,3 +106,18 @@ def test_token_mixture_dispatch_and_split_k_rules():
     assert F._weight_grad_splits(torch.bfloat16, 8192, 768, 768) == 8      # 18 tiles -> 148 // 18
     assert F._weight_grad_splits(torch.bfloat16, 262144, 1536, 768) == 4   # 36 tiles
     assert F._weight_grad_splits(torch.bfloat16, 256, 768, 768) == 1       # too few rows to split
+
+
+def test_a_cluster_beyond_eight_ctas_is_launched_only_where_the_device_holds_one():
+    """Eight CTAs are the most that every device promises.  Whoever asks for more asks first whether such a cluster fits, and says so
+    to its caller, which then takes the other kernels."""
+    text = open(os.path.join(ROOT, "memory_b200", "csrc", "router.cu")).read()
+    body = text[text.index("int launch_front("):]
+    body = body[:body.index("\n}\n")]
+    opt_in, asked, launched = (body.index(x) for x in ("NonPortableClusterSizeAllowed", "*done = resident_clusters(", "launch_clustered("))
+    assert opt_in < asked < body.index("if (!*done) return MOC_OK;") < launched
+    caller = text[text.index("int router_fwd_parts_impl("):]
+    assert "*q_done = one_launch;" in caller and "if ((parts & 1) && !one_launch)" in caller
+    for name in os.listdir(os.path.join(ROOT, "memory_b200", "csrc")):
+        if name != "router.cu":
+            assert "NonPortableClusterSizeAllowed" not in open(os.path.join(ROOT, "memory_b200", "csrc", name)).read(), name
