@@ -693,15 +693,16 @@ extern "C" int moc_gather_rows_fwd(const void* bank, int32_t bank_dtype, int64_t
   return MOC_OK;
 }
 
+constexpr int kSegmentSmemMost = 200 * 1024;
 extern "C" int moc_chapter_segments(const int32_t* comb_idx, int32_t n_pairs, int32_t num_chapters,
                                     int32_t* uniq, int32_t* seg_offsets, int32_t* seg_pairs,
                                     int32_t* pair_to_uniq, int32_t* num_unique, int32_t* status, void* stream_) {
   MOC_REQUIRE(comb_idx && uniq && seg_offsets && seg_pairs && pair_to_uniq && num_unique && status, "NULL buffer");
   MOC_REQUIRE(n_pairs > 0 && n_pairs <= 65536, "n_pairs out of range");
-  MOC_REQUIRE(num_chapters > 0 && static_cast<size_t>(num_chapters) * 12 <= 200 * 1024, "num_chapters too large");
+  MOC_REQUIRE(num_chapters > 0 && static_cast<size_t>(num_chapters) * 12 <= kSegmentSmemMost, "num_chapters too large");
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const size_t sm = static_cast<size_t>(num_chapters) * 12;
-  MOC_CUDA_OK(cudaFuncSetAttribute(chapter_segments_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm)));
+  MOC_CUDA_OK(allow_shared(chapter_segments_kernel, sm, kSegmentSmemMost));
   chapter_segments_kernel<<<1, 1024, sm, stream>>>(comb_idx, n_pairs, num_chapters, uniq, seg_offsets, seg_pairs,
                                                    pair_to_uniq, num_unique, status);
   MOC_CUDA_OK(cudaGetLastError());
@@ -722,13 +723,13 @@ extern "C" int moc_bank_grad_merge_to(const void* const* rank_rows, int32_t rows
   MOC_REQUIRE(rows_dtype == MOC_F32 || rows_dtype == MOC_BF16, "bad rows_dtype");
   const int n_pairs = world * per_rank;
   MOC_REQUIRE(n_pairs <= 65535, "too many list entries");
-  MOC_REQUIRE(num_chapters > 0 && num_chapters <= 65535 && static_cast<size_t>(num_chapters) * 8 <= 200 * 1024,
+  MOC_REQUIRE(num_chapters > 0 && num_chapters <= 65535 && static_cast<size_t>(num_chapters) * 8 <= kSegmentSmemMost,
               "num_chapters too large");
   const long long cap = n_pairs < num_chapters ? n_pairs : num_chapters;     // the union cannot be larger
   MOC_REQUIRE(rows_out_capacity >= cap * T, "rows_out too small for the largest possible union");
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const size_t sm = static_cast<size_t>(num_chapters) * 8;
-  MOC_CUDA_OK(cudaFuncSetAttribute(union_segments_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm)));
+  MOC_CUDA_OK(allow_shared(union_segments_kernel, sm, kSegmentSmemMost));
   union_segments_kernel<<<1, 256, sm, stream>>>(ids_all, counts, world, per_rank, num_chapters, uniq, seg_offsets,
                                                 seg_pairs, pair_to_uniq, num_unique, status);
   RankRows src;

@@ -152,7 +152,7 @@ int launch_gemm_rows(const moc_gemm_desc* g, const void* a, const void* b, void*
   if (static_cast<long long>(g->m) * g->n >= kMmaFrom) {
     const int sums = kMmaWarps * kMmaRows * kMmaCols * 4;
     const int bytes = std::max((kMmaRows + kMmaCols) * mma_stride(g->k), sums);
-    MOC_CUDA_OK(cudaFuncSetAttribute(gemm_rows_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    MOC_CUDA_OK(allow_shared(gemm_rows_mma_kernel, bytes, (kMmaRows + kMmaCols) * mma_stride(1024)));
     gemm_rows_mma_kernel<<<dim3(ceil_div(g->n, kMmaCols), ceil_div(g->m, kMmaRows)), 32 * kMmaWarps, bytes, stream>>>(
         static_cast<const __nv_bfloat16*>(a), g->lda, static_cast<const __nv_bfloat16*>(b), g->ldb, c, g->ldc,
         g->c_dtype == MOC_BF16, g->m, g->n, g->k);

@@ -515,6 +515,15 @@ inline int attn_key_split(int ctas, int key_tiles) {
   }
   return best;
 }
+// Dynamic shared memory of a kernel whose calls need different amounts, `most` at the most.  The limit belongs to the function on
+// its device and host threads share it, so every call sets the same one: set to a call's own need, another thread's smaller call
+// would lower it between this thread's setting and its launch.
+template <typename... Params>
+inline cudaError_t allow_shared(void (*kernel)(Params...), size_t bytes, int most) {
+  if (bytes > static_cast<size_t>(most)) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+constexpr int kSharedMost = 227 * 1024;      // of a CTA, with its static arrays
 // How many clusters of `cluster` CTAs of a kernel the device holds at once (0.2 us to ask).
 template <typename... Params>
 inline int resident_clusters(void (*kernel)(Params...), int threads, int smem, int cluster) {

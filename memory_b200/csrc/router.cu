@@ -668,7 +668,8 @@ select_kernel(const float* __restrict__ logits, long long ld, const float* __res
 // replayed, and those with work enough to hide the launches keep the kernels above.  The remaining CTAs, clusters of their own,
 // are a projection of as many rows that needs nothing of the routing: the step's queries, one warp a column.
 // One sequence, host and device overlapped: 52 -> 44 us a step, 7 launches -> 4.
-constexpr int kFrontCtas = 16, kFrontRows = 2;
+constexpr int kFrontCtas = 16, kFrontRows = 2, kFrontChapters = 9 * 1024;
+constexpr int kFrontSmemMost = (kFrontChapters + 2 * 1024) * 4;    // the selection's (the pooling takes 33 KiB, the pooled states 8)
 struct FrontParams {
   float *pooled, *logits, *probs;
   long long* idx;
@@ -1296,6 +1297,7 @@ __global__ void dh_broadcast_kernel(const float* __restrict__ d_pooled, T* __res
 
 // kManyRows rows are enough to fill the chip with CTAs of 1,024 threads twice over; from there on smaller ones win
 constexpr int kManyRows = 2 * 296;
+constexpr int kRowSmemMost = 200 * 1024;          // what check_shape lets a row of chapters and its lists take
 int launch_select(const float* logits, long long ld, const float* bias, float* probs, int64_t* idx, float* weights,
                   int* comb_idx, float* comb_w, float* row_stats, int B, int C, int k_sel, int S, float rho,
                   cudaStream_t stream) {
@@ -1307,7 +1309,7 @@ int launch_select(const float* logits, long long ld, const float* bias, float* p
   auto kern = small ? (C <= 5 * 256 ? select_kernel<5, 256> : C <= 17 * 256 ? select_kernel<17, 256> : select_kernel<33, 256>)
               : C <= 2 * 1024 ? select_kernel<2, 1024> : C <= 5 * 1024 ? select_kernel<5, 1024>
               : C <= 9 * 1024 ? select_kernel<9, 1024> : select_kernel<0, 1024>;
-  MOC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm)));
+  MOC_CUDA_OK(allow_shared(kern, sm, kRowSmemMost));
   kern<<<B, small ? 256 : 1024, sm, stream>>>(logits, ld, bias, probs, reinterpret_cast<long long*>(idx), weights, comb_idx,
                                               comb_w, row_stats, C, k_sel, S, rho);
   MOC_CUDA_OK(cudaGetLastError());
@@ -1328,7 +1330,7 @@ int launch_dlogits(const float* probs, const int64_t* idx, const float* weights,
   auto kern = terms != nullptr
                   ? (small ? dlogits_kernel<18, 256, true> : held ? dlogits_kernel<6, 1024, true> : dlogits_kernel<0, 1024, true>)
                   : (small ? dlogits_kernel<18, 256, false> : held ? dlogits_kernel<6, 1024, false> : dlogits_kernel<0, 1024, false>);
-  MOC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm)));
+  MOC_CUDA_OK(allow_shared(kern, sm, kRowSmemMost));
   kern<<<B, small ? 256 : 1024, sm, stream>>>(probs, reinterpret_cast<const long long*>(idx), weights, comb_w, row_stats,
                                               chapter_stats, d_weights, d_comb_w, d_losses, d_logits, terms, ld, B, C, k_sel, S,
                                               rho);
@@ -1341,7 +1343,7 @@ int launch_dlogits(const float* probs, const int64_t* idx, const float* weights,
 bool front_takes(const moc_router_shape* s, const void* h, const float* w, const float* pooled) {
   const int piece = s->h_dtype == MOC_F32 ? 4 : 8;
   return s->batch <= kFrontRows && s->seq <= kPoolSplits * kPoolOneMaxRows && s->hidden_dim % piece == 0 && s->hidden_dim % 4 == 0 &&
-         s->hidden_dim <= 1024 && s->num_chapters <= 9 * 1024 &&
+         s->hidden_dim <= 1024 && s->num_chapters <= kFrontChapters &&
          ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(pooled)) & 15) == 0;
 }
 template <typename T>
@@ -1356,8 +1358,7 @@ int launch_front(const T* h, const float* w, const float* bias, const FrontParam
   const size_t part = static_cast<size_t>(kPoolSplits) * (32 * (16 / sizeof(T)) + 4) * 4;
   const size_t sel = (static_cast<size_t>(p.C) + 2 * static_cast<size_t>(p.k_sel > 0 ? p.k_sel : 1)) * 4;
   const size_t bytes = std::max(std::max(part, sel), static_cast<size_t>(p.B) * p.d * 4);
-  if (bytes > 48 * 1024 - 9 * 1024)              // (9 KiB: the selection's static arrays)
-    MOC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+  MOC_CUDA_OK(allow_shared(kern, bytes, kFrontSmemMost));
   MOC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   *done = resident_clusters(kern, 1024, static_cast<int>(bytes), kFrontCtas) > 0;
   if (!*done) return MOC_OK;
@@ -1398,7 +1399,7 @@ inline int check_shape(const moc_router_shape* s) {
   MOC_REQUIRE(s->num_shared >= 0 && s->num_shared <= s->num_chapters, "exclude_prefix_chapters out of range");
   MOC_REQUIRE(s->top_k <= 1024, "top_k above 1024 is not supported");
   MOC_REQUIRE(s->h_dtype == MOC_F32 || s->h_dtype == MOC_BF16, "bad h_dtype");
-  MOC_REQUIRE((static_cast<size_t>(s->num_chapters) + 2 * 1024) * 4 <= 200 * 1024, "num_chapters too large");
+  MOC_REQUIRE((static_cast<size_t>(s->num_chapters) + 2 * 1024) * 4 <= kRowSmemMost, "num_chapters too large");
   return MOC_OK;
 }
 
@@ -1579,11 +1580,10 @@ int router_fwd_parts_impl(const moc_router_shape* s, const void* h, const float*
                   : d <= 768 ? (few ? logits_rows_kernel<6, 1> : logits_rows_kernel<6, 4>)
                              : (few ? logits_rows_kernel<8, 1> : logits_rows_kernel<8, 4>);
       const size_t bytes = few ? sm : 2 * sm;
-      if (bytes > 48 * 1024)
-        MOC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+      MOC_CUDA_OK(allow_shared(kern, bytes, 2 * 8 * 1024 * 4));
       kern<<<ceil_div(C, few ? 8 : 32), 256, bytes, stream>>>(pooled, w, bias, logits, B, d, C);
     } else {
-      MOC_CUDA_OK(cudaFuncSetAttribute(logits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm)));
+      MOC_CUDA_OK(allow_shared(logits_kernel, sm, kSharedMost));
       logits_kernel<<<ceil_div(C, 8), 256, sm, stream>>>(pooled, w, bias, logits, B, d, C);
     }
   }
@@ -1643,7 +1643,7 @@ extern "C" int moc_router_bwd_parts(const moc_router_shape* s, const float* w, c
     const size_t sm = static_cast<size_t>(8) * d * sizeof(float);
     const bool vec = d % 4 == 0 && ((reinterpret_cast<uintptr_t>(pooled) | reinterpret_cast<uintptr_t>(d_w)) & 15) == 0;
     auto kern = vec ? dweight_kernel<4> : dweight_kernel<1>;
-    MOC_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm)));
+    MOC_CUDA_OK(allow_shared(kern, sm, kSharedMost));
     kern<<<ceil_div(C, 8), 256, sm, stream>>>(d_logits, pooled, d_w, d_bias, B, d, C);
   }
   const int nchunks = ceil_div(C, kDpChunk);

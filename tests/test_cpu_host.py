@@ -121,3 +121,20 @@ def test_a_cluster_beyond_eight_ctas_is_launched_only_where_the_device_holds_one
     for name in os.listdir(os.path.join(ROOT, "memory_b200", "csrc")):
         if name != "router.cu":
             assert "NonPortableClusterSizeAllowed" not in open(os.path.join(ROOT, "memory_b200", "csrc", name)).read(), name
+
+
+def test_no_call_lowers_the_shared_memory_limit_of_another_threads_launch():
+    """A kernel's limit of dynamic shared memory is state of the function on its device.  Two host threads may stand between setting
+    it and their launches, so each kernel is given one limit that no call changes: a constant of the source."""
+    import re
+    csrc = os.path.join(ROOT, "memory_b200", "csrc")
+    limits = {}
+    for name in sorted(os.listdir(csrc)):
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, name)).read())
+        for kern, limit in re.findall(r"cudaFuncSetAttribute\((\w+(?:<[^>]*>)?), cudaFuncAttributeMaxDynamicSharedMemorySize, ([^;]*?)\)\)?;", text):
+            limits.setdefault((name, kern), set()).add(limit)
+            assert re.fullmatch(r"(C\w*::)?k\w+|most", limit), (name, kern, limit)
+        for kern, limit in re.findall(r"allow_shared\((\w+), \w+, (.*?)\)\);", text):
+            assert not set(re.findall(r"[A-Za-z_]\w*", limit)) - set(re.findall(r"\bk[A-Z]\w*|mma_stride", limit)), (name, kern, limit)
+        assert text.count("cudaFuncAttributeMaxDynamicSharedMemorySize") == sum(1 for n, _ in limits if n == name) or name == "moc_common.cuh"
+    assert limits
