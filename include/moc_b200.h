@@ -456,9 +456,10 @@ typedef struct {
   int32_t* status;
   void *stream, *side_stream;
   int32_t hidden_dim;      /* width of hidden; 0: that of the routing states */
+  int32_t launches;        /* written by the call: the kernels it launched */
 } moc_decode_step_desc;
 int64_t moc_decode_step_arena_bytes(const moc_decode_step_desc* s);
-int moc_decode_step(const moc_decode_step_desc* s);
+int moc_decode_step(moc_decode_step_desc* s);
 
 /* Token-routed memory attention with per-token chapter weights, projections included, in one call per pass (bf16 arithmetic,
  * head_dim 64, 64-row chapters): h [rows, hidden_dim], shared [shared_rows, hidden_dim] (shared_rows 0: none), routed

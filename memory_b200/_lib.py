@@ -89,7 +89,7 @@ class DecodeStepDesc(C.Structure):
     _fields_ = [("router", RouterShape), ("attn", DecodeShape)] + _fields(
         "i: hidden_dtype out_dim; l: bank_rows;"
         "p: routing_states hidden router_w router_b wq wo kv_bank idx weights comb_idx comb_w out arena status stream"
-        " side_stream; i: hidden_dim")
+        " side_stream; i: hidden_dim launches")
 
 
 class LayerDesc(C.Structure):

@@ -295,7 +295,7 @@ extern "C" int64_t moc_decode_step_arena_bytes(const moc_decode_step_desc* s) {
   return s ? carve(s, &a) : -1;
 }
 
-extern "C" int moc_decode_step(const moc_decode_step_desc* s) {
+extern "C" int moc_decode_step(moc_decode_step_desc* s) {
   MOC_REQUIRE(s && s->routing_states && s->hidden && s->router_w && s->wq && s->wo && s->kv_bank && s->out && s->arena &&
               s->status, "NULL decode-step buffer");
   MOC_REQUIRE(s->attn.head_dim == kDD, "decode attention needs head_dim 64");
@@ -319,15 +319,18 @@ extern "C" int moc_decode_step(const moc_decode_step_desc* s) {
   const bool few = rows <= 2 && d % 8 == 0 && d <= 1024 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(s->wq)) & 15) == 0;
   const RowsProduct q{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(s->wq), a.q, d, d, width,
                       static_cast<int>(rows), static_cast<int>(width), static_cast<int>(d)};
-  bool q_done = false;
-  if (few) MOC_TRY(route_fwd_impl(r, &q, &q_done));
-  if (!q_done) {
+  RouteRun run;
+  if (few) MOC_TRY(route_fwd_impl(r, &q, &run));
+  if (!run.q_done) {
     Gemm gq(MOC_BF16, rows, width, d, true, true, MOC_BF16);
     MOC_TRY(moc_gemm(&gq, x, s->wq, a.q, nullptr, nullptr, s->status, side));
   }
-  if (!few) MOC_TRY(moc_route_fwd(r));
+  if (!few) MOC_TRY(route_fwd_impl(r, nullptr, &run));
   MOC_TRY(join.done());
   MOC_TRY(moc_decode_attn(&s->attn, a.q, s->kv_bank, s->bank_rows, s->comb_idx, s->comb_w, a.o, nullptr, s->status, s->stream));
   Gemm go(MOC_BF16, rows, s->out_dim, width, true, true, s->hidden_dtype);
-  return moc_gemm(&go, a.o, s->wo, s->out, nullptr, nullptr, s->status, s->stream);
+  MOC_TRY(moc_gemm(&go, a.o, s->wo, s->out, nullptr, nullptr, s->status, s->stream));
+  // (the cast of fp32 states; the queries where the router did not take them along; attention and output projection)
+  s->launches = run.launches + (x != s->hidden ? 1 : 0) + (run.q_done ? 0 : 1) + 2;
+  return MOC_OK;
 }

@@ -54,12 +54,17 @@ struct RowsProduct {
   long long lda = 0, ldb = 0, ldc = 0;
   int m = 0, n = 0, k = 0;
 };
-// moc_router_fwd_parts / moc_route_fwd with one; *q_done says whether it ran
+// What a router call did: whether the projection given along ran, and the kernels of pooling, logits and selection
+struct RouteRun {
+  bool q_done = false;
+  int launches = 0;
+};
+// moc_router_fwd_parts / moc_route_fwd with one (q may be NULL), reporting to *run (may be NULL)
 int router_fwd_parts_impl(const moc_router_shape* s, const void* h, const float* w, const float* bias, float* pooled, float* logits,
                           float* probs, int64_t* idx, float* weights, int32_t* comb_idx, float* comb_w, float* row_stats,
                           float* chapter_stats, float* losses, void* workspace, size_t workspace_bytes, int32_t parts,
-                          const RowsProduct* q, bool* q_done, int32_t* status, void* stream);
-int route_fwd_impl(const moc_route_desc* s, const RowsProduct* q, bool* q_done);
+                          const RowsProduct* q, RouteRun* run, int32_t* status, void* stream);
+int route_fwd_impl(const moc_route_desc* s, const RowsProduct* q, RouteRun* run);
 
 // What the bf16 projection kernel can do beside moc_gemm_desc:
 // terms > 1: C = sum over t of op(A_t) op(B_t), all in one accumulator, the last term first; A_t / B_t start

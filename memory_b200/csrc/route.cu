@@ -44,7 +44,7 @@ extern "C" int64_t moc_route_bwd_scratch_bytes(const moc_route_desc* s) {
   return s ? carve_bwd(&s->shape, nullptr, &t) : -1;
 }
 
-int moc::route_fwd_impl(const moc_route_desc* s, const RowsProduct* q, bool* q_done) {
+int moc::route_fwd_impl(const moc_route_desc* s, const RowsProduct* q, RouteRun* run) {
   MOC_REQUIRE(s && s->h && s->w && s->comb_idx && s->comb_w && s->arena && s->status, "NULL router buffer");
   const moc_router_shape* r = &s->shape;
   Saved a;
@@ -57,7 +57,7 @@ int moc::route_fwd_impl(const moc_route_desc* s, const RowsProduct* q, bool* q_d
     parts |= 8;
   }
   return router_fwd_parts_impl(r, s->h, s->w, s->bias, a.pooled, a.logits, a.probs, s->idx, s->weights, s->comb_idx,
-                               s->comb_w, a.row_stats, a.chapter_stats, s->losses, a.ws, ws_bytes, parts, q, q_done, s->status,
+                               s->comb_w, a.row_stats, a.chapter_stats, s->losses, a.ws, ws_bytes, parts, q, run, s->status,
                                s->stream);
 }
 extern "C" int moc_route_fwd(const moc_route_desc* s) { return route_fwd_impl(s, nullptr, nullptr); }

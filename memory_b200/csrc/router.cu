@@ -1528,7 +1528,7 @@ namespace moc {
 int router_fwd_parts_impl(const moc_router_shape* s, const void* h, const float* w, const float* bias, float* pooled, float* logits,
                           float* probs, int64_t* idx, float* weights, int32_t* comb_idx, float* comb_w, float* row_stats,
                           float* chapter_stats, float* losses, void* workspace, size_t workspace_bytes, int32_t parts,
-                          const RowsProduct* q, bool* q_done, int32_t* status, void* stream_) {
+                          const RowsProduct* q, RouteRun* run, int32_t* status, void* stream_) {
   int rc = check_shape(s);
   if (rc != MOC_OK) return rc;
   const size_t front = ws_floats(s, (parts & 1) && !(parts & 8), false);
@@ -1553,12 +1553,16 @@ int router_fwd_parts_impl(const moc_router_shape* s, const void* h, const float*
                   S, s->routed_scale, *q};
     MOC_TRY(s->h_dtype == MOC_F32 ? launch_front(static_cast<const float*>(h), w, bias, p, stream, &one_launch)
                                   : launch_front(static_cast<const __nv_bfloat16*>(h), w, bias, p, stream, &one_launch));
-    *q_done = one_launch;
   }
+  RouteRun did;
+  did.q_done = one_launch;
+  did.launches = one_launch ? 1 : 0;
   if ((parts & 1) && !one_launch) {
+  did.launches = 1 + ((parts & 16) ? 0 : 1);
   if (!(parts & 8)) {      // bit 8: `pooled` already holds the pooled states (another pooling rule ran first)
   const int piece = s->h_dtype == MOC_F32 ? 4 : 8;
   const bool one = L <= kPoolSplits * kPoolOneMaxRows && d % piece == 0 && (reinterpret_cast<uintptr_t>(h) & 15) == 0;
+  did.launches += one ? 1 : 2;
   const dim3 og(B, ceil_div(d, 8 * piece));
   if (one && s->h_dtype == MOC_F32)
     pool_mean_kernel<float><<<og, 8 * kPoolSplits, 0, stream>>>(static_cast<const float*>(h), pooled, L, d);
@@ -1595,6 +1599,7 @@ int router_fwd_parts_impl(const moc_router_shape* s, const void* h, const float*
     launch_losses(s, probs, idx, row_stats, chapter_stats, losses, loss_partial, stream);
   }
   MOC_CUDA_OK(cudaGetLastError());
+  if (run != nullptr) *run = did;
   return MOC_OK;
 }
 

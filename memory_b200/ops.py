@@ -1313,16 +1313,12 @@ def decode_step(hidden: torch.Tensor, routing_states: torch.Tensor, router_w: to
             L.DecodeShape(b, n_q, num_heads, num_kv_heads, head_dim, num_shared + k, tokens_per_chapter, scale),
             L.dtype_code(h.dtype), wo.shape[0], kv_bank.shape[0], None, None, p(w), p(bias), p(wq), p(wo), p(kv_bank), None,
             None, None, None, None, None, p(L.status_word(dev)), stream, _side_stream(L.device_index(dev), stream), d)
-        # one or two rows: pooling, logits, selection and the queries in one launch (outside a capture)
-        one = (b * n_q <= 2 and window <= 1024 and max(d, rd) <= 1024 and d % 8 == 0 and c <= 9 * 1024
-               and rd % (4 if states.dtype == torch.float32 else 8) == 0)
-        plan = (bytes(s), _size("moc_decode_step_arena_bytes", s), (b, k), (b, num_shared + k), (b, n_q, wo.shape[0]),
-                3 if one else 5 + int(window <= 1024) + 2 * int(window > 1024) + int(h.dtype == torch.float32))
+        plan = bytes(s), _size("moc_decode_step_arena_bytes", s), (b, k), (b, num_shared + k), (b, n_q, wo.shape[0])
         if plans is not None:
             if len(plans) >= _DECODE_PLANS_MAX:
                 plans.clear()
             plans[key] = plan
-    image, arena_bytes, routed, joint, out_shape, launches = plan
+    image, arena_bytes, routed, joint, out_shape = plan
     f32 = torch.float32
     out = torch.empty(out_shape, dtype=h.dtype, device=dev)
     idx = torch.empty(routed, dtype=torch.int64, device=dev)
@@ -1337,7 +1333,7 @@ def decode_step(hidden: torch.Tensor, routing_states: torch.Tensor, router_w: to
           else _timed("decode_step", lambda: L.lib().moc_decode_step(C.byref(s))))
     if rc:
         L.check(rc, "moc_decode_step")
-    _report(launches, lambda: ("router_fwd:" + _TAG_OF_CODE[s.router.h_dtype], "gemm:bf16", "decode_attn:bf16", "gemm:bf16"))
+    _report(s.launches, lambda: ("router_fwd:" + _TAG_OF_CODE[s.router.h_dtype], "gemm:bf16", "decode_attn:bf16", "gemm:bf16"))
     return out, idx, weights, comb_idx, comb_w
 
 

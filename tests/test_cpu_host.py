@@ -117,7 +117,7 @@ def test_a_cluster_beyond_eight_ctas_is_launched_only_where_the_device_holds_one
     opt_in, asked, launched = (body.index(x) for x in ("NonPortableClusterSizeAllowed", "*done = resident_clusters(", "launch_clustered("))
     assert opt_in < asked < body.index("if (!*done) return MOC_OK;") < launched
     caller = text[text.index("int router_fwd_parts_impl("):]
-    assert "*q_done = one_launch;" in caller and "if ((parts & 1) && !one_launch)" in caller
+    assert "did.q_done = one_launch;" in caller and "if ((parts & 1) && !one_launch)" in caller
     for name in os.listdir(os.path.join(ROOT, "memory_b200", "csrc")):
         if name != "router.cu":
             assert "NonPortableClusterSizeAllowed" not in open(os.path.join(ROOT, "memory_b200", "csrc", name)).read(), name

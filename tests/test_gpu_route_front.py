@@ -50,3 +50,27 @@ def test_two_tokens_and_captured_steps(n_q):
         out, info = dec.step(one, s1)
     graph.replay()
     _check(out, info, want, wi, 1)
+
+
+def test_the_launches_of_a_step_are_those_it_made():
+    """One or two rows: router and queries, attention, output projection.  Captured steps, more rows and states that start off a
+    16-byte boundary take pooling (of long windows in two kernels), logits, selection and queries apart; fp32 states are cast first."""
+    from memory_b200 import ops
+    dec, rand = _decoder(128, 40, 8, 1)
+    h, states = rand(3, 1, 128).bfloat16(), rand(3, 1100, 128).bfloat16()
+
+    def launches(rows, window, dtype=torch.bfloat16, off=0):
+        r = torch.empty(rows * window * 128 + off, dtype=torch.bfloat16, device=h.device)[off:].view(rows, window, 128)
+        r.copy_(states[:rows, :window])
+        x = h[:rows].to(dtype).contiguous()
+        before = ops.LAUNCHES
+        dec.step(x, r)
+        return ops.LAUNCHES - before
+
+    assert launches(1, 50) == launches(2, 50) == 3
+    assert launches(1, 50, torch.float32) == 4
+    assert launches(3, 50) == 6 and launches(3, 50, torch.float32) == 7
+    assert launches(1, 50, off=1) == launches(1, 1100) == 7
+    with torch.cuda.graph(torch.cuda.CUDAGraph()):
+        captured = launches(1, 50)
+    assert captured == 6
