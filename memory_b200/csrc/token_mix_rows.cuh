@@ -52,12 +52,14 @@ struct RowGroup {
 };
 
 // ---- forward -------------------------------------------------------------------------------------------------
-// A warp an item: its chapter's K / V tile (TMA), blocks of 16 query rows (four rows a TMA gather, the next block's under this
-// one's products), S and P in registers, the outputs through the query block's place as whole lines.  Nothing is shared between
-// warps, so none waits for another.  10 warps an SM (20 KiB each); bound by their instructions' latency (36 % of issue slots) at 32
-// pairs a chapter and by HBM at one.  Against the 128-row kernel: 8,192 tokens 268 -> 231 us, 2,048 tokens 227 -> 146, 250 tokens
-// 151 -> 101 (uniform picks, 12 heads, 4,096 chapters, 16 slots).  Two warps on one tile (16 of them an SM) were no faster at
-// 32 pairs (237) and slower below (172, 120): an odd block leaves one of them idle.
+// A warp an item (a tile of up to 128 pairs of one chapter, and a head): its chapter's K / V tile (TMA), blocks of 16 query rows
+// (four rows a TMA gather, the next block's under this one's products), S and P in registers, the outputs through the query block's
+// place as whole lines.  Nothing is shared between warps, so none waits for another.  10 warps an SM (20 KiB each); bound by their
+// instructions' latency (36 % of issue slots) at 32 pairs a chapter and by HBM at one.  Two warps on one tile (16 of them an SM) were
+// no faster at 32 pairs and slower below: an odd block leaves one of them idle.
+// Tiles and not whole chapters: a warp that walks a popular chapter alone is what the call waits for.  8,192 tokens x 16 of 4,096
+// chapters, us with the sum over slots, whole chapters and tiles: uniform picks 272 and 273, a router's (up to 452 pairs a chapter) 340
+// and 312, all picks in 32 chapters 957 and 211.
 constexpr int kRowFwdWarps = 2;
 constexpr int kRowFwdRows = 16;                                    // pairs of a step
 constexpr int kRowFwdBytes = kRowFwdRows * kD * 2;                 // 2 KiB
@@ -67,7 +69,7 @@ constexpr int kRowFwdCtas = 5;                                     // an SM
 
 __global__ void __launch_bounds__(kRowFwdWarps * 32, kRowFwdCtas)
 token_mix_rows_fwd_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
-                          const __grid_constant__ CUtensorMap tmap_q, MixFwdParams p, RowItems items) {
+                          const __grid_constant__ CUtensorMap tmap_q, MixFwdParams p, PairDiv div) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t kv_bar[kRowFwdWarps], q_bar[kRowFwdWarps][2];
   __shared__ int abort_flag;
@@ -76,17 +78,27 @@ token_mix_rows_fwd_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
   const uint32_t k_s = smem_u32(base), v_s = k_s + kTileKV, q_s = v_s + kTileKV;
   const MixShape& x = p.x;
   const int G = x.HQ / x.HK, no_row = x.B * x.TQ;
+  if (p.ask && tiles_full(p.totals)) return;
   if (threadIdx.x == 0) {
     abort_flag = 0;
     for (int i = 0; i < kRowFwdWarps; ++i) { mbar_init(&kv_bar[i], 1); mbar_init(&q_bar[i][0], 1); mbar_init(&q_bar[i][1], 1); }
     fence_mbar_init();
   }
   __syncthreads();
-  const int step = gridDim.x * kRowFwdWarps;
-  auto no_empty = [](const RowGroup&) {};
-  RowGroup gi;
-  gi.item = blockIdx.x * kRowFwdWarps + warp;
-  gi.seek(p.x, p.x.HQ, items, step, no_empty);
+  const int step = gridDim.x * kRowFwdWarps, per_list = x.HQ / x.HI, n_items = p.totals[kTiles] * per_list;
+  auto open = [&](int item) {
+    RowGroup g;
+    g.item = item; g.n = 0;
+    if (item < n_items) {
+      const int tile = item / per_list, bkt = p.tile_bucket[tile], c = bkt % x.M, bh = bkt / x.M, hi = bh % x.HI;
+      g.head = hi * per_list + (item - tile * per_list);
+      g.kv_row = bh / x.HI * x.TK + c * kKeys;
+      g.first = p.tile_first[tile];
+      g.n = p.tile_cnt[tile];
+    }
+    return g;
+  };
+  RowGroup gi = open(blockIdx.x * kRowFwdWarps + warp);
 
   auto load_kv = [&](const RowGroup& g) {
     if (lane == 0) {
@@ -99,7 +111,7 @@ token_mix_rows_fwd_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
   // lanes 0 .. 15 know a row of the block each: its pair
   auto load_id = [&](const RowGroup& g, int blk) { return lane < kRowFwdRows && blk + lane < g.n ? p.entries[g.first + blk + lane] : -1; };
   auto load_rows = [&](int hq, int id, uint32_t buf) {
-    const int row = id < 0 ? no_row : token_of(items.div, id);       // (behind the last row: zeros)
+    const int row = id < 0 ? no_row : token_of(div, id);       // (behind the last row: zeros)
     if (lane == 0) mbar_arrive_expect_tx(&q_bar[warp][buf], kRowFwdBytes);
     const int from = (lane & 3) * 4;
     const int r0 = __shfl_sync(0xffffffffu, row, from), r1 = __shfl_sync(0xffffffffu, row, from + 1);
@@ -119,9 +131,7 @@ token_mix_rows_fwd_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
     load_rows(gi.head, id, 0);
   }
   while (gi.n && ok) {
-    RowGroup ng = gi;
-    ng.item += step;
-    ng.seek(x, x.HQ, items, step, no_empty);
+    const RowGroup ng = open(gi.item + step);
     ok = mbar_wait_w(&kv_bar[warp], n_groups & 1, &abort_flag, p.status);
     ++n_groups;
     const int hq = gi.head;
@@ -134,7 +144,7 @@ token_mix_rows_fwd_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
       int next_id = -1;
       if (more) next_id = last ? load_id(ng, 0) : load_id(gi, nblk);
       // row (token, slot) of the partial outputs and of the weights; rows lane / 4 and lane / 4 + 8 are this lane's in the products
-      const int pair = id < 0 ? 0 : id, tok = token_of(items.div, pair), slot = slot_of(items.div, pair);
+      const int pair = id < 0 ? 0 : id, tok = token_of(div, pair), slot = slot_of(div, pair);
       const long long at = static_cast<long long>(tok) * x.S + slot;
       const float w_own = id < 0 ? 0.f : p.w[at];
       ok = ok && mbar_wait_w(&q_bar[warp][buf], (it >> 1) & 1, &abort_flag, p.status);
@@ -266,6 +276,7 @@ token_mix_rows_bwd_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* rows = base + 4 * kTileKV;                            // two (dO, Q) row blocks behind two (K, V) tile pairs
   const MixShape& x = p.x;
+  if (p.ask && tiles_end_sooner(p.totals)) return;
   if (threadIdx.x == 0) {
     abort_flag = 0;
     for (int i = 0; i < 2; ++i) {

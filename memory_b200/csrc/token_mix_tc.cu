@@ -41,6 +41,7 @@ __device__ __forceinline__ float ex2(float x) {
 // pairs are numbered p = ((b * TQ + t) * HI + hi) * S + s (HI = 1: one chapter list per token for all heads;
 // HI = HK: a list per KV head); buckets are numbered (b * HI + hi) * M + chapter.
 struct IndexShape { int B, TQ, HI, S, M; };
+constexpr int kTiles = 0, kPairs = 1, kLargest = 2;      // of `totals`: tiles, pairs in buckets, pairs of the largest bucket
 
 __device__ __forceinline__ int bucket_of(const IndexShape& x, long long p, int chapter) {
   const long long bh = p / x.S;                       // (b * TQ + t) * HI + hi
@@ -58,14 +59,14 @@ __global__ void mix_count_kernel(const int* __restrict__ idx, IndexShape x, long
   atomicAdd(&cnt[bucket_of(x, p, c)], 1);
 }
 
-// exclusive scans of the bucket sizes and of the tiles per bucket; one CTA of 1024 threads
+// exclusive scans of the bucket sizes and of the tiles per bucket, and the largest bucket; one CTA of 1024 threads
 __global__ void mix_scan_kernel(const int* __restrict__ cnt, int n_buckets, int* __restrict__ bucket_off,
                                 int* __restrict__ tile_off, int* __restrict__ totals) {
-  __shared__ int warp_tot[2][32];
+  __shared__ int warp_tot[2][32], warp_max[32];
   const int per = (n_buckets + blockDim.x - 1) / blockDim.x;
   const int lo = threadIdx.x * per, hi = min(n_buckets, lo + per);
-  int s0 = 0, s1 = 0;
-  for (int i = lo; i < hi; ++i) { s0 += cnt[i]; s1 += (cnt[i] + kTok - 1) / kTok; }
+  int s0 = 0, s1 = 0, most = 0;
+  for (int i = lo; i < hi; ++i) { s0 += cnt[i]; s1 += (cnt[i] + kTok - 1) / kTok; most = max(most, cnt[i]); }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int i0 = s0, i1 = s1;
 #pragma unroll
@@ -73,7 +74,8 @@ __global__ void mix_scan_kernel(const int* __restrict__ cnt, int n_buckets, int*
     const int t0 = __shfl_up_sync(0xffffffffu, i0, o), t1 = __shfl_up_sync(0xffffffffu, i1, o);
     if (lane >= o) { i0 += t0; i1 += t1; }
   }
-  if (lane == 31) { warp_tot[0][warp] = i0; warp_tot[1][warp] = i1; }
+  most = __reduce_max_sync(0xffffffffu, most);
+  if (lane == 31) { warp_tot[0][warp] = i0; warp_tot[1][warp] = i1; warp_max[warp] = most; }
   __syncthreads();
   if (warp == 0) {
     int w0 = warp_tot[0][lane], w1 = warp_tot[1][lane];
@@ -83,6 +85,7 @@ __global__ void mix_scan_kernel(const int* __restrict__ cnt, int n_buckets, int*
       if (lane >= o) { w0 += t0; w1 += t1; }
     }
     warp_tot[0][lane] = w0; warp_tot[1][lane] = w1;
+    most = __reduce_max_sync(0xffffffffu, warp_max[lane]);
   }
   __syncthreads();
   int e0 = i0 - s0 + (warp > 0 ? warp_tot[0][warp - 1] : 0);
@@ -93,7 +96,7 @@ __global__ void mix_scan_kernel(const int* __restrict__ cnt, int n_buckets, int*
   }
   if (threadIdx.x == 0) {
     bucket_off[n_buckets] = warp_tot[0][31]; tile_off[n_buckets] = warp_tot[1][31];
-    totals[0] = warp_tot[1][31];       // number of tiles
+    totals[kTiles] = warp_tot[1][31]; totals[kPairs] = warp_tot[0][31]; totals[kLargest] = most;
   }
 }
 
@@ -241,9 +244,16 @@ struct MixFwdParams {
   __nv_bfloat16* partial;        // [B*TQ, S, HQ, 64]
   float* lse_slots;              // [B*TQ, HQ, S]
   const int *entries, *tile_bucket, *tile_first, *tile_cnt, *totals;
+  bool ask;                      // both kernels were launched; the buckets say whose call it is
   MixShape x;
   int* status;
 };
+// Whether the 128-row tiles are full enough for their kernel to be the faster one: 126 pairs a tile 177 and 211 us, 113: 64 and 66,
+// 102: 246 and 240 (the calls above kRowFwdPairs)
+constexpr int kFullTile = 108;
+__device__ __forceinline__ bool tiles_full(const int* totals) {
+  return totals[kPairs] >= static_cast<long long>(kFullTile) * totals[kTiles];
+}
 constexpr int kMixThreads = 160;                       // 4 row-owning warps + 1 control warp (TMA, MMA issue)
 constexpr int kFwdSmem = 2 * kTileQ + 2 * kTileKV + 1024;
 
@@ -263,6 +273,7 @@ token_mix_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
   uint8_t* o_s = v_s + kTileKV;
   const MixShape& x = p.x;
   const int G = x.HQ / x.HK;
+  if (p.ask && !tiles_full(p.totals)) return;
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
@@ -275,7 +286,7 @@ token_mix_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
-  const int n_tiles = p.totals[0];
+  const int n_tiles = p.totals[kTiles];
   uint32_t it = 0, kvn = 0, tile_no = 0;
   bool ok = true;
 
@@ -477,8 +488,9 @@ struct MixBwdParams {
   float* d_w_heads;              // [B*TQ, HQ, S]
   __nv_bfloat16 *d_k, *d_v;      // rows b*TK + key, row stride dkv_ld elements; head kh at column kh*64
   long long dkv_ld;
-  const int *entries, *bucket_off;
+  const int *entries, *bucket_off, *totals;
   int n_items, runs;             // (bucket, run of KV heads), runs per bucket
+  bool ask;                      // as in MixFwdParams
   MixShape x;
   int* status;
 };
@@ -519,6 +531,15 @@ struct GroupIter {
   }
 };
 
+// Whether the backward of 128-row tiles ends sooner where an item is one head of a bucket: whoever has the largest bucket walks it
+// alone.  In 0.1 us, a CTA alone on its SM takes 105 for a tile and one of the other kernel 34 for a step of 32 pairs; with the chip
+// full, one of two on an SM takes 95 for a tile, one of three 44 for a step.
+__device__ __forceinline__ bool tiles_end_sooner(const int* totals) {
+  const int tiles = totals[kTiles], pairs = totals[kPairs], largest = totals[kLargest];
+  const float steps = fmaxf((pairs / 32 + tiles / 2) * (44.f / (3 * 148)), ((largest + 31) / 32) * 34.f);
+  return fmaxf(tiles * (95.f / (2 * 148)), ((largest + kTok - 1) / kTok) * 105.f) < steps;
+}
+
 __global__ void __launch_bounds__(kMixThreads, 2)
 token_mix_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                         MixBwdParams p) {
@@ -535,6 +556,7 @@ token_mix_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
   uint8_t* kv_s = base + 4 * kTileQ;     // two (K, V) tile pairs: the next group's pair arrives under this group's work
   const MixShape& x = p.x;
   const int G = x.HQ / x.HK;
+  if (p.ask && !tiles_end_sooner(p.totals)) return;
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
@@ -779,12 +801,20 @@ int sm_count() {
   return n;
 }
 
-// Below these the kernels of token_mix_rows.cuh are the faster ones.  8,192 tokens x 16 chapters of as many as the figure says, 12
-// heads, us before (128-row tiles) and with them.  Forward, by pairs a chapter: 32: 268 -> 232, 64: 97 -> 104 (8 slots), 128: 208 -> 179,
-// 256: 195 and 206, 512: 131 and 202; with the uneven buckets that a router gives 32: 357 -> 270.  Backward, by rows (pairs x
-// query heads of a KV head) a chapter: 32: 1,064 -> 569, 128: 505 -> 391, 256: 442 -> 367, 384: 501 -> 382, 512: 406 and 397, 1,536: 387 and 466;
-// uneven, 32: 1,196 -> 607.
-constexpr long long kRowFwdPairs = 256, kRowBwdRowsMax = 512;
+// Which kernel a call takes, us with the sum over slots, 128-row tiles and the kernels of token_mix_rows.cuh; 12 heads.
+// Forward, 16 slots of as many chapters as the pairs a chapter say, 8,192 tokens, uniform picks and (behind the comma) a router's: 32
+// pairs 314 and 273, 416 and 312; 64: 234 and 240, 312 and 293; 128: 261 and 261, 234 and 246; 512: 183 and 224; 4 slots, 32: 99 and 85,
+// 153 and 99; 64: 70 and 79, 83 and 89.  So the line is between 32 and 64 pairs, and calls of few pairs, whose tiles leave
+// most of the chip idle, lie on this side of it whatever the chapters hold (512 tokens x 4 on 16 chapters: 54 and 25; 2,048 x 2 on
+// 32: 54 and 26; the same from some 32 K pairs on: 2,048 x 16 on 32: 64 and 66).
+// What the chapters hold is known on the device alone: where all picks fall on a few chapters (32 of 4,096: 177 and 211) the tiles are
+// full and theirs is the faster kernel again.  So both are launched and one of them leaves at once (`ask`).
+// Backward, by rows (pairs x query heads of a KV head) a chapter, 12 KV heads: 32 rows 1,126 and 621 (a router's 1,188 and 670), 128:
+// 560 and 443, 256: 487 and 412, 512: 457 and 402; 4 KV heads, 96 rows: 898 and 531, 384: 552 and 435, 768: 483 and 423, 1,536:
+// 433 and 445.  All picks in 32 chapters: 2,387 and 1,238 (12 KV heads), 4,165 and 1,436 (4).  A tile item is a run of up to four
+// heads; with one, few long items of tiles end sooner than as many of steps (one KV head, 32 chapters: 4,059 and 5,177): asked as well.
+constexpr long long kRowFwdPairs = 48, kRowBwdRowsMax = 512, kFewPairs = 24 * 1024;
+constexpr int kLongBucket = 512;         // (tokens a sequence; below, the longest item is short)
 
 int check_shape(const moc_sparse_attn_shape* s, int index_heads, MixShape* x) {
   MOC_REQUIRE(s != nullptr, "shape is NULL");
@@ -855,15 +885,19 @@ extern "C" int moc_token_mix_fwd(const moc_sparse_attn_shape* s, int32_t index_h
   p.partial = static_cast<__nv_bfloat16*>(partial); p.lse_slots = lse_slots;
   p.entries = ib.entries; p.tile_bucket = ib.tile_bucket; p.tile_first = ib.tile_first; p.tile_cnt = ib.tile_cnt;
   p.totals = ib.totals; p.x = x; p.status = status;
-  if (n_pairs < kRowFwdPairs * n_buckets && n_buckets * x.HQ < (1ll << 30)) {
+  const long long row_items = max_tiles(n_pairs, n_buckets) * (x.HQ / x.HI);
+  const bool row_blocks = (n_pairs < kRowFwdPairs * n_buckets || n_pairs < kFewPairs) && row_items < (1ll << 30);
+  p.ask = row_blocks && n_pairs >= kFewPairs;
+  if (row_blocks) {
     CUtensorMap mq;                                              // rows of one head, gathered four at a time
     const uint64_t q_cols = static_cast<uint64_t>(x.HQ) * kD;
     MOC_TRY(make_tmap_bf16_2d(&mq, q, static_cast<uint64_t>(x.B) * x.TQ, q_cols, q_cols, 1, kD));
-    const RowItems items{ib.bucket_off, static_cast<int>(n_buckets) * (x.HQ / x.HI), {fast_div(x.S), fast_div(x.HI)}};
     MOC_CUDA_OK(cudaFuncSetAttribute(token_mix_rows_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowFwdSmem));
-    const int grid = std::min((items.n + kRowFwdWarps - 1) / kRowFwdWarps, sm_count() * kRowFwdCtas);
-    token_mix_rows_fwd_kernel<<<grid, kRowFwdWarps * 32, kRowFwdSmem, st>>>(mk, mv, mq, p, items);
-  } else {
+    const long long grid = std::min<long long>((row_items + kRowFwdWarps - 1) / kRowFwdWarps, sm_count() * kRowFwdCtas);
+    token_mix_rows_fwd_kernel<<<static_cast<int>(grid), kRowFwdWarps * 32, kRowFwdSmem, st>>>(
+        mk, mv, mq, p, PairDiv{fast_div(x.S), fast_div(x.HI)});
+  }
+  if (!row_blocks || p.ask) {
     MOC_CUDA_OK(cudaFuncSetAttribute(token_mix_fwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem));
     const long long grid = std::min<long long>(max_tiles(n_pairs, n_buckets), static_cast<long long>(sm_count()) * 4);
     token_mix_fwd_tc_kernel<<<static_cast<int>(grid), kMixThreads, kFwdSmem, st>>>(mk, mv, p);
@@ -906,9 +940,13 @@ extern "C" int moc_token_mix_bwd(const moc_sparse_attn_shape* s, int32_t index_h
   p.w = weights; p.lse_slots = lse_slots;
   p.dq_partial = static_cast<__nv_bfloat16*>(dq_partial); p.d_w_heads = d_w_heads;
   p.d_k = static_cast<__nv_bfloat16*>(d_k); p.d_v = static_cast<__nv_bfloat16*>(d_v); p.dkv_ld = dkv_row_stride;
-  p.entries = ib.entries; p.bucket_off = ib.bucket_off;
+  p.entries = ib.entries; p.bucket_off = ib.bucket_off; p.totals = ib.totals;
   p.x = x; p.status = status;
-  if (n_pairs * (x.HQ / x.HK) < kRowBwdRowsMax * n_buckets) {
+  p.runs = x.HI == 1 ? (x.HK + kRunHeads - 1) / kRunHeads : 1;
+  p.n_items = static_cast<int>(n_buckets) * p.runs;
+  const bool row_steps = n_pairs * (x.HQ / x.HK) < kRowBwdRowsMax * n_buckets;
+  p.ask = row_steps && (x.HK == 1 || x.HI > 1) && x.TQ >= kLongBucket;
+  if (row_steps) {
     CUtensorMap mq, md;                                          // rows of one head, gathered four at a time
     const uint64_t q_rows = static_cast<uint64_t>(x.B) * x.TQ, q_cols = static_cast<uint64_t>(x.HQ) * kD;
     MOC_TRY(make_tmap_bf16_2d(&mq, q, q_rows, q_cols, q_cols, 1, kD));
@@ -917,9 +955,8 @@ extern "C" int moc_token_mix_bwd(const moc_sparse_attn_shape* s, int32_t index_h
     MOC_CUDA_OK(cudaFuncSetAttribute(token_mix_rows_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowBwdSmem));
     const int grid = std::min(items.n, sm_count() * kRowBwdCtas);
     token_mix_rows_bwd_kernel<<<grid, kRowBwdThreads, kRowBwdSmem, st>>>(mk, mv, mq, md, p, items);
-  } else {
-    p.runs = x.HI == 1 ? (x.HK + kRunHeads - 1) / kRunHeads : 1;
-    p.n_items = static_cast<int>(n_buckets) * p.runs;
+  }
+  if (!row_steps || p.ask) {
     MOC_CUDA_OK(cudaFuncSetAttribute(token_mix_bwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem));
     const int grid = std::min(p.n_items, sm_count() * 2);
     token_mix_bwd_tc_kernel<<<grid, kMixThreads, kBwdSmem, st>>>(mk, mv, p);

@@ -53,3 +53,11 @@ def test_warps_agree_about_their_waits(late):
         with pytest.raises(RuntimeError, match="timed out"):
             L.check_device_status(dev)
     L.check_device_status(dev)
+
+
+def test_no_warp_walks_a_whole_chapter_of_the_token_mixture_alone():
+    """Forward of chapters with few pairs: routing may send every pair to a few of them, so an item is a tile of the index (at most 128
+    pairs), as in the other kernel, and never a bucket."""
+    text = open(os.path.join(CSRC, "token_mix_rows.cuh")).read()
+    kernel = text[text.index("token_mix_rows_fwd_kernel("):text.index("// ---- backward")]
+    assert "g.n = p.tile_cnt[tile];" in kernel and "bucket_off" not in kernel and "seek(" not in kernel

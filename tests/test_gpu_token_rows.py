@@ -72,3 +72,48 @@ def test_an_infinite_key_stays_with_its_own_gradients(pairs, heads):
     for got, want, what in ((o, ref, "o"), (dk, kc.grad, "dk"), (dv, vc.grad, "dv"), (dw, wc.grad, "dw")):
         assert want.isfinite().all() and got.isfinite().all(), what
         assert_close_all_forms(got, want, 2e-2, what)           # (bf16 operands, as above)
+
+
+def _by_chapter(q, k, v, bi, w):
+    """Plain fp64 mixture, chapter by chapter: q [T, HQ, 64], k / v [M * 64, H, 64], bi [T, 1 or H, S], w [T, S]."""
+    h, per = k.shape[1], q.shape[1] // k.shape[1]
+    heads = []
+    for kh in range(h):
+        ids = bi[:, kh if bi.shape[1] > 1 else 0]
+        qh, out = q[:, kh * per:(kh + 1) * per], torch.zeros_like(q[:, :per])
+        for c in ids.unique().tolist():
+            t, s = (ids == c).nonzero(as_tuple=True)
+            p = torch.softmax(torch.einsum("ngd,md->ngm", qh[t], k[c * 64:(c + 1) * 64, kh]) * 0.125, -1)
+            out = out.index_add(0, t, w[t, s][:, None, None] * torch.einsum("ngm,md->ngd", p, v[c * 64:(c + 1) * 64, kh]))
+        heads.append(out)
+    return torch.cat(heads, 1)
+
+
+@pytest.mark.parametrize("heads,lists", [((2, 2), "token"), ((2, 2), "head"), ((4, 1), "token")], ids=["mha", "lists", "mqa"])
+@pytest.mark.parametrize("used", [16, 40, 600])
+def test_the_buckets_decide_between_the_kernels(used, heads, lists):
+    """Enough pairs for both kernels and few a chapter on average, all of them in 16 chapters (full tiles, one long item each), in 40, or
+    spread: whichever kernel takes the call, the results are the mixture's and repeats are the same bits."""
+    from memory_b200 import _lib as L, ops
+    dev = torch.device("cuda:0")
+    (hq, h), tokens, S, m = heads, 1600, 16, 600
+    g = torch.Generator(device=dev).manual_seed(used + hq)
+    rand = lambda *s: torch.randn(*s, generator=g, device=dev).bfloat16()
+    hi = 1 if lists == "token" else h
+    chosen = torch.randperm(m, generator=g, device=dev)[:used]
+    bi = chosen[torch.rand(tokens, hi, used, generator=g, device=dev).topk(S, -1).indices].int()
+    q, do, k, v = rand(1, tokens, hq, 64), rand(1, tokens, hq, 64), rand(1, m * 64, h, 64), rand(1, m * 64, h, 64)
+    w = torch.rand(1, tokens, S, generator=g, device=dev) + 0.1
+    qc, kc, vc, wc = (t[0].double().requires_grad_(True) for t in (q, k, v, w))
+    ref = _by_chapter(qc, kc, vc, bi.long(), wc)
+    ref.backward(do[0].double())
+    runs = []
+    for _ in range(2):
+        o, lse, ws = ops.token_mix_fwd(q, k, v, bi[None], w, 0.125)
+        dk, dv = (torch.full_like(t, float("nan")) for t in (k, v))
+        dq, dw = ops.token_mix_bwd(q, k, v, bi[None], w, lse, do, 0.125, 1.0, ws, dk, dv)
+        runs.append((o, dq, dk, dv, dw))
+    L.check_device_status(dev)
+    for got, want, what in zip(runs[0], (ref, qc.grad, kc.grad, vc.grad, wc.grad), ("o", "dq", "dk", "dv", "dw")):
+        assert_close_all_forms(got[0], want.float(), 2e-2, what)      # (bf16 operands, as above)
+    assert all(torch.equal(a, b) for a, b in zip(*runs))
