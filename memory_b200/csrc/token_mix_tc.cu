@@ -532,8 +532,9 @@ struct GroupIter {
 };
 
 // Whether the backward of 128-row tiles ends sooner where an item is one head of a bucket: whoever has the largest bucket walks it
-// alone.  In 0.1 us, a CTA alone on its SM takes 105 for a tile and one of the other kernel 34 for a step of 32 pairs; with the chip
-// full, one of two on an SM takes 95 for a tile, one of three 44 for a step.
+// alone.  In 0.1 us, three popular chapters one behind the other on a CTA (as the walk of 32 of them meets somewhere) take 105 a tile of
+// the largest, and 34 a step of 32 pairs in the other kernel; with the chip full, one of two CTAs on an SM takes 95 for a tile, one of
+// three 44 for a step.
 __device__ __forceinline__ bool tiles_end_sooner(const int* totals) {
   const int tiles = totals[kTiles], pairs = totals[kPairs], largest = totals[kLargest];
   const float steps = fmaxf((pairs / 32 + tiles / 2) * (44.f / (3 * 148)), ((largest + 31) / 32) * 34.f);
@@ -802,19 +803,23 @@ int sm_count() {
 }
 
 // Which kernel a call takes, us with the sum over slots, 128-row tiles and the kernels of token_mix_rows.cuh; 12 heads.
-// Forward, 16 slots of as many chapters as the pairs a chapter say, 8,192 tokens, uniform picks and (behind the comma) a router's: 32
-// pairs 314 and 273, 416 and 312; 64: 234 and 240, 312 and 293; 128: 261 and 261, 234 and 246; 512: 183 and 224; 4 slots, 32: 99 and 85,
-// 153 and 99; 64: 70 and 79, 83 and 89.  So the line is between 32 and 64 pairs, and calls of few pairs, whose tiles leave
-// most of the chip idle, lie on this side of it whatever the chapters hold (512 tokens x 4 on 16 chapters: 54 and 25; 2,048 x 2 on
-// 32: 54 and 26; the same from some 32 K pairs on: 2,048 x 16 on 32: 64 and 66).
-// What the chapters hold is known on the device alone: where all picks fall on a few chapters (32 of 4,096: 177 and 211) the tiles are
-// full and theirs is the faster kernel again.  So both are launched and one of them leaves at once (`ask`).
-// Backward, by rows (pairs x query heads of a KV head) a chapter, 12 KV heads: 32 rows 1,126 and 621 (a router's 1,188 and 670), 128:
+// Forward, 8,192 tokens x 16 slots, by the average of pairs a chapter, uniform picks and (behind the comma) a router's: 32 pairs 312 and
+// 271, 410 and 312; 48: 254 and 250, 326 and 284; 56: 240 and 242, 324 and 288; 80: 217 and 234, 293 and 265; 128: 261 and 261, 234
+// and 246; 512: 183 and 224.  4 slots, 32: 97 and 85, 148 and 99; 48: 101 and 80, 138 and 91; 56: 68 and 78, 134 and 105; 64: 70 and 78,
+// 82 and 89.  (A round of tiles is 592, what the chip holds, hence the steps.)  So the line is at 52 pairs, and calls whose tiles
+// leave most of the chip idle lie on this side of it whatever the chapters hold: 8,000 pairs 50 and 25, 24,000 62 to 74 and 52 to 78.
+// What the chapters hold is known on the device alone: where all picks fall on a few of them (32 of 4,096), the tiles are full and
+// theirs is the faster kernel again: 32,000 pairs 67 and 66, 48,000 78 and 87, 131,072 177 and 209.  So from 40 K pairs on both are
+// launched and one of them leaves at once (`ask`; 4 to 6 us).
+// Backward, by rows (pairs x query heads of a KV head) a chapter, 12 KV heads: 32 rows 1,115 and 618 (a router's 1,180 and 668), 128:
 // 560 and 443, 256: 487 and 412, 512: 457 and 402; 4 KV heads, 96 rows: 898 and 531, 384: 552 and 435, 768: 483 and 423, 1,536:
-// 433 and 445.  All picks in 32 chapters: 2,387 and 1,238 (12 KV heads), 4,165 and 1,436 (4).  A tile item is a run of up to four
-// heads; with one, few long items of tiles end sooner than as many of steps (one KV head, 32 chapters: 4,059 and 5,177): asked as well.
-constexpr long long kRowFwdPairs = 48, kRowBwdRowsMax = 512, kFewPairs = 24 * 1024;
-constexpr int kLongBucket = 512;         // (tokens a sequence; below, the longest item is short)
+// 433 and 445.  All picks in 32 chapters: 2,374 and 1,235 (12 KV heads), 4,149 and 1,438 (4).  A tile item is a run of up to four
+// heads.  With one, few items leave the chip idle either way and a walk of tiles is the shorter one (one KV head, 384 rows: 250
+// chapters 167 and 215, 1,000 320 and 332, 4,096 1,007 and 721; 192 rows: 500 chapters 155 and 146), and so it is for long items
+// (4,050 and 5,187 where all picks fall on 32): asked as well.
+constexpr long long kRowFwdPairs = 52, kFewPairs = 24 * 1024, kAskPairs = 40 * 1024;
+constexpr long long kRowBwdRowsMax = 512, kRowBwdRowsFewItems = 256, kFewItems = 1000;
+constexpr int kLongBucket = 256;         // (tokens a sequence; below, the longest item is short)
 
 int check_shape(const moc_sparse_attn_shape* s, int index_heads, MixShape* x) {
   MOC_REQUIRE(s != nullptr, "shape is NULL");
@@ -887,7 +892,7 @@ extern "C" int moc_token_mix_fwd(const moc_sparse_attn_shape* s, int32_t index_h
   p.totals = ib.totals; p.x = x; p.status = status;
   const long long row_items = max_tiles(n_pairs, n_buckets) * (x.HQ / x.HI);
   const bool row_blocks = (n_pairs < kRowFwdPairs * n_buckets || n_pairs < kFewPairs) && row_items < (1ll << 30);
-  p.ask = row_blocks && n_pairs >= kFewPairs;
+  p.ask = row_blocks && n_pairs >= kAskPairs;
   if (row_blocks) {
     CUtensorMap mq;                                              // rows of one head, gathered four at a time
     const uint64_t q_cols = static_cast<uint64_t>(x.HQ) * kD;
@@ -944,8 +949,15 @@ extern "C" int moc_token_mix_bwd(const moc_sparse_attn_shape* s, int32_t index_h
   p.x = x; p.status = status;
   p.runs = x.HI == 1 ? (x.HK + kRunHeads - 1) / kRunHeads : 1;
   p.n_items = static_cast<int>(n_buckets) * p.runs;
-  const bool row_steps = n_pairs * (x.HQ / x.HK) < kRowBwdRowsMax * n_buckets;
-  p.ask = row_steps && (x.HK == 1 || x.HI > 1) && x.TQ >= kLongBucket;
+  const bool one_head = x.HK == 1 || x.HI > 1;
+  const bool row_steps =
+      n_pairs * (x.HQ / x.HK) < (one_head && n_buckets < kFewItems ? kRowBwdRowsFewItems : kRowBwdRowsMax) * n_buckets;
+  p.ask = row_steps && one_head && x.TQ >= kLongBucket;
+  if (!row_steps || p.ask) {
+    MOC_CUDA_OK(cudaFuncSetAttribute(token_mix_bwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem));
+    const int grid = std::min(p.n_items, sm_count() * 2);
+    token_mix_bwd_tc_kernel<<<grid, kMixThreads, kBwdSmem, st>>>(mk, mv, p);
+  }
   if (row_steps) {
     CUtensorMap mq, md;                                          // rows of one head, gathered four at a time
     const uint64_t q_rows = static_cast<uint64_t>(x.B) * x.TQ, q_cols = static_cast<uint64_t>(x.HQ) * kD;
@@ -955,11 +967,6 @@ extern "C" int moc_token_mix_bwd(const moc_sparse_attn_shape* s, int32_t index_h
     MOC_CUDA_OK(cudaFuncSetAttribute(token_mix_rows_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowBwdSmem));
     const int grid = std::min(items.n, sm_count() * kRowBwdCtas);
     token_mix_rows_bwd_kernel<<<grid, kRowBwdThreads, kRowBwdSmem, st>>>(mk, mv, mq, md, p, items);
-  }
-  if (!row_steps || p.ask) {
-    MOC_CUDA_OK(cudaFuncSetAttribute(token_mix_bwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem));
-    const int grid = std::min(p.n_items, sm_count() * 2);
-    token_mix_bwd_tc_kernel<<<grid, kMixThreads, kBwdSmem, st>>>(mk, mv, p);
   }
   const long long rows = static_cast<long long>(x.B) * x.TQ;
   const long long threads = rows * x.HQ * (kD / 8);

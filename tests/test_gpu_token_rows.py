@@ -8,7 +8,8 @@ from util_cases import assert_close_all_forms
 
 pytestmark = pytest.mark.gpu
 
-# pairs of the first chapters (the rest nobody selects); 256 pairs a chapter on average and more: the 128-row kernels
+# pairs of the first chapters (the rest nobody selects); in the backward, 512 rows (pairs x query heads of a KV head; 256 with lists per head)
+# a chapter and more: the 128-row kernel.  So few pairs in all are the other kernel's in the forward: its tiles of up to 128 pairs are what the sizes meet.
 BUCKETS = {"edges": [1, 2, 15, 16, 17, 31, 32, 33, 48, 49, 64, 65], "one": [1], "tiles": [127, 128, 129, 300],
            "few_rows_side": [255, 255], "tile_side": [256, 256], "bwd_few_rows_side": [170, 170], "bwd_tile_side": [171, 171]}
 
@@ -90,13 +91,13 @@ def _by_chapter(q, k, v, bi, w):
 
 
 @pytest.mark.parametrize("heads,lists", [((2, 2), "token"), ((2, 2), "head"), ((4, 1), "token")], ids=["mha", "lists", "mqa"])
-@pytest.mark.parametrize("used", [16, 40, 600])
+@pytest.mark.parametrize("used", [26, 60, 1000])
 def test_the_buckets_decide_between_the_kernels(used, heads, lists):
-    """Enough pairs for both kernels and few a chapter on average, all of them in 16 chapters (full tiles, one long item each), in 40, or
+    """Enough pairs for both kernels and few a chapter on average, all of them in 26 chapters (full tiles, one long item each), in 60, or
     spread: whichever kernel takes the call, the results are the mixture's and repeats are the same bits."""
     from memory_b200 import _lib as L, ops
     dev = torch.device("cuda:0")
-    (hq, h), tokens, S, m = heads, 1600, 16, 600
+    (hq, h), tokens, S, m = heads, 1600, 26, 1000
     g = torch.Generator(device=dev).manual_seed(used + hq)
     rand = lambda *s: torch.randn(*s, generator=g, device=dev).bfloat16()
     hi = 1 if lists == "token" else h
@@ -117,3 +118,52 @@ def test_the_buckets_decide_between_the_kernels(used, heads, lists):
     for got, want, what in zip(runs[0], (ref, qc.grad, kc.grad, vc.grad, wc.grad), ("o", "dq", "dk", "dv", "dw")):
         assert_close_all_forms(got[0], want.float(), 2e-2, what)      # (bf16 operands, as above)
     assert all(torch.equal(a, b) for a, b in zip(*runs))
+
+
+@pytest.mark.parametrize("heads", [(2, 2), (6, 2)], ids=["mha", "gqa"])
+@pytest.mark.parametrize("lists", ["token", "head"])
+@pytest.mark.parametrize("B,tokens", [(5, 1801), (2, 75)], ids=["tiles", "few_rows"])
+def test_batches_slots_strided_rows_base_and_an_unselected_chapter(B, tokens, lists, heads):
+    """Sequences of three slots on six chapters, one that every token selects (a ragged last tile), one that nobody selects, K and V
+    halves of one row, a base under the outputs and the query gradients, bit-identical repeats, an id out of range.  27,015 pairs, 900 a
+    chapter on average: the 128-row kernels in both passes; 38 a chapter: those for chapters with few pairs."""
+    from memory_b200 import _lib as L, ops
+    dev = torch.device("cuda:0")
+    hq, h = heads
+    S, m, rho = 3, 6, 2.5
+    g = torch.Generator(device=dev).manual_seed(tokens + hq)
+    hi = 1 if lists == "token" else h
+    others = 1 + torch.rand(B, tokens, hi, m - 2, generator=g, device=dev).topk(S - 1, -1).indices
+    bi = torch.cat([torch.zeros_like(others[..., :1]), others], -1).int()
+    q, base, do, dq0 = (torch.randn(B, tokens, hq, 64, generator=g, device=dev).bfloat16() for _ in range(4))
+    # A value of dV sums thousands of products that are rounded to 2^-9: six of its standard deviations are 6 * 2^-9 / sqrt(3) of the
+    # values' rms, which a quarter of dO keeps near one.
+    do = do / 4
+    kv = torch.randn(B, m * 64, 2 * h * 64, generator=g, device=dev).bfloat16()
+    w = torch.rand(B, tokens, S, generator=g, device=dev) + 0.1
+    halves = lambda t: (t[..., :h * 64].unflatten(-1, (h, 64)), t[..., h * 64:].unflatten(-1, (h, 64)))
+    qc, kc, vc, wc = (t.double().requires_grad_(True) for t in (q, *halves(kv), w))
+    ref = base.double() + rho * torch.stack([_by_chapter(qc[b], kc[b], vc[b], bi[b].long(), wc[b]) for b in range(B)])
+    ref.backward(do.double())
+
+    def run():
+        o, lse, ws = ops.token_mix_fwd(q, *halves(kv), bi, w, 0.125, base=base, out_scale=rho)
+        d_kv = torch.full_like(kv, float("nan"))                 # the call writes every row
+        dq, dw = ops.token_mix_bwd(q, *halves(kv), bi, w, lse, do, 0.125, rho, ws, *halves(d_kv), d_q_base=dq0)
+        return o, dq, dw, d_kv
+
+    o, dq, dw, d_kv = run()
+    L.check_device_status(dev)
+    dk, dv = halves(d_kv)
+    # (bf16 operands and results, as above; the base's part of dQ is exact up to the rounding of the sum)
+    for got, want, what in ((o, ref, "o"), (dq, qc.grad + dq0.double(), "dq"), (dw, wc.grad, "dw"), (dk, kc.grad, "dk"), (dv, vc.grad, "dv")):
+        assert_close_all_forms(got, want.float(), 2e-2, what)
+    assert not d_kv[:, 5 * 64:].any(), "rows of a chapter nobody selected are zero"
+    assert all(torch.equal(a, b) for a, b in zip((o, dq, dw, d_kv), run()))
+    bi[1, 7, 0, 1] = m
+    o2, _, _ = ops.token_mix_fwd(q, *halves(kv), bi, w, 0.125, base=base, out_scale=rho)
+    same = torch.ones(B, tokens, dtype=torch.bool, device=dev)
+    same[1, 7] = False
+    assert torch.equal(o2[same], o[same])
+    with pytest.raises(RuntimeError, match="out of range"):
+        L.check_device_status(dev)
