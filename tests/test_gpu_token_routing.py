@@ -84,7 +84,8 @@ def test_token_layer_fp32_matches_reference_golden(name, dev):
 @pytest.mark.parametrize("name", ["token_gqa_rms", "token_multi_tile"])
 def test_token_layer_bf16_matches_reference_golden(name, dev):
     """64-row chapters and head_dim 64: projections, the shared branch and the per-token mixture on the tensor-core
-    kernels (``token_multi_tile``: chapters selected by more than 128 (token, slot) pairs)."""
+    kernels (``token_multi_tile``: chapters selected by more than 128 (token, slot) pairs; these are calls of the kernels for
+    chapters with few pairs)."""
     from memory_b200 import _lib as L
     case, gold = TOKEN_CASES[name], load_gold(name)
     idx, w, losses, out, grads = run_token_layer_gpu(case, torch.bfloat16, dev)
@@ -223,9 +224,9 @@ TC_SHAPES = {
 
 @pytest.mark.parametrize("shape", list(TC_SHAPES))
 def test_plugin_weighted_entry_point_tensor_core_path(shape, dev):
-    """bf16, head_dim 64, 64-row chapters: the chapter-stationary tcgen05 kernels (inverted index, gathered query
-    tiles, per-pair partial outputs summed in slot order).  Chapters hold fewer than, exactly and several times
-    128 (token, slot) pairs."""
+    """bf16, head_dim 64, 64-row chapters: the chapter-stationary kernels (inverted index, gathered query rows, per-pair
+    partial outputs summed in slot order).  Chapters hold fewer than, exactly and several times 128 (token, slot) pairs; what holds
+    more in fewer chapters, and so runs the kernels of 128-row tiles, is in test_gpu_token_rows.py."""
     from memory_b200 import _lib as L
     from memory_b200 import ops
     from memory_b200.plugin import FSA_topk_sparse_attention_weighted_bthd as fn
@@ -253,7 +254,7 @@ def test_plugin_weighted_entry_point_tensor_core_path(shape, dev):
 
 
 def test_token_mix_shared_lists_base_scale_and_reproducibility(dev):
-    """One chapter list per token for all heads (the module path): a base term, an output scale, a chapter that every
+    """One chapter list per token for all heads (the module path), few pairs a chapter: a base term, an output scale, a chapter that every
     token selects (several tiles), one nobody selects (its gradient rows stay zero), bit-identical repeats, and an
     out-of-range chapter id reported through the status word."""
     from memory_b200 import _lib as L
