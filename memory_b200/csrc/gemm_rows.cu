@@ -1,9 +1,9 @@
 // Projection of a few rows, C [M <= 256, N] = A [M, K] W [N, K]^T with bf16 operands and fp32 accumulation: the query and
 // output projections of a decoding step.  A 128-row tensor-core tile would leave all but a few SMs idle behind one serial
-// chain of K steps (10 us at K 768 whatever M is).  Bound by latency: up to eight rows the work goes to a warp per column, with
-// the weight row in registers and the sums of the eight rows reduced together (768 x 768: 9.5 -> 2.8 us for one row); with more
-// rows and columns, to CTAs of 16 columns and 32 rows on single-warp matrix instructions (64 rows: 7.9 -> 4.8 us, one behind the
-// other; 10.6 -> 6 in a decoding step).
+// chain of K steps (10 us at K 768 whatever M is).  Bound by latency: few outputs, and up to eight rows, go to a warp per column and
+// eight rows, with the weight row in registers and the sums of the eight rows reduced together (768 x 768: 9.5 -> 2.8 us for one
+// row); more of both, to CTAs of 16 columns and 32 rows on single-warp matrix instructions (64 rows: 7.9 -> 4.8 us, one behind the
+// other; 10.6 -> 6 in a decoding step).  by_mma says which.
 #include "rows_product.cuh"
 
 namespace moc {
@@ -135,21 +135,32 @@ gemm_rows_mma_kernel(const __nv_bfloat16* __restrict__ a, long long lda, const _
 
 }  // namespace
 
-// From here on the matrix instructions: 32 x 768 5.3 -> 4.8 us, 24 x 1,536 4.4 -> 3.9; below, the warps a column are faster (24 x 768:
-// 3.5 and 4.8, 64 x 256 over K 1,024: 5.2 and 5.6).
-constexpr long long kMmaFrom = 24 * 1024;
+// Whether the matrix instructions take a projection, us a warp a column and they: 24 x 768 3.6 and 4.8, 32 x 768 5.7 and 4.8, 24 x 1,536
+// 6.0 and 4.9, 64 x 256 over K 1,024 5.3 and 5.6, 256 x 64 3.6 and 4.8 (tensor-core tiles: 9.0).  Up to eight rows they would be three
+// quarters padding: 8 x 3,072 over K 256 / 512 / 768 / 1,024: 3.0 / 3.9 / 5.5 / 5.8 and 3.4 / 4.6 / 5.8 / 6.9.  Where fp32 FMAs of at most
+// 64 rows ran before them, results in fp32 stay theirs: 6.6e-8 from fp64 (2-norm, K 768) against 1.07e-7; rounded to bf16 both are
+// 1.65e-3 and agree to nine digits.  (The tensor-core tiles: 7.3e-7.)
+constexpr int kWarpRows = 64;
+constexpr long long kWarpOutputs = 64 * 1024, kMmaFrom = 24 * 1024;
+bool by_warps(const moc_gemm_desc* g) { return g->m <= kWarpRows && static_cast<long long>(g->m) * g->n <= kWarpOutputs; }
+bool by_mma(const moc_gemm_desc* g) {
+  return g->m > kRows && static_cast<long long>(g->m) * g->n >= kMmaFrom && !(by_warps(g) && g->c_dtype == MOC_F32);
+}
 
 // Whether the kernels take this projection: plain operands, rows of at most 1,024 (32 registers of operands a lane and row),
 // and few enough of them: their work grows with M N while the tensor-core tiles stay at the length of their K chain until N
-// fills the chip.  Here and there, us: 250 x 768 over K 768 7.3 and 10.0, 320 x 768 10.2 and 9.9; 128 x 1,536 over 512 5.9 and 8.1,
-// 250 x 1,536 9.5 and 8.2; 96 x 2,048 over 768 7.9 and 9.7, 128 x 2,048 10.9 and 10.0.
+// fills the chip.  The line is the CTAs of the matrix instructions, us there and here: 384 of them, 256 x 768 over K 768 9.8 and
+// 7.5, over 1,024 11.5 and 11.5; 128 x 1,536 9.9 and 7.6, 11.5 and 11.5; 480, 160 x 1,536 over 768 10.0 and 10.4; 512, 16 x 8,192
+// 9.8 and 10.4, 128 x 2,048 9.9 and 10.8; 1,024, 9 x 16,384 10.7 and 16.6.
+constexpr int kMmaCtas = 384;
 bool gemm_rows_supported(const moc_gemm_desc* g, const float* row_scale, const int32_t* a_row_blocks,
                          const int32_t* b_row_blocks) {
-  return g->m <= 256 && static_cast<long long>(g->m) * g->n <= 192 * 1024 && g->k <= 1024 && g->a_kmajor && g->b_kmajor && !g->accumulate && g->split_k <= 1 &&
+  const bool few = by_warps(g) || (g->m <= 256 && static_cast<long long>(ceil_div(g->m, kMmaRows)) * ceil_div(g->n, kMmaCols) <= kMmaCtas);
+  return few && g->k <= 1024 && g->a_kmajor && g->b_kmajor && !g->accumulate && g->split_k <= 1 &&
          g->residual == nullptr && row_scale == nullptr && a_row_blocks == nullptr && b_row_blocks == nullptr;
 }
 int launch_gemm_rows(const moc_gemm_desc* g, const void* a, const void* b, void* c, cudaStream_t stream) {
-  if (static_cast<long long>(g->m) * g->n >= kMmaFrom) {
+  if (by_mma(g)) {
     const int sums = kMmaWarps * kMmaRows * kMmaCols * 4;
     const int bytes = std::max((kMmaRows + kMmaCols) * mma_stride(g->k), sums);
     MOC_CUDA_OK(allow_shared(gemm_rows_mma_kernel, bytes, (kMmaRows + kMmaCols) * mma_stride(1024)));

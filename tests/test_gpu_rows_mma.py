@@ -8,7 +8,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("out", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("m,n,k", [(24, 1024, 768), (24, 1023, 768), (33, 1000, 8), (64, 771, 24), (63, 2048, 1024), (256, 768, 520),
-                                   (256, 769, 512), (250, 768, 768), (257, 512, 768), (100, 1700, 1000), (31, 800, 1032)])
+                                   (256, 769, 512), (250, 768, 768), (257, 512, 768), (100, 1700, 1000), (31, 800, 1032),
+                                   (8, 3072, 768), (9, 3071, 768), (1, 65536, 64), (3, 24001, 72), (16, 6145, 128), (65, 360, 520), (256, 64, 1024)])
 def test_projection(m, n, k, out):
     from memory_b200 import _lib as L, ops
     dev = torch.device("cuda:0")
