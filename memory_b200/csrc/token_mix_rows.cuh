@@ -24,9 +24,9 @@ struct PairDiv { FastDiv s, hi; };       // pair number -> (token row, list) -> 
 __device__ __forceinline__ int token_of(const PairDiv& d, int pair) { return div_of(div_of(pair, d.s), d.hi); }
 __device__ __forceinline__ int slot_of(const PairDiv& d, int pair) { return pair - div_of(pair, d.s) * d.s.d; }
 
-// A worker (a warp of the forward, a CTA of the backward) walks the (chapter bucket, head) items first, first + step, ...
+// A CTA of the backward walks the (chapter bucket, head) items first, first + step, ...: whole chapters, whose dK and dV it sums.
 // One head an item: buckets differ (at 32 pairs on average the largest have 300 to 500), and what evens them out is that
-// each worker has many.  8,192 tokens, backward, in-use buckets: runs of 12 / 4 / 2 / 1 heads 1,008 / 721 / 658 / 605 us; a CTA for each
+// each CTA has many.  8,192 tokens, in-use buckets: runs of 12 / 4 / 2 / 1 heads 1,008 / 721 / 658 / 605 us; a CTA for each
 // item instead of 444 that walk them 793 (every item then starts cold).
 struct RowItems {
   const int* bucket_off;
@@ -244,9 +244,9 @@ token_mix_rows_fwd_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
 // beside each step's rows where its results go.  A step is 32 pairs: each warp forms S^T and dP^T of eight of them against all 64
 // keys, so that a pair's delta stays inside a warp; Pw^T and dS^T go to shared memory (the one barrier of a step), and from there
 // each warp takes 16 keys of dV and dK (accumulated in registers over the item) and a quarter of dQ.
-// 8,192 tokens, 32 pairs a chapter, uniform: 1,066 -> 575 us; 250 tokens 711 -> 345, of which 246 are HBM.  What is left is shared
-// memory latency with 12 warps an SM (registers): splitting by keys instead (two barriers, less operand traffic) 576, eight
-// warps of half the registers 729.
+// 8,192 tokens, 32 pairs a chapter, uniform, with the sum over slots: 1,115 -> 633 us; 250 tokens 732 -> 359, of which 246 are HBM.
+// What is left is shared memory latency with 12 warps an SM (registers): splitting by keys instead (two barriers, less operand
+// traffic) made nothing faster, eight warps of half the registers took a quarter more.
 constexpr int kRowBwdThreads = 160;                                // 4 warps for the products, 1 for the copies
 constexpr int kRowBwdRows = 32;                                    // pairs of a step
 constexpr int kRowBwdBytes = kRowBwdRows * kD * 2;                 // 4 KiB
@@ -407,7 +407,9 @@ token_mix_rows_bwd_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
       // 16-pair halves of the step that hold pairs.  None where a wait ran out: the step's record and rows may never have been
       // written, so nothing of them is read or stored on the way to the meeting below, where every warp is awaited.
       const int halves = !ok ? 0 : st.pairs > 16 ? 2 : 1;
-      // S^T and dP^T: 64 keys x 8 pairs a warp; this lane's keys are 16 m + g8 and that + 8, its pairs c2 and the next
+      // S^T and dP^T: 64 keys x 8 pairs a warp; this lane's keys are 16 m + g8 and that + 8, its pairs c2 and the next.  A chain in the
+      // instruction's accumulator is truncated at each step, so two chains of 32 columns are added in fp32: dW (fp32) is 2.7e-7 from
+      // fp64 then, 3.1e-7 with chains of 64 columns, 2.75e-7 in the 128-row kernel.  (32 pairs a chapter: 621 -> 633 us.)
       if (warp < 2 * halves) {
         float sc[4][4], dp[4][4];
 #pragma unroll
@@ -417,15 +419,20 @@ token_mix_rows_bwd_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
           ldsm4(bd, from);
           ldsm4(bq, from + kRowBwdBytes);
 #pragma unroll
-          for (int k2 = 0; k2 < 2; ++k2) {
+          for (int m = 0; m < 4; ++m) {
+            uint32_t ak[4], av[4];
+            float ts[4], td[4];
+            const uint32_t a0 = ((k_s + la) ^ (kk << 5)) + 2048 * m, a1 = ((k_s + la) ^ ((kk + 1) << 5)) + 2048 * m;
+            ldsm4(ak, a0);
+            ldsm4(av, a0 + kTileKV);
+            mma_16816_new(ts, ak, bq[0], bq[1]); mma_16816_new(td, av, bd[0], bd[1]);
+            ldsm4(ak, a1);
+            ldsm4(av, a1 + kTileKV);
+            mma_16816(ts, ak, bq[2], bq[3]); mma_16816(td, av, bd[2], bd[3]);
 #pragma unroll
-            for (int m = 0; m < 4; ++m) {
-              uint32_t ak[4], av[4];
-              const uint32_t a = ((k_s + la) ^ ((kk + k2) << 5)) + 2048 * m;
-              ldsm4(ak, a);
-              ldsm4(av, a + kTileKV);
-              if (kk + k2 == 0) { mma_16816_new(sc[m], ak, bq[0], bq[1]); mma_16816_new(dp[m], av, bd[0], bd[1]); }
-              else { mma_16816(sc[m], ak, bq[2 * k2], bq[2 * k2 + 1]); mma_16816(dp[m], av, bd[2 * k2], bd[2 * k2 + 1]); }
+            for (int i = 0; i < 4; ++i) {
+              sc[m][i] = kk == 0 ? ts[i] : sc[m][i] + ts[i];
+              dp[m][i] = kk == 0 ? td[i] : dp[m][i] + td[i];
             }
           }
         }
