@@ -17,7 +17,8 @@ def _contig(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
     return None if t is None else (t if t.is_contiguous() else t.contiguous())
 
 
-# Kernel-launch accounting and optional per-call CUDA-event timing (used by the benchmark).
+# Kernel-launch accounting and optional per-call CUDA-event timing (used by the benchmark).  A kernel that leaves at once because the
+# call's chapters are the other one's (the token mixture asks them on the device) does not count.
 LAUNCHES = 0
 TIMER = None   # when a dict: name -> list of (start_event, end_event) on the current stream
 LAUNCH_HOOK = None   # when callable: called with "<operator>:<bf16|f32|...>" for every operator call (tests use it to
